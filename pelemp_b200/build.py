@@ -19,7 +19,7 @@ LIB = os.path.join(PKG, "libpmpspray.so")
 # arithmetic exactly, so their units are compiled without multiply-add
 # contraction (their multiply-adds are explicit fma() calls); the mixed and
 # learned forms allow it.
-SOURCES = [("pmp_spray.cu", "-fmad=false"), ("pmp_static.cu", "-fmad=false"),
+SOURCES = [("pmp_spray.cu", "-fmad=false"), ("pmp_store.cu", "-fmad=false"), ("pmp_static.cu", "-fmad=false"),
            ("pmp_mixed.cu", "-fmad=true"), ("pmp_learn.cu", "-fmad=true"),
            ("pmp_batch.cu", "-fmad=false"), ("batch/pmp_batch_b64.cu", "-fmad=false"),
            ("batch/pmp_batch_b128.cu", "-fmad=false"), ("batch/pmp_batch_b256.cu", "-fmad=false"),

@@ -424,6 +424,7 @@ extern "C" int pmp_spray_autotune(
   if (rc != PMP_OK) {
     return rc;
   }
+  pmp::quiesce(h);  // the droplets may have been packed on st just now
   const pmp_launch_config saved = h->batch.cfg;
   const std::string key = tune_key(h, nboxes, do_move, P.num_iter);
   if (cache_path) {

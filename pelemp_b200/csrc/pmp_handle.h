@@ -14,11 +14,19 @@ namespace pmp {
 constexpr int kBlock = 128;
 constexpr int kSortPad = 8;  // cells of margin in the sort key around a box
 
-struct BoxStore {
+// Device memory that the handle keeps between calls and exchanges for more
+// when a call needs it; given back with the handle.
+struct KeptBuffer {
+  void* p = nullptr;
+  size_t bytes = 0;
+};
+
+// One box's droplets handed over and not packed yet: n staging rows from
+// `row` of the spare buffer (pmp_store.cu); kept: in the store's order.
+struct StagedBox {
   long long n = 0;
-  double* d = nullptr;  // (3 + NR) * n doubles, sorted by cell
-  int* id = nullptr;
-  long long* perm = nullptr;  // sorted slot -> caller index
+  long long row = 0;
+  bool kept = false;
 };
 
 struct LearnState;  // learned form (pmp_learn.cu)
@@ -95,22 +103,24 @@ struct pmp_spray {
   int spec_perm[PMP_MAX_SPEC];  // species order of dmechf (see DevMechF)
   int fuel_first = 0;
   pmp::DevFuelF dfuelf;
-  // per-box staged droplets (before packing)
-  std::vector<pmp::BoxStore> staged;
+  // droplets handed over and not packed yet (per box)
+  std::vector<pmp::StagedBox> staged;
+  long long staged_rows = 0;
   std::vector<bool> box_set;
-  // packed droplets
+  // packed droplets: component arrays of length total and ids, in `store`;
+  // `spare` holds the staging rows, and the re-binned droplets, with which a
+  // re-binning exchanges the store
   bool packed = false;
   long long total = 0;
+  pmp::KeptBuffer store, spare, perm_b, fb_b, map_b, sort_scratch, transit;
   double* soa = nullptr;  // (3 + NR) arrays of length total
   int* ids = nullptr;
-  long long* perm = nullptr;
+  long long* perm() const { return static_cast<long long*>(perm_b.p); }  // slot -> caller's index in its box
   std::vector<long long> box_begin;
   int ncta = 0;
-  int cta_cap = 0;  // allocated entries of d_cta_box / d_cta_start
   int* d_cta_box = nullptr;
   long long* d_cta_start = nullptr;
   long long* d_box_begin = nullptr;
-  long long* fb_list = nullptr;  // fallback slots (mixed / learned forms)
   pmp::BoxEntry* h_boxes = nullptr;  // the box table of the call being prepared
   int boxes_cap = 0;
   pmp::TableSlot tables[pmp::kTableSlots];
@@ -156,15 +166,6 @@ struct pmp_spray {
   int* d_box_map = nullptr;
   void* mesh_scratch = nullptr;
   size_t mesh_scratch_bytes = 0;
-  // re-binning (pmp_spray_redistribute): its working arrays (sort keys and
-  // values, CUB's temporary storage), kept between calls, and a spare
-  // droplet store that the re-binned droplets are gathered into (the old
-  // store then becomes the spare); spare_cap droplets
-  void* rebin_scratch = nullptr;
-  size_t rebin_scratch_bytes = 0;
-  double* soa_spare = nullptr;
-  int* ids_spare = nullptr;
-  long long spare_cap = 0;
   // gas records of the grown boxes (BoxEntry::gr, FP32, mixed and learned
   // forms; BoxEntry::gr64, FP64 form): capacity in bytes, and the largest
   // grown box (cells) of the last prepared update
@@ -204,11 +205,19 @@ int run_update(
   pmp_spray* h, const pmp_box_view* state, const pmp_box_view* source, int nboxes,
   double flow_dt, int state_ghosts, int source_ghosts, int is_ghost, int do_move,
   double spray_cfl_lev, cudaStream_t st);
-// pack the staged droplets if needed
-int ensure_packed(pmp_spray* h);
-// after re-binning: the store (soa, ids, perm) already holds the droplets in
-// their new order; install the new box bounds and rebuild the CTA map
-int install_rebinned(pmp_spray* h, const std::vector<long long>& box_begin);
+// pmp_store.cu
+// pack the staged droplets if needed, on st
+int ensure_packed(pmp_spray* h, cudaStream_t st);
+int keep(pmp_spray* h, KeptBuffer& b, size_t bytes);
+size_t store_bytes(const pmp_spray* h, long long n);
+// soa and ids for n droplets in the store buffer
+void store_attach(pmp_spray* h, long long n);
+void store_reset(pmp_spray* h);
+void store_free(pmp_spray* h);
+int build_cta_map(pmp_spray* h, cudaStream_t st);
+// after re-binning: the store and perm already hold the droplets in
+// their new order; install the new box bounds and rebuild the CTA map on st
+int install_rebinned(pmp_spray* h, const std::vector<long long>& box_begin, cudaStream_t st);
 // pmp_mesh.cu
 void mesh_free(pmp_spray* h);
 // pmp_batch.cu

@@ -554,7 +554,7 @@ __global__ void k_rebin_perm(long long* perm, const long long* begin, int nb, lo
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// Offsets of the re-binning's working arrays in the handle's rebin_scratch:
+// Offsets of the re-binning's working arrays in the handle's sort_scratch:
 // keys, sorted keys, slot indices, sorted indices (the gather order), box
 // bounds, the box list, CUB's temporary storage.
 struct RebinLayout {
@@ -584,9 +584,6 @@ void mesh_free(pmp_spray* h)
   cudaFree(h->mesh_scratch);
   h->mesh_scratch = nullptr;
   h->mesh_scratch_bytes = 0;
-  cudaFree(h->rebin_scratch);
-  h->rebin_scratch = nullptr;
-  h->rebin_scratch_bytes = 0;
 }
 
 }  // namespace pmp
@@ -608,7 +605,7 @@ extern "C" int pmp_spray_est_timestep(pmp_spray* h, double cfl, double max_jet_v
     *dt = -1.;
     return PMP_OK;
   }
-  int rc = ensure_packed(h);
+  int rc = ensure_packed(h, st);
   if (rc != PMP_OK) {
     return rc;
   }
@@ -652,7 +649,7 @@ extern "C" int pmp_spray_derive(pmp_spray* h, const pmp_box_view* vars, int nbox
   cudaSetDevice(h->device);
   pmp::quiesce(h);
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = ensure_packed(h);
+  int rc = ensure_packed(h, st);
   if (rc != PMP_OK) {
     return rc;
   }
@@ -844,7 +841,7 @@ extern "C" int pmp_spray_transfer_source(pmp_spray* h, const pmp_box_view* tmp_s
 
 // The re-binning's keys, their sort and the box bounds (begin, host copy),
 // with K-bit keys over bits [0, end_bit) and V-bit slot indices; the sorted
-// indices (the gather order) stay in rebin_scratch at RebinLayout::perm.
+// indices (the gather order) stay in sort_scratch at RebinLayout::perm.
 template <typename K, typename V>
 static int rebin_sort(pmp_spray* h, cudaStream_t st, long long n, int nb, int shift, int end_bit,
                       std::vector<long long>& begin)
@@ -855,16 +852,11 @@ static int rebin_sort(pmp_spray* h, cudaStream_t st, long long n, int nb, int sh
                                     (int)n, 0, end_bit, st);
   }
   const RebinLayout L = rebin_layout(n, nb, sizeof(K), sizeof(V), tbytes);
-  if (h->rebin_scratch_bytes < L.total) {
-    cudaFree(h->rebin_scratch);
-    h->rebin_scratch = nullptr;
-    h->rebin_scratch_bytes = 0;
-    if (cudaMalloc(&h->rebin_scratch, L.total) != cudaSuccess) {
-      return set_err(h, PMP_ERR_CUDA, "redistribute: allocation failed");
-    }
-    h->rebin_scratch_bytes = L.total;
+  const int rk = keep(h, h->sort_scratch, L.total);
+  if (rk != PMP_OK) {
+    return rk;
   }
-  char* base = static_cast<char*>(h->rebin_scratch);
+  char* base = static_cast<char*>(h->sort_scratch.p);
   K* keys = reinterpret_cast<K*>(base);
   K* keys2 = reinterpret_cast<K*>(base + L.keys2);
   V* idx = reinterpret_cast<V*>(base + L.idx);
@@ -902,7 +894,7 @@ extern "C" int pmp_spray_redistribute(pmp_spray* h, long long* removed, void* st
   cudaSetDevice(h->device);
   pmp::quiesce(h);
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = ensure_packed(h);
+  int rc = ensure_packed(h, st);
   if (rc == PMP_OK) {
     rc = ensure_box_map(h, st);
   }
@@ -938,42 +930,38 @@ extern "C" int pmp_spray_redistribute(pmp_spray* h, long long* removed, void* st
   const long long live = begin[nb];
   // gather into the spare store (grown when too small), which then becomes
   // the store; the old store becomes the spare
-  if (h->spare_cap < live || !h->soa_spare) {
-    cudaFree(h->soa_spare);
-    cudaFree(h->ids_spare);
-    h->soa_spare = nullptr;
-    h->ids_spare = nullptr;
-    h->spare_cap = 0;
-    const long long lcap = std::max(live, 1LL);
-    if (cudaMalloc(&h->soa_spare, sizeof(double) * nc * lcap) != cudaSuccess ||
-        cudaMalloc(&h->ids_spare, sizeof(int) * lcap) != cudaSuccess) {
-      return set_err(h, PMP_ERR_CUDA, "redistribute: allocation failed");
-    }
-    h->spare_cap = lcap;
+  rc = keep(h, h->spare, store_bytes(h, std::max(live, 1LL)));
+  if (rc != PMP_OK) {
+    return rc;
   }
+  double* soa2 = static_cast<double*>(h->spare.p);
+  int* ids2 = reinterpret_cast<int*>(soa2 + (long long)nc * live);
   if (live > 0) {
     const RebinLayout Lr = rebin_layout(n, nb, narrow ? 4 : 8, narrow ? 4 : 8, 0);
-    const void* perm = static_cast<char*>(h->rebin_scratch) + Lr.perm;
-    const long long* d_begin = reinterpret_cast<const long long*>(static_cast<char*>(h->rebin_scratch) + Lr.begin);
+    const void* perm = static_cast<char*>(h->sort_scratch.p) + Lr.perm;
+    const long long* d_begin = reinterpret_cast<const long long*>(static_cast<char*>(h->sort_scratch.p) + Lr.begin);
     if (narrow) {
       k_gather_soa<<<nblk(live), 256, 0, st>>>(h->soa, n, h->ids, static_cast<const int*>(perm), live, nc,
-                                               h->soa_spare, h->ids_spare);
+                                               soa2, ids2);
     } else {
       k_gather_soa<<<nblk(live), 256, 0, st>>>(h->soa, n, h->ids, static_cast<const long long*>(perm), live, nc,
-                                               h->soa_spare, h->ids_spare);
+                                               soa2, ids2);
     }
-    // each box's new order is its caller order (h->perm holds >= n >= live slots)
-    k_rebin_perm<<<nblk(live), 256, 0, st>>>(h->perm, d_begin, nb, live);
+    // each box's new order is its caller order (h->perm_b holds >= n >= live slots)
+    k_rebin_perm<<<nblk(live), 256, 0, st>>>(h->perm(), d_begin, nb, live);
   }
   if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
     return set_err(h, PMP_ERR_CUDA, "redistribute: gather failed");
   }
-  const long long cap = std::max(n, 1LL);
-  std::swap(h->soa, h->soa_spare);
-  std::swap(h->ids, h->ids_spare);
-  h->spare_cap = cap;  // the old store
+  std::swap(h->store, h->spare);
+  store_attach(h, live);
   if (removed) {
     *removed = n - live;
   }
-  return install_rebinned(h, begin);
+  rc = install_rebinned(h, begin, st);
+  if (rc != PMP_OK) {
+    return rc;
+  }
+  PMP_TRY(h, cudaStreamSynchronize(st));
+  return PMP_OK;
 }

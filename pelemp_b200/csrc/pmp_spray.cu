@@ -1,14 +1,10 @@
 // pmp_spray.cu -- implementation of the C ABI in include/pmp_spray.h.
 //
 // The handle replaces SprayParticleContainer's static state
-// (Source/PP_Spray/SprayParticles.H:388-405) and its particle tiles.  Droplets
-// handed in per box are copied to the device, sorted by the cell that holds
-// them, and packed into one structure-of-arrays; the permutation back to the
-// caller's order is kept.  pmp_spray_update is updateParticles
+// (Source/PP_Spray/SprayParticles.H:388-405); its particle tiles are in
+// pmp_store.cu.  pmp_spray_update is updateParticles
 // (SprayParticles.cpp:142-502) for all boxes in one launch.
 #include <cuda_runtime.h>
-
-#include <cub/cub.cuh>
 
 #include <algorithm>
 #include <cmath>
@@ -36,9 +32,7 @@ using pmp::KParams;
 
 #include "pmp_handle.h"
 
-using pmp::BoxStore;
 using pmp::kBlock;
-using pmp::kSortPad;
 
 int pmp::set_err(pmp_spray* h, int code, const char* msg, int box, long long particle)
 {
@@ -67,134 +61,7 @@ using pmp::set_err;
   } while (0)
 
 // --------------------------------------------------------------------------
-// small data-movement kernels
-
-__global__ void k_aos_to_soa(const char* aos, long long n, int nr, double* soa, int* ids)
-{
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) {
-    return;
-  }
-  const size_t rec = sizeof(double) * (3 + nr) + 2 * sizeof(int);
-  const double* r = reinterpret_cast<const double*>(aos + i * rec);
-  for (int c = 0; c < 3 + nr; ++c) {
-    soa[c * n + i] = r[c];
-  }
-  ids[i] = *reinterpret_cast<const int*>(r + 3 + nr);
-}
-
-__global__ void k_soa_to_aos(const double* soa, const int* ids, long long n, int nr, char* aos)
-{
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) {
-    return;
-  }
-  const size_t rec = sizeof(double) * (3 + nr) + 2 * sizeof(int);
-  double* r = reinterpret_cast<double*>(aos + i * rec);
-  for (int c = 0; c < 3 + nr; ++c) {
-    r[c] = soa[c * n + i];
-  }
-  int* ip = reinterpret_cast<int*>(r + 3 + nr);
-  ip[0] = ids[i];
-  ip[1] = 0;
-}
-
-__global__ void k_cell_keys(
-  const double* x, const double* y, const double* z, long long n, double plo0, double plo1,
-  double plo2, double dxi0, double dxi1, double dxi2, int lo0, int lo1, int lo2, int nx, int ny,
-  int nz, unsigned* keys, long long* idx)
-{
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) {
-    return;
-  }
-  int c[3];
-  const double p[3] = {x[i], y[i], z[i]};
-  const double pl[3] = {plo0, plo1, plo2};
-  const double di[3] = {dxi0, dxi1, dxi2};
-  const int lo[3] = {lo0, lo1, lo2};
-  const int ext[3] = {nx, ny, nz};
-  for (int d = 0; d < 3; ++d) {
-    const double l = __dmul_rn(__dsub_rn(p[d], pl[d]), di[d]);
-    int v = static_cast<int>(floor(l)) - lo[d] + kSortPad;
-    v = v < 0 ? 0 : (v >= ext[d] ? ext[d] - 1 : v);
-    c[d] = v;
-  }
-  keys[i] = (unsigned)pmp::brick_key(c[0], c[1], c[2], ext[0], ext[1]);
-  idx[i] = i;
-}
-
-// dst[c][s] = src[c][perm[s]] for every component; ids likewise
-__global__ void k_gather(
-  const double* src, const int* sid, const long long* perm, long long n, int ncomp, double* dst,
-  int* did)
-{
-  const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (s >= n) {
-    return;
-  }
-  const long long j = perm[s];
-  for (int c = 0; c < ncomp; ++c) {
-    dst[c * n + s] = src[c * n + j];
-  }
-  did[s] = sid[j];
-}
-
-// dst[c][perm[s]] = src[c * stride + s]: back to the caller's order
-__global__ void k_unsort(
-  const double* src, long long stride, const int* sid, const long long* perm, long long n, int ncomp,
-  double* dst, int* did)
-{
-  const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (s >= n) {
-    return;
-  }
-  const long long j = perm[s];
-  for (int c = 0; c < ncomp; ++c) {
-    dst[c * n + j] = src[c * stride + s];
-  }
-  did[j] = sid[s];
-}
-
-inline unsigned nblk(long long n, int b = 256) { return (unsigned)((n + b - 1) / b); }
-
-// --------------------------------------------------------------------------
 // handle helpers
-
-void free_store(BoxStore& s)
-{
-  cudaFree(s.d);
-  cudaFree(s.id);
-  cudaFree(s.perm);
-  s = BoxStore{};
-}
-
-void free_packed(pmp_spray* h)
-{
-  cudaFree(h->soa);
-  cudaFree(h->ids);
-  cudaFree(h->perm);
-  cudaFree(h->d_cta_box);
-  cudaFree(h->d_cta_start);
-  cudaFree(h->d_box_begin);
-  cudaFree(h->fb_list);
-  cudaFree(h->soa_spare);
-  cudaFree(h->ids_spare);
-  h->soa_spare = nullptr;
-  h->ids_spare = nullptr;
-  h->spare_cap = 0;
-  h->soa = nullptr;
-  h->ids = nullptr;
-  h->perm = nullptr;
-  h->d_cta_box = nullptr;
-  h->d_cta_start = nullptr;
-  h->d_box_begin = nullptr;
-  h->fb_list = nullptr;
-  h->cta_cap = 0;
-  h->packed = false;
-  h->ncta = 0;
-  pmp::batch_reset(h);
-}
 
 // DevMech (species in mechanism order) and DevFuel from the mechanism and
 // SprayData.
@@ -418,106 +285,6 @@ int acquire_table(pmp_spray* h, int nboxes, cudaStream_t st, const BoxEntry** ou
   return PMP_OK;
 }
 
-int build_cta_map(pmp_spray* h);
-
-int pack(pmp_spray* h)
-{
-  if (h->packed) {
-    return PMP_OK;
-  }
-  const int nb = (int)h->boxes.size();
-  for (int b = 0; b < nb; ++b) {
-    if (!h->box_set[b]) {
-      return set_err(h, PMP_ERR_INVALID, "set_particles was not called for every box", b);
-    }
-  }
-  free_packed(h);
-  const int nc = h->ncomp();
-  long long total = 0;
-  h->box_begin.assign(nb + 1, 0);
-  for (int b = 0; b < nb; ++b) {
-    h->box_begin[b] = total;
-    total += h->staged[b].n;
-  }
-  h->box_begin[nb] = total;
-  h->total = total;
-  const long long cap = total > 0 ? total : 1;
-  PMP_CUDA(h, cudaMalloc(&h->soa, sizeof(double) * nc * cap));
-  PMP_CUDA(h, cudaMalloc(&h->ids, sizeof(int) * cap));
-  PMP_CUDA(h, cudaMalloc(&h->perm, sizeof(long long) * cap));
-  for (int b = 0; b < nb; ++b) {
-    BoxStore& s = h->staged[b];
-    const long long o = h->box_begin[b];
-    if (s.n > 0) {
-      PMP_CUDA(h, cudaMemcpy2D(h->soa + o, sizeof(double) * cap, s.d, sizeof(double) * s.n,
-                               sizeof(double) * s.n, nc, cudaMemcpyDeviceToDevice));
-      PMP_CUDA(h, cudaMemcpy(h->ids + o, s.id, sizeof(int) * s.n, cudaMemcpyDeviceToDevice));
-      PMP_CUDA(h, cudaMemcpy(h->perm + o, s.perm, sizeof(long long) * s.n, cudaMemcpyDeviceToDevice));
-    }
-    free_store(s);
-  }
-  return build_cta_map(h);
-}
-
-// CTA -> (box, first slot) map, box offsets and fallback list of the packed droplets
-int build_cta_map(pmp_spray* h)
-{
-  const int nb = (int)h->boxes.size();
-  const long long cap = h->total > 0 ? h->total : 1;
-  std::vector<int> cb;
-  std::vector<long long> cs;
-  for (int b = 0; b < nb; ++b) {
-    for (long long o = h->box_begin[b]; o < h->box_begin[b + 1]; o += kBlock) {
-      cb.push_back(b);
-      cs.push_back(o);
-    }
-  }
-  h->ncta = (int)cb.size();
-  if (h->ncta > h->cta_cap) {  // kept by a re-binning while large enough
-    cudaFree(h->d_cta_box);
-    cudaFree(h->d_cta_start);
-    h->d_cta_box = nullptr;
-    h->d_cta_start = nullptr;
-    h->cta_cap = 0;
-    PMP_CUDA(h, cudaMalloc(&h->d_cta_box, sizeof(int) * h->ncta));
-    PMP_CUDA(h, cudaMalloc(&h->d_cta_start, sizeof(long long) * h->ncta));
-    h->cta_cap = h->ncta;
-  }
-  if (h->ncta > 0) {
-    PMP_CUDA(h, cudaMemcpy(h->d_cta_box, cb.data(), sizeof(int) * h->ncta, cudaMemcpyHostToDevice));
-    PMP_CUDA(h, cudaMemcpy(h->d_cta_start, cs.data(), sizeof(long long) * h->ncta, cudaMemcpyHostToDevice));
-  }
-  if (!h->d_box_begin) {
-    PMP_CUDA(h, cudaMalloc(&h->d_box_begin, sizeof(long long) * (nb + 1)));
-  }
-  PMP_CUDA(h, cudaMemcpy(h->d_box_begin, h->box_begin.data(), sizeof(long long) * (nb + 1),
-                         cudaMemcpyHostToDevice));
-  if (!h->fb_list) {  // kept by a re-binning, whose droplet count only falls
-    PMP_CUDA(h, cudaMalloc(&h->fb_list, sizeof(long long) * cap));
-  }
-  h->packed = true;
-  return PMP_OK;
-}
-
-// Copy the droplets of box b (packed or staged) back into a device SoA of
-// caller order: out_d (nc * n doubles), out_id (n ints).
-int unsort_box(pmp_spray* h, int b, double* out_d, int* out_id, long long n)
-{
-  const int nc = h->ncomp();
-  if (n == 0) {
-    return PMP_OK;
-  }
-  if (h->packed) {
-    const long long o = h->box_begin[b];
-    k_unsort<<<nblk(n), 256>>>(h->soa + o, h->total, h->ids + o, h->perm + o, n, nc, out_d, out_id);
-  } else {
-    BoxStore& s = h->staged[b];
-    k_unsort<<<nblk(n), 256>>>(s.d, s.n, s.id, s.perm, n, nc, out_d, out_id);
-  }
-  PMP_CUDA(h, cudaGetLastError());
-  return PMP_OK;
-}
-
 // Device memory, managed memory or pinned (mapped) host memory; a plain host
 // pointer would fault in the kernel.
 bool device_accessible(const void* p)
@@ -730,7 +497,7 @@ int prepare_update_impl(
   if (!(flow_dt > 0.)) {
     return set_err(h, PMP_ERR_INVALID, "flow_dt must be positive");
   }
-  int rc = pack(h);
+  int rc = pmp::ensure_packed(h, st);
   if (rc != PMP_OK) {
     return rc;
   }
@@ -913,7 +680,7 @@ int prepare_update_impl(
   P.status = h->d_status;
   P.err_host = h->err_dev;
   P.box_begin = h->d_box_begin;
-  P.fb_list = h->fb_list;
+  P.fb_list = static_cast<long long*>(h->fb_b.p);
   P.fb_cap = h->total > 0 ? h->total : 1;
   P.nslots = h->total;
   return PMP_OK;
@@ -1239,6 +1006,8 @@ int pmp::sync_status(pmp_spray* h)
 {
   cudaStream_t st = h->last_stream;
   PMP_CUDA(h, cudaMemcpyAsync(h->h_status, h->d_status, sizeof(DevStatus), cudaMemcpyDeviceToHost, st));
+  // cleared behind the copy: an error is reported once, and later calls run again
+  PMP_CUDA(h, cudaMemsetAsync(h->d_status, 0, sizeof(DevStatus), st));
   PMP_CUDA(h, cudaStreamSynchronize(st));
   h->pending = false;
   const long long T = h->total;
@@ -1256,7 +1025,7 @@ int pmp::sync_status(pmp_spray* h)
     long long caller = -1;
     const long long slot = h->h_status->slot;
     if (slot >= 0 && slot < h->total) {
-      cudaMemcpy(&caller, h->perm + slot, sizeof(long long), cudaMemcpyDeviceToHost);
+      cudaMemcpy(&caller, h->perm() + slot, sizeof(long long), cudaMemcpyDeviceToHost);
     }
     double pos[3] = {0, 0, 0};
     for (int d = 0; d < 3; ++d) {
@@ -1265,9 +1034,6 @@ int pmp::sync_status(pmp_spray* h)
     static const char* names[] = {"ok", "droplet left the domain", "state box too small",
                                   "source box too small", "unsupported droplet state", "timeout"};
     const int code = h->h_status->code;
-    // clear the status (the error is reported once; later calls run again)
-    PMP_CUDA(h, cudaMemsetAsync(h->d_status, 0, sizeof(DevStatus), st));
-    PMP_CUDA(h, cudaStreamSynchronize(st));
     *reinterpret_cast<volatile int*>(h->err_host) = 0;
     set_err(h, code, code < 6 ? names[code] : "error", b, caller);
     for (int d = 0; d < 3; ++d) {
@@ -1275,8 +1041,6 @@ int pmp::sync_status(pmp_spray* h)
     }
     return code;
   }
-  PMP_CUDA(h, cudaMemsetAsync(h->d_status, 0, sizeof(DevStatus), st));
-  PMP_CUDA(h, cudaStreamSynchronize(st));
   memset(&h->last_err, 0, sizeof(h->last_err));
   h->last_err.particle = -1;
   return PMP_OK;
@@ -1296,23 +1060,12 @@ int pmp::prepare_update(
   return PMP_OK;
 }
 
-int pmp::ensure_packed(pmp_spray* h) { return pack(h); }
-
-int pmp::install_rebinned(pmp_spray* h, const std::vector<long long>& box_begin)
+int pmp::install_rebinned(pmp_spray* h, const std::vector<long long>& box_begin, cudaStream_t st)
 {
-  const int nb = (int)h->boxes.size();
   h->box_begin = box_begin;
-  h->total = box_begin[nb];
-  for (int b = 0; b < nb; ++b) {
-    free_store(h->staged[b]);
-    h->staged[b].n = box_begin[b + 1] - box_begin[b];
-    h->box_set[b] = true;
-  }
-  // the CTA map and the box bounds of the new counts (their arrays, perm and
-  // the fallback list keep their capacity: the droplet count only falls)
   h->ncta = 0;
   pmp::batch_reset(h);
-  return build_cta_map(h);
+  return build_cta_map(h, st);
 }
 
 int pmp::enqueue_update(pmp_spray* h, const KParams& P, int nboxes, cudaStream_t st)
@@ -1479,10 +1232,7 @@ int pmp_spray_destroy(pmp_spray* h)
   }
   cudaSetDevice(h->device);
   pmp::quiesce(h);
-  for (auto& s : h->staged) {
-    free_store(s);
-  }
-  free_packed(h);
+  pmp::store_free(h);
   pmp::learn_free(h);
   pmp::batch_free(h);
   pmp::mesh_free(h);
@@ -1691,210 +1441,13 @@ int pmp_spray_set_grids(pmp_spray* h, int nboxes, const pmp_box* boxes)
   }
   cudaSetDevice(h->device);
   pmp::quiesce(h);
-  for (auto& s : h->staged) {
-    free_store(s);
-  }
-  free_packed(h);
+  pmp::store_reset(h);
   h->boxes.assign(boxes, boxes + nboxes);
   h->grids_version += 1;
-  h->staged.assign(nboxes, BoxStore{});
+  h->staged.assign(nboxes, pmp::StagedBox{});
+  h->staged_rows = 0;
   h->box_set.assign(nboxes, false);
   return PMP_OK;
-}
-
-int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
-{
-  if (!h || !p || box < 0 || box >= (int)h->boxes.size() || p->n < 0) {
-    return PMP_ERR_INVALID;
-  }
-  if (!h->have_geom) {
-    return set_err(h, PMP_ERR_INVALID, "set_geometry must precede set_particles");
-  }
-  cudaSetDevice(h->device);
-  pmp::quiesce(h);
-  // unpack the other boxes first if the layout changes
-  if (h->packed) {
-    const int nb = (int)h->boxes.size();
-    const int nc = h->ncomp();
-    for (int b = 0; b < nb; ++b) {
-      const long long n = h->box_begin[b + 1] - h->box_begin[b];
-      BoxStore s;
-      s.n = n;
-      if (n > 0) {
-        PMP_CUDA(h, cudaMalloc(&s.d, sizeof(double) * nc * n));
-        PMP_CUDA(h, cudaMalloc(&s.id, sizeof(int) * n));
-        PMP_CUDA(h, cudaMalloc(&s.perm, sizeof(long long) * n));
-        const long long o = h->box_begin[b];
-        PMP_CUDA(h, cudaMemcpy2D(s.d, sizeof(double) * n, h->soa + o, sizeof(double) * h->total,
-                                 sizeof(double) * n, nc, cudaMemcpyDeviceToDevice));
-        PMP_CUDA(h, cudaMemcpy(s.id, h->ids + o, sizeof(int) * n, cudaMemcpyDeviceToDevice));
-        PMP_CUDA(h, cudaMemcpy(s.perm, h->perm + o, sizeof(long long) * n, cudaMemcpyDeviceToDevice));
-      }
-      h->staged[b] = s;
-    }
-    free_packed(h);
-  }
-  BoxStore& s = h->staged[box];
-  free_store(s);
-  const long long n = p->n;
-  const int nc = h->ncomp();
-  const int nr = h->nr();
-  s.n = n;
-  h->box_set[box] = true;
-  if (n == 0) {
-    return PMP_OK;
-  }
-  double* raw = nullptr;
-  int* rid = nullptr;
-  PMP_CUDA(h, cudaMalloc(&raw, sizeof(double) * nc * n));
-  PMP_CUDA(h, cudaMalloc(&rid, sizeof(int) * n));
-  const cudaMemcpyKind kind =
-    p->where == PMP_WHERE_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
-  if (p->layout == PMP_LAYOUT_SOA) {
-    for (int d = 0; d < 3; ++d) {
-      if (!p->pos[d]) {
-        cudaFree(raw);
-        cudaFree(rid);
-        return set_err(h, PMP_ERR_INVALID, "missing position array");
-      }
-      PMP_CUDA(h, cudaMemcpy(raw + (long long)d * n, p->pos[d], sizeof(double) * n, kind));
-    }
-    for (int r = 0; r < nr; ++r) {
-      if (p->rdata[r]) {
-        PMP_CUDA(h, cudaMemcpy(raw + (long long)(3 + r) * n, p->rdata[r], sizeof(double) * n, kind));
-      } else {
-        PMP_CUDA(h, cudaMemset(raw + (long long)(3 + r) * n, 0, sizeof(double) * n));
-      }
-    }
-    if (!p->id) {
-      cudaFree(raw);
-      cudaFree(rid);
-      return set_err(h, PMP_ERR_INVALID, "missing id array");
-    }
-    PMP_CUDA(h, cudaMemcpy(rid, p->id, sizeof(int) * n, kind));
-  } else if (p->layout == PMP_LAYOUT_AOS) {
-    const size_t rec = sizeof(double) * nc + 2 * sizeof(int);
-    char* tmp = nullptr;
-    PMP_CUDA(h, cudaMalloc(&tmp, rec * n));
-    PMP_CUDA(h, cudaMemcpy(tmp, p->aos, rec * n, kind));
-    k_aos_to_soa<<<nblk(n), 256>>>(tmp, n, nr, raw, rid);
-    PMP_CUDA(h, cudaGetLastError());
-    PMP_CUDA(h, cudaDeviceSynchronize());
-    cudaFree(tmp);
-  } else {
-    cudaFree(raw);
-    cudaFree(rid);
-    return set_err(h, PMP_ERR_INVALID, "unknown particle layout");
-  }
-  // sort by the cell holding the droplet, in brick order (margin kSortPad
-  // around the box)
-  const pmp_box& bx = h->boxes[box];
-  const int ext[3] = {bx.hi[0] - bx.lo[0] + 1 + 2 * kSortPad, bx.hi[1] - bx.lo[1] + 1 + 2 * kSortPad,
-                      bx.hi[2] - bx.lo[2] + 1 + 2 * kSortPad};
-  unsigned *keys = nullptr, *keys2 = nullptr;
-  long long* idx = nullptr;
-  PMP_CUDA(h, cudaMalloc(&keys, sizeof(unsigned) * n));
-  PMP_CUDA(h, cudaMalloc(&keys2, sizeof(unsigned) * n));
-  PMP_CUDA(h, cudaMalloc(&idx, sizeof(long long) * n));
-  PMP_CUDA(h, cudaMalloc(&s.perm, sizeof(long long) * n));
-  const pmp_geometry& g = h->geom;
-  k_cell_keys<<<nblk(n), 256>>>(raw, raw + n, raw + 2 * n, n, g.plo[0], g.plo[1], g.plo[2],
-                                1. / g.dx[0], 1. / g.dx[1], 1. / g.dx[2], bx.lo[0], bx.lo[1],
-                                bx.lo[2], ext[0], ext[1], ext[2], keys, idx);
-  PMP_CUDA(h, cudaGetLastError());
-  size_t tbytes = 0;
-  const long long maxkey = (long long)pmp::brick_key_count(ext[0], ext[1], ext[2]);
-  if (maxkey >= (1LL << 32)) {
-    cudaFree(raw);
-    cudaFree(rid);
-    cudaFree(keys);
-    cudaFree(keys2);
-    cudaFree(idx);
-    return set_err(h, PMP_ERR_INVALID, "box too large for the droplet sort key", box);
-  }
-  int end_bit = 1;
-  while ((1LL << end_bit) < maxkey && end_bit < 32) {
-    ++end_bit;
-  }
-  PMP_CUDA(h, cub::DeviceRadixSort::SortPairs(nullptr, tbytes, keys, keys2, idx, s.perm, (int)n, 0, end_bit));
-  void* tmp = nullptr;
-  PMP_CUDA(h, cudaMalloc(&tmp, tbytes));
-  PMP_CUDA(h, cub::DeviceRadixSort::SortPairs(tmp, tbytes, keys, keys2, idx, s.perm, (int)n, 0, end_bit));
-  PMP_CUDA(h, cudaMalloc(&s.d, sizeof(double) * nc * n));
-  PMP_CUDA(h, cudaMalloc(&s.id, sizeof(int) * n));
-  k_gather<<<nblk(n), 256>>>(raw, rid, s.perm, n, nc, s.d, s.id);
-  PMP_CUDA(h, cudaGetLastError());
-  PMP_CUDA(h, cudaDeviceSynchronize());
-  cudaFree(tmp);
-  cudaFree(keys);
-  cudaFree(keys2);
-  cudaFree(idx);
-  cudaFree(raw);
-  cudaFree(rid);
-  return PMP_OK;
-}
-
-int pmp_spray_num_particles(const pmp_spray* h, int box, long long* n)
-{
-  if (!h || !n || box < 0 || box >= (int)h->boxes.size()) {
-    return PMP_ERR_INVALID;
-  }
-  *n = h->packed ? h->box_begin[box + 1] - h->box_begin[box] : h->staged[box].n;
-  return PMP_OK;
-}
-
-int pmp_spray_get_particles(pmp_spray* h, int box, pmp_particles* out)
-{
-  if (!h || !out || box < 0 || box >= (int)h->boxes.size()) {
-    return PMP_ERR_INVALID;
-  }
-  cudaSetDevice(h->device);
-  pmp::quiesce(h);
-  long long n = 0;
-  pmp_spray_num_particles(h, box, &n);
-  if (out->n != n) {
-    return set_err(h, PMP_ERR_INVALID, "output count differs from the box's droplet count", box);
-  }
-  if (n == 0) {
-    return PMP_OK;
-  }
-  const int nc = h->ncomp();
-  const int nr = h->nr();
-  double* d = nullptr;
-  int* id = nullptr;
-  PMP_CUDA(h, cudaMalloc(&d, sizeof(double) * nc * n));
-  PMP_CUDA(h, cudaMalloc(&id, sizeof(int) * n));
-  int rc = unsort_box(h, box, d, id, n);
-  if (rc == PMP_OK) {
-    const cudaMemcpyKind kind =
-      out->where == PMP_WHERE_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
-    if (out->layout == PMP_LAYOUT_SOA) {
-      for (int dd = 0; dd < 3; ++dd) {
-        if (out->pos[dd]) {
-          PMP_CUDA(h, cudaMemcpy(out->pos[dd], d + (long long)dd * n, sizeof(double) * n, kind));
-        }
-      }
-      for (int r = 0; r < nr; ++r) {
-        if (out->rdata[r]) {
-          PMP_CUDA(h, cudaMemcpy(out->rdata[r], d + (long long)(3 + r) * n, sizeof(double) * n, kind));
-        }
-      }
-      if (out->id) {
-        PMP_CUDA(h, cudaMemcpy(out->id, id, sizeof(int) * n, kind));
-      }
-    } else {
-      const size_t rec = sizeof(double) * nc + 2 * sizeof(int);
-      char* tmp = nullptr;
-      PMP_CUDA(h, cudaMalloc(&tmp, rec * n));
-      k_soa_to_aos<<<nblk(n), 256>>>(d, id, n, nr, tmp);
-      PMP_CUDA(h, cudaGetLastError());
-      PMP_CUDA(h, cudaMemcpy(out->aos, tmp, rec * n, kind));
-      cudaFree(tmp);
-    }
-  }
-  cudaFree(d);
-  cudaFree(id);
-  return rc;
 }
 
 int pmp_spray_update(

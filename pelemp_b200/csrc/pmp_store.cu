@@ -1,0 +1,947 @@
+// pmp_store.cu -- the droplet store: hand-over (pmp_spray_set_particles),
+// packing into the cell-sorted structure of arrays the update kernels read,
+// and write-back (pmp_spray_get_particles).
+//
+// A box's droplets are handed over into staging rows (one 128- or 160-byte
+// row per droplet: the reals, the id and the caller's index), whatever the
+// caller's layout.  The first operation that needs the droplets packs all
+// boxes at once: one key per row (box, then cell), one radix sort over every
+// box, one gather of whole rows into the store's component arrays.  A row is
+// whole 32-byte sectors, so the gather in sorted (random) order moves no byte
+// it does not use, where gathering 8 bytes from each of 14-17 component
+// arrays read four times the data; write-back to records goes the same way
+// round.  Staging rows, store, sort arrays and maps stay with the handle
+// between calls (KeptBuffer), so that a caller who hands its droplets over
+// for every call allocates nothing in the steady state.  Measured, hand-over,
+// FP64 update and write-back: 2M two-fuel droplets in 8 boxes 56.0 -> 4.25 ms
+// (3.48 ms of it the update; with a cudaMalloc and cudaFree per array and box
+// the allocator took 46 ms and moving droplets 1.8 ms), 0.78M droplets in 64
+// uneven boxes 72.9 -> 2.37 ms, 8M droplets in the mixed form 79.9 -> 4.89 ms.
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include <cub/cub.cuh>
+
+#include <algorithm>
+#include <cstdio>
+#include <cstring>
+#include <vector>
+
+#include "pmp_handle.h"
+
+namespace pmp {
+
+namespace {
+
+int check(pmp_spray* h, cudaError_t e, const char* what)
+{
+  if (e != cudaSuccess) {
+    char b[160];
+    snprintf(b, sizeof(b), "%s: %s", what, cudaGetErrorString(e));
+    cudaGetLastError();  // reported here, not by the next call
+    return set_err(h, PMP_ERR_CUDA, b);
+  }
+  return PMP_OK;
+}
+
+#define PMP_TRY(h, call)                        \
+  do {                                          \
+    const int rc_ = check((h), (call), #call);  \
+    if (rc_ != PMP_OK) {                        \
+      return rc_;                               \
+    }                                           \
+  } while (0)
+
+constexpr int kTile = 128;  // droplets per CTA of the kernels below
+constexpr int kMaxWords = 4 + PMP_PSTATE_NUM(PMP_MAX_FUEL);
+
+// A droplet's staging row: 3 + NR reals, then {id, caller's index} in one
+// word, padded to whole sectors.
+template <int NF>
+struct Row {
+  static constexpr int kReals = 3 + PMP_PSTATE_NUM(NF);
+  static constexpr int kWords = kReals + 1;
+  static constexpr int kStride = (kWords + 3) / 4 * 4;  // doubles
+  static constexpr int kPieces = (kWords + 1) / 2;      // 16-byte pieces that hold words
+  static constexpr int kPitch = kWords | 1;             // shared-memory tile: odd, so that a column is conflict-free
+};
+int row_stride(int nf) { return (PMP_PSTATE_NUM(nf) + 4 + 3) / 4 * 4; }
+
+struct Columns {
+  double* c[kMaxWords - 1];
+  int* id;
+};
+
+__device__ __forceinline__ double pack_ints(int lo, int hi) { return __hiloint2double(hi, lo); }
+
+// tile[r][w] of the CTA's rows -> staging rows, 16 bytes a lane
+template <int NF>
+__device__ __forceinline__ void tile_to_rows(const double (*tile)[Row<NF>::kPitch], double* rows, int m)
+{
+  using R = Row<NF>;
+  for (int i = threadIdx.x; i < m * R::kPieces; i += kTile) {
+    const int r = i / R::kPieces, w = 2 * (i % R::kPieces);
+    double2 v;
+    v.x = tile[r][w];
+    v.y = w + 1 < R::kWords ? tile[r][w + 1] : 0.;
+    *reinterpret_cast<double2*>(rows + (long long)r * R::kStride + w) = v;
+  }
+}
+
+// AMReX records {pos[3], rdata[10 + F], id, cpu} -> rows.  Records are read as
+// one stream of words (the caller's buffer is 8-byte aligned, a record with
+// one fuel is 120 bytes), and turned in shared memory.
+template <int NF>
+__global__ void __launch_bounds__(kTile) k_aos_to_rows(const double* aos, long long n, double* rows)
+{
+  using R = Row<NF>;
+  __shared__ double tile[kTile][R::kPitch];
+  const long long s0 = (long long)blockIdx.x * kTile;
+  const int m = (int)min((long long)kTile, n - s0);
+  const double* src = aos + s0 * R::kWords;
+  for (int i = threadIdx.x; i < m * R::kWords; i += kTile) {
+    tile[i / R::kWords][i % R::kWords] = __ldcs(src + i);
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < m) {
+    const int id = __double2loint(tile[threadIdx.x][R::kReals]);
+    tile[threadIdx.x][R::kReals] = pack_ints(id, (int)(s0 + threadIdx.x));
+  }
+  __syncthreads();
+  tile_to_rows<NF>(tile, rows + s0 * R::kStride, m);
+}
+
+// component arrays -> rows; a null component is zero.  caller: the droplets'
+// caller indices, or null for 0, 1, ...
+template <int NF>
+__global__ void __launch_bounds__(kTile) k_columns_to_rows(const Columns C, const long long* caller, long long n, double* rows)
+{
+  using R = Row<NF>;
+  __shared__ double tile[kTile][R::kPitch];
+  const long long s0 = (long long)blockIdx.x * kTile;
+  const int m = (int)min((long long)kTile, n - s0);
+  const long long s = s0 + threadIdx.x;
+  if ((int)threadIdx.x < m) {
+#pragma unroll
+    for (int c = 0; c < R::kReals; ++c) {
+      tile[threadIdx.x][c] = C.c[c] ? __ldcs(C.c[c] + s) : 0.;
+    }
+    tile[threadIdx.x][R::kReals] = pack_ints(C.id[s], caller ? (int)caller[s] : (int)s);
+  }
+  __syncthreads();
+  tile_to_rows<NF>(tile, rows + s0 * R::kStride, m);
+}
+
+// One box's staging rows, in the order of the packed store (box by box).
+struct Region {
+  long long row;    // first staging row
+  long long begin;  // first slot of the box
+  int lo[3], ext[3];
+  int kept;         // rows already in the store's order (a repack): keep it
+  int pad;
+};
+
+__device__ __forceinline__ int region_of(const Region* reg, int nb, long long s)
+{
+  int lo = 0, hi = nb;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) / 2;
+    if (reg[mid].begin <= s) {
+      lo = mid;
+    } else {
+      hi = mid;
+    }
+  }
+  return lo;
+}
+
+// The sort key of each row: its box above `shift` bits of its cell's place in
+// the box's sort order (brick_key over the box and kSortPad cells around it).
+template <typename K, typename V>
+__global__ void __launch_bounds__(256) k_row_keys(const double* rows, int stride, const Region* reg, int nb, long long n,
+                                                  double plo0, double plo1, double plo2, double dxi0, double dxi1,
+                                                  double dxi2, int shift, K* keys, V* idx)
+{
+  const long long s = blockIdx.x * 256LL + threadIdx.x;
+  if (s >= n) {
+    return;
+  }
+  const int b = region_of(reg, nb, s);
+  const Region& g = reg[b];
+  const long long r = g.row + (s - g.begin);
+  unsigned long long cell = 0;
+  if (!g.kept) {
+    const double* q = rows + r * stride;
+    const double2 xy = *reinterpret_cast<const double2*>(q);
+    const double p[3] = {xy.x, xy.y, q[2]};
+    const double pl[3] = {plo0, plo1, plo2}, di[3] = {dxi0, dxi1, dxi2};
+    int c[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int v = static_cast<int>(floor(__dmul_rn(__dsub_rn(p[d], pl[d]), di[d]))) - g.lo[d] + kSortPad;
+      c[d] = v < 0 ? 0 : (v >= g.ext[d] ? g.ext[d] - 1 : v);
+    }
+    cell = brick_key(c[0], c[1], c[2], g.ext[0], g.ext[1]);
+  }
+  keys[s] = ((K)b << shift) | (K)cell;
+  idx[s] = (V)r;
+}
+
+// rows in sorted order -> the store.  Eight or nine lanes read one row.
+template <int NF, typename V>
+__global__ void __launch_bounds__(kTile) k_rows_to_store(const double* rows, const V* order, long long n, double* soa,
+                                                         int* ids, long long* perm)
+{
+  using R = Row<NF>;
+  __shared__ double tile[kTile][R::kPitch];
+  const long long s0 = (long long)blockIdx.x * kTile;
+  const int m = (int)min((long long)kTile, n - s0);
+#pragma unroll
+  for (int it = 0; it < R::kPieces; ++it) {
+    const int i = it * kTile + threadIdx.x;
+    const int r = i / R::kPieces, w = 2 * (i % R::kPieces);
+    if (r < m) {
+      const double2 v = __ldcs(reinterpret_cast<const double2*>(rows + (long long)order[s0 + r] * R::kStride + w));
+      tile[r][w] = v.x;
+      if (w + 1 < R::kWords) {
+        tile[r][w + 1] = v.y;
+      }
+    }
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < m) {
+    const long long s = s0 + threadIdx.x;
+#pragma unroll
+    for (int c = 0; c < R::kReals; ++c) {
+      soa[c * n + s] = tile[threadIdx.x][c];
+    }
+    const double t = tile[threadIdx.x][R::kReals];
+    ids[s] = __double2loint(t);
+    perm[s] = (long long)__double2hiint(t);
+  }
+}
+
+// the store's slots of one box -> records in the caller's order: whole
+// records per droplet, turned in shared memory
+template <int NF>
+__global__ void __launch_bounds__(kTile) k_store_to_aos(const double* soa, long long total, const int* ids,
+                                                        const long long* perm, long long n, double* aos)
+{
+  using R = Row<NF>;
+  __shared__ double tile[kTile][R::kPitch];
+  __shared__ long long at[kTile];
+  const long long s0 = (long long)blockIdx.x * kTile;
+  const int m = (int)min((long long)kTile, n - s0);
+  if ((int)threadIdx.x < m) {
+    const long long s = s0 + threadIdx.x;
+#pragma unroll
+    for (int c = 0; c < R::kReals; ++c) {
+      tile[threadIdx.x][c] = __ldcs(soa + c * total + s);
+    }
+    tile[threadIdx.x][R::kReals] = pack_ints(ids[s], 0);
+    at[threadIdx.x] = perm[s] * R::kWords;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < m * R::kWords; i += kTile) {
+    const int r = i / R::kWords, w = i % R::kWords;
+    aos[at[r] + w] = tile[r][w];
+  }
+}
+
+// the store's slots of one box -> component arrays in the caller's order, a
+// component per blockIdx.y: the CTAs in flight then write one or two
+// components of the box, which stay in L2 until their sectors are full (with
+// every component in flight, k_unsort's 8-byte stores left L2 as partial
+// sectors: 2929 us of GPU time for 8M droplets of 17 words)
+__global__ void __launch_bounds__(256) k_store_to_columns(const double* soa, long long total, const int* ids,
+                                                          const long long* perm, long long n, int nreal, const Columns C)
+{
+  const long long s = blockIdx.x * 256LL + threadIdx.x;
+  if (s >= n) {
+    return;
+  }
+  const int c = blockIdx.y;
+  if (c < nreal) {
+    if (C.c[c]) {
+      C.c[c][perm[s]] = __ldcs(soa + c * total + s);
+    }
+  } else if (C.id) {
+    C.id[perm[s]] = ids[s];
+  }
+}
+
+// staging rows of one box (not packed yet) -> the caller's order
+__global__ void __launch_bounds__(256) k_rows_out(const double* rows, int stride, int nreal, long long n, const Columns C,
+                                                  double* aos)
+{
+  const long long s = blockIdx.x * 256LL + threadIdx.x;
+  if (s >= n) {
+    return;
+  }
+  const double* q = rows + s * stride;
+  const int id = __double2loint(q[nreal]);
+  const long long j = (long long)__double2hiint(q[nreal]);
+  if (aos) {
+    double* o = aos + j * (nreal + 1);
+    for (int c = 0; c < nreal; ++c) {
+      o[c] = q[c];
+    }
+    o[nreal] = pack_ints(id, 0);
+    return;
+  }
+  for (int c = 0; c < nreal; ++c) {
+    if (C.c[c]) {
+      C.c[c][j] = q[c];
+    }
+  }
+  if (C.id) {
+    C.id[j] = id;
+  }
+}
+
+// (box, first slot) of each CTA of the update's map: kBlock slots of one box
+__global__ void __launch_bounds__(256) k_cta_map(const long long* box_begin, const int* first, int nb, int ncta,
+                                                 int* cta_box, long long* cta_start)
+{
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= ncta) {
+    return;
+  }
+  int lo = 0, hi = nb;  // the box b with first[b] <= i < first[b + 1]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) / 2;
+    if (first[mid] <= i) {
+      lo = mid;
+    } else {
+      hi = mid;
+    }
+  }
+  cta_box[i] = lo;
+  cta_start[i] = box_begin[lo] + (long long)(i - first[lo]) * kBlock;
+}
+
+#define PMP_BY_FUELS(h, CALL) \
+  switch ((h)->nfuel) {       \
+    case 1: {                 \
+      constexpr int F = 1;    \
+      CALL;                   \
+    } break;                  \
+    case 2: {                 \
+      constexpr int F = 2;    \
+      CALL;                   \
+    } break;                  \
+    case 3: {                 \
+      constexpr int F = 3;    \
+      CALL;                   \
+    } break;                  \
+    default: {                \
+      constexpr int F = 4;    \
+      CALL;                   \
+    } break;                  \
+  }
+
+unsigned nblk(long long n, int b) { return (unsigned)((n + b - 1) / b); }
+
+size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+size_t row_bytes(const pmp_spray* h) { return sizeof(double) * row_stride(h->nfuel); }
+
+double* staged_row(const pmp_spray* h, long long r)
+{
+  return reinterpret_cast<double*>(static_cast<char*>(h->spare.p) + (size_t)r * row_bytes(h));
+}
+
+// Room for n more staging rows in the spare buffer; the live boxes' rows move
+// to its front when it is exchanged for a larger one.
+int stage_room(pmp_spray* h, long long n)
+{
+  const size_t rb = row_bytes(h);
+  if ((size_t)(h->staged_rows + n) * rb <= h->spare.bytes) {
+    return PMP_OK;
+  }
+  long long live = 0;
+  for (const StagedBox& s : h->staged) {
+    live += s.n;
+  }
+  // the first boxes of a hand-over say little about the rest of it: doubling,
+  // so that many boxes exchange the buffer a few times only
+  const size_t need = (size_t)(live + n) * rb;
+  KeptBuffer nw;
+  nw.bytes = live > 0 ? 2 * need : need;
+  if (cudaMalloc(&nw.p, nw.bytes) != cudaSuccess) {
+    cudaGetLastError();
+    nw.bytes = need;
+    PMP_TRY(h, cudaMalloc(&nw.p, nw.bytes));
+  }
+  long long at = 0;
+  for (StagedBox& s : h->staged) {
+    if (s.n > 0) {
+      const cudaError_t e = cudaMemcpy(static_cast<char*>(nw.p) + (size_t)at * rb, staged_row(h, s.row),
+                                       (size_t)s.n * rb, cudaMemcpyDeviceToDevice);
+      if (e != cudaSuccess) {
+        cudaFree(nw.p);
+        return check(h, e, "cudaMemcpy (staged droplets)");
+      }
+      s.row = at;
+      at += s.n;
+    }
+  }
+  h->staged_rows = at;
+  cudaFree(h->spare.p);  // waits for the copies
+  h->spare = nw;
+  return PMP_OK;
+}
+
+// The packed droplets back into staging rows, in the store's order (which a
+// later pack keeps), except box `skip`, whose droplets are being replaced.
+int unpack(pmp_spray* h, int skip)
+{
+  const int nb = (int)h->boxes.size();
+  const int nc = h->ncomp();
+  const long long T = h->total;
+  h->staged_rows = 0;
+  for (int b = 0; b < nb; ++b) {
+    h->staged[b] = StagedBox{};
+  }
+  long long n = T - (h->box_begin[skip + 1] - h->box_begin[skip]);
+  int rc = stage_room(h, n);
+  if (rc != PMP_OK) {
+    return rc;
+  }
+  for (int b = 0; b < nb; ++b) {
+    const long long o = h->box_begin[b], m = h->box_begin[b + 1] - o;
+    if (b == skip || m == 0) {
+      continue;
+    }
+    StagedBox& s = h->staged[b];
+    s.n = m;
+    s.row = h->staged_rows;
+    s.kept = true;
+    h->staged_rows += m;
+    Columns C;
+    memset(&C, 0, sizeof(C));
+    for (int c = 0; c < nc; ++c) {
+      C.c[c] = h->soa + (long long)c * T + o;
+    }
+    C.id = h->ids + o;
+    PMP_BY_FUELS(h, (k_columns_to_rows<F><<<nblk(m, kTile), kTile>>>(C, h->perm() + o, m, staged_row(h, s.row))));
+  }
+  PMP_TRY(h, cudaGetLastError());
+  store_reset(h);
+  return PMP_OK;
+}
+
+// Ranges of device allocations of the handle's GPU that a call has seen: a
+// caller's array inside one, and suitably aligned, is read or written by the
+// kernels directly.  Everything else (host, managed or another GPU's memory,
+// a range that leaves its allocation) goes through cudaMemcpy, which accepts
+// or refuses it.
+class DeviceRanges {
+ public:
+  explicit DeviceRanges(int device) : device_(device) {}
+  bool holds(const void* p, size_t bytes, size_t align)
+  {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    if (!p || a % align != 0) {
+      return false;
+    }
+    if (a >= lo_ && a + bytes <= hi_) {
+      return true;
+    }
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (at.type != cudaMemoryTypeDevice || at.device != device_) {
+      return false;
+    }
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    if (!range_of() || range_of()(&base, &size, (CUdeviceptr)a) != CUDA_SUCCESS) {
+      return false;
+    }
+    lo_ = (uintptr_t)base;
+    hi_ = lo_ + size;
+    return a + bytes <= hi_;
+  }
+
+ private:
+  using RangeFn = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+  static RangeFn range_of()
+  {
+    static const RangeFn fn = [] {
+      void* p = nullptr;
+      cudaDriverEntryPointQueryResult q;
+      if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &p, cudaEnableDefault, &q) != cudaSuccess ||
+          q != cudaDriverEntryPointSuccess) {
+        cudaGetLastError();
+        p = nullptr;
+      }
+      return reinterpret_cast<RangeFn>(p);
+    }();
+    return fn;
+  }
+  int device_;
+  uintptr_t lo_ = 1, hi_ = 0;
+};
+
+// A device buffer for droplets on their way from or to memory the kernels do
+// not touch directly; given back when it grew large.
+struct Transit {
+  pmp_spray* h;
+  explicit Transit(pmp_spray* handle) : h(handle) {}
+  ~Transit()
+  {
+    if (h->transit.bytes > ((size_t)64 << 20)) {
+      cudaFree(h->transit.p);
+      h->transit = KeptBuffer{};
+    }
+  }
+};
+
+// columns of nreal components of n doubles, then n ids, in one buffer
+Columns columns_in(void* base, int nreal, long long n)
+{
+  Columns C;
+  memset(&C, 0, sizeof(C));
+  double* d = static_cast<double*>(base);
+  for (int c = 0; c < nreal; ++c) {
+    C.c[c] = d + (long long)c * n;
+  }
+  C.id = reinterpret_cast<int*>(d + (long long)nreal * n);
+  return C;
+}
+
+// the sort of every box's rows: the sorted row indices at *order
+template <typename K, typename V>
+int sort_rows(pmp_spray* h, const Region* d_reg, int nb, long long n, int shift, int end_bit, cudaStream_t st,
+              const V** order)
+{
+  using N = V;  // the count type decides CUB's offsets
+  size_t tbytes = 0;
+  PMP_TRY(h, (cub::DeviceRadixSort::SortPairs(nullptr, tbytes, (const K*)nullptr, (K*)nullptr, (const V*)nullptr,
+                                              (V*)nullptr, (N)n, 0, end_bit, st)));
+  const size_t kb = align256(sizeof(K) * n), vb = align256(sizeof(V) * n);
+  const int rc = keep(h, h->sort_scratch, 2 * kb + 2 * vb + tbytes);
+  if (rc != PMP_OK) {
+    return rc;
+  }
+  char* base = static_cast<char*>(h->sort_scratch.p);
+  K* keys = reinterpret_cast<K*>(base);
+  K* keys2 = reinterpret_cast<K*>(base + kb);
+  V* idx = reinterpret_cast<V*>(base + 2 * kb);
+  V* idx2 = reinterpret_cast<V*>(base + 2 * kb + vb);
+  const pmp_geometry& g = h->geom;
+  k_row_keys<K, V><<<nblk(n, 256), 256, 0, st>>>(staged_row(h, 0), row_stride(h->nfuel), d_reg, nb, n, g.plo[0],
+                                                 g.plo[1], g.plo[2], 1. / g.dx[0], 1. / g.dx[1], 1. / g.dx[2], shift,
+                                                 keys, idx);
+  PMP_TRY(h, cudaGetLastError());
+  PMP_TRY(h, cub::DeviceRadixSort::SortPairs(base + 2 * kb + 2 * vb, tbytes, keys, keys2, idx, idx2, (N)n, 0, end_bit, st));
+  *order = idx2;
+  return PMP_OK;
+}
+
+// sort-key extent of a box: its cells and kSortPad around them
+void sort_extent(const pmp_box& bx, int* ext)
+{
+  for (int d = 0; d < 3; ++d) {
+    ext[d] = bx.hi[d] - bx.lo[d] + 1 + 2 * kSortPad;
+  }
+}
+
+}  // namespace
+
+// A kept buffer of at least `bytes`: exchanged when too small, and when it is
+// large and mostly unused (its content is not kept).
+int keep(pmp_spray* h, KeptBuffer& b, size_t bytes)
+{
+  const bool idle = b.bytes > ((size_t)256 << 20) && b.bytes / 4 > bytes;
+  if (b.p && b.bytes >= bytes && !idle) {
+    return PMP_OK;
+  }
+  cudaFree(b.p);
+  b = KeptBuffer{};
+  const size_t want = std::max(bytes, (size_t)256);
+  PMP_TRY(h, cudaMalloc(&b.p, want));
+  b.bytes = want;
+  return PMP_OK;
+}
+
+size_t store_bytes(const pmp_spray* h, long long n) { return (size_t)n * (sizeof(double) * h->ncomp() + sizeof(int)); }
+
+void store_attach(pmp_spray* h, long long n)
+{
+  h->total = n;
+  h->soa = static_cast<double*>(h->store.p);
+  h->ids = reinterpret_cast<int*>(h->soa + (long long)h->ncomp() * n);
+}
+
+void store_reset(pmp_spray* h)
+{
+  h->soa = nullptr;
+  h->ids = nullptr;
+  h->packed = false;
+  h->ncta = 0;
+  batch_reset(h);
+}
+
+void store_free(pmp_spray* h)
+{
+  store_reset(h);
+  for (KeptBuffer* b : {&h->store, &h->spare, &h->perm_b, &h->fb_b, &h->map_b, &h->sort_scratch, &h->transit}) {
+    cudaFree(b->p);
+    *b = KeptBuffer{};
+  }
+}
+
+// Box offsets and the CTA -> (box, first slot) map of the packed droplets,
+// and the fallback list, enqueued on st.
+int build_cta_map(pmp_spray* h, cudaStream_t st)
+{
+  const int nb = (int)h->boxes.size();
+  std::vector<int> first(nb + 1, 0);
+  for (int b = 0; b < nb; ++b) {
+    const long long n = h->box_begin[b + 1] - h->box_begin[b];
+    first[b + 1] = first[b] + (int)((n + kBlock - 1) / kBlock);
+  }
+  h->ncta = first[nb];
+  // {box_begin[nb + 1], first[nb + 1]} uploaded, then cta_start, cta_box
+  const size_t bb = sizeof(long long) * (nb + 1), fb = align256(sizeof(int) * (nb + 1));
+  const size_t cs = align256(bb + fb), cb = align256(sizeof(long long) * h->ncta);
+  int rc = keep(h, h->map_b, cs + cb + sizeof(int) * (size_t)h->ncta);
+  if (rc == PMP_OK) {
+    rc = keep(h, h->fb_b, sizeof(long long) * (size_t)std::max(h->total, 1LL));
+  }
+  if (rc != PMP_OK) {
+    return rc;
+  }
+  char* base = static_cast<char*>(h->map_b.p);
+  std::vector<char> up(bb + fb);
+  memcpy(up.data(), h->box_begin.data(), bb);
+  memcpy(up.data() + bb, first.data(), sizeof(int) * (nb + 1));
+  PMP_TRY(h, cudaMemcpyAsync(base, up.data(), bb + sizeof(int) * (nb + 1), cudaMemcpyHostToDevice, st));
+  h->d_box_begin = reinterpret_cast<long long*>(base);
+  h->d_cta_start = reinterpret_cast<long long*>(base + cs);
+  h->d_cta_box = reinterpret_cast<int*>(base + cs + cb);
+  if (h->ncta > 0) {
+    k_cta_map<<<nblk(h->ncta, 256), 256, 0, st>>>(h->d_box_begin, reinterpret_cast<const int*>(base + bb), nb, h->ncta,
+                                                  h->d_cta_box, h->d_cta_start);
+    PMP_TRY(h, cudaGetLastError());
+  }
+  h->packed = true;
+  return PMP_OK;
+}
+
+// The staged boxes packed into the store on st.  No work of the handle is
+// pending (whoever staged droplets waited for it).
+int ensure_packed(pmp_spray* h, cudaStream_t st)
+{
+  if (h->packed) {
+    return PMP_OK;
+  }
+  const int nb = (int)h->boxes.size();
+  for (int b = 0; b < nb; ++b) {
+    if (!h->box_set[b]) {
+      return set_err(h, PMP_ERR_INVALID, "set_particles was not called for every box", b);
+    }
+  }
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  PMP_TRY(h, cudaStreamIsCapturing(st, &cap));
+  const bool capturing = cap != cudaStreamCaptureStatusNone;
+  if (capturing) {
+    // packing is not part of the caller's graph: it runs at once, beside the
+    // capture, where the capture's mode lets a call allocate
+    void* p = nullptr;
+    PMP_TRY(h, cudaMalloc(&p, 256));
+    cudaFree(p);
+    st = nullptr;
+  }
+  std::vector<Region> reg(nb);
+  h->box_begin.assign(nb + 1, 0);
+  int shift = 0;
+  for (int b = 0; b < nb; ++b) {
+    const pmp_box& bx = h->boxes[b];
+    Region& r = reg[b];
+    memset(&r, 0, sizeof(r));
+    r.row = h->staged[b].row;
+    r.begin = h->box_begin[b];
+    r.kept = h->staged[b].kept ? 1 : 0;
+    sort_extent(bx, r.ext);
+    for (int d = 0; d < 3; ++d) {
+      r.lo[d] = bx.lo[d];
+    }
+    const unsigned long long cells = brick_key_count(r.ext[0], r.ext[1], r.ext[2]);
+    while (shift < 40 && (1ULL << shift) < cells) {
+      ++shift;
+    }
+    h->box_begin[b + 1] = h->box_begin[b] + h->staged[b].n;
+  }
+  const long long n = h->box_begin[nb];
+  int rc = keep(h, h->store, store_bytes(h, std::max(n, 1LL)));
+  if (rc == PMP_OK) {
+    rc = keep(h, h->perm_b, sizeof(long long) * (size_t)std::max(n, 1LL));
+  }
+  if (rc == PMP_OK) {
+    rc = keep(h, h->map_b, sizeof(Region) * (size_t)std::max(nb, 1));
+  }
+  if (rc != PMP_OK) {
+    return rc;
+  }
+  store_attach(h, n);
+  if (n > 0) {
+    // the regions are read before build_cta_map reuses the buffer, in stream order
+    const Region* d_reg = static_cast<const Region*>(h->map_b.p);
+    PMP_TRY(h, cudaMemcpyAsync(h->map_b.p, reg.data(), sizeof(Region) * nb, cudaMemcpyHostToDevice, st));
+    int end_bit = shift;
+    while (end_bit < 63 && (1LL << (end_bit - shift)) < nb) {
+      ++end_bit;
+    }
+    end_bit = std::max(end_bit, 1);
+    if (end_bit <= 32 && h->staged_rows < (1LL << 31)) {
+      const int* order = nullptr;
+      rc = sort_rows<unsigned, int>(h, d_reg, nb, n, shift, end_bit, st, &order);
+      if (rc == PMP_OK) {
+        PMP_BY_FUELS(h, (k_rows_to_store<F, int><<<nblk(n, kTile), kTile, 0, st>>>(staged_row(h, 0), order, n, h->soa,
+                                                                                  h->ids, h->perm())));
+      }
+    } else {
+      const long long* order = nullptr;
+      rc = sort_rows<unsigned long long, long long>(h, d_reg, nb, n, shift, end_bit, st, &order);
+      if (rc == PMP_OK) {
+        PMP_BY_FUELS(h, (k_rows_to_store<F, long long><<<nblk(n, kTile), kTile, 0, st>>>(staged_row(h, 0), order, n,
+                                                                                        h->soa, h->ids, h->perm())));
+      }
+    }
+    if (rc != PMP_OK) {
+      return rc;
+    }
+    PMP_TRY(h, cudaGetLastError());
+  }
+  rc = build_cta_map(h, st);
+  if (rc != PMP_OK) {
+    return rc;
+  }
+  for (StagedBox& s : h->staged) {
+    s = StagedBox{};
+  }
+  h->staged_rows = 0;
+  if (capturing) {
+    PMP_TRY(h, cudaStreamSynchronize(st));
+    return PMP_OK;
+  }
+  // entry points on other streams wait for the store
+  PMP_TRY(h, cudaEventRecord(h->ev_done, st));
+  h->last_stream = st;
+  h->pending = true;
+  return PMP_OK;
+}
+
+}  // namespace pmp
+
+using namespace pmp;
+
+extern "C" {
+
+int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
+{
+  if (!h || !p || box < 0 || box >= (int)h->boxes.size() || p->n < 0) {
+    return PMP_ERR_INVALID;
+  }
+  if (!h->have_geom) {
+    return set_err(h, PMP_ERR_INVALID, "set_geometry must precede set_particles");
+  }
+  cudaSetDevice(h->device);
+  pmp::quiesce(h);
+  int rc = PMP_OK;
+  if (h->packed) {
+    rc = unpack(h, box);
+    if (rc != PMP_OK) {
+      return rc;
+    }
+  }
+  const long long n = p->n;
+  StagedBox& s = h->staged[box];
+  if (s.n > 0 && s.row + s.n == h->staged_rows) {
+    h->staged_rows = s.row;  // its rows are the last ones
+  }
+  s = StagedBox{};
+  h->box_set[box] = false;  // until its droplets are in
+  int ext[3];
+  sort_extent(h->boxes[box], ext);
+  if (n > 0 && brick_key_count(ext[0], ext[1], ext[2]) >= (1ULL << 32)) {
+    return set_err(h, PMP_ERR_INVALID, "box too large for the droplet sort key", box);
+  }
+  if (n >= (1LL << 31)) {
+    return set_err(h, PMP_ERR_INVALID, "2^31 droplets or more in one box", box);
+  }
+  if (n == 0) {
+    h->box_set[box] = true;
+    return PMP_OK;
+  }
+  if (p->layout != PMP_LAYOUT_SOA && p->layout != PMP_LAYOUT_AOS) {
+    return set_err(h, PMP_ERR_INVALID, "unknown particle layout");
+  }
+  rc = stage_room(h, n);
+  if (rc != PMP_OK) {
+    return rc;
+  }
+  const int nc = h->ncomp();
+  const int nr = h->nr();
+  double* rows = staged_row(h, h->staged_rows);
+  const cudaMemcpyKind kind = p->where == PMP_WHERE_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
+  DeviceRanges ranges(h->device);
+  Transit transit(h);
+  if (p->layout == PMP_LAYOUT_SOA) {
+    Columns C;
+    memset(&C, 0, sizeof(C));
+    for (int d = 0; d < 3; ++d) {
+      if (!p->pos[d]) {
+        return set_err(h, PMP_ERR_INVALID, "missing position array");
+      }
+      C.c[d] = const_cast<double*>(p->pos[d]);
+    }
+    for (int r = 0; r < nr; ++r) {
+      C.c[3 + r] = const_cast<double*>(p->rdata[r]);
+    }
+    if (!p->id) {
+      return set_err(h, PMP_ERR_INVALID, "missing id array");
+    }
+    C.id = const_cast<int*>(p->id);
+    bool direct = p->where == PMP_WHERE_DEVICE && ranges.holds(C.id, sizeof(int) * n, sizeof(int));
+    for (int c = 0; c < nc && direct; ++c) {
+      direct = !C.c[c] || ranges.holds(C.c[c], sizeof(double) * n, sizeof(double));
+    }
+    if (!direct) {
+      rc = keep(h, h->transit, store_bytes(h, n));
+      if (rc != PMP_OK) {
+        return rc;
+      }
+      Columns D = columns_in(h->transit.p, nc, n);
+      for (int c = 0; c < nc; ++c) {
+        if (C.c[c]) {
+          PMP_TRY(h, cudaMemcpy(D.c[c], C.c[c], sizeof(double) * n, kind));
+        } else {
+          D.c[c] = nullptr;
+        }
+      }
+      PMP_TRY(h, cudaMemcpy(D.id, C.id, sizeof(int) * n, kind));
+      C = D;
+    }
+    PMP_BY_FUELS(h, (k_columns_to_rows<F><<<nblk(n, kTile), kTile>>>(C, nullptr, n, rows)));
+  } else {
+    const size_t bytes = sizeof(double) * (nc + 1) * (size_t)n;
+    const double* src = static_cast<const double*>(p->aos);
+    if (p->where != PMP_WHERE_DEVICE || !ranges.holds(p->aos, bytes, sizeof(double))) {
+      rc = keep(h, h->transit, bytes);
+      if (rc != PMP_OK) {
+        return rc;
+      }
+      PMP_TRY(h, cudaMemcpy(h->transit.p, p->aos, bytes, kind));
+      src = static_cast<const double*>(h->transit.p);
+    }
+    PMP_BY_FUELS(h, (k_aos_to_rows<F><<<nblk(n, kTile), kTile>>>(src, n, rows)));
+  }
+  PMP_TRY(h, cudaGetLastError());
+  // the caller's arrays are read when the call returns
+  PMP_TRY(h, cudaStreamSynchronize(nullptr));
+  s.n = n;
+  s.row = h->staged_rows;
+  h->staged_rows += n;
+  h->box_set[box] = true;
+  return PMP_OK;
+}
+
+int pmp_spray_num_particles(const pmp_spray* h, int box, long long* n)
+{
+  if (!h || !n || box < 0 || box >= (int)h->boxes.size()) {
+    return PMP_ERR_INVALID;
+  }
+  *n = h->packed ? h->box_begin[box + 1] - h->box_begin[box] : h->staged[box].n;
+  return PMP_OK;
+}
+
+int pmp_spray_get_particles(pmp_spray* h, int box, pmp_particles* out)
+{
+  if (!h || !out || box < 0 || box >= (int)h->boxes.size()) {
+    return PMP_ERR_INVALID;
+  }
+  cudaSetDevice(h->device);
+  pmp::quiesce(h);
+  long long n = 0;
+  pmp_spray_num_particles(h, box, &n);
+  if (out->n != n) {
+    return set_err(h, PMP_ERR_INVALID, "output count differs from the box's droplet count", box);
+  }
+  if (n == 0) {
+    return PMP_OK;
+  }
+  const int nc = h->ncomp();
+  const int nr = h->nr();
+  const bool soa = out->layout == PMP_LAYOUT_SOA;
+  const size_t rec_bytes = sizeof(double) * (nc + 1) * (size_t)n;
+  const cudaMemcpyKind kind = out->where == PMP_WHERE_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
+  DeviceRanges ranges(h->device);
+  Transit transit(h);
+  Columns user;
+  memset(&user, 0, sizeof(user));
+  bool direct = out->where == PMP_WHERE_DEVICE;
+  if (soa) {
+    for (int d = 0; d < 3; ++d) {
+      user.c[d] = out->pos[d];
+    }
+    for (int r = 0; r < nr; ++r) {
+      user.c[3 + r] = out->rdata[r];
+    }
+    user.id = out->id;
+    direct = direct && (!user.id || ranges.holds(user.id, sizeof(int) * n, sizeof(int)));
+    for (int c = 0; c < nc && direct; ++c) {
+      direct = !user.c[c] || ranges.holds(user.c[c], sizeof(double) * n, sizeof(double));
+    }
+  } else {
+    direct = direct && ranges.holds(out->aos, rec_bytes, sizeof(double));
+  }
+  Columns C = user;
+  double* aos = static_cast<double*>(out->aos);
+  if (!direct) {
+    const int rc = keep(h, h->transit, soa ? store_bytes(h, n) : rec_bytes);
+    if (rc != PMP_OK) {
+      return rc;
+    }
+    aos = static_cast<double*>(h->transit.p);
+    C = columns_in(h->transit.p, nc, n);
+  }
+  if (!h->packed) {
+    k_rows_out<<<nblk(n, 256), 256>>>(staged_row(h, h->staged[box].row), row_stride(h->nfuel), nc, n, C,
+                                      soa ? nullptr : aos);
+  } else {
+    const long long o = h->box_begin[box];
+    const long long T = h->total;
+    if (soa) {
+      const dim3 grid(nblk(n, 256), (unsigned)(nc + 1));
+      k_store_to_columns<<<grid, 256>>>(h->soa + o, T, h->ids + o, h->perm() + o, n, nc, C);
+    } else {
+      PMP_BY_FUELS(h, (k_store_to_aos<F><<<nblk(n, kTile), kTile>>>(h->soa + o, T, h->ids + o, h->perm() + o, n, aos)));
+    }
+  }
+  PMP_TRY(h, cudaGetLastError());
+  if (!direct) {
+    if (soa) {
+      for (int c = 0; c < nc; ++c) {
+        if (user.c[c]) {
+          PMP_TRY(h, cudaMemcpy(user.c[c], C.c[c], sizeof(double) * n, kind));
+        }
+      }
+      if (user.id) {
+        PMP_TRY(h, cudaMemcpy(user.id, C.id, sizeof(int) * n, kind));
+      }
+    } else {
+      PMP_TRY(h, cudaMemcpy(out->aos, aos, rec_bytes, kind));
+    }
+  }
+  // the droplets are there when the call returns
+  PMP_TRY(h, cudaStreamSynchronize(nullptr));
+  return PMP_OK;
+}
+
+}  // extern "C"
