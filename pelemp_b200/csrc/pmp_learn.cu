@@ -21,21 +21,13 @@
 #include "learn/learn_common.cuh"
 #include "learn/mlp_mma.cuh"
 #include "learn/mlp_tc.cuh"
+#include "learn/train_step.cuh"
 #include "pmp_handle.h"
 #include "spray_kernels.cuh"
 
 namespace pmp {
 
 // flat parameter layout
-constexpr int kP_W1 = 0;               // 64 x 16 (inputs padded to 16)
-constexpr int kP_B1 = kP_W1 + 64 * 16;
-constexpr int kP_W2 = kP_B1 + 64;      // 64 x 64
-constexpr int kP_B2 = kP_W2 + 64 * 64;
-constexpr int kP_W3 = kP_B2 + 64;      // 64 x 64
-constexpr int kP_B3 = kP_W3 + 64 * 64;
-constexpr int kP_W4 = kP_B3 + 64;      // 8 x 64 (outputs padded to 8)
-constexpr int kP_B4 = kP_W4 + 8 * 64;
-constexpr int kP_N = kP_B4 + 8;
 constexpr int kTupleW = 16;            // x[10], y[5], pad
 
 struct LearnParams {
@@ -59,10 +51,8 @@ struct LearnState {
   float* grads = nullptr;
   float* adam_m = nullptr;
   float* adam_v = nullptr;
-  // training work buffers
-  int bcap = 0;
-  float *X = nullptr, *Yt = nullptr, *H1 = nullptr, *A1 = nullptr, *H2 = nullptr, *A2 = nullptr;
-  float *H3 = nullptr, *A3 = nullptr, *Yp = nullptr, *dY = nullptr, *dA = nullptr, *dH = nullptr;
+  // partial gradients of k_train_rows, one per CTA; rows given to the gradient check
+  float *part = nullptr, *X = nullptr, *Yt = nullptr;
   double* d_stats = nullptr;
   double* d_loss = nullptr;
   // inference
@@ -80,20 +70,10 @@ struct LearnState {
 // ---------------------------------------------------------------------------
 // helpers
 
-__host__ __device__ inline unsigned long long mix64(unsigned long long z)
-{
-  z += 0x9e3779b97f4a7c15ULL;
-  z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ULL;
-  z = (z ^ (z >> 27)) * 0x94d049bb133111ebULL;
-  return z ^ (z >> 31);
-}
-
 __host__ __device__ inline double u01(unsigned long long a, unsigned long long b, unsigned long long c)
 {
   return (double)(mix64(a ^ mix64(b ^ mix64(c))) >> 11) * (1.0 / 9007199254740992.0);
 }
-
-__device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 static float host_bf16r(float x)
 {
@@ -454,314 +434,33 @@ __global__ void k_resid_range(const float* t, long long n, LearnNorm nrm, float*
   }
 }
 
-// batch rows: normalised inputs (16 columns, 10 used) and normalised
-// residual targets about the baseline (8, 5 used)
-__global__ void k_gather_batch(
-  const float* t, long long ntrain, long long base, int B, unsigned long long seed, long long step, int random,
-  LearnNorm nrm, float* X, float* Y)
-{
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= B) {
-    return;
-  }
-  long long i;
-  if (random) {
-    i = (long long)(mix64(seed ^ mix64((unsigned long long)step * 1315423911ULL + r)) % (unsigned long long)ntrain);
-  } else {
-    i = base + r;
-  }
-  const float* o = t + i * kTupleW;
-  float xn[kLearnIn];
-  for (int k = 0; k < kLearnIn; ++k) {
-    xn[k] = (o[k] - nrm.x_mean[k]) * nrm.x_inv_std[k];
-  }
-  for (int k = 0; k < 16; ++k) {
-    X[r * 16 + k] = k < kLearnIn ? xn[k] : 0.f;
-  }
-  const BaseVars bv = base_vars(o, nrm);
-  for (int k = 0; k < 8; ++k) {
-    Y[r * 8 + k] = k < kLearnOut ? (o[kLearnIn + k] - learn_base(nrm, k, xn, bv) - nrm.y_mean[k]) / nrm.y_std[k] : 0.f;
-  }
-}
-
-// C[MxN] (+)= op(A) op(B); A is MxK (TA: stored KxM), B is KxN (TB: stored NxK).
-// blockIdx.z splits K; with more than one split the partial sums are atomically added.
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) k_gemm(
-  int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C, int ldc, int kchunk)
-{
-  __shared__ float As[16][68];
-  __shared__ float Bs[16][68];
-  const int tx = threadIdx.x & 15;
-  const int ty = threadIdx.x >> 4;
-  const int row0 = blockIdx.y * 64;
-  const int col0 = blockIdx.x * 64;
-  const int kbeg = blockIdx.z * kchunk;
-  const int kend = min(K, kbeg + kchunk);
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      acc[i][j] = 0.f;
-    }
-  }
-  for (int k0 = kbeg; k0 < kend; k0 += 16) {
-    for (int i = threadIdx.x; i < 1024; i += 256) {
-      int r, kk;
-      if (TA) {
-        r = i & 63;
-        kk = i >> 6;
-      } else {
-        r = i >> 4;
-        kk = i & 15;
-      }
-      const int gr = row0 + r;
-      const int gk = k0 + kk;
-      float v = 0.f;
-      if (gr < M && gk < kend) {
-        v = TA ? A[(size_t)gk * lda + gr] : A[(size_t)gr * lda + gk];
-      }
-      As[kk][r] = v;
-    }
-    for (int i = threadIdx.x; i < 1024; i += 256) {
-      int c, kk;
-      if (TB) {
-        c = i >> 4;
-        kk = i & 15;
-      } else {
-        c = i & 63;
-        kk = i >> 6;
-      }
-      const int gc = col0 + c;
-      const int gk = k0 + kk;
-      float v = 0.f;
-      if (gc < N && gk < kend) {
-        v = TB ? B[(size_t)gc * ldb + gk] : B[(size_t)gk * ldb + gc];
-      }
-      Bs[kk][c] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        a[i] = As[kk][ty * 4 + i];
-        b[i] = Bs[kk][tx * 4 + i];
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = row0 + ty * 4 + i;
-    if (r >= M) {
-      continue;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int cc = col0 + tx * 4 + j;
-      if (cc < N) {
-        if (gridDim.z > 1) {
-          atomicAdd(&C[(size_t)r * ldc + cc], acc[i][j]);
-        } else {
-          C[(size_t)r * ldc + cc] = acc[i][j];
-        }
-      }
-    }
-  }
-}
-
-__device__ __forceinline__ float silu_exact(float x) { return x / (1.f + expf(-x)); }
-
-// silu(x) as the inference kernel rounds it (mlp_mma.cuh): h = bf16(x/2),
-// bf16(fma(h, bf16(tanh h), h))
-__device__ __forceinline__ float silu_bf16(float x)
-{
-  const float h = bf16r(0.5f * x);
-  return bf16r(fmaf(h, bf16r(tanhf(h)), h));
-}
-
-// H += bias; A = silu(H), with the inference's bf16 roundings when quant
-__global__ void k_bias_act(float* H, float* A, const float* bias, int B, int N, int act, int quant)
-{
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= (long long)B * N) {
-    return;
-  }
-  const int n = (int)(i % N);
-  const float h = H[i] + bias[n];
-  H[i] = h;
-  if (act) {
-    A[i] = quant ? silu_bf16(h) : silu_exact(h);
-  }
-}
-
-// dY = 2 (Yp - Y) / (B * 5) on the 5 used outputs; loss partial sums
-__global__ void k_mse(const float* Yp, const float* Y, float* dY, int B, double* loss)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  float l = 0.f;
-  if (i < B * 8) {
-    const int k = i & 7;
-    if (k < kLearnOut) {
-      const float d = Yp[i] - Y[i];
-      dY[i] = 2.f * d / (float)(B * kLearnOut);
-      l = d * d;
-    } else {
-      dY[i] = 0.f;
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    l += __shfl_down_sync(0xffffffffu, l, o);
-  }
-  if ((threadIdx.x & 31) == 0 && loss) {
-    atomicAdd(loss, (double)l);
-  }
-}
-
-// dH = dA * silu'(H)
-__global__ void k_act_bwd(const float* dA, const float* H, float* dH, long long n)
-{
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) {
-    return;
-  }
-  const float h = H[i];
-  const float s = 1.f / (1.f + expf(-h));
-  dH[i] = dA[i] * s * (1.f + h * (1.f - s));
-}
-
-// db[n] += sum over rows of dH[:, n]
-__global__ void k_colsum(const float* dH, float* db, int B, int N)
-{
-  const int n = blockIdx.x;
-  float s = 0.f;
-  for (int r = threadIdx.x; r < B; r += blockDim.x) {
-    s += dH[(size_t)r * N + n];
-  }
-  __shared__ float red[256];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) {
-      red[threadIdx.x] += red[threadIdx.x + o];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    db[n] += red[0];
-  }
-}
-
-// Adam; wq = the bf16-rounded weights used by the forward pass (biases exact)
-__global__ void k_adam(
-  float* p, float* wq, const float* g, float* m, float* v, int n, float lr, float b1, float b2, float eps,
-  float bc1, float bc2, int quant)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) {
-    return;
-  }
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gi;
-  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float pi = p[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-  p[i] = pi;
-  const bool is_bias = (i >= kP_B1 && i < kP_W2) || (i >= kP_B2 && i < kP_W3) || (i >= kP_B3 && i < kP_W4) ||
-                       (i >= kP_B4);
-  wq[i] = (quant && !is_bias) ? bf16r(pi) : pi;
-}
-
-__global__ void k_quantize(const float* p, float* wq, int n, int quant)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) {
-    return;
-  }
-  const bool is_bias = (i >= kP_B1 && i < kP_W2) || (i >= kP_B2 && i < kP_W3) || (i >= kP_B3 && i < kP_W4) ||
-                       (i >= kP_B4);
-  wq[i] = (quant && !is_bias) ? bf16r(p[i]) : p[i];
-}
-
 // ---------------------------------------------------------------------------
 // host-side training driver
 
-template <bool TA, bool TB>
-static void gemm(int M, int N, int K, const float* A, int lda, const float* Bm, int ldb, float* C, int ldc,
-                 cudaStream_t st, bool accumulate_split)
-{
-  const int kchunk = accumulate_split ? 256 : ((K + 15) / 16) * 16;
-  dim3 grid((N + 63) / 64, (M + 63) / 64, accumulate_split ? (K + kchunk - 1) / kchunk : 1);
-  k_gemm<TA, TB><<<grid, 256, 0, st>>>(M, N, K, A, lda, Bm, ldb, C, ldc, kchunk);
-}
-
 static unsigned nb(long long n, int b = 256) { return (unsigned)((n + b - 1) / b); }
 
-// forward of a batch in the training buffers (X -> Yp); quant rounds activations
-static void forward(LearnState* L, const float* w, int B, int quant, cudaStream_t st)
+// k_train_rows: one CTA per SM at most (its tile takes 173 KB of shared memory)
+constexpr int kTrainCtas = 148;
+
+static int train_ctas(long long rows) { return (int)std::min<long long>((rows + kTrainRows - 1) / kTrainRows, kTrainCtas); }
+
+template <bool BACK>
+static cudaError_t train_rows(const TrainBatch& T, const LearnNorm& nrm, const float* w, int quant, float* part,
+                              double* loss, double* val, cudaStream_t st)
 {
-  gemm<false, true>(B, 64, 16, L->X, 16, w + kP_W1, 16, L->H1, 64, st, false);
-  k_bias_act<<<nb((long long)B * 64), 256, 0, st>>>(L->H1, L->A1, w + kP_B1, B, 64, 1, quant);
-  gemm<false, true>(B, 64, 64, L->A1, 64, w + kP_W2, 64, L->H2, 64, st, false);
-  k_bias_act<<<nb((long long)B * 64), 256, 0, st>>>(L->H2, L->A2, w + kP_B2, B, 64, 1, quant);
-  gemm<false, true>(B, 64, 64, L->A2, 64, w + kP_W3, 64, L->H3, 64, st, false);
-  k_bias_act<<<nb((long long)B * 64), 256, 0, st>>>(L->H3, L->A3, w + kP_B3, B, 64, 1, quant);
-  gemm<false, true>(B, 8, 64, L->A3, 64, w + kP_W4, 64, L->Yp, 8, st, false);
-  k_bias_act<<<nb((long long)B * 8), 256, 0, st>>>(L->Yp, nullptr, w + kP_B4, B, 8, 0, 0);
+  const cudaError_t e = cudaFuncSetAttribute(k_train_rows<BACK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(TrainSmem));
+  if (e != cudaSuccess) {
+    return e;
+  }
+  k_train_rows<BACK><<<train_ctas(T.rows), kTrainThreads, sizeof(TrainSmem), st>>>(T, nrm, w, quant, part, loss, val);
+  return cudaGetLastError();
 }
 
-// backward of the MSE loss into L->grads (zeroed here)
-static void backward(LearnState* L, const float* w, int B, cudaStream_t st)
+static void train_update(LearnState* L, int parts, int apply, const AdamStep& A, int quant, cudaStream_t st)
 {
-  cudaMemsetAsync(L->grads, 0, sizeof(float) * kP_N, st);
-  // output layer
-  gemm<true, false>(8, 64, B, L->dY, 8, L->A3, 64, L->grads + kP_W4, 64, st, true);
-  k_colsum<<<8, 256, 0, st>>>(L->dY, L->grads + kP_B4, B, 8);
-  gemm<false, false>(B, 64, 8, L->dY, 8, w + kP_W4, 64, L->dA, 64, st, false);
-  k_act_bwd<<<nb((long long)B * 64), 256, 0, st>>>(L->dA, L->H3, L->dH, (long long)B * 64);
-  // layer 3
-  gemm<true, false>(64, 64, B, L->dH, 64, L->A2, 64, L->grads + kP_W3, 64, st, true);
-  k_colsum<<<64, 256, 0, st>>>(L->dH, L->grads + kP_B3, B, 64);
-  gemm<false, false>(B, 64, 64, L->dH, 64, w + kP_W3, 64, L->dA, 64, st, false);
-  k_act_bwd<<<nb((long long)B * 64), 256, 0, st>>>(L->dA, L->H2, L->dH, (long long)B * 64);
-  // layer 2
-  gemm<true, false>(64, 64, B, L->dH, 64, L->A1, 64, L->grads + kP_W2, 64, st, true);
-  k_colsum<<<64, 256, 0, st>>>(L->dH, L->grads + kP_B2, B, 64);
-  gemm<false, false>(B, 64, 64, L->dH, 64, w + kP_W2, 64, L->dA, 64, st, false);
-  k_act_bwd<<<nb((long long)B * 64), 256, 0, st>>>(L->dA, L->H1, L->dH, (long long)B * 64);
-  // layer 1
-  gemm<true, false>(64, 16, B, L->dH, 64, L->X, 16, L->grads + kP_W1, 16, st, true);
-  k_colsum<<<64, 256, 0, st>>>(L->dH, L->grads + kP_B1, B, 64);
-}
-
-static int ensure_batch(LearnState* L, int B)
-{
-  if (L->bcap >= B) {
-    return 0;
-  }
-  float** bufs[] = {&L->X, &L->Yt, &L->H1, &L->A1, &L->H2, &L->A2, &L->H3, &L->A3, &L->Yp, &L->dY, &L->dA, &L->dH};
-  const int widths[] = {16, 8, 64, 64, 64, 64, 64, 64, 8, 8, 64, 64};
-  for (int i = 0; i < 12; ++i) {
-    cudaFree(*bufs[i]);
-    *bufs[i] = nullptr;
-    if (cudaMalloc(bufs[i], sizeof(float) * (size_t)B * widths[i]) != cudaSuccess) {
-      return -1;
-    }
-  }
-  L->bcap = B;
-  return 0;
+  k_train_update<<<nb(kP_N, 32), 256, 0, st>>>(L->part, parts, L->params, L->wq, L->grads, L->adam_m, L->adam_v, apply, A,
+                                               quant);
 }
 
 static int ensure_params(LearnState* L)
@@ -775,7 +474,8 @@ static int ensure_params(LearnState* L)
       return -1;
     }
   }
-  if (cudaMalloc(&L->d_stats, sizeof(double) * 64) != cudaSuccess ||
+  if (cudaMalloc(&L->part, sizeof(float) * kP_N * (size_t)kTrainCtas) != cudaSuccess ||
+      cudaMalloc(&L->d_stats, sizeof(double) * 64) != cudaSuccess ||
       cudaMalloc(&L->d_loss, sizeof(double)) != cudaSuccess ||
       cudaMalloc(&L->d_mlp, sizeof(MlpSmem)) != cudaSuccess ||
       cudaMalloc(&L->d_mlp_tc, sizeof(tc::TcMlp)) != cudaSuccess ||
@@ -1653,9 +1353,8 @@ bool learn_audit_on(const pmp_spray* h) { return h->learn && h->learn->audit_fra
 
 static void free_state(LearnState* L)
 {
-  void* bufs[] = {L->tuples, L->d_count, L->params, L->wq, L->grads, L->adam_m, L->adam_v, L->X, L->Yt,
-                  L->H1, L->A1, L->H2, L->A2, L->H3, L->A3, L->Yp, L->dY, L->dA, L->dH, L->d_stats,
-                  L->d_loss, L->d_mlp, L->d_mlp_tc, L->d_audit};
+  void* bufs[] = {L->tuples, L->d_count, L->params, L->wq, L->grads, L->adam_m, L->adam_v, L->part, L->X, L->Yt,
+                  L->d_stats, L->d_loss, L->d_mlp, L->d_mlp_tc, L->d_audit};
   for (void* p : bufs) {
     cudaFree(p);
   }
@@ -1930,9 +1629,6 @@ extern "C" int pmp_spray_learn_train(pmp_spray* h, const pmp_learn_config* cfg, 
     return set_err(h, PMP_ERR_CUDA, "allocation failed");
   }
   const int B = cfg->batch > 0 ? cfg->batch : 8192;
-  if (ensure_batch(L, B) != 0) {
-    return set_err(h, PMP_ERR_CUDA, "allocation failed");
-  }
   cudaStream_t st = nullptr;
   const auto t0 = std::chrono::steady_clock::now();
   // normalisation from all tuples
@@ -2019,20 +1715,19 @@ extern "C" int pmp_spray_learn_train(pmp_spray* h, const pmp_learn_config* cfg, 
   const double lr_end = lr0 * 0.01;
   double loss_first = -1., loss_last = -1.;
   for (long long it = 0; it < steps; ++it) {
-    k_gather_batch<<<nb(B), 256>>>(L->tuples, ntrain, 0, B, L->seed, it, 1, nrm, L->X, L->Yt);
-    forward(L, L->wq, B, quant, st);
     const bool track = (it == 0 || it == steps - 1 || (it % 200) == 0);
     if (track) {
       cudaMemsetAsync(L->d_loss, 0, sizeof(double), st);
     }
-    k_mse<<<nb((long long)B * 8), 256>>>(L->Yp, L->Yt, L->dY, B, track ? L->d_loss : nullptr);
-    backward(L, L->wq, B, st);
+    const TrainBatch T{L->tuples, ntrain, 0, L->seed, it, 1, nullptr, nullptr, B};
+    if (train_rows<true>(T, nrm, L->wq, quant, L->part, track ? L->d_loss : nullptr, nullptr, st) != cudaSuccess) {
+      return set_err(h, PMP_ERR_CUDA, "training failed");
+    }
     const double lr = lr0 * pow(lr_end / lr0, (double)it / (double)steps);
     const double b1 = 0.9, b2 = 0.999;
     const double bc1 = 1. - pow(b1, (double)(it + 1));
     const double bc2 = 1. - pow(b2, (double)(it + 1));
-    k_adam<<<nb(kP_N), 256>>>(L->params, L->wq, L->grads, L->adam_m, L->adam_v, kP_N, (float)lr, (float)b1,
-                              (float)b2, 1e-8f, (float)bc1, (float)bc2, quant);
+    train_update(L, train_ctas(B), 1, {(float)lr, (float)b1, (float)b2, 1e-8f, (float)bc1, (float)bc2}, quant, st);
     if (track) {
       double l = 0.;
       cudaMemcpy(&l, L->d_loss, sizeof(double), cudaMemcpyDeviceToHost);
@@ -2047,24 +1742,12 @@ extern "C" int pmp_spray_learn_train(pmp_spray* h, const pmp_learn_config* cfg, 
     return set_err(h, PMP_ERR_CUDA, "training failed");
   }
   // validation: normalised RMSE per output on the held-out tuples
-  double se[kLearnOut] = {0}, sy[kLearnOut] = {0};
-  std::vector<float> yp((size_t)B * 8), yt((size_t)B * 8);
-  long long done = 0;
-  while (done < nval) {
-    const int bb = (int)std::min((long long)B, nval - done);
-    k_gather_batch<<<nb(bb), 256>>>(L->tuples, n, ntrain + done, bb, 0, 0, 0, nrm, L->X, L->Yt);
-    forward(L, L->wq, bb, quant, st);
-    cudaMemcpy(yp.data(), L->Yp, sizeof(float) * bb * 8, cudaMemcpyDeviceToHost);
-    cudaMemcpy(yt.data(), L->Yt, sizeof(float) * bb * 8, cudaMemcpyDeviceToHost);
-    for (int r = 0; r < bb; ++r) {
-      for (int k = 0; k < kLearnOut; ++k) {
-        const double a = yp[r * 8 + k] * nrm.y_std[k] + nrm.y_mean[k];
-        const double t = yt[r * 8 + k] * nrm.y_std[k] + nrm.y_mean[k];
-        se[k] += (a - t) * (a - t);
-        sy[k] += t * t;
-      }
-    }
-    done += bb;
+  double se[kLearnOut] = {0};
+  cudaMemsetAsync(L->d_stats, 0, sizeof(se), st);
+  const TrainBatch V{L->tuples, n, ntrain, 0, 0, 0, nullptr, nullptr, nval};
+  if (train_rows<false>(V, nrm, L->wq, quant, nullptr, nullptr, L->d_stats, st) != cudaSuccess ||
+      cudaMemcpy(se, L->d_stats, sizeof(se), cudaMemcpyDeviceToHost) != cudaSuccess) {
+    return set_err(h, PMP_ERR_CUDA, "validation failed");
   }
   // inference weights
   std::vector<float> pw(kP_N);
@@ -2170,7 +1853,8 @@ extern "C" int pmp_learn_debug_grad(
     return PMP_ERR_INVALID;
   }
   LearnState* L = new LearnState();
-  if (ensure_params(L) != 0 || ensure_batch(L, n) != 0) {
+  if (ensure_params(L) != 0 || cudaMalloc(&L->X, sizeof(float) * 16 * (size_t)n) != cudaSuccess ||
+      cudaMalloc(&L->Yt, sizeof(float) * 8 * (size_t)n) != cudaSuccess) {
     free_state(L);
     return PMP_ERR_CUDA;
   }
@@ -2188,10 +1872,13 @@ extern "C" int pmp_learn_debug_grad(
   cudaMemcpy(L->params, params, sizeof(float) * kP_N, cudaMemcpyHostToDevice);
   k_quantize<<<nb(kP_N), 256>>>(L->params, L->wq, kP_N, quant);
   cudaMemset(L->d_loss, 0, sizeof(double));
-  forward(L, L->wq, n, quant, nullptr);
-  k_mse<<<nb((long long)n * 8), 256>>>(L->Yp, L->Yt, L->dY, n, L->d_loss);
-  backward(L, L->wq, n, nullptr);
+  const TrainBatch T{nullptr, 0, 0, 0, 0, 0, L->X, L->Yt, n};
   int rc = PMP_OK;
+  if (train_rows<true>(T, L->norm, L->wq, quant, L->part, L->d_loss, nullptr, nullptr) != cudaSuccess) {
+    rc = PMP_ERR_CUDA;
+  } else {
+    train_update(L, train_ctas(n), 0, {}, quant, nullptr);
+  }
   if (cudaDeviceSynchronize() != cudaSuccess) {
     rc = PMP_ERR_CUDA;
   } else {
