@@ -37,6 +37,7 @@ struct LearnParams {
   long long audit_stride;
   long long audit_offset;
   double* audit;  // [0] count, [1..5] sum of squared errors, [6..10] sum of squared targets
+  int* next;      // counter of the items taken beyond the first per CTA, zeroed before the launch
   int ncta;       // items of the CTA map
 };
 
@@ -62,6 +63,7 @@ struct LearnState {
   bool trained = false;
   double gate_margin = 0.05;
   double audit_fraction = 0.0;
+  int* d_next = nullptr;  // next map item of the learned kernel's CTAs
   double* d_audit = nullptr;
   unsigned long long seed = 1;
   double target_std[kLearnOut] = {1., 1., 1., 1., 1.};  // of the raw targets (report)
@@ -479,6 +481,7 @@ static int ensure_params(LearnState* L)
       cudaMalloc(&L->d_loss, sizeof(double)) != cudaSuccess ||
       cudaMalloc(&L->d_mlp, sizeof(MlpSmem)) != cudaSuccess ||
       cudaMalloc(&L->d_mlp_tc, sizeof(tc::TcMlp)) != cudaSuccess ||
+      cudaMalloc(&L->d_next, sizeof(int)) != cudaSuccess ||
       cudaMalloc(&L->d_audit, sizeof(double) * 16) != cudaSuccess) {
     return -1;
   }
@@ -645,13 +648,21 @@ __global__ void __launch_bounds__(BLOCK, PMP_LEARNED_MIN_BLOCKS)
   __shared__ BoxEntry sB[TILES];
   Counters c;
   bool tc_dead = false;  // a timed-out MMA wait stops the CTA (uniform)
-  for (int it = blockIdx.x; it * TILES < L.ncta && !tc_dead; it += gridDim.x) {
+  // items beyond the first are taken from a counter: a CTA that starts late (its
+  // SM held by the FP64 list kernel beside it) leaves its share to the others.
+  // Measured, 1M droplets: 236 us, and 327 us with a fixed share per CTA when
+  // both kernels start together
+  __shared__ int s_next;
+  for (int it = blockIdx.x; it * TILES < L.ncta && !tc_dead; it = s_next) {
     const int item = it * TILES + threadIdx.x / kBlock;
     const bool item_ok = item < L.ncta;
     const int b = item_ok ? P.cta_box[item] : 0;
     // this item's box entry, staged in shared memory (after the previous
     // item's readers are done)
     __syncthreads();
+    if (threadIdx.x == 0) {
+      s_next = (int)gridDim.x + atomicAdd(L.next, 1);
+    }
     {
       const int h = threadIdx.x / kBlock;
       const int* src = reinterpret_cast<const int*>(P.boxes + b);
@@ -1326,6 +1337,10 @@ int launch_learned(pmp_spray* h, const KParams& P, cudaStream_t st, int first, i
   LP.mlp = L->d_mlp;
   LP.mlp_tc = L->d_mlp_tc;
   LP.audit = L->d_audit;
+  LP.next = L->d_next;
+  if (cudaMemsetAsync(L->d_next, 0, sizeof(int), st) != cudaSuccess) {
+    return PMP_ERR_CUDA;
+  }
   LP.ncta = count;
   LP.audit_stride = 0;
   if (L->audit_fraction > 0. && count == h->ncta) {
@@ -1354,7 +1369,7 @@ bool learn_audit_on(const pmp_spray* h) { return h->learn && h->learn->audit_fra
 static void free_state(LearnState* L)
 {
   void* bufs[] = {L->tuples, L->d_count, L->params, L->wq, L->grads, L->adam_m, L->adam_v, L->part, L->X, L->Yt,
-                  L->d_stats, L->d_loss, L->d_mlp, L->d_mlp_tc, L->d_audit};
+                  L->d_stats, L->d_loss, L->d_mlp, L->d_mlp_tc, L->d_next, L->d_audit};
   for (void* p : bufs) {
     cudaFree(p);
   }
