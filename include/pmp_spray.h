@@ -606,6 +606,15 @@ int pmp_learn_debug_solve_baseline(const double* acc, float* coef);
 int pmp_measure_peaks(int device, double* fp64_tflops, double* fp32_tflops,
                       double* sfu_gops);
 
+/* Check of the FP64 kernels' arithmetic (no counterpart in the reference): fn
+ * of x[i] (and y[i]) by the branch-free functions of the update kernels and by
+ * pmp_math.h and IEEE division, and where the former hand over to the latter
+ * (odd[i] = 1).  fn: 0 exp, 1 log, 2 pow, 3 cbrt, 4 log1p, 5 (1 + x)^0.7,
+ * 6 x / y, 7 1 / x, 8 x / y for y near 1, 9 x / y for a launch constant y.
+ * Host arrays of n; runs on the current device. */
+int pmp_debug_math(int fn, const double* x, const double* y, long long n,
+                   double* fast, double* plain, int* odd);
+
 #ifdef __cplusplus
 }
 #endif

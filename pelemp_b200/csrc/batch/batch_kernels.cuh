@@ -31,15 +31,17 @@ __global__ void __launch_bounds__(BLOCK, MINB)
   spray_update_fp64_grid(const __grid_constant__ KParams P, const WorkArgs W)
 {
   __shared__ BoxEntry sB;
+  __shared__ double stash[fp64_stash(NF) * BLOCK];
   const int item = blockIdx.x;
   const int b = W.box[item];
+  stage_math_tables();
   if (stage_box(P, b, sB)) {
     return;
   }
   const long long s = W.start[item] + threadIdx.x;
   Counters c;
   if (s < sB.p_end) {
-    update_one<NS, NF, Form::FP64>(P, sB, b, s, c);
+    update_one<NS, NF, Form::FP64, false, false, MathFast>(P, sB, b, s, c, stash + threadIdx.x, BLOCK);
   }
   flush_counters(P, c);
 }
@@ -49,7 +51,9 @@ __global__ void __launch_bounds__(BLOCK, MINB)
   spray_update_fp64_persistent(const __grid_constant__ KParams P, const WorkArgs W)
 {
   __shared__ int s_item;
+  __shared__ double stash[fp64_stash(NF) * BLOCK];
   Counters c;
+  stage_math_tables();
   if (cta_call_failed(P)) {
     return;
   }
@@ -66,7 +70,7 @@ __global__ void __launch_bounds__(BLOCK, MINB)
     const int b = W.box[item];
     const long long end = min(W.start[item] + W.chunk, P.boxes[b].p_end);
     for (long long s = W.start[item] + threadIdx.x; s < end; s += BLOCK) {
-      update_one<NS, NF, Form::FP64>(P, P.boxes[b], b, s, c);
+      update_one<NS, NF, Form::FP64, false, false, MathFast>(P, P.boxes[b], b, s, c, stash + threadIdx.x, BLOCK);
     }
   }
   flush_counters(P, c);

@@ -53,6 +53,11 @@ struct DevMech {
   double mu[kMaxSpec][4];            // ln mu(lnT), CGS
   double lam[kMaxSpec][4];           // ln lambda(lnT), CGS
   double dbin[kMaxFuel][kMaxSpec][4];// ln(P D_{indx[f],j})(lnT), fuel rows
+  // the same rows without the fuel itself (j ascending), and reciprocals of
+  // the weights (divisors of the FP64 kernels, math_fast64.cuh)
+  double dbo[kMaxFuel][kMaxSpec - 1][4];
+  double inv_mw_kg[kMaxSpec];
+  double inv_mw_g[kMaxSpec];
 };
 
 struct DevFuel {
@@ -64,6 +69,9 @@ struct DevFuel {
   double psat_coef[4 * kMaxFuel];
   double rho_coef[4 * kMaxFuel];
   double hboil_ref[kMaxFuel];  // ref_latent * ((critT-ref_T)/(critT-boilT))^-0.38
+  double hboil_mw[kMaxFuel];   // hboil_ref times the fuel's weight, and its reciprocal
+  double inv_hboil_mw[kMaxFuel];
+  double inv_boilT[kMaxFuel];
   int indx[kMaxFuel];          // gas species of fuel f
   int dep[kMaxFuel];           // deposit species of fuel f
   double ln10;                 // pmp_log(10.), as pmp_pow(10., y) uses it
@@ -74,6 +82,26 @@ struct DevFuel {
   int mom_trans;
   int fixed_parts;
 };
+
+// The derived entries of the FP64 tables, from the others
+inline void finish_tables(DevMech& m, DevFuel& F, int ns, int nf)
+{
+  for (int k = 0; k < ns; ++k) {
+    m.inv_mw_kg[k] = 1. / m.mw_kg[k];
+    m.inv_mw_g[k] = 1. / m.mw_g[k];
+  }
+  for (int f = 0; f < nf; ++f) {
+    const int i = F.indx[f];
+    for (int j = 0; j + 1 < ns; ++j) {
+      for (int n = 0; n < 4; ++n) {
+        m.dbo[f][j][n] = m.dbin[f][j < i ? j : j + 1][n];
+      }
+    }
+    F.hboil_mw[f] = F.hboil_ref[f] * m.mw_kg[i];
+    F.inv_hboil_mw[f] = 1. / F.hboil_mw[f];
+    F.inv_boilT[f] = 1. / F.boilT[f];
+  }
+}
 
 // FP32 copies of the tables for the mixed-precision and learned forms
 // (converted once on the host; scaled where the physics always scales them)

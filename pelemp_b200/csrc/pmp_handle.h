@@ -134,7 +134,7 @@ struct pmp_spray {
   int* err_dev = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // stream-ordered updates: the stream of the last call and an event after
-  // its device work; pending = work enqueued since the last pmp_spray_sync
+  // its device work; pending = work enqueued that nothing has waited for since
   cudaStream_t last_stream = nullptr;
   cudaEvent_t ev_done = nullptr;
   bool pending = false;

@@ -131,6 +131,7 @@ int build_device_tables(pmp_spray* h)
   F.mass_trans = d.mass_trans;
   F.mom_trans = d.mom_trans;
   F.fixed_parts = d.fixed_parts;
+  pmp::finish_tables(m, F, NS, NF);
   // FP32 tables of the mixed / learned forms, fuels' species first when
   // every fuel deposits into its own species
   h->fuel_first = 1;
@@ -989,6 +990,7 @@ void pmp::quiesce(pmp_spray* h)
 {
   if (h->pending && h->ev_done) {
     cudaEventSynchronize(h->ev_done);
+    h->pending = false;
   }
 }
 

@@ -95,6 +95,8 @@ __global__ void __launch_bounds__(kStaticBlock, PMP_FP64_MIN_BLOCKS)
   __shared__ DevParts sD;
   __shared__ int s_box;
   __shared__ long long s_n;
+  __shared__ double stash[fp64_stash(NF) * kStaticBlock];
+  stage_math_tables();
   if (threadIdx.x == 0) {
     int lo = 0;
     int hi = P.nboxes;  // cta_prefix[lo] <= blockIdx.x < cta_prefix[hi]
@@ -128,7 +130,7 @@ __global__ void __launch_bounds__(kStaticBlock, PMP_FP64_MIN_BLOCKS)
   const long long s = (long long)(blockIdx.x - scr->cta_prefix[b]) * kStaticBlock + threadIdx.x;
   Counters c;
   if (s < s_n) {
-    update_one<NS, NF, Form::FP64>(P, sD, sB, b, s, c);
+    update_one<NS, NF, Form::FP64, false, false, MathFastPlanes>(P, sD, sB, b, s, c, stash + threadIdx.x, kStaticBlock);
   }
   flush_counters(P, c);
 }
@@ -309,6 +311,7 @@ extern "C" int pmp_spray_update_static(
   P.f.mass_trans = data->mass_trans;
   P.f.mom_trans = data->mom_trans;
   P.f.fixed_parts = data->fixed_parts;
+  pmp::finish_tables(P.m, P.f, NS, NF);
   for (int d = 0; d < 3; ++d) {
     if (!(geom->dx[d] > 0.)) {
       return fail(err, PMP_ERR_INVALID, "bad geometry");

@@ -20,7 +20,7 @@
 
 #include <cfloat>
 
-#include "phys/pmp_math.h"
+#include "phys/math_fast64.cuh"
 #include "pmp_device.cuh"
 
 namespace pmp {
@@ -78,20 +78,11 @@ __device__ __forceinline__ double rhoL(const DevFuel& f, double T, int spf)
   return a + T * (b + T * (c + T * d));
 }
 
-// log1p(x) and (1 + x)^0.7 sharing one log(1 + x); bit-identical to
-// pmp_log1p(x) and pmp_pow(1. + x, 0.7) for x > -1
-__device__ __forceinline__ void log1p_pow07(double x, double& l1p, double& p07)
-{
-  const double u = 1. + x;
-  const double lu = pmp_log(u);
-  l1p = (fabs(x) < 0.0078125) ? pmp_log1p_core(x) : pmp_log1p_from(x, u, lu);
-  p07 = pmp_exp(0.7 * lu);
-}
-
 // calcHeatCoeff (Drag.H:6-45); pow(BM1, phi) = exp(phi log BM1) with the
 // loop-invariant log hoisted (bit-identical to pmp_pow)
+template <class Math>
 __device__ __forceinline__ double heat_coeff(
-  double ratio, double B_M, double B_eps, double C_eps, double Nu_0)
+  Math& M, double ratio, double B_M, double B_eps, double C_eps, double Nu_0)
 {
   if (B_M <= C_eps) {
     return 0.;
@@ -99,31 +90,31 @@ __device__ __forceinline__ double heat_coeff(
   const int maxIter = 100;
   const double NU2 = Nu_0 - 2.;
   const double BM1 = 1. + B_M;
-  const double lnBM1 = pmp_log(BM1);
-  double phi = ratio / Nu_0;
-  double B_T_old = pmp_exp(phi * lnBM1) - 1.;
-  double logB, p07;
-  log1p_pow07(B_T_old, logB, p07);
-  double invFT = B_T_old / (logB * p07);
-  double Nu_num = 2. + NU2 * invFT;
-  phi = ratio / Nu_num;
-  double B_T = pmp_exp(phi * lnBM1) - 1.;
-  double error = fabs(B_T - B_T_old);
-  int k = 0;
-  while (k < maxIter && error > B_eps) {
-    B_T_old = B_T;
-    log1p_pow07(B_T, logB, p07);
-    invFT = B_T / (logB * p07);
-    Nu_num = 2. + NU2 * invFT;
-    phi = ratio / Nu_num;
-    B_T = pmp_exp(phi * lnBM1) - 1.;
-    error = fabs(B_T - B_T_old);
-    k++;
+  const double lnBM1 = M.log(BM1);
+  // one copy of the step for the start value, the iterations and the final
+  // evaluation: B_T from Nu_0, a first step, up to maxIter more
+  double B_T = M.exp(M.div(ratio, Nu_0) * lnBM1) - 1.;
+  bool go = true;
+  for (int k = 0;; k++) {
+    double logB, p07;
+    M.log1p_pow07(B_T, logB, p07);
+    const double invFT = M.div(B_T, logB * p07);
+    const double Nu_num = 2. + NU2 * invFT;
+    if (!go) {
+      return M.div(Nu_num * logB, B_T);
+    }
+    const double phi = M.div(ratio, Nu_num);
+    const double B_T_old = B_T;
+    B_T = M.exp(phi * lnBM1) - 1.;
+    const double error = fabs(B_T - B_T_old);
+    go = k < maxIter && error > B_eps;
   }
-  log1p_pow07(B_T, logB, p07);
-  invFT = B_T / (logB * p07);
-  Nu_num = 2. + NU2 * invFT;
-  return Nu_num * logB / B_T;
+}
+
+__device__ __forceinline__ double heat_coeff(double ratio, double B_M, double B_eps, double C_eps, double Nu_0)
+{
+  MathPlain M;
+  return heat_coeff(M, ratio, B_M, B_eps, C_eps, Nu_0);
 }
 
 // eos.T2Cpi / eos.T2Hi of species n at T (pmp_thermo.h, same operation
@@ -180,9 +171,9 @@ __device__ __forceinline__ double ey2t(const DevMech& m, double e, const double*
 // (this thread's shared-memory slots, stride sxs), the parcel count, the
 // start mass and the start composition wait there across the inner
 // sub-steps instead of in registers: the same values, fewer spills.
-template <int NS, int NF, bool PELEC = false>
+template <int NS, int NF, bool PELEC, class Math>
 __device__ __forceinline__ int spray_source_fp64(
-  const KParams& P, double flow_dt, GasVals<NS, NF>& gpv, double* vel_io, double& T_io,
+  Math& M, const KParams& P, double flow_dt, GasVals<NS, NF>& gpv, double* vel_io, double& T_io,
   double& dia_io, double* Y_io, double num_ppp, int& id, const double* cBoilT,
   double* sx = nullptr, int sxs = 0)
 {
@@ -217,13 +208,13 @@ __device__ __forceinline__ int spray_source_fp64(
 #pragma unroll
   for (int spf = 0; spf < NF; ++spf) {
     Y_part[spf] = Y_io[spf];
-    rho_part += Y_part[spf] / rhoL(fdat, dmin(T_part, cBoilT[spf]), spf);
+    rho_part += M.div(Y_part[spf], rhoL(fdat, dmin(T_part, cBoilT[spf]), spf));
   }
-  rho_part = 1. / rho_part;
+  rho_part = M.inv(rho_part);
   double dt = flow_dt;
   int isub = 1;
   int nsub = 1;
-  double pmass = PMP_PI / 6. * rho_part * pmp_pow(dia_part, 3.);
+  double pmass = PMP_PI / 6. * rho_part * M.pow(dia_part, 3.);
   double startmass = pmass;
   if (sx) {
     sx[3 * sxs] = num_ppp_;
@@ -245,9 +236,9 @@ __device__ __forceinline__ int spray_source_fp64(
     for (int spf = 0; spf < NF; ++spf) {
       Tboil += Y_part[spf] * cBoilT[spf];
       cp_part += Y_part[spf] * fdat.cp[spf];
-      mw_part += Y_part[spf] / m.mw_kg[fdat.indx[spf]];
+      mw_part += M.divk(Y_part[spf], m.mw_kg[fdat.indx[spf]], m.inv_mw_kg[fdat.indx[spf]]);
     }
-    mw_part = 1. / mw_part;
+    mw_part = M.inv(mw_part);
     const double delT = dmax(gpv.T - T_part, 0.);
     double T_skin = gpv.T;
     if (fdat.mass_trans) {
@@ -268,30 +259,31 @@ __device__ __forceinline__ int spray_source_fp64(
       // calcVaporState (Drag.H:48-135)
       const double RU = kRuCgs * Units<PELEC>::ru;
       const double PATM = kPatmCgs * Units<PELEC>::pres;
+      const Divisor by_p = M.divisor(gpv.p);
       double mbar_vap = 0.;
 #pragma unroll
       for (int spf = 0; spf < NF; ++spf) {
         const int fspec = fdat.indx[spf];
         const int fdspec = fdat.dep[spf];
-        const double boilT_ref = fdat.boilT[spf];
         const double mw_fuel = m.mw_kg[fspec];
+        const double inv_mw = m.inv_mw_kg[fspec];
         const double Tp = dmin(T_part, 0.99 * cBoilT[spf]);
         const double part_latent = h_mks<PELEC>(m, fspec, T_part) + fdat.latent[spf] - fdat.cp[spf] * (Tp - fdat.ref_T);
         L_fuel[spf] = part_latent;
         double pres_sat = 0.;
         if (fdat.psat_coef[4 * spf + 3] == 0.) {
-          pres_sat = PATM * pmp_exp(part_latent * mw_fuel / RU * (1. / boilT_ref - 1. / Tp));
+          pres_sat = PATM * M.exp(M.divk(part_latent * mw_fuel, RU, 1. / RU) * (fdat.inv_boilT[spf] - M.inv(Tp)));
         } else {
           const double a = fdat.psat_coef[4 * spf];
           const double b = fdat.psat_coef[4 * spf + 1];
           const double c = fdat.psat_coef[4 * spf + 2];
           const double d = fdat.psat_coef[4 * spf + 3];
-          pres_sat = d * pmp_exp((a - b / (Tp + c)) * fdat.ln10);
+          pres_sat = d * M.exp((a - M.div(b, Tp + c)) * fdat.ln10);
         }
-        const double X_fluid = sel(gpv.Y, fdspec) * gpv.mw_mix / mw_fuel;
+        const double X_fluid = M.divk(sel(gpv.Y, fdspec) * gpv.mw_mix, mw_fuel, inv_mw);
         if (pres_sat > X_fluid * gpv.p) {
-          const double Xl = Y_part[spf] * mw_part / mw_fuel;
-          const double Xv = Xl * pres_sat / gpv.p;
+          const double Xl = M.divk(Y_part[spf] * mw_part, mw_fuel, inv_mw);
+          const double Xv = M.div(Xl * pres_sat, by_p);
           mbar_vap += Xv * mw_fuel;
           sumXVap += Xv;
           X_vapor[spf] = Xv;
@@ -299,7 +291,7 @@ __device__ __forceinline__ int spray_source_fp64(
           X_vapor[spf] = 0.;
         }
       }
-      const double totalmwx = mbar_vap + (1. - sumXVap) * gpv.mw_mix;
+      const Divisor totalmwx = M.divisor(mbar_vap + (1. - sumXVap) * gpv.mw_mix);
       double sumYSkin = 0.;
       double sumYfFluid = 0.;
       double sumYVap = 0.;
@@ -308,7 +300,7 @@ __device__ __forceinline__ int spray_source_fp64(
         if (X_vapor[spf] > 0.) {
           const int fspec = fdat.indx[spf];
           const double mw_fuel = m.mw_kg[fspec];
-          const double Yfv = X_vapor[spf] * mw_fuel / totalmwx;
+          const double Yfv = M.div(X_vapor[spf] * mw_fuel, totalmwx);
           sumYVap += Yfv;
           const double gasY = sel(gpv.Y, fdat.dep[spf]);
           sumYfFluid += gasY;
@@ -317,17 +309,17 @@ __device__ __forceinline__ int spray_source_fp64(
           sumYSkin += Ysk;
         }
       }
-      const double renorm = (1. - sumYSkin) / (1. - sumYfFluid);
+      const double renorm = M.div(1. - sumYSkin, M.divisor_near1(1. - sumYfFluid));
 #pragma unroll
       for (int n = 0; n < NS; ++n) {
         if (Y_skin[n] == 0.) {
           Y_skin[n] = gpv.Y[n] * renorm;
         }
         cp_skin += Y_skin[n] * cp_mks<PELEC>(m, n, T_skin);
-        mw_skin += Y_skin[n] / m.mw_kg[n];
+        mw_skin += M.divk(Y_skin[n], m.mw_kg[n], m.inv_mw_kg[n]);
       }
-      mw_skin = 1. / mw_skin;
-      B_M = (sumYVap - sumYfFluid) / dmax(C_eps, (1. - sumYVap));
+      mw_skin = M.inv(mw_skin);
+      B_M = M.div(sumYVap - sumYfFluid, M.divisor_near1(dmax(C_eps, (1. - sumYVap))));
       B_M = dmin(20., B_M);
     } else {
 #pragma unroll
@@ -341,7 +333,7 @@ __device__ __forceinline__ int spray_source_fp64(
     double mu_skin = 0.;
     double rho_skin = gpv.rho;
     if (fdat.mass_trans) {
-      rho_skin = mw_skin * gpv.p / (kRuCgs * Units<PELEC>::ru * T_skin);
+      rho_skin = M.div(mw_skin * gpv.p, kRuCgs * Units<PELEC>::ru * T_skin);
     }
     // trans.transport at (T_skin, Y_skin) (pmp_thermo.h), fuel rows of Ddiag
     {
@@ -349,25 +341,25 @@ __device__ __forceinline__ int spray_source_fp64(
       double sumYW = 0.;
 #pragma unroll
       for (int k = 0; k < NS; ++k) {
-        sumYW += Y_skin[k] / m.mw_g[k];
+        sumYW += M.divk(Y_skin[k], m.mw_g[k], m.inv_mw_g[k]);
       }
-      const double wbar = 1.0 / sumYW;
+      const double wbar = M.inv(sumYW);
 #pragma unroll
       for (int k = 0; k < NS; ++k) {
-        X[k] = Y_skin[k] * wbar / m.mw_g[k];
+        X[k] = M.divk(Y_skin[k] * wbar, m.mw_g[k], m.inv_mw_g[k]);
       }
-      const double lnT = pmp_log(T_skin);
+      const double lnT = M.log(T_skin);
       double s = 0.0;
 #pragma unroll
       for (int k = 0; k < NS; ++k) {
-        s = fma(X[k], pmp_exp(6.0 * cubic(m.mu[k], lnT)), s);
+        s = fma(X[k], M.exp(6.0 * cubic(m.mu[k], lnT)), s);
       }
-      mu_skin = pmp_exp(pmp_log(s) * (1.0 / 6.0));
+      mu_skin = M.exp(M.log(s) * (1.0 / 6.0));
       if (fdat.mass_trans) {
         double sl = 0.0;
 #pragma unroll
         for (int k = 0; k < NS; ++k) {
-          sl = fma(X[k], pmp_exp(0.25 * cubic(m.lam[k], lnT)), sl);
+          sl = fma(X[k], M.exp(0.25 * cubic(m.lam[k], lnT)), sl);
         }
         const double s2 = sl * sl;
         lambda_skin = s2 * s2;
@@ -378,13 +370,12 @@ __device__ __forceinline__ int spray_source_fp64(
           double term1 = 0.0;
           double term2 = 0.0;
 #pragma unroll
-          for (int j = 0; j < NS; ++j) {
-            if (j != i) {
-              term1 += Y_skin[j];
-              term2 = fma(X[j], pmp_exp(-cubic(m.dbin[f][j], lnT)), term2);
-            }
+          for (int j = 0; j + 1 < NS; ++j) {
+            const bool below = j < i;  // the other species, in order
+            term1 += below ? Y_skin[j] : Y_skin[j + 1];
+            term2 = fma(below ? X[j] : X[j + 1], M.exp(-cubic(m.dbo[f][j], lnT)), term2);
           }
-          Ddiag[f] = m.mw_g[i] * term1 / (term2 * rt);
+          Ddiag[f] = M.div(m.mw_g[i] * term1, term2 * rt);
         }
       }
     }
@@ -397,20 +388,21 @@ __device__ __forceinline__ int spray_source_fp64(
     }
     const double diff_vel_mag =
       sqrt(diff_vel[0] * diff_vel[0] + diff_vel[1] * diff_vel[1] + diff_vel[2] * diff_vel[2]);
-    const double Reyn = rho_skin * diff_vel_mag * dia_part / mu_skin;
-    const double inv_pmass = 1. / pmass;
+    const double Reyn = M.div(rho_skin * diff_vel_mag * dia_part, mu_skin);
+    M.check_finite(Reyn);
+    const double inv_pmass = M.inv(pmass);
     double drag_coef = 0.;
     if (Reyn > 1000.) {
       drag_coef = 0.424;
     } else if (Reyn > 1.) {
-      drag_coef = 24. / Reyn * (1. + pmp_cbrt(Reyn * Reyn) / 6.);
+      drag_coef = M.div(24., Reyn) * (1. + M.divk(M.cbrt(Reyn * Reyn), 6., 1. / 6.));
     } else if (Reyn > 0.) {
-      drag_coef = 24. / Reyn;
+      drag_coef = M.div(24., Reyn);
     }
     drag_coef *= (1. + 2.6432 * 0.);
     const double drag_force =
       0.125 * rho_skin * drag_coef * PMP_PI * dia_part * dia_part * diff_vel_mag;
-    const double drag_force_p = 0.75 * rho_skin * drag_coef * diff_vel_mag / (dia_part * rho_part);
+    const double drag_force_p = M.div(0.75 * rho_skin * drag_coef * diff_vel_mag, dia_part * rho_part);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       part_vel_src[d] = drag_force_p * diff_vel[d] + fdat.body_force[d];
@@ -435,36 +427,38 @@ __device__ __forceinline__ int spray_source_fp64(
     double part_temp_src = 0.;
     double m_dot = 0.;
     if (fdat.mass_trans) {
-      const double Pr_skin = mu_skin * cp_skin / lambda_skin;
-      const double powR = dmax(pmp_pow(dmin(400., Reyn), 0.077), 1.);
+      const Divisor by_lambda = M.divisor(lambda_skin);
+      const double Pr_skin = M.div(mu_skin * cp_skin, by_lambda);
+      const double powR = dmax(M.pow(dmin(400., Reyn), 0.077), 1.);
       double Nu_num = 0.;
       double sumL = 0.;
-      const double Nu_0 = 1. + powR * pmp_cbrt(1. + Reyn * Pr_skin);
+      const double Nu_0 = 1. + powR * M.cbrt(1. + Reyn * Pr_skin);
       if (sumXVap > 0.) {
         double rhoDtotal = 0.;
         double cp_fuel = 0.;
         double sumYSkin = 0.;
+        const Divisor by_sumX = M.divisor(sumXVap);
 #pragma unroll
         for (int spf = 0; spf < NF; ++spf) {
           const int fspec = fdat.indx[spf];
-          Ddiag[spf] *= mw_skin / m.mw_kg[fspec] * Units<PELEC>::rhod;
-          const double X_norm = X_vapor[spf] / sumXVap;
+          Ddiag[spf] *= M.divk(mw_skin, m.mw_kg[fspec], m.inv_mw_kg[fspec]) * Units<PELEC>::rhod;
+          const double X_norm = M.div(X_vapor[spf], by_sumX);
           Ddiag[spf] *= X_norm;
           rhoDtotal += Ddiag[spf];
           const double ysk = sel(Y_skin, fspec);
           cp_fuel += ysk * cp_mks<PELEC>(m, fspec, T_skin);
           sumYSkin += ysk;
         }
-        cp_fuel /= sumYSkin;
-        const double Sc_skin = mu_skin / rhoDtotal;
+        cp_fuel = M.div(cp_fuel, sumYSkin);
+        const double Sc_skin = M.div(mu_skin, rhoDtotal);
         double logB, pBM07;
-        log1p_pow07(B_M, logB, pBM07);
-        const double invFM = B_M / (logB * pBM07);
-        const double Sh_0 = 1. + powR * pmp_cbrt(1. + Reyn * Sc_skin);
+        M.log1p_pow07(B_M, logB, pBM07);
+        const double invFM = M.div(B_M, logB * pBM07);
+        const double Sh_0 = 1. + powR * M.cbrt(1. + Reyn * Sc_skin);
         const double Sh_num = 2. + (Sh_0 - 2.) * invFM;
         const double mdotcoeff = PMP_PI * dia_part * Sh_num * logB;
-        const double ratio = cp_fuel * Sh_num * rhoDtotal / lambda_skin;
-        Nu_num = heat_coeff(ratio, B_M, B_eps, C_eps, Nu_0);
+        const double ratio = M.div(cp_fuel * Sh_num * rhoDtotal, by_lambda);
+        Nu_num = heat_coeff(M, ratio, B_M, B_eps, C_eps, Nu_0);
 #pragma unroll
         for (int spf = 0; spf < NF; ++spf) {
           if (X_vapor[spf] > 0.) {
@@ -478,10 +472,10 @@ __device__ __forceinline__ int spray_source_fp64(
       }
       const double conv_src = PMP_PI * lambda_skin * dia_part * delT * Nu_num;
       gpv.eng_src += nppp() * conv_src;
-      part_temp_src = (sumL + conv_src) * inv_pmass / cp_part;
+      part_temp_src = M.div((sumL + conv_src) * inv_pmass, cp_part);
       if (isub == 1 && delT > C_eps) {
-        const double inv_tau_d = -m_dot / (0.2 * pmass);
-        const double inv_tau_T = conv_src * inv_pmass / (cp_part * delT);
+        const double inv_tau_d = M.div(-m_dot, 0.2 * pmass);
+        const double inv_tau_T = M.div(conv_src * inv_pmass, cp_part * delT);
         nsub = min(
           max(nsub, max(static_cast<int>(flow_dt * inv_tau_d), static_cast<int>(flow_dt * inv_tau_T)) + 1),
           nSubMax);
@@ -505,25 +499,27 @@ __device__ __forceinline__ int spray_source_fp64(
         if (NF > 1) {
           rho_part = 0.;
           double sumY = 0.;
+          const Divisor by_mass = M.divisor(new_mass);
 #pragma unroll
           for (int spf = 0; spf < NF; ++spf) {
-            Y_part[spf] = dmin(1., dmax(0., (Y_part[spf] * pmass + mi_dot[spf] * part_dt) / new_mass));
+            Y_part[spf] = dmin(1., dmax(0., M.div(Y_part[spf] * pmass + mi_dot[spf] * part_dt, by_mass)));
             if (Y_part[spf] <= 1.E-12) {
               Y_part[spf] = 0.;
             }
             sumY += Y_part[spf];
           }
+          const Divisor by_sumY = M.divisor_near1(sumY);
 #pragma unroll
           for (int spf = 0; spf < NF; ++spf) {
-            Y_part[spf] /= sumY;
-            rho_part += Y_part[spf] / rhoL(fdat, dmin(T_part, cBoilT[spf]), spf);
+            Y_part[spf] = M.div(Y_part[spf], by_sumY);
+            rho_part += M.div(Y_part[spf], rhoL(fdat, dmin(T_part, cBoilT[spf]), spf));
           }
-          rho_part = 1. / rho_part;
+          rho_part = M.inv(rho_part);
         } else {
           rho_part = rhoL(fdat, dmin(T_part, cBoilT[0]), 0);
         }
         pmass = new_mass;
-        dia_part = pmp_cbrt(6. * pmass / (PMP_PI * rho_part));
+        dia_part = M.cbrt(M.div(6. * pmass, PMP_PI * rho_part));
       } else {
         pmass = 0.;
         id = -1;
@@ -549,7 +545,7 @@ __device__ __forceinline__ int spray_source_fp64(
     startmass = vx[4 * sxs];
   }
   const double np_end = nppp();
-  const double mdot_total = (pmass - startmass) / (fdat.dtmod * flow_dt);
+  const double mdot_total = M.divk(pmass - startmass, fdat.dtmod * flow_dt, P.inv_dtf);
   gpv.mass_src = np_end * mdot_total;
   if (PELEC) {
     // kinetic energy of the exchanged mass (Drag.H:418-421, PeleC branch)
@@ -567,7 +563,7 @@ __device__ __forceinline__ int spray_source_fp64(
   for (int spf = 0; spf < NF; ++spf) {
     const double oldY = Y0[spf];
     const double newY = Y_part[spf];
-    const double midot = (newY * pmass - oldY * startmass) / (fdat.dtmod * flow_dt);
+    const double midot = M.divk(newY * pmass - oldY * startmass, fdat.dtmod * flow_dt, P.inv_dtf);
     gpv.Ydot[spf] = np_end * midot;
     gpv.eng_src += np_end * midot * h_mks<PELEC>(m, fdat.dep[spf], T_h);
     Y_io[spf] = Y_part[spf];

@@ -162,6 +162,280 @@ __device__ __forceinline__ void cell_of(const KParams& P, const double* pos, dou
   }
 }
 
+// InterpolateGasPhase (SprayInterpolation.H:99-150) of a stencil with upper
+// cell ijk and factors ssv, FP64: false when a cell with a weight lies outside
+// the box's state.
+template <int NS, int NF, bool PELEC>
+__device__ __forceinline__ bool gather_fp64(const KParams& P, const BoxEntry& B, const int* ijk, const double (&ssv)[2][3],
+                                            GasVals<NS, NF>& gpv, const CellTile<double2>* tile64)
+{
+  bool state_ok = true;
+  gpv.rho = 0.;
+  gpv.T = 0.;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    gpv.vel[d] = 0.;
+    gpv.mom_src[d] = 0.;
+  }
+#pragma unroll
+  for (int n = 0; n < NS; ++n) {
+    gpv.Y[n] = 0.;
+  }
+#pragma unroll
+  for (int spf = 0; spf < NF; ++spf) {
+    gpv.Ydot[spf] = 0.;
+  }
+  gpv.eng_src = 0.;
+  gpv.mass_src = 0.;
+        const int tb = tile_base(tile64, ijk);
+  #pragma unroll
+        for (int kk = -1; kk < 1; ++kk) {
+  #pragma unroll
+          for (int jj = -1; jj < 1; ++jj) {
+  #pragma unroll
+            for (int ii = -1; ii < 1; ++ii) {
+              const double cw = __dmul_rn(__dmul_rn(ssv[ii + 1][0], ssv[jj + 1][1]), ssv[kk + 1][2]);
+              if (cw > 0.) {
+                const int ci = ijk[0] + ii;
+                const int cj = ijk[1] + jj;
+                const int ck = ijk[2] + kk;
+                if (!in_box(B.state_lo, B.state_hi, ci, cj, ck)) {
+                  state_ok = false;
+                } else if (B.gr64) {
+                  // the cell's record holds the same per-cell terms the plane
+                  // gather below forms (k_gas_records64), so the sums are equal
+                  constexpr int R2 = gas_rec2(NS);
+                  double rec[2 * R2];
+                  if (tb >= 0) {
+                    const double2* r = tile64->rec + (tb + (kk + 1) * tile64->nxy + (jj + 1) * tile64->nx + (ii + 1)) * R2;
+  #pragma unroll
+                    for (int m = 0; m < R2; ++m) {
+                      const double2 v = r[m];
+                      rec[2 * m] = v.x;
+                      rec[2 * m + 1] = v.y;
+                    }
+                  } else {
+                    load_gas_rec64<R2>(B, ci, cj, ck, rec);
+                  }
+                  gpv.rho = __dadd_rn(gpv.rho, __dmul_rn(cw, rec[0]));
+  #pragma unroll
+                  for (int n = 0; n < NS; ++n) {
+                    gpv.Y[n] = __dadd_rn(gpv.Y[n], __dmul_rn(cw, rec[5 + n]));
+                  }
+  #pragma unroll
+                  for (int dir = 0; dir < 3; ++dir) {
+                    gpv.vel[dir] = __dadd_rn(gpv.vel[dir], __dmul_rn(cw, rec[2 + dir]));
+                  }
+                  gpv.T = __dadd_rn(gpv.T, __dmul_rn(cw, rec[1]));
+                } else {
+                  const double* q = B.st + ((ci - B.st_lo[0]) + (cj - B.st_lo[1]) * B.st_j32 + (ck - B.st_lo[2]) * B.st_k32);
+                  const double cur_rho = __ldg(q + P.c_rho * B.st_n32);
+                  gpv.rho = __dadd_rn(gpv.rho, __dmul_rn(cw, cur_rho));
+                  const double inv_rho = 1. / cur_rho;
+                  if (!PELEC) {
+  #pragma unroll
+                    for (int n = 0; n < NS; ++n) {
+                      const double cur_mf = __dmul_rn(__ldg(q + (P.c_spec + n) * B.st_n32), inv_rho);
+                      gpv.Y[n] = __dadd_rn(gpv.Y[n], __dmul_rn(cw, cur_mf));
+                    }
+  #pragma unroll
+                    for (int dir = 0; dir < 3; ++dir) {
+                      gpv.vel[dir] =
+                        __dadd_rn(gpv.vel[dir], __dmul_rn(cw, __ldg(q + (P.c_mom + dir) * B.st_n32)));
+                    }
+                    gpv.T = __dadd_rn(gpv.T, __dmul_rn(cw, __ldg(q + P.c_T * B.st_n32)));
+                  } else {
+                    // PeleC branch (SprayInterpolation.H:111-146): velocity from
+                    // momentum, T from the internal energy (eos.EY2T, the cell's
+                    // T as the guess)
+                    double mass_frac[NS];
+  #pragma unroll
+                    for (int n = 0; n < NS; ++n) {
+                      const double cur_mf = __dmul_rn(__ldg(q + (P.c_spec + n) * B.st_n32), inv_rho);
+                      gpv.Y[n] = __dadd_rn(gpv.Y[n], __dmul_rn(cw, cur_mf));
+                      mass_frac[n] = cur_mf;
+                    }
+                    double ke = 0.;
+  #pragma unroll
+                    for (int dir = 0; dir < 3; ++dir) {
+                      const double vel = __dmul_rn(__ldg(q + (P.c_mom + dir) * B.st_n32), inv_rho);
+                      gpv.vel[dir] = __dadd_rn(gpv.vel[dir], __dmul_rn(cw, vel));
+                      ke = __dadd_rn(ke, __dmul_rn(vel, vel) / 2.);
+                    }
+                    const double intEng = __dsub_rn(__dmul_rn(__ldg(q + P.c_eng * B.st_n32), inv_rho), ke);
+                    const double T_i = ey2t<NS>(P.m, intEng, mass_frac, __ldg(q + P.c_T * B.st_n32));
+                    gpv.T = __dadd_rn(gpv.T, __dmul_rn(cw, T_i));
+                  }
+                }
+              }
+            }
+          }
+        }
+  return state_ok;
+}
+
+// gather_fp64 from the records of a stencil's cells lo .. hi, without a branch
+// per cell.  A cell of weight zero (a droplet on a cell plane or at a wall) is
+// left out by lo == hi in that direction: the same cell again, times zero, so
+// the sums are the same.
+template <int NS, int NF>
+__device__ __forceinline__ void gather_fp64_inner(const BoxEntry& B, const int* lo, const int* hi,
+                                                  const double (&ssv)[2][3], GasVals<NS, NF>& gpv)
+{
+  constexpr int R2 = gas_rec2(NS);
+  double acc[5 + NS];
+#pragma unroll
+  for (int i = 0; i < 5 + NS; ++i) {
+    acc[i] = 0.;
+  }
+  const double2* r0 =
+    B.gr64 + ((lo[2] - B.state_lo[2]) * B.gr_k + (lo[1] - B.state_lo[1]) * B.gr_j + (lo[0] - B.state_lo[0])) * R2;
+  const int dx = (hi[0] - lo[0]) * R2;
+  const int dy = (hi[1] - lo[1]) * B.gr_j * R2;
+  const int dz = (hi[2] - lo[2]) * B.gr_k * R2;
+#pragma unroll
+  for (int kk = 0; kk < 2; ++kk) {
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj) {
+#pragma unroll
+      for (int ii = 0; ii < 2; ++ii) {
+        const double2* r = r0 + (kk ? dz : 0) + (jj ? dy : 0) + (ii ? dx : 0);
+        double2 v[R2];
+#pragma unroll
+        for (int m = 0; m < R2; ++m) {
+          v[m] = __ldg(r + m);
+        }
+        const double cw = __dmul_rn(__dmul_rn(ssv[ii][0], ssv[jj][1]), ssv[kk][2]);
+#pragma unroll
+        for (int i = 0; i < 5 + NS; ++i) {
+          acc[i] = __dadd_rn(acc[i], __dmul_rn(cw, i % 2 ? v[i / 2].y : v[i / 2].x));
+        }
+      }
+    }
+  }
+  gpv.rho = acc[0];
+  gpv.T = acc[1];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    gpv.vel[d] = acc[2 + d];
+    gpv.mom_src[d] = 0.;
+  }
+#pragma unroll
+  for (int n = 0; n < NS; ++n) {
+    gpv.Y[n] = acc[5 + n];
+  }
+#pragma unroll
+  for (int spf = 0; spf < NF; ++spf) {
+    gpv.Ydot[spf] = 0.;
+  }
+  gpv.eng_src = 0.;
+  gpv.mass_src = 0.;
+}
+
+// GasPhaseVals::define and calcBoilT (SprayFuelData.H:178-200)
+template <int NS, int NF, bool PELEC, class Math>
+__device__ __forceinline__ void define_gas(Math& M, const KParams& P, GasVals<NS, NF>& gpv, double* cBoilT)
+{
+        double mw_mix = 0.;
+  #pragma unroll
+        for (int n = 0; n < NS; ++n) {
+          mw_mix = __dadd_rn(mw_mix, M.divk(gpv.Y[n], P.m.mw_kg[n], P.m.inv_mw_kg[n]));
+        }
+        gpv.p = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(gpv.rho, kRuCgs), mw_mix), gpv.T), Units<PELEC>::ru);
+        gpv.mw_mix = M.inv(mw_mix);
+              {
+          const double RU = kRuCgs * Units<PELEC>::ru;
+          const double PATM = kPatmCgs * Units<PELEC>::pres;
+          const double lp = M.log(M.div(PATM, gpv.p));
+  #pragma unroll
+          for (int spf = 0; spf < NF; ++spf) {
+                  const double cc = M.inv(
+        __dadd_rn(M.divk(__dmul_rn(lp, RU), P.f.hboil_mw[spf], P.f.inv_hboil_mw[spf]), P.f.inv_boilT[spf]));
+      cBoilT[spf] = dmin(P.f.critT[spf], cc);
+          }
+        }
+}
+
+// trilinear_interp (SprayInterpolation.H:158-199)
+__device__ __forceinline__ void stencil_factors(const double* lx, const int* ijk, const int* bflags, double (&ssv)[2][3])
+{
+#pragma unroll
+  for (int dir = 0; dir < 3; ++dir) {
+    const double sx_hi = __dsub_rn(lx[dir], static_cast<double>(ijk[dir]));
+    const double sx_lo = __dsub_rn(1., sx_hi);
+    if (bflags[dir] > 1) {
+      ssv[0][dir] = 1.;
+      ssv[1][dir] = 0.;
+    } else if (bflags[dir] < -1) {
+      ssv[0][dir] = 0.;
+      ssv[1][dir] = 1.;
+    } else {
+      ssv[0][dir] = sx_lo;
+      ssv[1][dir] = sx_hi;
+    }
+  }
+}
+
+// Doubles a thread keeps in shared memory across the FP64 droplet physics
+// (stride: the CTA's threads): position, parcel count, start mass, start
+// composition, and the start velocity, temperature and diameter.
+__host__ __device__ constexpr int fp64_stash(int nf) { return 10 + nf; }
+
+// What a sub-cycle's physics leaves
+template <int NF>
+struct SubcycleOut {
+  double vel[3], T, dia, Y[NF];
+  SrcD<NF> src;
+  int id, nsub;
+};
+
+// One sub-cycle of a droplet again, from its stash, with MathPlain: for the
+// rare arguments that MathFast does not take, and for a stencil that leaves
+// the state.  False when a cell with a weight lies outside the
+// box's state.  A call, so that its code stays out of the update's.
+template <int NS, int NF, bool PELEC>
+__device__ __noinline__ bool redo_subcycle(const KParams& P, const BoxEntry& B, const double* sx, int sxs, int b0, int b1,
+                                           int b2, SubcycleOut<NF>* out)
+{
+  MathPlain M;
+  double pos[3], lx[3], ssv[2][3];
+  int ijk[3], ijkc[3];
+  const int bflags[3] = {b0, b1, b2};
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    pos[d] = sx[d * sxs];
+    out->vel[d] = sx[(5 + NF + d) * sxs];
+  }
+  const double num_ppp = sx[3 * sxs];
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    out->Y[f] = sx[(5 + f) * sxs];
+  }
+  out->T = sx[(8 + NF) * sxs];
+  out->dia = sx[(9 + NF) * sxs];
+  cell_of(P, pos, lx, ijk, ijkc);
+  stencil_factors(lx, ijk, bflags, ssv);
+  GasVals<NS, NF> gpv;
+  double cBoilT[NF];
+  if (!gather_fp64<NS, NF, PELEC>(P, B, ijk, ssv, gpv, nullptr)) {
+    return false;
+  }
+  define_gas<NS, NF, PELEC>(M, P, gpv, cBoilT);
+  out->nsub = spray_source_fp64<NS, NF, PELEC>(M, P, P.sub_dt, gpv, out->vel, out->T, out->dia, out->Y, num_ppp, out->id,
+                                               cBoilT);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    out->src.mom[d] = gpv.mom_src[d];
+  }
+  out->src.mass = gpv.mass_src;
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    out->src.Ydot[f] = gpv.Ydot[f];
+  }
+  out->src.eng = gpv.eng_src;
+  return true;
+}
+
 // One droplet slot s of box b through the whole call.  D holds the droplet
 // arrays (the library's packed SoA, or a caller's per-box arrays in the
 // allocation-free entry point).  B is box b's entry: the kernel passes a copy
@@ -183,7 +457,7 @@ __device__ __forceinline__ void cell_of(const KParams& P, const double* pos, dou
 #define PMP_STD(p, v) (*(p) = (v))
 #endif
 
-template <int NS, int NF, Form FORM, bool FF = false, bool PELEC = false>
+template <int NS, int NF, Form FORM, bool FF = false, bool PELEC = false, class Math = MathPlain>
 __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, const BoxEntry& B, int b,
                                            long long s, Counters& c, double* sx = nullptr, int sxs = 0,
                                            const CellTile<double2>* tile64 = nullptr,
@@ -242,23 +516,8 @@ __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, 
         sx[d * sxs] = pos[d];
       }
     }
-    // trilinear_interp (SprayInterpolation.H:158-199)
     double ssv[2][3];
-#pragma unroll
-    for (int dir = 0; dir < 3; ++dir) {
-      const double sx_hi = __dsub_rn(lx[dir], static_cast<double>(ijk[dir]));
-      const double sx_lo = __dsub_rn(1., sx_hi);
-      if (bflags[dir] > 1) {
-        ssv[0][dir] = 1.;
-        ssv[1][dir] = 0.;
-      } else if (bflags[dir] < -1) {
-        ssv[0][dir] = 0.;
-        ssv[1][dir] = 1.;
-      } else {
-        ssv[0][dir] = sx_lo;
-        ssv[1][dir] = sx_hi;
-      }
-    }
+    stencil_factors(lx, ijk, bflags, ssv);
     // InterpolateGasPhase (SprayInterpolation.H:99-150), PeleLMeX branch, then
     // GasPhaseVals::define, calcBoilT and the droplet physics of the form
     SrcD<NF> src;
@@ -266,132 +525,42 @@ __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, 
     bool state_ok = true;
     if (FORM == Form::FP64) {
       GasVals<NS, NF> gpv;
-      gpv.rho = 0.;
-      gpv.T = 0.;
+      Math M;
+      if (Math::records) {
+        // a stencil that leaves the state, or no records: the whole sub-cycle
+        // in redo_subcycle
+        int lo[3], hi[3];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        gpv.vel[d] = 0.;
-        gpv.mom_src[d] = 0.;
-      }
-#pragma unroll
-      for (int n = 0; n < NS; ++n) {
-        gpv.Y[n] = 0.;
-      }
-#pragma unroll
-      for (int spf = 0; spf < NF; ++spf) {
-        gpv.Ydot[spf] = 0.;
-      }
-      gpv.eng_src = 0.;
-      gpv.mass_src = 0.;
-      const int tb = tile_base(tile64, ijk);
-#pragma unroll
-      for (int kk = -1; kk < 1; ++kk) {
-#pragma unroll
-        for (int jj = -1; jj < 1; ++jj) {
-#pragma unroll
-          for (int ii = -1; ii < 1; ++ii) {
-            const double cw = __dmul_rn(__dmul_rn(ssv[ii + 1][0], ssv[jj + 1][1]), ssv[kk + 1][2]);
-            if (cw > 0.) {
-              const int ci = ijk[0] + ii;
-              const int cj = ijk[1] + jj;
-              const int ck = ijk[2] + kk;
-              if (!in_box(B.state_lo, B.state_hi, ci, cj, ck)) {
-                state_ok = false;
-              } else if (B.gr64) {
-                // the cell's record holds the same per-cell terms the plane
-                // gather below forms (k_gas_records64), so the sums are equal
-                constexpr int R2 = gas_rec2(NS);
-                double rec[2 * R2];
-                if (tb >= 0) {
-                  const double2* r = tile64->rec + (tb + (kk + 1) * tile64->nxy + (jj + 1) * tile64->nx + (ii + 1)) * R2;
-#pragma unroll
-                  for (int m = 0; m < R2; ++m) {
-                    const double2 v = r[m];
-                    rec[2 * m] = v.x;
-                    rec[2 * m + 1] = v.y;
-                  }
-                } else {
-                  load_gas_rec64<R2>(B, ci, cj, ck, rec);
-                }
-                gpv.rho = __dadd_rn(gpv.rho, __dmul_rn(cw, rec[0]));
-#pragma unroll
-                for (int n = 0; n < NS; ++n) {
-                  gpv.Y[n] = __dadd_rn(gpv.Y[n], __dmul_rn(cw, rec[5 + n]));
-                }
-#pragma unroll
-                for (int dir = 0; dir < 3; ++dir) {
-                  gpv.vel[dir] = __dadd_rn(gpv.vel[dir], __dmul_rn(cw, rec[2 + dir]));
-                }
-                gpv.T = __dadd_rn(gpv.T, __dmul_rn(cw, rec[1]));
-              } else {
-                const double* q = B.st + ((ci - B.st_lo[0]) + (cj - B.st_lo[1]) * B.st_j32 + (ck - B.st_lo[2]) * B.st_k32);
-                const double cur_rho = __ldg(q + P.c_rho * B.st_n32);
-                gpv.rho = __dadd_rn(gpv.rho, __dmul_rn(cw, cur_rho));
-                const double inv_rho = 1. / cur_rho;
-                if (!PELEC) {
-#pragma unroll
-                  for (int n = 0; n < NS; ++n) {
-                    const double cur_mf = __dmul_rn(__ldg(q + (P.c_spec + n) * B.st_n32), inv_rho);
-                    gpv.Y[n] = __dadd_rn(gpv.Y[n], __dmul_rn(cw, cur_mf));
-                  }
-#pragma unroll
-                  for (int dir = 0; dir < 3; ++dir) {
-                    gpv.vel[dir] =
-                      __dadd_rn(gpv.vel[dir], __dmul_rn(cw, __ldg(q + (P.c_mom + dir) * B.st_n32)));
-                  }
-                  gpv.T = __dadd_rn(gpv.T, __dmul_rn(cw, __ldg(q + P.c_T * B.st_n32)));
-                } else {
-                  // PeleC branch (SprayInterpolation.H:111-146): velocity from
-                  // momentum, T from the internal energy (eos.EY2T, the cell's
-                  // T as the guess)
-                  double mass_frac[NS];
-#pragma unroll
-                  for (int n = 0; n < NS; ++n) {
-                    const double cur_mf = __dmul_rn(__ldg(q + (P.c_spec + n) * B.st_n32), inv_rho);
-                    gpv.Y[n] = __dadd_rn(gpv.Y[n], __dmul_rn(cw, cur_mf));
-                    mass_frac[n] = cur_mf;
-                  }
-                  double ke = 0.;
-#pragma unroll
-                  for (int dir = 0; dir < 3; ++dir) {
-                    const double vel = __dmul_rn(__ldg(q + (P.c_mom + dir) * B.st_n32), inv_rho);
-                    gpv.vel[dir] = __dadd_rn(gpv.vel[dir], __dmul_rn(cw, vel));
-                    ke = __dadd_rn(ke, __dmul_rn(vel, vel) / 2.);
-                  }
-                  const double intEng = __dsub_rn(__dmul_rn(__ldg(q + P.c_eng * B.st_n32), inv_rho), ke);
-                  const double T_i = ey2t<NS>(P.m, intEng, mass_frac, __ldg(q + P.c_T * B.st_n32));
-                  gpv.T = __dadd_rn(gpv.T, __dmul_rn(cw, T_i));
-                }
-              }
-            }
-          }
+        for (int dir = 0; dir < 3; ++dir) {
+          lo[dir] = ssv[0][dir] > 0. ? ijk[dir] - 1 : ijk[dir];
+          hi[dir] = ssv[1][dir] > 0. ? ijk[dir] : ijk[dir] - 1;
         }
+        if (B.gr64 && in_box(B.state_lo, B.state_hi, lo[0], lo[1], lo[2]) &&
+            in_box(B.state_lo, B.state_hi, hi[0], hi[1], hi[2])) {
+          gather_fp64_inner<NS, NF>(B, lo, hi, ssv, gpv);
+        } else {
+          M.odd = true;
+          gpv = GasVals<NS, NF>{};
+        }
+      } else {
+        state_ok = gather_fp64<NS, NF, PELEC>(P, B, ijk, ssv, gpv, tile64);
       }
       if (!state_ok) {
         set_error(P, PMP_ERR_STATE_BOX, b, s);
         ok = false;
         break;
       }
-      double mw_mix = 0.;
-#pragma unroll
-      for (int n = 0; n < NS; ++n) {
-        mw_mix = __dadd_rn(mw_mix, gpv.Y[n] / P.m.mw_kg[n]);
-      }
-      gpv.p = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(gpv.rho, kRuCgs), mw_mix), gpv.T), Units<PELEC>::ru);
-      gpv.mw_mix = 1. / mw_mix;
       double cBoilT[NF];
-      {
-        const double RU = kRuCgs * Units<PELEC>::ru;
-        const double PATM = kPatmCgs * Units<PELEC>::pres;
-        const double lp = pmp_log(PATM / gpv.p);
+      define_gas<NS, NF, PELEC>(M, P, gpv, cBoilT);
+      if (Math::fast) {
 #pragma unroll
-        for (int spf = 0; spf < NF; ++spf) {
-          const double mw_fuel = P.m.mw_kg[P.f.indx[spf]];
-          const double cc = 1. / __dadd_rn(__dmul_rn(lp, RU) / (P.f.hboil_ref[spf] * mw_fuel), 1. / P.f.boilT[spf]);
-          cBoilT[spf] = dmin(P.f.critT[spf], cc);
+        for (int d = 0; d < 3; ++d) {
+          sx[(5 + NF + d) * sxs] = vel[d];
         }
+        sx[(8 + NF) * sxs] = T;
+        sx[(9 + NF) * sxs] = dia;
       }
-      nsub = spray_source_fp64<NS, NF, PELEC>(P, P.sub_dt, gpv, vel, T, dia, Y, num_ppp, id, cBoilT, sx, sxs);
+      nsub = spray_source_fp64<NS, NF, PELEC>(M, P, P.sub_dt, gpv, vel, T, dia, Y, num_ppp, id, cBoilT, sx, sxs);
       if (sx) {
         // the position and the cell it gives, back from shared memory
         const volatile double* vx = sx;
@@ -411,6 +580,28 @@ __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, 
         src.Ydot[spf] = gpv.Ydot[spf];
       }
       src.eng = gpv.eng_src;
+      if (Math::fast && M.odd) {
+        SubcycleOut<NF> o;
+        o.id = D.id[s];
+        if (!redo_subcycle<NS, NF, PELEC>(P, B, sx, sxs, bflags[0], bflags[1], bflags[2], &o)) {
+          set_error(P, PMP_ERR_STATE_BOX, b, s);
+          ok = false;
+          break;
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          vel[d] = o.vel[d];
+        }
+        T = o.T;
+        dia = o.dia;
+#pragma unroll
+        for (int spf = 0; spf < NF; ++spf) {
+          Y[spf] = o.Y[spf];
+        }
+        src = o.src;
+        id = o.id;
+        nsub = o.nsub;
+      }
     } else {
       // FP32 gather of the cells' gas records (weights from the FP64 position)
       constexpr int R4 = gas_rec4(NS);
@@ -571,13 +762,13 @@ __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, 
 }
 
 // update_one over the library's packed droplet arrays
-template <int NS, int NF, Form FORM, bool FF = false, bool PELEC = false>
+template <int NS, int NF, Form FORM, bool FF = false, bool PELEC = false, class Math = MathPlain>
 __device__ __forceinline__ void update_one(const KParams& P, const BoxEntry& B, int b, long long s, Counters& c,
                                            double* sx = nullptr, int sxs = 0,
                                            const CellTile<double2>* tile64 = nullptr,
                                            const CellTile<float4>* tile32 = nullptr)
 {
-  update_one<NS, NF, FORM, FF, PELEC>(P, P.parts, B, b, s, c, sx, sxs, tile64, tile32);
+  update_one<NS, NF, FORM, FF, PELEC, Math>(P, P.parts, B, b, s, c, sx, sxs, tile64, tile32);
 }
 
 __device__ __forceinline__ void flush_counters(const KParams& P, Counters& c)
@@ -600,7 +791,11 @@ __device__ __forceinline__ void flush_counters(const KParams& P, Counters& c)
 }
 
 #ifndef PMP_FP64_MIN_BLOCKS
-#define PMP_FP64_MIN_BLOCKS 5  /* 96 registers: 5 CTAs of 128 per SM (measured best) */
+/* 128 registers: 4 CTAs of 128 per SM.  Few spills, and the update's code
+   (about 90 KB) stays in the instruction cache: with 4 / 5 / 6 CTAs two
+   fuels (2M droplets, 4 sub-cycles) take 2.19 / 2.20 / 2.21 ms, the PeleC
+   coupling (300k) 141 / 152 / 162 us */
+#define PMP_FP64_MIN_BLOCKS 4
 #endif
 #ifndef PMP_MIXED_MIN_BLOCKS
 #define PMP_MIXED_MIN_BLOCKS 7  /* 72 registers: 7 CTAs of 128 per SM (measured best against 6 and 8
@@ -684,13 +879,12 @@ __device__ __forceinline__ void fp64_cta(const KParams& P)
   const int b = P.cta_box[blockIdx.x];
   const long long s = P.cta_start[blockIdx.x] + threadIdx.x;
   prefetch_droplet<NF>(P, s);
+  stage_math_tables();
   if (stage_box(P, b, sB)) {
     return;
   }
   Counters c;
-  // per thread: position, parcel count, start mass, composition, across the
-  // droplet physics (update_one, spray_source_fp64)
-  __shared__ double stash[(5 + NF) * BLOCK];
+  __shared__ double stash[fp64_stash(NF) * BLOCK];
   double* sx = stash + threadIdx.x;
 #if PMP_GATHER_TILE
   constexpr int R2 = gas_rec2(NS);
@@ -701,11 +895,11 @@ __device__ __forceinline__ void fp64_cta(const KParams& P)
     stage_tile<R2, PMP_TILE64_CELLS, BLOCK>(P, P.parts, sB, s, s < sB.p_end, sB.gr64, tile, tile_rec);
   }
   if (s < sB.p_end) {
-    update_one<NS, NF, Form::FP64, false, PELEC>(P, sB, b, s, c, sx, BLOCK, tiled ? &tile : nullptr);
+    update_one<NS, NF, Form::FP64, false, PELEC, MathFast>(P, sB, b, s, c, sx, BLOCK, tiled ? &tile : nullptr);
   }
 #else
   if (s < sB.p_end) {
-    update_one<NS, NF, Form::FP64, false, PELEC>(P, sB, b, s, c, sx, BLOCK);
+    update_one<NS, NF, Form::FP64, false, PELEC, MathFast>(P, sB, b, s, c, sx, BLOCK);
   }
 #endif
   flush_counters(P, c);
@@ -910,9 +1104,11 @@ __global__ void __launch_bounds__(256) k_gas_records64(const __grid_constant__ K
 template <int NS, int NF, int BLOCK, bool PELEC = false>
 __global__ void __launch_bounds__(BLOCK, PMP_FP64_MIN_BLOCKS) spray_update_fp64_list(const __grid_constant__ KParams P)
 {
+  stage_math_tables();
   if (cta_call_failed(P)) {
     return;
   }
+  __shared__ double stash[fp64_stash(NF) * BLOCK];
   const unsigned long long n =
     *reinterpret_cast<volatile unsigned long long*>(P.list_back ? &P.status->fb_gate : &P.status->fb_count);
   Counters c;
@@ -923,7 +1119,7 @@ __global__ void __launch_bounds__(BLOCK, PMP_FP64_MIN_BLOCKS) spray_update_fp64_
     if (P.list_nbox > 0 && (b < P.list_box0 || b >= P.list_box0 + P.list_nbox)) {
       continue;
     }
-    update_one<NS, NF, Form::FP64, false, PELEC>(P, P.boxes[b], b, s, c);
+    update_one<NS, NF, Form::FP64, false, PELEC, MathFastPlanes>(P, P.boxes[b], b, s, c, stash + threadIdx.x, BLOCK);
   }
   flush_counters(P, c);
 }
