@@ -151,15 +151,94 @@ __device__ __forceinline__ int tile_base(const CellTile<Rec>* T, const int* ijk)
   return in ? (ijk[2] - 1 - T->lo[2]) * T->nxy + (ijk[1] - 1 - T->lo[1]) * T->nx + (ijk[0] - 1 - T->lo[0]) : -1;
 }
 
-__device__ __forceinline__ void cell_of(const KParams& P, const double* pos, double* lx, int* ijk, int* ijkc)
+// Cell coordinates of a position: lx = (x - plo) / dx + 1/2, ijk = floor(lx)
+// (the stencil's upper cell), fx = lx - ijk, ijkc = floor((x - plo) / dx) (the
+// cell holding it).  A floor is one addition of 1.5 2^52 rounded down: its low
+// word is the integer, exactly, below 2^31 (floor and conversion are two
+// conversion instructions, which run at a quarter of the FP64 rate); further
+// out, and for NaN, the conversion's saturated integers.
+__device__ __forceinline__ void cell_of(const KParams& P, const double* pos, double* lx, int* ijk, int* ijkc, double* fx)
 {
+  constexpr double kMagic = 6755399441055744.0;
+  bool far = false;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const double l = __dmul_rn(__dsub_rn(pos[d], P.plo[d]), P.dxi[d]);
     lx[d] = __dadd_rn(l, 0.5);
-    ijk[d] = static_cast<int>(floor(lx[d]));
-    ijkc[d] = static_cast<int>(floor(l));
+    const double t = __dadd_rd(lx[d], kMagic);
+    ijk[d] = __double2loint(t);
+    fx[d] = __dsub_rn(lx[d], __dsub_rn(t, kMagic));
+    ijkc[d] = __double2loint(__dadd_rd(l, kMagic));
+    far |= (__double2hiint(l) & 0x7fffffff) >= 0x41d00000;  // |l| >= 2^30 or NaN
   }
+  if (far) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double l = __dmul_rn(__dsub_rn(pos[d], P.plo[d]), P.dxi[d]);
+      ijk[d] = static_cast<int>(floor(lx[d]));
+      ijkc[d] = static_cast<int>(floor(l));
+      fx[d] = __dsub_rn(lx[d], static_cast<double>(ijk[d]));
+    }
+  }
+}
+
+__device__ __forceinline__ void cell_of(const KParams& P, const double* pos, double* lx, int* ijk, int* ijkc)
+{
+  double fx[3];
+  cell_of(P, pos, lx, ijk, ijkc, fx);
+}
+
+// Where a stencil's eight cells of records lie (the gather then has no branch
+// per cell, and its 16-24 loads are in flight together: with the branches the
+// mixed kernel waited 3.5 cycles per issue on loads; 8M two-fuel droplets,
+// mixed, 2.83 -> 2.51 ms): the first, and the steps to
+// the upper cell in each direction.  A cell of weight zero (a droplet on a
+// cell plane or at a wall) is left out by a step of zero: the neighbour again,
+// times zero, so that no cell outside the weights is read and the sums are
+// the same.  in: every cell with a weight is inside the box's state.
+template <typename Rec>
+struct StencilAt {
+  const Rec* r0;
+  int dx, dy, dz;
+  bool in;
+};
+
+template <int R, typename Rec>
+__device__ __forceinline__ StencilAt<Rec> stencil_at(const BoxEntry& B, const Rec* records, const CellTile<Rec>* tile,
+                                                     const int* ijk, const double (&ssv)[2][3])
+{
+  int lo[3], hi[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    lo[d] = ssv[0][d] > 0. ? ijk[d] - 1 : ijk[d];
+    hi[d] = ssv[1][d] > 0. ? ijk[d] : ijk[d] - 1;
+  }
+  StencilAt<Rec> S;
+  S.in = in_box(B.state_lo, B.state_hi, lo[0], lo[1], lo[2]) && in_box(B.state_lo, B.state_hi, hi[0], hi[1], hi[2]);
+  const int tb = tile_base(tile, ijk);
+  if (tb >= 0) {
+    S.r0 = tile->rec + tb * R;
+    S.dx = R;
+    S.dy = tile->nx * R;
+    S.dz = tile->nxy * R;
+    return S;
+  }
+  S.r0 = records + ((lo[2] - B.state_lo[2]) * B.gr_k + (lo[1] - B.state_lo[1]) * B.gr_j + (lo[0] - B.state_lo[0])) * R;
+  S.dx = (hi[0] - lo[0]) * R;
+  S.dy = (hi[1] - lo[1]) * B.gr_j * R;
+  S.dz = (hi[2] - lo[2]) * B.gr_k * R;
+  return S;
+}
+
+// a record's words: from the tile in shared memory when the build has one
+template <typename Rec>
+__device__ __forceinline__ Rec load_rec(const Rec* p)
+{
+#if PMP_GATHER_TILE
+  return *p;
+#else
+  return __ldg(p);
+#endif
 }
 
 // InterpolateGasPhase (SprayInterpolation.H:99-150) of a stencil with upper
@@ -274,13 +353,10 @@ __device__ __forceinline__ bool gather_fp64(const KParams& P, const BoxEntry& B,
   return state_ok;
 }
 
-// gather_fp64 from the records of a stencil's cells lo .. hi, without a branch
-// per cell.  A cell of weight zero (a droplet on a cell plane or at a wall) is
-// left out by lo == hi in that direction: the same cell again, times zero, so
-// the sums are the same.
+// gather_fp64 from records, without a branch per cell
 template <int NS, int NF>
-__device__ __forceinline__ void gather_fp64_inner(const BoxEntry& B, const int* lo, const int* hi,
-                                                  const double (&ssv)[2][3], GasVals<NS, NF>& gpv)
+__device__ __forceinline__ void gather_fp64_inner(const StencilAt<double2>& S, const double (&ssv)[2][3],
+                                                  GasVals<NS, NF>& gpv)
 {
   constexpr int R2 = gas_rec2(NS);
   double acc[5 + NS];
@@ -288,22 +364,17 @@ __device__ __forceinline__ void gather_fp64_inner(const BoxEntry& B, const int* 
   for (int i = 0; i < 5 + NS; ++i) {
     acc[i] = 0.;
   }
-  const double2* r0 =
-    B.gr64 + ((lo[2] - B.state_lo[2]) * B.gr_k + (lo[1] - B.state_lo[1]) * B.gr_j + (lo[0] - B.state_lo[0])) * R2;
-  const int dx = (hi[0] - lo[0]) * R2;
-  const int dy = (hi[1] - lo[1]) * B.gr_j * R2;
-  const int dz = (hi[2] - lo[2]) * B.gr_k * R2;
 #pragma unroll
   for (int kk = 0; kk < 2; ++kk) {
 #pragma unroll
     for (int jj = 0; jj < 2; ++jj) {
 #pragma unroll
       for (int ii = 0; ii < 2; ++ii) {
-        const double2* r = r0 + (kk ? dz : 0) + (jj ? dy : 0) + (ii ? dx : 0);
+        const double2* r = S.r0 + (kk ? S.dz : 0) + (jj ? S.dy : 0) + (ii ? S.dx : 0);
         double2 v[R2];
 #pragma unroll
         for (int m = 0; m < R2; ++m) {
-          v[m] = __ldg(r + m);
+          v[m] = load_rec(r + m);
         }
         const double cw = __dmul_rn(__dmul_rn(ssv[ii][0], ssv[jj][1]), ssv[kk][2]);
 #pragma unroll
@@ -357,11 +428,11 @@ __device__ __forceinline__ void define_gas(Math& M, const KParams& P, GasVals<NS
 }
 
 // trilinear_interp (SprayInterpolation.H:158-199)
-__device__ __forceinline__ void stencil_factors(const double* lx, const int* ijk, const int* bflags, double (&ssv)[2][3])
+__device__ __forceinline__ void stencil_factors(const double* fx, const int* bflags, double (&ssv)[2][3])
 {
 #pragma unroll
   for (int dir = 0; dir < 3; ++dir) {
-    const double sx_hi = __dsub_rn(lx[dir], static_cast<double>(ijk[dir]));
+    const double sx_hi = fx[dir];
     const double sx_lo = __dsub_rn(1., sx_hi);
     if (bflags[dir] > 1) {
       ssv[0][dir] = 1.;
@@ -378,8 +449,12 @@ __device__ __forceinline__ void stencil_factors(const double* lx, const int* ijk
 
 // Doubles a thread keeps in shared memory across the FP64 droplet physics
 // (stride: the CTA's threads): position, parcel count, start mass, start
-// composition, and the start velocity, temperature and diameter.
-__host__ __device__ constexpr int fp64_stash(int nf) { return 10 + nf; }
+// composition, the start velocity, temperature and diameter, and the source
+// cell's offset (last).
+__host__ __device__ constexpr int fp64_stash(int nf) { return 11 + nf; }
+// The same of the mixed form: position, parcel count, start mass, start
+// composition, offset.
+__host__ __device__ constexpr int mixed_stash(int nf) { return 6 + nf; }
 
 // What a sub-cycle's physics leaves
 template <int NF>
@@ -398,7 +473,7 @@ __device__ __noinline__ bool redo_subcycle(const KParams& P, const BoxEntry& B, 
                                            int b2, SubcycleOut<NF>* out)
 {
   MathPlain M;
-  double pos[3], lx[3], ssv[2][3];
+  double pos[3], lx[3], fx[3], ssv[2][3];
   int ijk[3], ijkc[3];
   const int bflags[3] = {b0, b1, b2};
 #pragma unroll
@@ -413,8 +488,8 @@ __device__ __noinline__ bool redo_subcycle(const KParams& P, const BoxEntry& B, 
   }
   out->T = sx[(8 + NF) * sxs];
   out->dia = sx[(9 + NF) * sxs];
-  cell_of(P, pos, lx, ijk, ijkc);
-  stencil_factors(lx, ijk, bflags, ssv);
+  cell_of(P, pos, lx, ijk, ijkc, fx);
+  stencil_factors(fx, bflags, ssv);
   GasVals<NS, NF> gpv;
   double cBoilT[NF];
   if (!gather_fp64<NS, NF, PELEC>(P, B, ijk, ssv, gpv, nullptr)) {
@@ -457,12 +532,13 @@ __device__ __noinline__ bool redo_subcycle(const KParams& P, const BoxEntry& B, 
 #define PMP_STD(p, v) (*(p) = (v))
 #endif
 
-template <int NS, int NF, Form FORM, bool FF = false, bool PELEC = false, class Math = MathPlain>
+template <int NS, int NF, Form FORM, bool FF = false, bool PELEC = false, class Math = MathFast>
 __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, const BoxEntry& B, int b,
-                                           long long s, Counters& c, double* sx = nullptr, int sxs = 0,
+                                           long long s, Counters& c, double* sx, int sxs,
                                            const CellTile<double2>* tile64 = nullptr,
                                            const CellTile<float4>* tile32 = nullptr)
 {
+  constexpr int stash = FORM == Form::FP64 ? fp64_stash(NF) : mixed_stash(NF);
   int id = PMP_LDD(&D.id[s]);
   if (!(id > 0)) {
     return;
@@ -504,20 +580,25 @@ __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, 
   for (int cur_iter = 0; ok && cur_iter < P.num_iter && id > 0; ++cur_iter) {
     // cell of the droplet, from its position at the start of the sub-cycle
     // (recomputed rather than carried, so that it is not live across the physics)
-    double lx[3];
+    double lx[3], fx[3];
     int ijk[3], ijkc[3];
-    cell_of(P, pos, lx, ijk, ijkc);
-    if (sx) {
-      // the position waits in shared memory across the droplet physics (sx:
-      // this thread's slots, stride sxs), which does not read it: fewer
-      // registers live there, fewer spills
+    cell_of(P, pos, lx, ijk, ijkc, fx);
+    // the position and the source cell's offset (-1: outside the sources) wait
+    // in shared memory across the droplet physics (sx: this thread's slots,
+    // stride sxs), which does not read them: fewer registers live there,
+    // fewer spills
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        sx[d * sxs] = pos[d];
-      }
+    for (int d = 0; d < 3; ++d) {
+      sx[d * sxs] = pos[d];
+    }
+    {
+      const bool in = in_box(B.src_lo, B.src_hi, ijkc[0], ijkc[1], ijkc[2]) ||
+                      (P.is_ghost && in_box(B.sr_alo, B.sr_ahi, ijkc[0], ijkc[1], ijkc[2]));
+      const int q = (ijkc[0] - B.sr_lo[0]) + (ijkc[1] - B.sr_lo[1]) * B.sr_j32 + (ijkc[2] - B.sr_lo[2]) * B.sr_k32;
+      *reinterpret_cast<int*>(sx + (stash - 1) * sxs) = in ? q : -1;
     }
     double ssv[2][3];
-    stencil_factors(lx, ijk, bflags, ssv);
+    stencil_factors(fx, bflags, ssv);
     // InterpolateGasPhase (SprayInterpolation.H:99-150), PeleLMeX branch, then
     // GasPhaseVals::define, calcBoilT and the droplet physics of the form
     SrcD<NF> src;
@@ -529,15 +610,9 @@ __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, 
       if (Math::records) {
         // a stencil that leaves the state, or no records: the whole sub-cycle
         // in redo_subcycle
-        int lo[3], hi[3];
-#pragma unroll
-        for (int dir = 0; dir < 3; ++dir) {
-          lo[dir] = ssv[0][dir] > 0. ? ijk[dir] - 1 : ijk[dir];
-          hi[dir] = ssv[1][dir] > 0. ? ijk[dir] : ijk[dir] - 1;
-        }
-        if (B.gr64 && in_box(B.state_lo, B.state_hi, lo[0], lo[1], lo[2]) &&
-            in_box(B.state_lo, B.state_hi, hi[0], hi[1], hi[2])) {
-          gather_fp64_inner<NS, NF>(B, lo, hi, ssv, gpv);
+        const StencilAt<double2> S = stencil_at<gas_rec2(NS)>(B, static_cast<const double2*>(B.gr64), tile64, ijk, ssv);
+        if (B.gr64 && S.in) {
+          gather_fp64_inner<NS, NF>(S, ssv, gpv);
         } else {
           M.odd = true;
           gpv = GasVals<NS, NF>{};
@@ -552,24 +627,13 @@ __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, 
       }
       double cBoilT[NF];
       define_gas<NS, NF, PELEC>(M, P, gpv, cBoilT);
-      if (Math::fast) {
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          sx[(5 + NF + d) * sxs] = vel[d];
-        }
-        sx[(8 + NF) * sxs] = T;
-        sx[(9 + NF) * sxs] = dia;
+      for (int d = 0; d < 3; ++d) {
+        sx[(5 + NF + d) * sxs] = vel[d];
       }
+      sx[(8 + NF) * sxs] = T;
+      sx[(9 + NF) * sxs] = dia;
       nsub = spray_source_fp64<NS, NF, PELEC>(M, P, P.sub_dt, gpv, vel, T, dia, Y, num_ppp, id, cBoilT, sx, sxs);
-      if (sx) {
-        // the position and the cell it gives, back from shared memory
-        const volatile double* vx = sx;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          pos[d] = vx[d * sxs];
-        }
-        cell_of(P, pos, lx, ijk, ijkc);
-      }
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
         src.mom[d] = gpv.mom_src[d];
@@ -580,7 +644,7 @@ __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, 
         src.Ydot[spf] = gpv.Ydot[spf];
       }
       src.eng = gpv.eng_src;
-      if (Math::fast && M.odd) {
+      if (M.odd) {
         SubcycleOut<NF> o;
         o.id = D.id[s];
         if (!redo_subcycle<NS, NF, PELEC>(P, B, sx, sxs, bflags[0], bflags[1], bflags[2], &o)) {
@@ -610,57 +674,42 @@ __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, 
       for (int n = 0; n < NS; ++n) {
         Yg[n] = 0.f;
       }
-      const int tb = tile_base(tile32, ijk);
-      // FP32 weights from the FP64 factors; a corner is gathered when all
-      // three factors are positive (the FP64 product's test, which FP32
-      // products could underflow); one bounds check for the whole stencil,
-      // per corner only when the stencil crosses the grown state box
+      // FP32 weights from the FP64 factors
       float wf[2][3];
 #pragma unroll
       for (int dir = 0; dir < 3; ++dir) {
         wf[0][dir] = (float)ssv[0][dir];
         wf[1][dir] = (float)ssv[1][dir];
       }
-      const bool stencil_in = in_box(B.state_lo, B.state_hi, ijk[0] - 1, ijk[1] - 1, ijk[2] - 1) &&
-                              in_box(B.state_lo, B.state_hi, ijk[0], ijk[1], ijk[2]);
+      const StencilAt<float4> S = stencil_at<R4>(B, static_cast<const float4*>(B.gr), tile32, ijk, ssv);
+      state_ok = S.in;
+      if (S.in) {
 #pragma unroll
-      for (int kk = -1; kk < 1; ++kk) {
+        for (int kk = 0; kk < 2; ++kk) {
 #pragma unroll
-        for (int jj = -1; jj < 1; ++jj) {
+          for (int jj = 0; jj < 2; ++jj) {
 #pragma unroll
-          for (int ii = -1; ii < 1; ++ii) {
-            if (ssv[ii + 1][0] > 0. && ssv[jj + 1][1] > 0. && ssv[kk + 1][2] > 0.) {
-              const int ci = ijk[0] + ii;
-              const int cj = ijk[1] + jj;
-              const int ck = ijk[2] + kk;
-              if (!stencil_in && !in_box(B.state_lo, B.state_hi, ci, cj, ck)) {
-                state_ok = false;
-              } else {
-                float rec[4 * R4];
-                if (tb >= 0) {
-                  const float4* r = tile32->rec + (tb + (kk + 1) * tile32->nxy + (jj + 1) * tile32->nx + (ii + 1)) * R4;
+            for (int ii = 0; ii < 2; ++ii) {
+              const float4* r = S.r0 + (kk ? S.dz : 0) + (jj ? S.dy : 0) + (ii ? S.dx : 0);
+              float rec[4 * R4];
 #pragma unroll
-                  for (int m = 0; m < R4; ++m) {
-                    const float4 v = r[m];
-                    rec[4 * m] = v.x;
-                    rec[4 * m + 1] = v.y;
-                    rec[4 * m + 2] = v.z;
-                    rec[4 * m + 3] = v.w;
-                  }
-                } else {
-                  load_gas_rec<R4>(B, ci, cj, ck, rec);
-                }
-                const float w = wf[ii + 1][0] * wf[jj + 1][1] * wf[kk + 1][2];
-                rho = fmaf(w, rec[0], rho);
-                Tg = fmaf(w, rec[1], Tg);
+              for (int m = 0; m < R4; ++m) {
+                const float4 v = load_rec(r + m);
+                rec[4 * m] = v.x;
+                rec[4 * m + 1] = v.y;
+                rec[4 * m + 2] = v.z;
+                rec[4 * m + 3] = v.w;
+              }
+              const float w = wf[ii][0] * wf[jj][1] * wf[kk][2];
+              rho = fmaf(w, rec[0], rho);
+              Tg = fmaf(w, rec[1], Tg);
 #pragma unroll
-                for (int dir = 0; dir < 3; ++dir) {
-                  vel_g[dir] = fmaf(w, rec[2 + dir], vel_g[dir]);
-                }
+              for (int dir = 0; dir < 3; ++dir) {
+                vel_g[dir] = fmaf(w, rec[2 + dir], vel_g[dir]);
+              }
 #pragma unroll
-                for (int n = 0; n < NS; ++n) {
-                  Yg[n] = fmaf(w, rec[5 + n], Yg[n]);
-                }
+              for (int n = 0; n < NS; ++n) {
+                Yg[n] = fmaf(w, rec[5 + n], Yg[n]);
               }
             }
           }
@@ -693,29 +742,26 @@ __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, 
         cBoilT[spf] = fminf(P.ff.critT[spf], fdiv(1.f, fmaf(lp, P.ff.hb[spf], P.ff.inv_boilT[spf])));
       }
       nsub = spray_source_mixed<NS, NF, FF, PELEC>(P, P.sub_dt, g, cBoilT, vel, T, dia, Y, num_ppp, id, src, sx, sxs);
-      {
-        // the position and the cell it gives, back from shared memory
-        const volatile double* vx = sx;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          pos[d] = vx[d * sxs];
-        }
-        cell_of(P, pos, lx, ijk, ijkc);
-      }
     }
     c.sub += 1;
     c.inner += static_cast<unsigned>(nsub);
     // source scatter into the cell holding the droplet (SprayParticles.cpp:419-441)
     const double cur_coef = P.cur_coef;  // -(1/V) sub_dt / flow_dt, computed on the host
-    if (!in_box(B.src_lo, B.src_hi, ijkc[0], ijkc[1], ijkc[2])) {
-      if (!P.is_ghost || !in_box(B.sr_alo, B.sr_ahi, ijkc[0], ijkc[1], ijkc[2])) {
-        set_error(P, PMP_ERR_SOURCE_BOX, b, s);
-        ok = false;
-        break;
+    const int qoff = *reinterpret_cast<const volatile int*>(sx + (stash - 1) * sxs);
+    if (qoff < 0) {
+      set_error(P, PMP_ERR_SOURCE_BOX, b, s);
+      ok = false;
+      break;
+    }
+    double* q = B.sr + qoff;
+    deposit<NF>(P, q, B.sr_n32, cur_coef, src.mom, src.mass, src.Ydot, src.eng);
+    {
+      const volatile double* vx = sx;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        pos[d] = vx[d * sxs];
       }
     }
-    double* q = B.sr + ((ijkc[0] - B.sr_lo[0]) + (ijkc[1] - B.sr_lo[1]) * B.sr_j32 + (ijkc[2] - B.sr_lo[2]) * B.sr_k32);
-    deposit<NF>(P, q, B.sr_n32, cur_coef, src.mom, src.mass, src.Ydot, src.eng);
     // move (SprayParticles.cpp:444-476)
     if (P.do_move && !P.f.fixed_parts && id > 0) {
 #pragma unroll
@@ -762,9 +808,9 @@ __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, 
 }
 
 // update_one over the library's packed droplet arrays
-template <int NS, int NF, Form FORM, bool FF = false, bool PELEC = false, class Math = MathPlain>
+template <int NS, int NF, Form FORM, bool FF = false, bool PELEC = false, class Math = MathFast>
 __device__ __forceinline__ void update_one(const KParams& P, const BoxEntry& B, int b, long long s, Counters& c,
-                                           double* sx = nullptr, int sxs = 0,
+                                           double* sx, int sxs,
                                            const CellTile<double2>* tile64 = nullptr,
                                            const CellTile<float4>* tile32 = nullptr)
 {
@@ -798,12 +844,14 @@ __device__ __forceinline__ void flush_counters(const KParams& P, Counters& c)
 #define PMP_FP64_MIN_BLOCKS 4
 #endif
 #ifndef PMP_MIXED_MIN_BLOCKS
-#define PMP_MIXED_MIN_BLOCKS 7  /* 72 registers: 7 CTAs of 128 per SM (measured best against 6 and 8
-                                   with the FP32 gas records and the shared-memory stash) */
+/* 72 registers: 7 CTAs of 128 per SM.  8M two-fuel droplets, 4 sub-cycles,
+   with 6 / 7 / 8 CTAs: 2.53 / 2.49 / 2.73 ms (4M, one sub-cycle: 0.42 / 0.40 / 0.42 ms) */
+#define PMP_MIXED_MIN_BLOCKS 7
 #endif
 #ifndef PMP_MIXED_MIN_BLOCKS_SMALL
-#define PMP_MIXED_MIN_BLOCKS_SMALL 8  /* one fuel, <= 3 species: 64 registers, 8 CTAs per SM (config 5:
-                                         +3 % against 7; the 5-species, 2-fuel kernel loses 7 % at 8) */
+/* one fuel, <= 3 species: 64 registers, 8 CTAs per SM (4M droplets: 334 us, 341
+   with 7; the 5-species, 2-fuel kernel is slower with 8) */
+#define PMP_MIXED_MIN_BLOCKS_SMALL 8
 #endif
 __host__ __device__ constexpr int mixed_min_blocks(int ns, int nf)
 {
@@ -931,7 +979,7 @@ __global__ void __launch_bounds__(BLOCK, mixed_min_blocks(NS, NF)) spray_update_
   Counters c;
   // per thread: position, parcel count, start mass, composition (update_one,
   // spray_source_mixed)
-  __shared__ double stash[(5 + NF) * BLOCK];
+  __shared__ double stash[mixed_stash(NF) * BLOCK];
   double* sx = stash + threadIdx.x;
 #if PMP_GATHER_TILE
   constexpr int R4 = gas_rec4(NS);
