@@ -11,7 +11,9 @@
 // and by launches when each product, activation and column sum is a kernel
 // of its own: 25 launches and 350 us a step, the split-K weight gradients
 // 45 us each (32 CTAs, FP32 atomics) and the column sums 11 us each (64
-// CTAs).  Now 36 us for the rows and 4 us for the update.  Every product's sums run in the order of the reduction index, as
+// CTAs).  Now 33 us for the rows and 4 us for the update (256 threads a CTA
+// with 4 x 4 outputs each: 36 us); 42 % of the issue slots, the waits are on
+// shared memory.  Every product's sums run in the order of the reduction index, as
 // an FP32 multiply-add chain; only the gradients' sum over rows is split (64
 // rows, then the CTAs' partials).
 #pragma once
@@ -54,7 +56,7 @@ __device__ __forceinline__ float silu_bf16(float x)
 }
 
 constexpr int kTrainRows = 64;      // batch rows per tile
-constexpr int kTrainThreads = 256;  // 16 x 16, 4 x 4 outputs each
+constexpr int kTrainThreads = 512;  // 2 x 4 outputs each; weight gradients 4 x 4 over half of the rows each
 constexpr int kTP = 68;             // pitch of 64-wide tiles: 16-byte rows, 4 banks apart
 constexpr int kTX = 20;             // pitch of the 16-wide input tile
 constexpr int kTY = 12;             // pitch of the output gradients
@@ -82,7 +84,7 @@ struct TrainSmem {
   float H3[kTrainRows * kTP], A3[kTrainRows * kTP];
   float dH[kTrainRows * kTP];
   float bell[kTrainRows], bg[kTrainRows];
-  float red[4 * 64];
+  float red[8 * 64];
   double val[kLearnOut];
 };
 
@@ -90,25 +92,28 @@ __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast
 __device__ __forceinline__ float at4(const float4& v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
 
 // rows [r][n] = sum_k A[r][k] W[n][k] of a hidden layer, bias and SiLU: this
-// thread's rows 4 ty + i and columns tx + 16 j (the W rows of 16 neighbouring
+// thread's rows 2 ty + i and columns tx + 16 j (the W rows of 16 neighbouring
 // lanes are then 4 banks apart)
 template <int K, int PA>
 __device__ __forceinline__ void layer_fwd(const float* A, const float* W, const float* b, float* H, float* Act, int tx,
                                           int ty, int quant)
 {
-  float acc[4][4] = {};
+  float acc[2][4] = {};
 #pragma unroll 4
   for (int k = 0; k < K; k += 4) {
-    float4 a[4], w[4];
+    float4 a[2], w[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      a[i] = ld4(A + (4 * ty + i) * PA + k);
-      w[i] = ld4(W + (tx + 16 * i) * PA + k);
+    for (int i = 0; i < 2; ++i) {
+      a[i] = ld4(A + (2 * ty + i) * PA + k);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      w[j] = ld4(W + (tx + 16 * j) * PA + k);
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < 2; ++i) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           acc[i][j] = fmaf(at4(a[i], q), at4(w[j], q), acc[i][j]);
@@ -117,23 +122,24 @@ __device__ __forceinline__ void layer_fwd(const float* A, const float* W, const 
     }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < 2; ++i) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int n = tx + 16 * j;
       const float h = acc[i][j] + b[n];
-      const int o = (4 * ty + i) * kTP + n;
+      const int o = (2 * ty + i) * kTP + n;
       H[o] = h;
       Act[o] = quant ? silu_bf16(h) : silu_exact(h);
     }
   }
 }
 
-// acc[n][k] += sum_r dH[r][n] A[r][k]: rows n = 4 ty + i, columns 4 tx + j
-__device__ __forceinline__ void layer_dw(const float* dH, const float* A, float (&acc)[4][4], int tx, int ty)
+// acc[n][k] += sum over rows [r0, r0 + 32) of dH[r][n] A[r][k]: rows n = 4 ty + i,
+// columns 4 tx + j
+__device__ __forceinline__ void layer_dw(const float* dH, const float* A, float (&acc)[4][4], int tx, int ty, int r0)
 {
 #pragma unroll 4
-  for (int r = 0; r < kTrainRows; ++r) {
+  for (int r = r0; r < r0 + kTrainRows / 2; ++r) {
     const float4 d = ld4(dH + r * kTP + 4 * ty);
     const float4 a = ld4(A + r * kTP + 4 * tx);
 #pragma unroll
@@ -151,19 +157,19 @@ __device__ __forceinline__ void layer_dw(const float* dH, const float* A, float 
 template <int N, int PD>
 __device__ __forceinline__ void layer_bwd(const float* D, const float* W, const float* H, float* dH, int tx, int ty)
 {
-  float acc[4][4] = {};
+  float acc[2][4] = {};
 #pragma unroll 2
   for (int n = 0; n < N; n += 4) {
-    float4 d[4];
+    float4 d[2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      d[i] = ld4(D + (4 * ty + i) * PD + n);
+    for (int i = 0; i < 2; ++i) {
+      d[i] = ld4(D + (2 * ty + i) * PD + n);
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const float4 w = ld4(W + (n + q) * kTP + 4 * tx);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < 2; ++i) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           acc[i][j] = fmaf(at4(d[i], q), at4(w, j), acc[i][j]);
@@ -173,8 +179,8 @@ __device__ __forceinline__ void layer_bwd(const float* D, const float* W, const 
   }
   __syncthreads();  // every reader of dH is done
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int o = (4 * ty + i) * kTP + 4 * tx;
+  for (int i = 0; i < 2; ++i) {
+    const int o = (2 * ty + i) * kTP + 4 * tx;
     const float4 h4 = ld4(H + o);
     float v[4];
 #pragma unroll
@@ -188,12 +194,12 @@ __device__ __forceinline__ void layer_bwd(const float* D, const float* W, const 
   __syncthreads();
 }
 
-// sum of 16 of the tile's rows of column n (part p of 4)
+// sum of 8 of the tile's rows of column n (part p of 8)
 __device__ __forceinline__ float col_part(const float* D, int pitch, int n, int p)
 {
   float s = 0.f;
 #pragma unroll 4
-  for (int r = 16 * p; r < 16 * p + 16; ++r) {
+  for (int r = 8 * p; r < 8 * p + 8; ++r) {
     s += D[r * pitch + n];
   }
   return s;
@@ -210,6 +216,8 @@ __global__ void __launch_bounds__(kTrainThreads) k_train_rows(const __grid_const
   extern __shared__ __align__(16) unsigned char train_smem[];
   TrainSmem& S = *reinterpret_cast<TrainSmem*>(train_smem);
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  // weight gradients: the CTA's halves take half of the rows each
+  const int ht = tid & 255, wy = ht >> 4, hr0 = (tid >> 8) * (kTrainRows / 2);
   for (int i = tid; i < 64 * 64; i += kTrainThreads) {
     S.W2[(i >> 6) * kTP + (i & 63)] = w[kP_W2 + i];
     S.W3[(i >> 6) * kTP + (i & 63)] = w[kP_W3 + i];
@@ -277,9 +285,11 @@ __global__ void __launch_bounds__(kTrainThreads) k_train_rows(const __grid_const
         }
       }
       __syncthreads();
-      // residual targets: one (row, output) a thread
-      for (int i = tid; i < kTrainRows * 8; i += kTrainThreads) {
-        const int r = i >> 3, k = i & 7;
+      // residual targets: one (row, output) a thread, the output the same over
+      // a warp (the baseline's coefficients are read from the constant bank)
+      {
+        static_assert(kTrainThreads == kTrainRows * 8, "one (row, output) a thread");
+        const int k = tid / kTrainRows, r = tid % kTrainRows;
         float y = 0.f;
         if (k < kLearnOut && r0 + r < T.rows) {
           float xn[kLearnIn];
@@ -290,9 +300,9 @@ __global__ void __launch_bounds__(kTrainThreads) k_train_rows(const __grid_const
           BaseVars bv;
           bv.ell = S.bell[r];
           bv.g = S.bg[r];
-          y = (S.Y[i] - learn_base(nrm, k, xn, bv) - nrm.y_mean[k]) / nrm.y_std[k];
+          y = (S.Y[r * 8 + k] - learn_base(nrm, k, xn, bv) - nrm.y_mean[k]) / nrm.y_std[k];
         }
-        S.Y[i] = y;
+        S.Y[r * 8 + k] = y;
       }
     } else {
       for (int i = tid; i < kTrainRows * 16; i += kTrainThreads) {
@@ -310,11 +320,10 @@ __global__ void __launch_bounds__(kTrainThreads) k_train_rows(const __grid_const
     __syncthreads();
     layer_fwd<64, kTP>(S.A2, S.W3, S.b3, S.H3, S.A3, tx, ty, quant);
     __syncthreads();
-    // output layer and the loss: two (row, output) a thread
+    // output layer and the loss: one (row, output) a thread
     float l = 0.f;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int r = tid >> 2, k = (tid & 3) + 4 * q;
+    {
+      const int r = tid >> 3, k = tid & 7;
       float acc = 0.f;
 #pragma unroll 4
       for (int c = 0; c < 64; c += 4) {
@@ -354,32 +363,32 @@ __global__ void __launch_bounds__(kTrainThreads) k_train_rows(const __grid_const
       }
     }
     __syncthreads();
-    // layer 4: 8 x 64, output tid / 32, columns 2 (tid % 32)
+    // layer 4: 8 x 64, output ht / 32, columns 2 (ht % 32)
     {
-      const int n = tid >> 5, c = 2 * (tid & 31);
+      const int n = ht >> 5, c = 2 * (ht & 31);
 #pragma unroll 4
-      for (int r = 0; r < kTrainRows; ++r) {
+      for (int r = hr0; r < hr0 + kTrainRows / 2; ++r) {
         const float d = S.dY[r * kTY + n];
         const float2 a = *reinterpret_cast<const float2*>(S.A3 + r * kTP + c);
         g4[0] = fmaf(d, a.x, g4[0]);
         g4[1] = fmaf(d, a.y, g4[1]);
       }
-      if (tid < 32) {
+      if (tid < 64) {
         gb4 += col_part(S.dY, kTY, tid & 7, tid >> 3);
       }
     }
     layer_bwd<8, kTY>(S.dY, S.W4, S.H3, S.dH, tx, ty);
-    layer_dw(S.dH, S.A2, g3, tx, ty);
+    layer_dw(S.dH, S.A2, g3, tx, wy, hr0);
     gb3 += col_part(S.dH, kTP, tid & 63, tid >> 6);
     layer_bwd<64, kTP>(S.dH, S.W3, S.H2, S.dH, tx, ty);
-    layer_dw(S.dH, S.A1, g2, tx, ty);
+    layer_dw(S.dH, S.A1, g2, tx, wy, hr0);
     gb2 += col_part(S.dH, kTP, tid & 63, tid >> 6);
     layer_bwd<64, kTP>(S.dH, S.W2, S.H1, S.dH, tx, ty);
-    // layer 1: 64 x 16, output tid / 4, columns 4 (tid % 4)
+    // layer 1: 64 x 16, output ht / 4, columns 4 (ht % 4)
     {
-      const int n = tid >> 2, c = 4 * (tid & 3);
+      const int n = ht >> 2, c = 4 * (ht & 3);
 #pragma unroll 4
-      for (int r = 0; r < kTrainRows; ++r) {
+      for (int r = hr0; r < hr0 + kTrainRows / 2; ++r) {
         const float d = S.dH[r * kTP + n];
         const float4 x = ld4(S.X + r * kTX + c);
         g1[0] = fmaf(d, x.x, g1[0]);
@@ -397,33 +406,58 @@ __global__ void __launch_bounds__(kTrainThreads) k_train_rows(const __grid_const
     }
     return;
   }
-  float* P = part + (size_t)blockIdx.x * kP_N;
+  // the second half's sums to the first through the activations' tiles
+  float* X = S.H1;
+  __syncthreads();
+  if (tid >= 256) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int o = (4 * ty + i) * 64 + 4 * tx;
-    *reinterpret_cast<float4*>(P + kP_W2 + o) = make_float4(g2[i][0], g2[i][1], g2[i][2], g2[i][3]);
-    *reinterpret_cast<float4*>(P + kP_W3 + o) = make_float4(g3[i][0], g3[i][1], g3[i][2], g3[i][3]);
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        X[(4 * i + j) * 256 + ht] = g2[i][j];
+        X[(16 + 4 * i + j) * 256 + ht] = g3[i][j];
+      }
+      X[(32 + i) * 256 + ht] = g1[i];
+    }
+    X[36 * 256 + ht] = g4[0];
+    X[37 * 256 + ht] = g4[1];
   }
-  *reinterpret_cast<float4*>(P + kP_W1 + 4 * tid) = make_float4(g1[0], g1[1], g1[2], g1[3]);
-  *reinterpret_cast<float2*>(P + kP_W4 + 2 * tid) = make_float2(g4[0], g4[1]);
-  const float gb[3] = {gb1, gb2, gb3};
-  const int at[3] = {kP_B1, kP_B2, kP_B3};
+  __syncthreads();
+  float* P = part + (size_t)blockIdx.x * kP_N;
+  if (tid < 256) {
 #pragma unroll
-  for (int q = 0; q < 3; ++q) {
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        g2[i][j] += X[(4 * i + j) * 256 + ht];
+        g3[i][j] += X[(16 + 4 * i + j) * 256 + ht];
+      }
+      g1[i] += X[(32 + i) * 256 + ht];
+      const int o = (4 * wy + i) * 64 + 4 * tx;
+      *reinterpret_cast<float4*>(P + kP_W2 + o) = make_float4(g2[i][0], g2[i][1], g2[i][2], g2[i][3]);
+      *reinterpret_cast<float4*>(P + kP_W3 + o) = make_float4(g3[i][0], g3[i][1], g3[i][2], g3[i][3]);
+    }
+    g4[0] += X[36 * 256 + ht];
+    g4[1] += X[37 * 256 + ht];
+    *reinterpret_cast<float4*>(P + kP_W1 + 4 * ht) = make_float4(g1[0], g1[1], g1[2], g1[3]);
+    *reinterpret_cast<float2*>(P + kP_W4 + 2 * ht) = make_float2(g4[0], g4[1]);
+  }
+  const float gb[4] = {gb1, gb2, gb3, gb4};
+  const int at[4] = {kP_B1, kP_B2, kP_B3, kP_B4};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int cols = q < 3 ? 64 : 8;  // the output layer's parts lie in the first 64 threads
     __syncthreads();
     S.red[tid] = gb[q];
     __syncthreads();
-    if (tid < 64) {
-      P[at[q] + tid] = (S.red[tid] + S.red[64 + tid]) + (S.red[128 + tid] + S.red[192 + tid]);
+    if (tid < cols) {
+      float v = 0.f;
+#pragma unroll
+      for (int p = 0; p < 8; ++p) {
+        v += S.red[p * cols + tid];
+      }
+      P[at[q] + tid] = v;
     }
-  }
-  __syncthreads();
-  if (tid < 32) {
-    S.red[tid] = gb4;
-  }
-  __syncthreads();
-  if (tid < 8) {
-    P[kP_B4 + tid] = (S.red[tid] + S.red[8 + tid]) + (S.red[16 + tid] + S.red[24 + tid]);
   }
 }
 

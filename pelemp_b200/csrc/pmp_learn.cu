@@ -200,240 +200,244 @@ __global__ void k_learn_tuples(
 // ---------------------------------------------------------------------------
 // training kernels
 
-// column statistics: sum, sum of squares, min, max of the 15 tuple columns
-__global__ void k_tuple_stats(const float* t, long long n, double* st)
+// sum of v over the warp, in lane 0
+template <typename T>
+__device__ __forceinline__ T warp_sum(T v)
 {
-  __shared__ double ssum[15], ssq[15];
-  __shared__ float smin[15], smax[15];
-  if (threadIdx.x < 15) {
-    ssum[threadIdx.x] = 0.;
-    ssq[threadIdx.x] = 0.;
-    smin[threadIdx.x] = 3.4e38f;
-    smax[threadIdx.x] = -3.4e38f;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    v += __shfl_down_sync(0xffffffffu, v, o);
+  }
+  return v;
+}
+__device__ __forceinline__ float warp_min(float v)
+{
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    v = fminf(v, __shfl_down_sync(0xffffffffu, v, o));
+  }
+  return v;
+}
+
+// *p = min(*p, v), *p a double
+__device__ __forceinline__ void atomic_min_d(double* p, double v)
+{
+  unsigned long long* q = reinterpret_cast<unsigned long long*>(p);
+  unsigned long long old = *q, assumed;
+  do {
+    assumed = old;
+    if (__longlong_as_double(assumed) <= v) {
+      return;
+    }
+    old = atomicCAS(q, assumed, __double_as_longlong(v));
+  } while (old != assumed);
+}
+
+// Sums, sums of squares, minima and minima of the negatives of C columns,
+// from this thread's l (sum), q (squares), lo, nhi into st[0..C), st[C..2C),
+// st[2C..3C) and st[3C..4C): warp shuffles, one value per warp, one atomic
+// per CTA (block-wide shared-memory atomics on doubles took 176 us for 131k
+// tuples, now 8).
+template <int C>
+__device__ __forceinline__ void reduce_columns(const double* l, const double* q, const float* lo, const float* nhi, double* st)
+{
+  __shared__ double sl[8][C], sq[8][C];
+  __shared__ float smn[8][C], smx[8][C];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const double a = warp_sum(l[c]), b = warp_sum(q[c]);
+    const float mn = warp_min(lo[c]), mx = warp_min(nhi[c]);
+    if (lane == 0) {
+      sl[warp][c] = a;
+      sq[warp][c] = b;
+      smn[warp][c] = mn;
+      smx[warp][c] = mx;
+    }
   }
   __syncthreads();
+  const int t = threadIdx.x;
+  if (t < 2 * C) {
+    double (*src)[C] = t < C ? sl : sq;
+    double v = 0.;
+    for (int w = 0; w < 8; ++w) {
+      v += src[w][t % C];
+    }
+    atomicAdd(&st[t], v);
+  } else if (t < 4 * C) {
+    float (*src)[C] = t < 3 * C ? smn : smx;
+    float v = src[0][t % C];
+    for (int w = 1; w < 8; ++w) {
+      v = fminf(v, src[w][t % C]);
+    }
+    atomic_min_d(&st[t], (double)v);
+  }
+}
+
+// a tuple's 16 floats
+__device__ __forceinline__ void load_tuple(const float* t, long long i, float* o)
+{
+  const float4* p = reinterpret_cast<const float4*>(t + i * kTupleW);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float4 v = __ldg(p + q);
+    o[4 * q] = v.x;
+    o[4 * q + 1] = v.y;
+    o[4 * q + 2] = v.z;
+    o[4 * q + 3] = v.w;
+  }
+}
+
+// column statistics of the 15 tuple columns (reduce_columns)
+__global__ void __launch_bounds__(256) k_tuple_stats(const float* t, long long n, double* st)
+{
   double ls[15], lq[15];
-  float lmin[15], lmax[15];
+  float lo[15], nhi[15];
+#pragma unroll
   for (int c = 0; c < 15; ++c) {
     ls[c] = 0.;
     lq[c] = 0.;
-    lmin[c] = 3.4e38f;
-    lmax[c] = -3.4e38f;
+    lo[c] = 3.4e38f;
+    nhi[c] = 3.4e38f;
   }
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+    float o[16];
+    load_tuple(t, i, o);
+#pragma unroll
     for (int c = 0; c < 15; ++c) {
-      const float v = t[i * kTupleW + c];
+      const float v = o[c];
       ls[c] += v;
       lq[c] += (double)v * v;
-      lmin[c] = fminf(lmin[c], v);
-      lmax[c] = fmaxf(lmax[c], v);
+      lo[c] = fminf(lo[c], v);
+      nhi[c] = fminf(nhi[c], -v);
     }
   }
-  for (int c = 0; c < 15; ++c) {
-    atomicAdd(&ssum[c], ls[c]);
-    atomicAdd(&ssq[c], lq[c]);
-    // float min/max through the ordered integer view
-    const float mn = lmin[c], mx = lmax[c];
-    if (mn >= 0.f) {
-      atomicMin(reinterpret_cast<int*>(&smin[c]), __float_as_int(mn));
-    } else {
-      atomicMax(reinterpret_cast<unsigned*>(&smin[c]), __float_as_uint(mn));
-    }
-    if (mx >= 0.f) {
-      atomicMax(reinterpret_cast<int*>(&smax[c]), __float_as_int(mx));
-    } else {
-      atomicMin(reinterpret_cast<unsigned*>(&smax[c]), __float_as_uint(mx));
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < 15) {
-    const int c = threadIdx.x;
-    atomicAdd(&st[c], ssum[c]);
-    atomicAdd(&st[15 + c], ssq[c]);
-    // global min/max kept as doubles through a CAS loop
-    unsigned long long* pmn = reinterpret_cast<unsigned long long*>(&st[30 + c]);
-    unsigned long long* pmx = reinterpret_cast<unsigned long long*>(&st[45 + c]);
-    unsigned long long old = *pmn, assumed;
-    do {
-      assumed = old;
-      if (__longlong_as_double(assumed) <= (double)smin[c]) {
-        break;
-      }
-      old = atomicCAS(pmn, assumed, __double_as_longlong((double)smin[c]));
-    } while (old != assumed);
-    old = *pmx;
-    do {
-      assumed = old;
-      if (__longlong_as_double(assumed) >= (double)smax[c]) {
-        break;
-      }
-      old = atomicCAS(pmx, assumed, __double_as_longlong((double)smax[c]));
-    } while (old != assumed);
-  }
+  reduce_columns<15>(ls, lq, lo, nhi, st);
 }
 
 // Normal equations of the baseline fit in FP64: the upper triangle of F^T F
 // (kBaseTerms x kBaseTerms) and F^T Y (kBaseTerms x kLearnOut) over every
 // stride-th tuple, F the baseline features of the normalised inputs and Y the
-// raw targets.  A block of 256 threads stages 128 tuples' features and
-// targets in shared memory; each thread sums fixed entries over them.
+// raw targets.  A CTA stages 64 tuples' features and targets as doubles in
+// shared memory, and a thread sums one 4 x 4 block of entries over half of
+// them: 8 loads for 16 multiply-adds (one entry a thread converted both
+// factors for every product: 115 us for 131k tuples, bound by the conversions).
 constexpr int kBaseCols = kBaseTerms + kLearnOut;
 constexpr int kBaseTri = kBaseTerms * (kBaseTerms + 1) / 2;
 constexpr int kBaseEntries = kBaseTri + kBaseTerms * kLearnOut;
-__global__ void __launch_bounds__(256) k_base_normal(const float* t, long long n, long long stride,
-                                                     LearnNorm nrm, double* out)
+constexpr int kBaseTiles = (kBaseCols + 3) / 4;
+constexpr int kBaseBlocks = kBaseTiles * (kBaseTiles + 1) / 2;
+constexpr int kBaseThreads = (2 * kBaseBlocks + 31) / 32 * 32;
+__global__ void __launch_bounds__(kBaseThreads) k_base_normal(const float* t, long long n, long long stride,
+                                                              const __grid_constant__ LearnNorm nrm, double* out)
 {
-  constexpr int kChunk = 128;  // tuples staged per pass (shared memory)
-  __shared__ float F[kChunk][kBaseCols + 1];
-  constexpr int kPer = (kBaseEntries + 255) / 256;
-  int ea[kPer], eb[kPer];
-  double acc[kPer];
-#pragma unroll
-  for (int q = 0; q < kPer; ++q) {
-    const int e = threadIdx.x + 256 * q;
-    int a = -1, b = -1;
-    if (e < kBaseTri) {
-      int r = e;
-      a = 0;
-      while (r >= kBaseTerms - a) {
-        r -= kBaseTerms - a;
-        ++a;
-      }
-      b = a + r;
-    } else if (e < kBaseEntries) {
-      const int r = e - kBaseTri;
-      a = r / kLearnOut;
-      b = kBaseTerms + r % kLearnOut;
-    }
-    ea[q] = a;
-    eb[q] = b;
-    acc[q] = 0.;
+  constexpr int kChunk = 64;  // tuples staged per pass
+  __shared__ double F[kChunk][4 * kBaseTiles];
+  // block (ta, tb), ta <= tb, and half of the rows
+  const int half = threadIdx.x / kBaseBlocks;
+  int ta = 0, tb = threadIdx.x % kBaseBlocks;
+  while (tb >= kBaseTiles - ta) {
+    tb -= kBaseTiles - ta;
+    ++ta;
   }
+  tb += ta;
+  double acc[4][4] = {};
   const long long m = (n + stride - 1) / stride;
   for (long long c0 = (long long)blockIdx.x * kChunk; c0 < m; c0 += (long long)gridDim.x * kChunk) {
-    const long long i = c0 + threadIdx.x;
-    float* row = F[threadIdx.x % kChunk];
-    if (threadIdx.x >= kChunk) {
-      // the second half of the block only sums
-    } else if (i < m) {
-      const float* o = t + (i * stride) * kTupleW;
-      float xn[kLearnIn];
-      for (int k = 0; k < kLearnIn; ++k) {
-        xn[k] = (o[k] - nrm.x_mean[k]) * nrm.x_inv_std[k];
-      }
-      base_features(xn, base_vars(o, nrm), row);
-      for (int k = 0; k < kLearnOut; ++k) {
-        row[kBaseTerms + k] = o[kLearnIn + k];
-      }
-    } else {
-      for (int k = 0; k < kBaseCols; ++k) {
-        row[k] = 0.f;
-      }
-    }
     __syncthreads();
+    if (threadIdx.x < kChunk) {
+      double* row = F[threadIdx.x];
+      const long long i = c0 + threadIdx.x;
+      float f[kBaseTerms];
+      float o[16] = {};
+      if (i < m) {
+        load_tuple(t, i * stride, o);
+        float xn[kLearnIn];
 #pragma unroll
-    for (int q = 0; q < kPer; ++q) {
-      if (ea[q] >= 0) {
-        double s = 0.;
-        for (int r = 0; r < kChunk; ++r) {
-          s = fma((double)F[r][ea[q]], (double)F[r][eb[q]], s);
+        for (int k = 0; k < kLearnIn; ++k) {
+          xn[k] = (o[k] - nrm.x_mean[k]) * nrm.x_inv_std[k];
         }
-        acc[q] += s;
+        base_features(xn, base_vars(o, nrm), f);
+      }
+#pragma unroll
+      for (int k = 0; k < kBaseTerms; ++k) {
+        row[k] = i < m ? (double)f[k] : 0.;
+      }
+#pragma unroll
+      for (int k = kBaseTerms; k < 4 * kBaseTiles; ++k) {
+        row[k] = k < kBaseCols ? (double)o[kLearnIn + k - kBaseTerms] : 0.;
       }
     }
     __syncthreads();
-  }
+    if (half < 2) {
+#pragma unroll 2
+      for (int r = half * (kChunk / 2); r < (half + 1) * (kChunk / 2); ++r) {
+        double x[4], y[4];
 #pragma unroll
-  for (int q = 0; q < kPer; ++q) {
-    if (ea[q] >= 0) {
-      atomicAdd(&out[threadIdx.x + 256 * q], acc[q]);
+        for (int i = 0; i < 4; ++i) {
+          x[i] = F[r][4 * ta + i];
+          y[i] = F[r][4 * tb + i];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            acc[i][j] = fma(x[i], y[j], acc[i][j]);
+          }
+        }
+      }
+    }
+  }
+  if (half < 2) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int a = 4 * ta + i, b = 4 * tb + j;
+        if (a < kBaseTerms && b < kBaseCols && a <= b) {
+          const int e = b < kBaseTerms ? a * kBaseTerms - a * (a - 1) / 2 + (b - a)
+                                       : kBaseTri + a * kLearnOut + (b - kBaseTerms);
+          atomicAdd(&out[e], acc[i][j]);
+        }
+      }
     }
   }
 }
 
-// Sum and sum of squares of each target's residual about the baseline
-// (st[0..4], st[5..9]).
-__global__ void k_resid_stats(const float* t, long long n, LearnNorm nrm, double* st)
+// Each target's residual about the baseline: sums, sums of squares and range
+// (reduce_columns)
+__global__ void __launch_bounds__(256) k_resid_stats(const float* t, long long n, const __grid_constant__ LearnNorm nrm, double* st)
 {
-  __shared__ double ss[2 * kLearnOut];
-  if (threadIdx.x < 2 * kLearnOut) {
-    ss[threadIdx.x] = 0.;
-  }
-  __syncthreads();
   double ls[kLearnOut], lq[kLearnOut];
+  float lo[kLearnOut], nhi[kLearnOut];
+#pragma unroll
   for (int k = 0; k < kLearnOut; ++k) {
     ls[k] = 0.;
     lq[k] = 0.;
+    lo[k] = 3.4e38f;
+    nhi[k] = 3.4e38f;
   }
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float* o = t + i * kTupleW;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+    float o[16];
+    load_tuple(t, i, o);
     float xn[kLearnIn];
+#pragma unroll
     for (int k = 0; k < kLearnIn; ++k) {
       xn[k] = (o[k] - nrm.x_mean[k]) * nrm.x_inv_std[k];
     }
     const BaseVars bv = base_vars(o, nrm);
+#pragma unroll
     for (int k = 0; k < kLearnOut; ++k) {
-      const double r = (double)o[kLearnIn + k] - (double)learn_base(nrm, k, xn, bv);
+      const float base = learn_base(nrm, k, xn, bv);
+      const double r = (double)o[kLearnIn + k] - (double)base;
       ls[k] += r;
       lq[k] += r * r;
+      const float f = o[kLearnIn + k] - base;
+      lo[k] = fminf(lo[k], f);
+      nhi[k] = fminf(nhi[k], -f);
     }
   }
-  for (int k = 0; k < kLearnOut; ++k) {
-    atomicAdd(&ss[k], ls[k]);
-    atomicAdd(&ss[kLearnOut + k], lq[k]);
-  }
-  __syncthreads();
-  if (threadIdx.x < 2 * kLearnOut) {
-    atomicAdd(&st[threadIdx.x], ss[threadIdx.x]);
-  }
-}
-
-// float min / max through the ordered integer view (mn, mx start at +/-3.4e38)
-__device__ __forceinline__ void atomic_min_max_f(float* mn, float* mx, float lo, float hi)
-{
-  if (lo >= 0.f) {
-    atomicMin(reinterpret_cast<int*>(mn), __float_as_int(lo));
-  } else {
-    atomicMax(reinterpret_cast<unsigned*>(mn), __float_as_uint(lo));
-  }
-  if (hi >= 0.f) {
-    atomicMax(reinterpret_cast<int*>(mx), __float_as_int(hi));
-  } else {
-    atomicMin(reinterpret_cast<unsigned*>(mx), __float_as_uint(hi));
-  }
-}
-
-// Range of each target's normalised residual about the baseline over the
-// tuples (mm[0..4] min, mm[5..9] max): the residual gate's bounds.
-__global__ void k_resid_range(const float* t, long long n, LearnNorm nrm, float* mm)
-{
-  float lo[kLearnOut], hi[kLearnOut];
-  for (int k = 0; k < kLearnOut; ++k) {
-    lo[k] = 3.4e38f;
-    hi[k] = -3.4e38f;
-  }
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float* o = t + i * kTupleW;
-    float xn[kLearnIn];
-    for (int k = 0; k < kLearnIn; ++k) {
-      xn[k] = (o[k] - nrm.x_mean[k]) * nrm.x_inv_std[k];
-    }
-    const BaseVars bv = base_vars(o, nrm);
-    for (int k = 0; k < kLearnOut; ++k) {
-      const float r = (o[kLearnIn + k] - learn_base(nrm, k, xn, bv) - nrm.y_mean[k]) / nrm.y_std[k];
-      lo[k] = fminf(lo[k], r);
-      hi[k] = fmaxf(hi[k], r);
-    }
-  }
-  for (int k = 0; k < kLearnOut; ++k) {
-    for (int off = 16; off > 0; off >>= 1) {
-      lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], off));
-      hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], off));
-    }
-    if ((threadIdx.x & 31) == 0) {
-      atomic_min_max_f(&mm[k], &mm[kLearnOut + k], lo[k], hi[k]);
-    }
-  }
+  reduce_columns<kLearnOut>(ls, lq, lo, nhi, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -1547,7 +1551,8 @@ static bool fit_baseline(LearnState* L, long long n, LearnNorm& nrm)
     return false;
   }
   cudaMemset(d_acc, 0, sizeof(double) * kBaseEntries);
-  k_base_normal<<<592, 256>>>(L->tuples, n, stride, nrm, d_acc);
+  const long long rows = (n + stride - 1) / stride;
+  k_base_normal<<<(int)std::min<long long>(296, (rows + 63) / 64), kBaseThreads>>>(L->tuples, n, stride, nrm, d_acc);
   std::vector<double> acc(kBaseEntries);
   const bool ok = cudaMemcpy(acc.data(), d_acc, sizeof(double) * kBaseEntries, cudaMemcpyDeviceToHost) == cudaSuccess;
   cudaFree(d_acc);
@@ -1646,14 +1651,14 @@ extern "C" int pmp_spray_learn_train(pmp_spray* h, const pmp_learn_config* cfg, 
   const int B = cfg->batch > 0 ? cfg->batch : 8192;
   cudaStream_t st = nullptr;
   const auto t0 = std::chrono::steady_clock::now();
-  // normalisation from all tuples
+  // normalisation from all tuples (a few rows a thread)
+  const int sgrid = (int)std::min<long long>(592, (n + 1023) / 1024);
   std::vector<double> init(64, 0.);
-  for (int c = 0; c < 15; ++c) {
-    init[30 + c] = 1e300;
-    init[45 + c] = -1e300;
+  for (int c = 30; c < 60; ++c) {
+    init[c] = 1e300;  // minima, of the columns and of their negatives
   }
   cudaMemcpy(L->d_stats, init.data(), sizeof(double) * 64, cudaMemcpyHostToDevice);
-  k_tuple_stats<<<592, 256>>>(L->tuples, n, L->d_stats);
+  k_tuple_stats<<<sgrid, 256>>>(L->tuples, n, L->d_stats);
   double stt[64];
   if (cudaMemcpy(stt, L->d_stats, sizeof(stt), cudaMemcpyDeviceToHost) != cudaSuccess) {
     return set_err(h, PMP_ERR_CUDA, "statistics failed");
@@ -1664,7 +1669,7 @@ extern "C" int pmp_spray_learn_train(pmp_spray* h, const pmp_learn_config* cfg, 
     const double mean = stt[k] / n;
     const double var = std::max(0., stt[15 + k] / n - mean * mean);
     const double sd = sqrt(var);
-    const double lo = stt[30 + k], hi = stt[45 + k];
+    const double lo = stt[30 + k], hi = -stt[45 + k];
     const double span = hi - lo;
     nrm.x_mean[k] = (float)mean;
     nrm.x_inv_std[k] = (float)(sd > 1e-12 * (fabs(mean) + 1e-30) && sd > 0. ? 1. / sd : 1.);
@@ -1681,9 +1686,12 @@ extern "C" int pmp_spray_learn_train(pmp_spray* h, const pmp_learn_config* cfg, 
     const double var = std::max(0., stt[15 + kLearnIn + k] / n - mean * mean);
     L->target_std[k] = var > 0. ? sqrt(var) : 1.;
   }
-  cudaMemset(L->d_stats, 0, sizeof(double) * 64);
-  k_resid_stats<<<592, 256>>>(L->tuples, n, nrm, L->d_stats);
-  if (cudaMemcpy(stt, L->d_stats, sizeof(double) * 2 * kLearnOut, cudaMemcpyDeviceToHost) != cudaSuccess) {
+  for (int c = 0; c < 4 * kLearnOut; ++c) {
+    init[c] = c < 2 * kLearnOut ? 0. : 1e300;
+  }
+  cudaMemcpy(L->d_stats, init.data(), sizeof(double) * 4 * kLearnOut, cudaMemcpyHostToDevice);
+  k_resid_stats<<<sgrid, 256>>>(L->tuples, n, nrm, L->d_stats);
+  if (cudaMemcpy(stt, L->d_stats, sizeof(double) * 4 * kLearnOut, cudaMemcpyDeviceToHost) != cudaSuccess) {
     return set_err(h, PMP_ERR_CUDA, "statistics failed");
   }
   for (int k = 0; k < kLearnOut; ++k) {
@@ -1692,24 +1700,14 @@ extern "C" int pmp_spray_learn_train(pmp_spray* h, const pmp_learn_config* cfg, 
     nrm.y_mean[k] = (float)mean;
     nrm.y_std[k] = (float)(var > 0. ? sqrt(var) : 1.);
   }
-  // the residual gate's range: the training residuals', widened by the margin
-  {
-    float mm[2 * kLearnOut];
-    for (int k = 0; k < kLearnOut; ++k) {
-      mm[k] = 3.4e38f;
-      mm[kLearnOut + k] = -3.4e38f;
-    }
-    float* d_mm = reinterpret_cast<float*>(L->d_stats);
-    cudaMemcpy(d_mm, mm, sizeof(mm), cudaMemcpyHostToDevice);
-    k_resid_range<<<592, 256>>>(L->tuples, n, nrm, d_mm);
-    if (cudaMemcpy(mm, d_mm, sizeof(mm), cudaMemcpyDeviceToHost) != cudaSuccess) {
-      return set_err(h, PMP_ERR_CUDA, "statistics failed");
-    }
-    for (int k = 0; k < kLearnOut; ++k) {
-      const double span = std::max(0., (double)mm[kLearnOut + k] - (double)mm[k]);
-      nrm.r_lo[k] = (float)(mm[k] - margin * span);
-      nrm.r_hi[k] = (float)(mm[kLearnOut + k] + margin * span);
-    }
+  // the residual gate's range: the training residuals', normalised (as the
+  // kernels normalise them) and widened by the margin
+  for (int k = 0; k < kLearnOut; ++k) {
+    const float lo = ((float)stt[2 * kLearnOut + k] - nrm.y_mean[k]) / nrm.y_std[k];
+    const float hi = ((float)-stt[3 * kLearnOut + k] - nrm.y_mean[k]) / nrm.y_std[k];
+    const double span = std::max(0., (double)hi - (double)lo);
+    nrm.r_lo[k] = (float)(lo - margin * span);
+    nrm.r_hi[k] = (float)(hi + margin * span);
   }
   L->gate_margin = margin;
   L->audit_fraction = cfg->audit_fraction;
