@@ -263,63 +263,123 @@ struct DeriveArgs {
 // component offsets (relative to start) in the reference's order
 enum { kMass = 0, kDens, kNum, kVol, kSurf, kVolf, kD10, kD32, kWfh, kWfm, kTemp, kNump, kVel, kSpec = kVel + 3 };
 
-__global__ void k_derive(const DeriveArgs A)
+// The droplets are sorted by cell, so a warp's neighbouring lanes deposit into
+// the same cell: each run of lanes with one cell is summed by shuffles into its
+// first lane, which alone adds to the cell.  One FP64 atomic per droplet and
+// field (34M for 2M two-fuel droplets) held k_derive at L2's atomic rate,
+// 180 us; a run is 4-8 droplets at the usual densities.
+template <int NF>
+__global__ void __launch_bounds__(128) k_derive(const __grid_constant__ DeriveArgs A)
 {
-  const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (s >= A.n || !(A.id[s] > 0)) {
-    return;
+  constexpr int NV = 13 + (NF > 1 ? NF : 0);  // deposited fields, in the order of `comp`
+  const long long s = blockIdx.x * 128LL + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  double v[NV];
+  double* cell = nullptr;  // field A.start of the droplet's cell; null: nothing to deposit
+  int stride = 0;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    v[i] = 0.;
   }
-  const int b = find_box(A.box_begin, A.nboxes, s);
-  const View32& V = A.views[b];
-  int c[3];
+  // every field of the droplet is asked for before the first one is used
+  const bool held = s < A.n;
+  const int id = held ? __ldcs(A.id + s) : 0;
+  double pos[3], vel[3], Y[NF];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    c[d] = static_cast<int>(floor(__dmul_rn(__dsub_rn(A.pos[d][s], A.plo[d]), A.dxi[d])));
+    pos[d] = held ? __ldcs(A.pos[d] + s) : 0.;
+    vel[d] = held ? __ldcs(A.vel[d] + s) : 0.;
   }
-  if (!inside(V, c[0], c[1], c[2])) {
-    atomicCAS(A.error, 0, (int)min(s + 1, 0x7fffffffLL));
-    return;
+  const double T_part = held ? __ldcs(A.T + s) : 1.;
+  const double dia_part = held ? __ldcs(A.dia + s) : 0.;
+#pragma unroll
+  for (int spf = 0; spf < NF; ++spf) {
+    Y[spf] = held ? __ldcs(A.Y[spf] + s) : 0.;
   }
-  const double T_part = A.T[s];
-  const double dia_part = A.dia[s];
-  double rho_part = 0.;
-  for (int spf = 0; spf < A.nf; ++spf) {
-    const double* rc = A.rho_coef + 4 * spf;
-    rho_part += A.Y[spf][s] / (rc[0] + T_part * (rc[1] + T_part * (rc[2] + T_part * rc[3])));
-  }
-  rho_part = 1. / rho_part;
-  const double surf = PMP_PI * dia_part * dia_part;
-  const double vol = PMP_PI / 6. * (dia_part * dia_part * dia_part);
-  const double pmass = vol * rho_part;
-  const double num_ppp = A.numdens[s];
-  const double curvol = A.cell_vol;
-  const double face_area = A.dx[0] * A.dx[0];
-  const double film = A.film[s];
-  auto add = [&](int comp, double v) { atomicAdd(at(V, c[0], c[1], c[2], A.start + comp), v); };
-  if (film == 0.) {
-    add(kMass, num_ppp * pmass);
-    add(kDens, num_ppp * pmass / curvol);
-    add(kNum, num_ppp);
-    add(kVol, num_ppp * vol);
-    add(kSurf, num_ppp * surf);
-    add(kVolf, num_ppp * vol / curvol);
-    add(kD10, num_ppp * dia_part);
-    add(kD32, num_ppp * vol * 6.);
-    add(kTemp, num_ppp * pmass * T_part);
-    add(kNump, 1.);
+  const double num_ppp = held ? __ldcs(A.numdens + s) : 0.;
+  const double film = held ? __ldcs(A.film + s) : 0.;
+  if (id > 0) {
+    const int b = find_box(A.box_begin, A.nboxes, s);
+    const View32& V = A.views[b];
+    int c[3];
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
-      add(kVel + d, num_ppp * pmass * A.vel[d][s]);
+      c[d] = static_cast<int>(floor(__dmul_rn(__dsub_rn(pos[d], A.plo[d]), A.dxi[d])));
     }
-    if (A.species) {
-      for (int spf = 0; spf < A.nf; ++spf) {
-        add(kSpec + spf, A.Y[spf][s] * pmass);  // no parcel count, as the reference
+    if (!inside(V, c[0], c[1], c[2])) {
+      atomicCAS(A.error, 0, (int)min(s + 1, 0x7fffffffLL));
+    } else {
+      double rho_part = 0.;
+#pragma unroll
+      for (int spf = 0; spf < NF; ++spf) {
+        const double* rc = A.rho_coef + 4 * spf;
+        rho_part += Y[spf] / (rc[0] + T_part * (rc[1] + T_part * (rc[2] + T_part * rc[3])));
+      }
+      rho_part = 1. / rho_part;
+      const double surf = PMP_PI * dia_part * dia_part;
+      const double vol = PMP_PI / 6. * (dia_part * dia_part * dia_part);
+      const double pmass = vol * rho_part;
+      double* at0 = at(V, c[0], c[1], c[2], A.start);
+      if (film == 0.) {
+        cell = at0;
+        stride = V.ns;
+        v[0] = num_ppp * pmass;
+        v[1] = num_ppp * pmass / A.cell_vol;
+        v[2] = num_ppp;
+        v[3] = num_ppp * vol;
+        v[4] = num_ppp * surf;
+        v[5] = num_ppp * vol / A.cell_vol;
+        v[6] = num_ppp * dia_part;
+        v[7] = num_ppp * vol * 6.;
+        v[8] = num_ppp * pmass * T_part;
+        v[9] = 1.;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          v[10 + d] = num_ppp * pmass * vel[d];
+        }
+        if (NF > 1) {
+#pragma unroll
+          for (int spf = 0; spf < NF; ++spf) {
+            v[NF > 1 ? 13 + spf : 0] = Y[spf] * pmass;  // no parcel count, as the reference
+          }
+        }
+      } else {
+        const double face_area = A.dx[0] * A.dx[0];
+        const double rad2 = (0.5 * dia_part) * (0.5 * dia_part);
+        const double cur_vol = PMP_PI / 6. * film * (3. * rad2 + film * film);
+        atomicAdd(at0 + kWfh * V.ns, cur_vol / face_area);
+        atomicAdd(at0 + kWfm * V.ns, rho_part * cur_vol);
       }
     }
-  } else {
-    const double rad2 = (0.5 * dia_part) * (0.5 * dia_part);
-    const double cur_vol = PMP_PI / 6. * film * (3. * rad2 + film * film);
-    add(kWfh, cur_vol / face_area);
-    add(kWfm, rho_part * cur_vol);
+  }
+  // runs of neighbouring lanes with the same cell
+  const unsigned all = 0xffffffffu;
+  const unsigned long long key = reinterpret_cast<unsigned long long>(cell);
+  const unsigned long long before = __shfl_up_sync(all, key, 1);
+  const unsigned heads = __ballot_sync(all, lane == 0 || key != before);
+  const unsigned after = lane == 31 ? 0u : heads >> (lane + 1);
+  const int end = after ? lane + __ffs(after) - 1 : 31;  // last lane of this lane's run
+  const int longest = (int)__reduce_max_sync(all, cell ? (unsigned)(end - lane) : 0u);
+  for (int o = 1; o <= longest; o <<= 1) {
+    const bool take = lane + o <= end;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const double t = __shfl_down_sync(all, v[i], o);
+      v[i] = take ? v[i] + t : v[i];
+    }
+  }
+  if (cell && (heads >> lane & 1u)) {
+    constexpr int comp[13] = {kMass, kDens, kNum, kVol, kSurf, kVolf, kD10, kD32, kTemp, kNump, kVel, kVel + 1, kVel + 2};
+#pragma unroll
+    for (int i = 0; i < 13; ++i) {
+      red_add(cell + comp[i] * stride, v[i]);
+    }
+    if (NF > 1 && A.species) {
+#pragma unroll
+      for (int spf = 0; spf < NF; ++spf) {
+        red_add(cell + (kSpec + spf) * stride, v[NF > 1 ? 13 + spf : 0]);
+      }
+    }
   }
 }
 
@@ -713,7 +773,21 @@ extern "C" int pmp_spray_derive(pmp_spray* h, const pmp_box_view* vars, int nbox
   A.cell_vol = g.dx[0] * g.dx[1] * g.dx[2];
   A.error = d_err;
   if (n > 0) {
-    k_derive<<<nblk(n, 128), 128, 0, st>>>(A);
+    const unsigned grid = nblk(n, 128);
+    switch (nf) {
+      case 1:
+        k_derive<1><<<grid, 128, 0, st>>>(A);
+        break;
+      case 2:
+        k_derive<2><<<grid, 128, 0, st>>>(A);
+        break;
+      case 3:
+        k_derive<3><<<grid, 128, 0, st>>>(A);
+        break;
+      default:
+        k_derive<4><<<grid, 128, 0, st>>>(A);
+        break;
+    }
   }
   if (prefix[nboxes] > 0) {
     k_protected_divide<<<nblk(prefix[nboxes]), 256, 0, st>>>(d_views, d_prefix, nboxes, prefix[nboxes], start_indx);
