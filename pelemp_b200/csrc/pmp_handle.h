@@ -12,7 +12,11 @@
 namespace pmp {
 
 constexpr int kBlock = 128;
-constexpr int kSortPad = 8;  // cells of margin in the sort key around a box
+// cells of margin in the sort key around a box: droplets that left it by up to
+// this much (a state has 3 ghost cells as a rule) still sort by their own cell.
+// 4 keeps the key of a 32^3 box within 16 bits, two radix passes (8: three,
+// 14 us of a hand-over of 100k droplets)
+constexpr int kSortPad = 4;
 
 // Device memory that the handle keeps between calls and exchanges for more
 // when a call needs it; given back with the handle.
@@ -107,12 +111,13 @@ struct pmp_spray {
   std::vector<pmp::StagedBox> staged;
   long long staged_rows = 0;
   std::vector<bool> box_set;
+  int sort_shift = 0, sort_bits = 1;  // sort keys of the grids: a cell's bits, and the box's above them
   // packed droplets: component arrays of length total and ids, in `store`;
   // `spare` holds the staging rows, and the re-binned droplets, with which a
   // re-binning exchanges the store
   bool packed = false;
   long long total = 0;
-  pmp::KeptBuffer store, spare, perm_b, fb_b, map_b, sort_scratch, transit;
+  pmp::KeptBuffer store, spare, row_keys, perm_b, fb_b, map_b, sort_scratch, transit;
   double* soa = nullptr;  // (3 + NR) arrays of length total
   int* ids = nullptr;
   long long* perm() const { return static_cast<long long*>(perm_b.p); }  // slot -> caller's index in its box
@@ -212,6 +217,7 @@ int keep(pmp_spray* h, KeptBuffer& b, size_t bytes);
 size_t store_bytes(const pmp_spray* h, long long n);
 // soa and ids for n droplets in the store buffer
 void store_attach(pmp_spray* h, long long n);
+void store_layout(pmp_spray* h);
 void store_reset(pmp_spray* h);
 void store_free(pmp_spray* h);
 int build_cta_map(pmp_spray* h, cudaStream_t st);

@@ -1448,6 +1448,7 @@ int pmp_spray_set_grids(pmp_spray* h, int nboxes, const pmp_box* boxes)
   h->grids_version += 1;
   h->staged.assign(nboxes, pmp::StagedBox{});
   h->staged_rows = 0;
+  pmp::store_layout(h);
   h->box_set.assign(nboxes, false);
   return PMP_OK;
 }

@@ -3,9 +3,9 @@
 // and write-back (pmp_spray_get_particles).
 //
 // A box's droplets are handed over into staging rows (one 128- or 160-byte
-// row per droplet: the reals, the id and the caller's index), whatever the
-// caller's layout.  The first operation that needs the droplets packs all
-// boxes at once: one key per row (box, then cell), one radix sort over every
+// row per droplet: the reals, the id and the caller's index) and a sort key
+// each (box, then cell), whatever the caller's layout.  The first operation
+// that needs the droplets packs all boxes at once: one radix sort over every
 // box, one gather of whole rows into the store's component arrays.  A row is
 // whole 32-byte sectors, so the gather in sorted (random) order moves no byte
 // it does not use, where gathering 8 bytes from each of 14-17 component
@@ -72,6 +72,38 @@ struct Columns {
   int* id;
 };
 
+// The sort key of a droplet of one box: the box above `shift` bits of its
+// cell's place in the box's sort order (brick_key over the box and kSortPad
+// cells around it; a droplet further out counts to the edge).
+struct KeyOf {
+  double plo[3], dxi[3];
+  int lo[3], ext[3];
+  unsigned long long base;  // box << shift
+  int kept;                 // the rows are in the store's order: keep it
+};
+__device__ __forceinline__ unsigned long long sort_key(const KeyOf& k, double x, double y, double z)
+{
+  if (k.kept) {
+    return k.base;
+  }
+  const double p[3] = {x, y, z};
+  int c[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int v = static_cast<int>(floor(__dmul_rn(__dsub_rn(p[d], k.plo[d]), k.dxi[d]))) - k.lo[d] + kSortPad;
+    c[d] = v < 0 ? 0 : (v >= k.ext[d] ? k.ext[d] - 1 : v);
+  }
+  return k.base | brick_key(c[0], c[1], c[2], k.ext[0], k.ext[1]);
+}
+
+// Where a staging kernel leaves each row's key and index (narrow keys; null:
+// formed from the rows when they are packed)
+struct KeyOut {
+  unsigned* keys;
+  int* idx;
+  long long row0;  // index of the kernel's first row
+};
+
 __device__ __forceinline__ double pack_ints(int lo, int hi) { return __hiloint2double(hi, lo); }
 
 // tile[r][w] of the CTA's rows -> staging rows, 16 bytes a lane
@@ -92,7 +124,8 @@ __device__ __forceinline__ void tile_to_rows(const double (*tile)[Row<NF>::kPitc
 // one stream of words (the caller's buffer is 8-byte aligned, a record with
 // one fuel is 120 bytes), and turned in shared memory.
 template <int NF>
-__global__ void __launch_bounds__(kTile) k_aos_to_rows(const double* aos, long long n, double* rows)
+__global__ void __launch_bounds__(kTile) k_aos_to_rows(const double* aos, long long n, double* rows,
+                                                       const __grid_constant__ KeyOf key, const KeyOut out)
 {
   using R = Row<NF>;
   __shared__ double tile[kTile][R::kPitch];
@@ -104,8 +137,13 @@ __global__ void __launch_bounds__(kTile) k_aos_to_rows(const double* aos, long l
   }
   __syncthreads();
   if ((int)threadIdx.x < m) {
-    const int id = __double2loint(tile[threadIdx.x][R::kReals]);
-    tile[threadIdx.x][R::kReals] = pack_ints(id, (int)(s0 + threadIdx.x));
+    double* t = tile[threadIdx.x];
+    const int id = __double2loint(t[R::kReals]);
+    t[R::kReals] = pack_ints(id, (int)(s0 + threadIdx.x));
+    if (out.keys) {
+      out.keys[s0 + threadIdx.x] = (unsigned)sort_key(key, t[0], t[1], t[2]);
+      out.idx[s0 + threadIdx.x] = (int)(out.row0 + s0 + threadIdx.x);
+    }
   }
   __syncthreads();
   tile_to_rows<NF>(tile, rows + s0 * R::kStride, m);
@@ -114,7 +152,9 @@ __global__ void __launch_bounds__(kTile) k_aos_to_rows(const double* aos, long l
 // component arrays -> rows; a null component is zero.  caller: the droplets'
 // caller indices, or null for 0, 1, ...
 template <int NF>
-__global__ void __launch_bounds__(kTile) k_columns_to_rows(const Columns C, const long long* caller, long long n, double* rows)
+__global__ void __launch_bounds__(kTile) k_columns_to_rows(const __grid_constant__ Columns C, const long long* caller,
+                                                           long long n, double* rows,
+                                                           const __grid_constant__ KeyOf key, const KeyOut out)
 {
   using R = Row<NF>;
   __shared__ double tile[kTile][R::kPitch];
@@ -126,7 +166,12 @@ __global__ void __launch_bounds__(kTile) k_columns_to_rows(const Columns C, cons
     for (int c = 0; c < R::kReals; ++c) {
       tile[threadIdx.x][c] = C.c[c] ? __ldcs(C.c[c] + s) : 0.;
     }
-    tile[threadIdx.x][R::kReals] = pack_ints(C.id[s], caller ? (int)caller[s] : (int)s);
+    double* t = tile[threadIdx.x];
+    t[R::kReals] = pack_ints(C.id[s], caller ? (int)caller[s] : (int)s);
+    if (out.keys) {
+      out.keys[s] = (unsigned)sort_key(key, t[0], t[1], t[2]);
+      out.idx[s] = (int)(out.row0 + s);
+    }
   }
   __syncthreads();
   tile_to_rows<NF>(tile, rows + s0 * R::kStride, m);
@@ -136,9 +181,7 @@ __global__ void __launch_bounds__(kTile) k_columns_to_rows(const Columns C, cons
 struct Region {
   long long row;    // first staging row
   long long begin;  // first slot of the box
-  int lo[3], ext[3];
-  int kept;         // rows already in the store's order (a repack): keep it
-  int pad;
+  KeyOf key;
 };
 
 __device__ __forceinline__ int region_of(const Region* reg, int nb, long long s)
@@ -155,36 +198,32 @@ __device__ __forceinline__ int region_of(const Region* reg, int nb, long long s)
   return lo;
 }
 
-// The sort key of each row: its box above `shift` bits of its cell's place in
-// the box's sort order (brick_key over the box and kSortPad cells around it).
-template <typename K, typename V>
+// Wide keys (the boxes' bits do not fit 32, or 2^31 rows and more), from the
+// rows, and the rows' indices.
 __global__ void __launch_bounds__(256) k_row_keys(const double* rows, int stride, const Region* reg, int nb, long long n,
-                                                  double plo0, double plo1, double plo2, double dxi0, double dxi1,
-                                                  double dxi2, int shift, K* keys, V* idx)
+                                                  unsigned long long* keys, long long* idx)
 {
   const long long s = blockIdx.x * 256LL + threadIdx.x;
   if (s >= n) {
     return;
   }
-  const int b = region_of(reg, nb, s);
-  const Region& g = reg[b];
+  const Region& g = reg[region_of(reg, nb, s)];
   const long long r = g.row + (s - g.begin);
-  unsigned long long cell = 0;
-  if (!g.kept) {
-    const double* q = rows + r * stride;
-    const double2 xy = *reinterpret_cast<const double2*>(q);
-    const double p[3] = {xy.x, xy.y, q[2]};
-    const double pl[3] = {plo0, plo1, plo2}, di[3] = {dxi0, dxi1, dxi2};
-    int c[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const int v = static_cast<int>(floor(__dmul_rn(__dsub_rn(p[d], pl[d]), di[d]))) - g.lo[d] + kSortPad;
-      c[d] = v < 0 ? 0 : (v >= g.ext[d] ? g.ext[d] - 1 : v);
+  const double* q = rows + r * stride;
+  keys[s] = sort_key(g.key, q[0], q[1], q[2]);
+  idx[s] = r;
+}
+
+// rows [0, n): key (keys null: unchanged) and their own index
+__global__ void __launch_bounds__(256) k_fill_keys(unsigned* keys, int* idx, long long row0, long long n, unsigned key)
+{
+  const long long i = blockIdx.x * 256LL + threadIdx.x;
+  if (i < n) {
+    if (keys) {
+      keys[row0 + i] = key;
     }
-    cell = brick_key(c[0], c[1], c[2], g.ext[0], g.ext[1]);
+    idx[row0 + i] = (int)(row0 + i);
   }
-  keys[s] = ((K)b << shift) | (K)cell;
-  idx[s] = (V)r;
 }
 
 // rows in sorted order -> the store.  Eight or nine lanes read one row.
@@ -351,12 +390,48 @@ double* staged_row(const pmp_spray* h, long long r)
   return reinterpret_cast<double*>(static_cast<char*>(h->spare.p) + (size_t)r * row_bytes(h));
 }
 
-// Room for n more staging rows in the spare buffer; the live boxes' rows move
-// to its front when it is exchanged for a larger one.
+// sort-key extent of a box: its cells and kSortPad around them
+void sort_extent(const pmp_box& bx, int* ext)
+{
+  for (int d = 0; d < 3; ++d) {
+    ext[d] = bx.hi[d] - bx.lo[d] + 1 + 2 * kSortPad;
+  }
+}
+
+KeyOf key_of(const pmp_spray* h, int box, bool kept)
+{
+  KeyOf k;
+  memset(&k, 0, sizeof(k));
+  const pmp_box& bx = h->boxes[box];
+  sort_extent(bx, k.ext);
+  for (int d = 0; d < 3; ++d) {
+    k.plo[d] = h->geom.plo[d];
+    k.dxi[d] = 1. / h->geom.dx[d];
+    k.lo[d] = bx.lo[d];
+  }
+  k.base = (unsigned long long)box << h->sort_shift;
+  k.kept = kept ? 1 : 0;
+  return k;
+}
+
+// 32-bit keys: every box's fit below 2^31, the key of rows given up lies above
+bool narrow_keys(const pmp_spray* h) { return h->sort_bits <= 31; }
+
+// the narrow keys and indices of the staging rows, from row `row` on
+KeyOut key_out(const pmp_spray* h, long long row)
+{
+  const long long cap = (long long)(h->row_keys.bytes / (2 * sizeof(unsigned)));
+  unsigned* keys = static_cast<unsigned*>(h->row_keys.p);
+  return {keys + row, reinterpret_cast<int*>(keys + cap) + row, row};
+}
+
+// Room for n more staging rows in the spare buffer (and their keys); the live
+// boxes' rows move to its front when it is exchanged for a larger one.
 int stage_room(pmp_spray* h, long long n)
 {
   const size_t rb = row_bytes(h);
-  if ((size_t)(h->staged_rows + n) * rb <= h->spare.bytes) {
+  const size_t kb = 2 * sizeof(unsigned);
+  if ((size_t)(h->staged_rows + n) * rb <= h->spare.bytes && (size_t)(h->staged_rows + n) * kb <= h->row_keys.bytes) {
     return PMP_OK;
   }
   long long live = 0;
@@ -365,30 +440,52 @@ int stage_room(pmp_spray* h, long long n)
   }
   // the first boxes of a hand-over say little about the rest of it: doubling,
   // so that many boxes exchange the buffer a few times only
-  const size_t need = (size_t)(live + n) * rb;
-  KeptBuffer nw;
-  nw.bytes = live > 0 ? 2 * need : need;
-  if (cudaMalloc(&nw.p, nw.bytes) != cudaSuccess) {
+  size_t rows = (size_t)(live > 0 ? 2 * (live + n) : n);
+  KeptBuffer nw, nk;
+  if (cudaMalloc(&nw.p, rows * rb) != cudaSuccess) {
     cudaGetLastError();
-    nw.bytes = need;
-    PMP_TRY(h, cudaMalloc(&nw.p, nw.bytes));
+    rows = (size_t)(live + n);
+    PMP_TRY(h, cudaMalloc(&nw.p, rows * rb));
   }
+  nw.bytes = rows * rb;
+  nk.bytes = rows * kb;
+  cudaError_t e = cudaMalloc(&nk.p, nk.bytes);
+  const KeptBuffer old_rows = h->spare, old_keys = h->row_keys;
+  const KeyOut from = key_out(h, 0);
+  h->row_keys = nk;
+  const KeyOut to = key_out(h, 0);
   long long at = 0;
+  for (const StagedBox& s : h->staged) {
+    if (s.n > 0 && e == cudaSuccess) {
+      e = cudaMemcpy(static_cast<char*>(nw.p) + (size_t)at * rb, staged_row(h, s.row), (size_t)s.n * rb,
+                     cudaMemcpyDeviceToDevice);
+      if (e == cudaSuccess) {
+        e = cudaMemcpy(to.keys + at, from.keys + s.row, sizeof(unsigned) * s.n, cudaMemcpyDeviceToDevice);
+      }
+      at += s.n;
+    }
+  }
+  if (e == cudaSuccess && at > 0) {
+    k_fill_keys<<<nblk(at, 256), 256>>>(nullptr, to.idx, 0, at, 0);
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) {
+    h->row_keys = old_keys;
+    cudaFree(nw.p);
+    cudaFree(nk.p);
+    return check(h, e, "staging rows");
+  }
+  at = 0;
   for (StagedBox& s : h->staged) {
     if (s.n > 0) {
-      const cudaError_t e = cudaMemcpy(static_cast<char*>(nw.p) + (size_t)at * rb, staged_row(h, s.row),
-                                       (size_t)s.n * rb, cudaMemcpyDeviceToDevice);
-      if (e != cudaSuccess) {
-        cudaFree(nw.p);
-        return check(h, e, "cudaMemcpy (staged droplets)");
-      }
       s.row = at;
       at += s.n;
     }
   }
   h->staged_rows = at;
-  cudaFree(h->spare.p);  // waits for the copies
   h->spare = nw;
+  cudaFree(old_rows.p);  // waits for the copies
+  cudaFree(old_keys.p);
   return PMP_OK;
 }
 
@@ -418,13 +515,16 @@ int unpack(pmp_spray* h, int skip)
     s.row = h->staged_rows;
     s.kept = true;
     h->staged_rows += m;
+    const KeyOf key = key_of(h, b, true);
+    const KeyOut out = narrow_keys(h) ? key_out(h, s.row) : KeyOut{};
     Columns C;
     memset(&C, 0, sizeof(C));
     for (int c = 0; c < nc; ++c) {
       C.c[c] = h->soa + (long long)c * T + o;
     }
     C.id = h->ids + o;
-    PMP_BY_FUELS(h, (k_columns_to_rows<F><<<nblk(m, kTile), kTile>>>(C, h->perm() + o, m, staged_row(h, s.row))));
+    PMP_BY_FUELS(h, (k_columns_to_rows<F><<<nblk(m, kTile), kTile>>>(C, h->perm() + o, m, staged_row(h, s.row), key,
+                                                                   out)));
   }
   PMP_TRY(h, cudaGetLastError());
   store_reset(h);
@@ -513,41 +613,28 @@ Columns columns_in(void* base, int nreal, long long n)
   return C;
 }
 
-// the sort of every box's rows: the sorted row indices at *order
+// the sort of m keyed rows: the sorted row indices at *order
 template <typename K, typename V>
-int sort_rows(pmp_spray* h, const Region* d_reg, int nb, long long n, int shift, int end_bit, cudaStream_t st,
+int sort_rows(pmp_spray* h, const K* keys, const V* idx, long long m, int end_bit, size_t used, cudaStream_t st,
               const V** order)
 {
   using N = V;  // the count type decides CUB's offsets
-  size_t tbytes = 0;
-  PMP_TRY(h, (cub::DeviceRadixSort::SortPairs(nullptr, tbytes, (const K*)nullptr, (K*)nullptr, (const V*)nullptr,
-                                              (V*)nullptr, (N)n, 0, end_bit, st)));
-  const size_t kb = align256(sizeof(K) * n), vb = align256(sizeof(V) * n);
-  const int rc = keep(h, h->sort_scratch, 2 * kb + 2 * vb + tbytes);
-  if (rc != PMP_OK) {
-    return rc;
-  }
-  char* base = static_cast<char*>(h->sort_scratch.p);
-  K* keys = reinterpret_cast<K*>(base);
-  K* keys2 = reinterpret_cast<K*>(base + kb);
-  V* idx = reinterpret_cast<V*>(base + 2 * kb);
-  V* idx2 = reinterpret_cast<V*>(base + 2 * kb + vb);
-  const pmp_geometry& g = h->geom;
-  k_row_keys<K, V><<<nblk(n, 256), 256, 0, st>>>(staged_row(h, 0), row_stride(h->nfuel), d_reg, nb, n, g.plo[0],
-                                                 g.plo[1], g.plo[2], 1. / g.dx[0], 1. / g.dx[1], 1. / g.dx[2], shift,
-                                                 keys, idx);
-  PMP_TRY(h, cudaGetLastError());
-  PMP_TRY(h, cub::DeviceRadixSort::SortPairs(base + 2 * kb + 2 * vb, tbytes, keys, keys2, idx, idx2, (N)n, 0, end_bit, st));
-  *order = idx2;
+  const size_t kb = align256(sizeof(K) * m), vb = align256(sizeof(V) * m);
+  char* base = static_cast<char*>(h->sort_scratch.p) + used;
+  size_t tbytes = h->sort_scratch.bytes - used - kb - vb;
+  PMP_TRY(h, (cub::DeviceRadixSort::SortPairs(base + kb + vb, tbytes, keys, reinterpret_cast<K*>(base), idx,
+                                              reinterpret_cast<V*>(base + kb), (N)m, 0, end_bit, st)));
+  *order = reinterpret_cast<V*>(base + kb);
   return PMP_OK;
 }
 
-// sort-key extent of a box: its cells and kSortPad around them
-void sort_extent(const pmp_box& bx, int* ext)
+template <typename K, typename V>
+size_t sort_bytes(long long m, int end_bit)
 {
-  for (int d = 0; d < 3; ++d) {
-    ext[d] = bx.hi[d] - bx.lo[d] + 1 + 2 * kSortPad;
-  }
+  size_t tbytes = 0;
+  cub::DeviceRadixSort::SortPairs(nullptr, tbytes, (const K*)nullptr, (K*)nullptr, (const V*)nullptr, (V*)nullptr, (V)m, 0,
+                                  end_bit, nullptr);
+  return align256(sizeof(K) * m) + align256(sizeof(V) * m) + align256(std::max(tbytes, (size_t)1));
 }
 
 }  // namespace
@@ -577,6 +664,26 @@ void store_attach(pmp_spray* h, long long n)
   h->ids = reinterpret_cast<int*>(h->soa + (long long)h->ncomp() * n);
 }
 
+// Sort-key layout of new grids: bits of a cell's place in its box, and of the
+// box above them.
+void store_layout(pmp_spray* h)
+{
+  int sh = 0;
+  for (const pmp_box& bx : h->boxes) {
+    int ext[3];
+    sort_extent(bx, ext);
+    const unsigned long long cells = brick_key_count(ext[0], ext[1], ext[2]);
+    while (sh < 40 && (1ULL << sh) < cells) {
+      ++sh;
+    }
+  }
+  h->sort_shift = sh;
+  h->sort_bits = std::max(sh, 1);
+  while (h->sort_bits < 63 && (1ULL << (h->sort_bits - sh)) < h->boxes.size()) {
+    ++h->sort_bits;
+  }
+}
+
 void store_reset(pmp_spray* h)
 {
   h->soa = nullptr;
@@ -589,7 +696,8 @@ void store_reset(pmp_spray* h)
 void store_free(pmp_spray* h)
 {
   store_reset(h);
-  for (KeptBuffer* b : {&h->store, &h->spare, &h->perm_b, &h->fb_b, &h->map_b, &h->sort_scratch, &h->transit}) {
+  for (KeptBuffer* b : {&h->store, &h->spare, &h->row_keys, &h->perm_b, &h->fb_b, &h->map_b, &h->sort_scratch,
+                        &h->transit}) {
     cudaFree(b->p);
     *b = KeptBuffer{};
   }
@@ -657,24 +765,8 @@ int ensure_packed(pmp_spray* h, cudaStream_t st)
     cudaFree(p);
     st = nullptr;
   }
-  std::vector<Region> reg(nb);
   h->box_begin.assign(nb + 1, 0);
-  int shift = 0;
   for (int b = 0; b < nb; ++b) {
-    const pmp_box& bx = h->boxes[b];
-    Region& r = reg[b];
-    memset(&r, 0, sizeof(r));
-    r.row = h->staged[b].row;
-    r.begin = h->box_begin[b];
-    r.kept = h->staged[b].kept ? 1 : 0;
-    sort_extent(bx, r.ext);
-    for (int d = 0; d < 3; ++d) {
-      r.lo[d] = bx.lo[d];
-    }
-    const unsigned long long cells = brick_key_count(r.ext[0], r.ext[1], r.ext[2]);
-    while (shift < 40 && (1ULL << shift) < cells) {
-      ++shift;
-    }
     h->box_begin[b + 1] = h->box_begin[b] + h->staged[b].n;
   }
   const long long n = h->box_begin[nb];
@@ -682,32 +774,43 @@ int ensure_packed(pmp_spray* h, cudaStream_t st)
   if (rc == PMP_OK) {
     rc = keep(h, h->perm_b, sizeof(long long) * (size_t)std::max(n, 1LL));
   }
-  if (rc == PMP_OK) {
-    rc = keep(h, h->map_b, sizeof(Region) * (size_t)std::max(nb, 1));
-  }
   if (rc != PMP_OK) {
     return rc;
   }
   store_attach(h, n);
   if (n > 0) {
-    // the regions are read before build_cta_map reuses the buffer, in stream order
-    const Region* d_reg = static_cast<const Region*>(h->map_b.p);
-    PMP_TRY(h, cudaMemcpyAsync(h->map_b.p, reg.data(), sizeof(Region) * nb, cudaMemcpyHostToDevice, st));
-    int end_bit = shift;
-    while (end_bit < 63 && (1LL << (end_bit - shift)) < nb) {
-      ++end_bit;
-    }
-    end_bit = std::max(end_bit, 1);
-    if (end_bit <= 32 && h->staged_rows < (1LL << 31)) {
+    const int end_bit = h->sort_bits;
+    if (narrow_keys(h) && h->staged_rows < (1LL << 31)) {
+      // rows given up carry the key of no box, above every other
+      const long long m = h->staged_rows;
+      const int bits = m == n ? end_bit : 32;
+      rc = keep(h, h->sort_scratch, sort_bytes<unsigned, int>(m, bits));
+      const KeyOut k = key_out(h, 0);
       const int* order = nullptr;
-      rc = sort_rows<unsigned, int>(h, d_reg, nb, n, shift, end_bit, st, &order);
+      if (rc == PMP_OK) {
+        rc = sort_rows<unsigned, int>(h, k.keys, k.idx, m, bits, 0, st, &order);
+      }
       if (rc == PMP_OK) {
         PMP_BY_FUELS(h, (k_rows_to_store<F, int><<<nblk(n, kTile), kTile, 0, st>>>(staged_row(h, 0), order, n, h->soa,
                                                                                   h->ids, h->perm())));
       }
     } else {
+      std::vector<Region> reg(nb);
+      for (int b = 0; b < nb; ++b) {
+        reg[b] = Region{h->staged[b].row, h->box_begin[b], key_of(h, b, h->staged[b].kept)};
+      }
+      const size_t kb = align256(sizeof(unsigned long long) * n), used = 2 * kb + align256(sizeof(Region) * nb);
+      rc = keep(h, h->sort_scratch, used + sort_bytes<unsigned long long, long long>(n, end_bit));
       const long long* order = nullptr;
-      rc = sort_rows<unsigned long long, long long>(h, d_reg, nb, n, shift, end_bit, st, &order);
+      if (rc == PMP_OK) {
+        char* base = static_cast<char*>(h->sort_scratch.p);
+        unsigned long long* keys = reinterpret_cast<unsigned long long*>(base);
+        long long* idx = reinterpret_cast<long long*>(base + kb);
+        Region* d_reg = reinterpret_cast<Region*>(base + 2 * kb);
+        PMP_TRY(h, cudaMemcpyAsync(d_reg, reg.data(), sizeof(Region) * nb, cudaMemcpyHostToDevice, st));
+        k_row_keys<<<nblk(n, 256), 256, 0, st>>>(staged_row(h, 0), row_stride(h->nfuel), d_reg, nb, n, keys, idx);
+        rc = sort_rows<unsigned long long, long long>(h, keys, idx, n, end_bit, used, st, &order);
+      }
       if (rc == PMP_OK) {
         PMP_BY_FUELS(h, (k_rows_to_store<F, long long><<<nblk(n, kTile), kTile, 0, st>>>(staged_row(h, 0), order, n,
                                                                                         h->soa, h->ids, h->perm())));
@@ -764,6 +867,11 @@ int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
   StagedBox& s = h->staged[box];
   if (s.n > 0 && s.row + s.n == h->staged_rows) {
     h->staged_rows = s.row;  // its rows are the last ones
+  } else if (s.n > 0 && narrow_keys(h)) {
+    // given up: the key above every box's
+    const KeyOut k = key_out(h, 0);
+    k_fill_keys<<<nblk(s.n, 256), 256>>>(k.keys, k.idx, s.row, s.n, 0xffffffffu);
+    PMP_TRY(h, cudaGetLastError());
   }
   s = StagedBox{};
   h->box_set[box] = false;  // until its droplets are in
@@ -789,6 +897,8 @@ int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
   const int nc = h->ncomp();
   const int nr = h->nr();
   double* rows = staged_row(h, h->staged_rows);
+  const KeyOf key = key_of(h, box, false);
+  const KeyOut out = narrow_keys(h) ? key_out(h, h->staged_rows) : KeyOut{};
   const cudaMemcpyKind kind = p->where == PMP_WHERE_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
   DeviceRanges ranges(h->device);
   Transit transit(h);
@@ -828,7 +938,7 @@ int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
       PMP_TRY(h, cudaMemcpy(D.id, C.id, sizeof(int) * n, kind));
       C = D;
     }
-    PMP_BY_FUELS(h, (k_columns_to_rows<F><<<nblk(n, kTile), kTile>>>(C, nullptr, n, rows)));
+    PMP_BY_FUELS(h, (k_columns_to_rows<F><<<nblk(n, kTile), kTile>>>(C, nullptr, n, rows, key, out)));
   } else {
     const size_t bytes = sizeof(double) * (nc + 1) * (size_t)n;
     const double* src = static_cast<const double*>(p->aos);
@@ -840,7 +950,7 @@ int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
       PMP_TRY(h, cudaMemcpy(h->transit.p, p->aos, bytes, kind));
       src = static_cast<const double*>(h->transit.p);
     }
-    PMP_BY_FUELS(h, (k_aos_to_rows<F><<<nblk(n, kTile), kTile>>>(src, n, rows)));
+    PMP_BY_FUELS(h, (k_aos_to_rows<F><<<nblk(n, kTile), kTile>>>(src, n, rows, key, out)));
   }
   PMP_TRY(h, cudaGetLastError());
   // the caller's arrays are read when the call returns

@@ -161,3 +161,24 @@ def test_refused():
     sp.set_particles(0, *droplets(np.random.default_rng(0), 4, 1, *prob.boxes[0], prob.dx[0]))
     p.layout, p.n = capi.PMP_LAYOUT_SOA, 3
     assert L.pmp_spray_get_particles(h, 0, C.byref(p)) == capi.PMP_ERR_INVALID  # another count
+
+
+def test_wide_keys():
+    """Boxes whose cells and count need more than 31 key bits together (64-bit keys)."""
+    prob = level(1)
+    n = 512
+    prob.boxes = [((n * i, 0, 0), (n * i + n - 1, n - 1, n - 1)) for i in range(20)]
+    prob.domain_hi = (20 * n - 1, n - 1, n - 1)
+    prob.phi = prob.dx * np.array([20 * n, n, n])
+    sp = from_problem(prob, set_droplets=False)
+    rng = np.random.default_rng(8)
+    drs = [droplets(rng, 300 + b, 1, lo, hi, prob.dx[0]) for b, (lo, hi) in enumerate(prob.boxes)]
+    for b, d in enumerate(drs):
+        sp.set_particles(b, *d)
+    sp.est_timestep(0.5)
+    drs[3] = droplets(rng, 50, 1, *prob.boxes[3], prob.dx[0])
+    sp.set_particles(3, *drs[3])  # the others keep their order
+    v = np.concatenate([d[1][:3] for d in drs], axis=1)
+    assert sp.est_timestep(0.5) == np.min(0.5 / np.max(np.abs(v) * (1.0 / prob.dx)[:, None], axis=0))
+    for b, d in enumerate(drs):
+        check_box(sp, b, d, 1, capi.PMP_LAYOUT_SOA, capi.PMP_WHERE_DEVICE)
