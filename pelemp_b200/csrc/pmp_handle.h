@@ -132,7 +132,9 @@ struct pmp_spray {
   unsigned long long table_clock = 0;
   int cur_table = -1;  // slot of the last prepared call's table
   pmp::DevStatus* d_status = nullptr;
-  pmp::DevStatus* h_status = nullptr;
+  pmp::DevStatus* h_status = nullptr;  // page-locked, kSmall bytes more behind it
+  static constexpr size_t kSmall = 64;
+  void* h_small() const { return h_status + 1; }  // for the few bytes an operation reads back
   // the first device error code, written by the kernels into page-locked
   // host memory mapped into the device (err_dev: its device address)
   int* err_host = nullptr;

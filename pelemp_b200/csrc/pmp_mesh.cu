@@ -205,33 +205,68 @@ __device__ __forceinline__ int owner(const int* map, const Domain& D, int* c)
 // --------------------------------------------------------------------------
 // estTimestep
 
-__global__ void k_est_dt(const double* vx, const double* vy, const double* vz, const int* id, long long n,
-                         double dxi0, double dxi1, double dxi2, double cfl, double* partial)
+// A double as an unsigned integer of the same order (no NaN), and back
+__host__ __device__ inline unsigned long long ordered(double v)
 {
+  unsigned long long u;
+#ifdef __CUDA_ARCH__
+  u = (unsigned long long)__double_as_longlong(v);
+#else
+  memcpy(&u, &v, sizeof(u));
+#endif
+  return u >> 63 ? ~u : u | (1ULL << 63);
+}
+inline double from_ordered(unsigned long long k)
+{
+  const unsigned long long u = k >> 63 ? k & ~(1ULL << 63) : ~k;
+  double v;
+  memcpy(&v, &u, sizeof(v));
+  return v;
+}
+
+// The minimum over the droplets into *out (an ordered double): four droplets a
+// thread, all their fields asked for first (one at a time, the loads of a
+// thread waited for one another: 43 us for 4M droplets, 2.6 TB/s).
+constexpr int kEstPer = 4;
+__global__ void __launch_bounds__(256) k_est_dt(const double* vx, const double* vy, const double* vz, const int* id,
+                                                long long n, double dxi0, double dxi1, double dxi2, double cfl,
+                                                unsigned long long* out)
+{
+  const long long base = blockIdx.x * (256LL * kEstPer) + threadIdx.x;
+  int live[kEstPer];
+  double u[kEstPer][3];
+#pragma unroll
+  for (int q = 0; q < kEstPer; ++q) {
+    const long long i = base + 256 * q;
+    live[q] = i < n ? __ldg(id + i) : 1;
+    u[q][0] = i < n ? __ldg(vx + i) : 0.;
+    u[q][1] = i < n ? __ldg(vy + i) : 0.;
+    u[q][2] = i < n ? __ldg(vz + i) : 0.;
+  }
   double m = DBL_MAX;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+#pragma unroll
+  for (int q = 0; q < kEstPer; ++q) {
     double v = -1.;
-    if (id[i] > 0) {
-      const double mv = fmax(fmax(fabs(vx[i]) * dxi0, fabs(vy[i]) * dxi1), fabs(vz[i]) * dxi2);
+    if (live[q] > 0) {
+      const double mv = fmax(fmax(fabs(u[q][0]) * dxi0, fabs(u[q][1]) * dxi1), fabs(u[q][2]) * dxi2);
       v = mv > 0. ? cfl / mv : 1.E50;
     }
-    m = fmin(m, v);
+    m = base + 256 * q < n ? fmin(m, v) : m;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     m = fmin(m, __shfl_down_sync(0xffffffffu, m, o));
   }
-  __shared__ double red[32];
+  __shared__ double red[8];
   if ((threadIdx.x & 31) == 0) {
     red[threadIdx.x >> 5] = m;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    double r = red[0];
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-      r = fmin(r, red[w]);
+    for (int w = 1; w < 8; ++w) {
+      m = fmin(m, red[w]);
     }
-    partial[blockIdx.x] = r;
+    atomicMin(out, ordered(m));
   }
 }
 
@@ -453,53 +488,52 @@ struct AddMap {
   int dep[PMP_MAX_FUEL];
 };
 
-// MultiFab::Add or addSpraySrc over each box grown by nghost
-__global__ void k_add_source(const View32* tmp, const View32* act, const pmp_box* boxes, const long long* prefix, int nb,
-                             long long total, int ng, const AddMap M)
+// MultiFab::Add or addSpraySrc over each box grown by nghost, and the reset of
+// the temporary over its whole view, in one pass: a thread per cell of the view
+// (consecutive threads, consecutive cells of a component).  As two kernels, the
+// reset one thread per value with a 64-bit division each, 60 us for 8 boxes of
+// 64 x 32 x 32 and 7 components.
+__global__ void __launch_bounds__(256) k_add_reset(const View32* tmp, const View32* act, const pmp_box* boxes,
+                                                   const long long* prefix, int nb, long long total, int ng,
+                                                   const __grid_constant__ AddMap M)
 {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long t = blockIdx.x * 256LL + threadIdx.x;
   if (t >= total) {
     return;
   }
   const int b = find_box(prefix, nb, t);
-  const pmp_box& bx = boxes[b];
-  const long long l = t - prefix[b];
-  const int nx = bx.hi[0] - bx.lo[0] + 1 + 2 * ng, ny = bx.hi[1] - bx.lo[1] + 1 + 2 * ng;
-  const int i = bx.lo[0] - ng + (int)(l % nx);
-  const int j = bx.lo[1] - ng + (int)((l / nx) % ny);
-  const int k = bx.lo[2] - ng + (int)(l / ((long long)nx * ny));
   const View32& S = tmp[b];
-  const View32& A = act[b];
-  if (M.same) {
-    for (int n = 0; n < A.ncomp; ++n) {
-      *at(A, i, j, k, n) += *at(S, i, j, k, n);
+  const pmp_box& bx = boxes[b];
+  const unsigned l = (unsigned)(t - prefix[b]);  // a view spans fewer than 2^31 elements
+  const unsigned nx = (unsigned)(S.hi[0] - S.lo[0] + 1), ny = (unsigned)(S.hi[1] - S.lo[1] + 1);
+  const unsigned row = l / nx;
+  const int i = S.lo[0] + (int)(l - row * nx);
+  const int k = S.lo[2] + (int)(row / ny);
+  const int j = S.lo[1] + (int)(row - row / ny * ny);
+  double* s = at(S, i, j, k, 0);
+  const bool in = i >= bx.lo[0] - ng && i <= bx.hi[0] + ng && j >= bx.lo[1] - ng && j <= bx.hi[1] + ng &&
+                  k >= bx.lo[2] - ng && k <= bx.hi[2] + ng;
+  if (in) {
+    const View32& A = act[b];
+    double* a = at(A, i, j, k, 0);
+    if (M.same) {
+      for (int n = 0; n < A.ncomp; ++n) {
+        a[n * A.ns] += s[n * S.ns];
+      }
+    } else {
+      for (int d = 0; d < 3; ++d) {
+        a[(M.mom + d) * A.ns] += s[(M.mom_src + d) * S.ns];
+      }
+      a[M.rho * A.ns] += s[M.rho_src * S.ns];
+      a[M.eng * A.ns] += s[M.eng_src * S.ns];
+      for (int sp = 0; sp < M.nf; ++sp) {
+        a[(M.spec + M.dep[sp]) * A.ns] += s[(M.spec_src + sp) * S.ns];
+      }
     }
-    return;
   }
-  for (int d = 0; d < 3; ++d) {
-    *at(A, i, j, k, M.mom + d) += *at(S, i, j, k, M.mom_src + d);
+  for (int n = 0; n < S.ncomp; ++n) {
+    s[n * S.ns] = 0.;
   }
-  *at(A, i, j, k, M.rho) += *at(S, i, j, k, M.rho_src);
-  *at(A, i, j, k, M.eng) += *at(S, i, j, k, M.eng_src);
-  for (int sp = 0; sp < M.nf; ++sp) {
-    *at(A, i, j, k, M.spec + M.dep[sp]) += *at(S, i, j, k, M.spec_src + sp);
-  }
-}
-
-__global__ void k_zero_views(const View32* v, const long long* prefix, int nb, long long total)
-{
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= total) {
-    return;
-  }
-  const int b = find_box(prefix, nb, t);
-  const View32& V = v[b];
-  const long long l = t - prefix[b];
-  const int nx = V.hi[0] - V.lo[0] + 1, ny = V.hi[1] - V.lo[1] + 1, nz = V.hi[2] - V.lo[2] + 1;
-  const long long cells = (long long)nx * ny * nz;
-  const int n = (int)(l / cells);
-  const long long r = l % cells;
-  *at(V, V.lo[0] + (int)(r % nx), V.lo[1] + (int)((r / nx) % ny), V.lo[2] + (int)(r / ((long long)nx * ny)), n) = 0.;
 }
 
 // --------------------------------------------------------------------------
@@ -673,22 +707,20 @@ extern "C" int pmp_spray_est_timestep(pmp_spray* h, double cfl, double max_jet_v
   double r = DBL_MAX;
   const long long n = h->total;
   if (n > 0) {
-    const int nblocks = (int)std::min<long long>(nblk(n, 256), 148 * 8);
     void* sp = nullptr;
-    rc = scratch(h, sizeof(double) * nblocks, &sp);
+    rc = scratch(h, sizeof(unsigned long long), &sp);
     if (rc != PMP_OK) {
       return rc;
     }
-    double* partial = static_cast<double*>(sp);
+    unsigned long long* least = static_cast<unsigned long long*>(sp);
+    unsigned long long* hl = reinterpret_cast<unsigned long long*>(h->h_small());
+    PMP_TRY(h, cudaMemsetAsync(least, 0xff, sizeof(*least), st));
     const double* vel = h->soa + 3 * n;  // rdata component 0 follows the positions
-    k_est_dt<<<nblocks, 256, 0, st>>>(vel, vel + n, vel + 2 * n, h->ids, n, 1. / g.dx[0], 1. / g.dx[1], 1. / g.dx[2],
-                                      cfl, partial);
-    std::vector<double> hp(nblocks);
-    PMP_TRY(h, cudaMemcpyAsync(hp.data(), partial, sizeof(double) * nblocks, cudaMemcpyDeviceToHost, st));
+    k_est_dt<<<nblk(n, 256 * kEstPer), 256, 0, st>>>(vel, vel + n, vel + 2 * n, h->ids, n, 1. / g.dx[0], 1. / g.dx[1],
+                                                     1. / g.dx[2], cfl, least);
+    PMP_TRY(h, cudaMemcpyAsync(hl, least, sizeof(*hl), cudaMemcpyDeviceToHost, st));
     PMP_TRY(h, cudaStreamSynchronize(st));
-    for (double v : hp) {
-      r = std::min(r, v);
-    }
+    r = std::min(r, from_ordered(*hl));
   }
   if (max_jet_vel > 0.) {
     r = std::min(r, cfl * g.dx[0] / max_jet_vel);
@@ -735,12 +767,14 @@ extern "C" int pmp_spray_derive(pmp_spray* h, const pmp_box_view* vars, int nbox
   if (rc != PMP_OK) {
     return rc;
   }
+  // {error word, views, cell prefix} in one upload
+  std::vector<char> up(need, 0);
+  memcpy(up.data() + 16, hv.data(), sizeof(View32) * nboxes);
+  memcpy(up.data() + 16 + sizeof(View32) * nboxes, prefix.data(), sizeof(long long) * (nboxes + 1));
   int* d_err = static_cast<int*>(sp);
   View32* d_views = reinterpret_cast<View32*>(static_cast<char*>(sp) + 16);
   long long* d_prefix = reinterpret_cast<long long*>(d_views + nboxes);
-  PMP_TRY(h, cudaMemsetAsync(d_err, 0, sizeof(int), st));
-  PMP_TRY(h, cudaMemcpyAsync(d_views, hv.data(), sizeof(View32) * nboxes, cudaMemcpyHostToDevice, st));
-  PMP_TRY(h, cudaMemcpyAsync(d_prefix, prefix.data(), sizeof(long long) * (nboxes + 1), cudaMemcpyHostToDevice, st));
+  PMP_TRY(h, cudaMemcpyAsync(sp, up.data(), need, cudaMemcpyHostToDevice, st));
   const long long n = h->total;
   const pmp_geometry& g = h->geom;
   DeriveArgs A;
@@ -792,10 +826,11 @@ extern "C" int pmp_spray_derive(pmp_spray* h, const pmp_box_view* vars, int nbox
   if (prefix[nboxes] > 0) {
     k_protected_divide<<<nblk(prefix[nboxes]), 256, 0, st>>>(d_views, d_prefix, nboxes, prefix[nboxes], start_indx);
   }
-  int herr = 0;
+  int* hp = reinterpret_cast<int*>(h->h_small());
   PMP_TRY(h, cudaGetLastError());
-  PMP_TRY(h, cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  PMP_TRY(h, cudaMemcpyAsync(hp, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
   PMP_TRY(h, cudaStreamSynchronize(st));
+  const int herr = *hp;
   if (herr != 0) {
     return set_err(h, PMP_ERR_SOURCE_BOX, "derive view does not hold a droplet's cell", -1, herr - 1);
   }
@@ -821,7 +856,7 @@ extern "C" int pmp_spray_transfer_source(pmp_spray* h, const pmp_box_view* tmp_s
   const int g = source_ghosts;
   const int ng = std::min(act_ghosts, source_ghosts);
   std::vector<View32> ht(nboxes), ha(nboxes);
-  std::vector<long long> pg(nboxes + 1, 0), pa(nboxes + 1, 0), pz(nboxes + 1, 0);
+  std::vector<long long> pg(nboxes + 1, 0), pz(nboxes + 1, 0);
   int ncomp = -1;
   for (int b = 0; b < nboxes; ++b) {
     const pmp_box& bx = h->boxes[b];
@@ -846,9 +881,8 @@ extern "C" int pmp_spray_transfer_source(pmp_spray* h, const pmp_box_view* tmp_s
              (bx.hi[2] - bx.lo[2] + 1 + 2 * grow);
     };
     pg[b + 1] = pg[b] + cells(g);
-    pa[b + 1] = pa[b] + cells(ng);
     const pmp_box_view& v = tmp_source[b];
-    pz[b + 1] = pz[b] + (long long)(v.hi[0] - v.lo[0] + 1) * (v.hi[1] - v.lo[1] + 1) * (v.hi[2] - v.lo[2] + 1) * v.ncomp;
+    pz[b + 1] = pz[b] + (long long)(v.hi[0] - v.lo[0] + 1) * (v.hi[1] - v.lo[1] + 1) * (v.hi[2] - v.lo[2] + 1);
   }
   const pmp_spray_comps& c = h->comps;
   AddMap M;
@@ -881,32 +915,30 @@ extern "C" int pmp_spray_transfer_source(pmp_spray* h, const pmp_box_view* tmp_s
       }
     }
   }
-  const size_t need = 2 * sizeof(View32) * nboxes + 3 * sizeof(long long) * (nboxes + 1) + sizeof(pmp_box) * nboxes;
+  // {source views, destination views, cell prefixes, boxes} in one upload
+  const size_t vb = sizeof(View32) * nboxes, xb = sizeof(long long) * (nboxes + 1), bb = sizeof(pmp_box) * nboxes;
+  std::vector<char> up(2 * vb + 2 * xb + bb);
+  memcpy(up.data(), ht.data(), vb);
+  memcpy(up.data() + vb, ha.data(), vb);
+  memcpy(up.data() + 2 * vb, pg.data(), xb);
+  memcpy(up.data() + 2 * vb + xb, pz.data(), xb);
+  memcpy(up.data() + 2 * vb + 2 * xb, h->boxes.data(), bb);
   void* sp = nullptr;
-  if ((rc = scratch(h, need, &sp)) != PMP_OK) {
+  if ((rc = scratch(h, up.size(), &sp)) != PMP_OK) {
     return rc;
   }
   View32* d_t = static_cast<View32*>(sp);
   View32* d_a = d_t + nboxes;
   long long* d_pg = reinterpret_cast<long long*>(d_a + nboxes);
-  long long* d_pa = d_pg + nboxes + 1;
-  long long* d_pz = d_pa + nboxes + 1;
+  long long* d_pz = d_pg + nboxes + 1;
   pmp_box* d_boxes = reinterpret_cast<pmp_box*>(d_pz + nboxes + 1);
-  PMP_TRY(h, cudaMemcpyAsync(d_t, ht.data(), sizeof(View32) * nboxes, cudaMemcpyHostToDevice, st));
-  PMP_TRY(h, cudaMemcpyAsync(d_a, ha.data(), sizeof(View32) * nboxes, cudaMemcpyHostToDevice, st));
-  PMP_TRY(h, cudaMemcpyAsync(d_pg, pg.data(), sizeof(long long) * (nboxes + 1), cudaMemcpyHostToDevice, st));
-  PMP_TRY(h, cudaMemcpyAsync(d_pa, pa.data(), sizeof(long long) * (nboxes + 1), cudaMemcpyHostToDevice, st));
-  PMP_TRY(h, cudaMemcpyAsync(d_pz, pz.data(), sizeof(long long) * (nboxes + 1), cudaMemcpyHostToDevice, st));
-  PMP_TRY(h, cudaMemcpyAsync(d_boxes, h->boxes.data(), sizeof(pmp_box) * nboxes, cudaMemcpyHostToDevice, st));
+  PMP_TRY(h, cudaMemcpyAsync(sp, up.data(), up.size(), cudaMemcpyHostToDevice, st));
   const Domain D = domain_of(h);
   if (g > 0 && pg[nboxes] > 0) {
     k_sum_boundary<<<nblk(pg[nboxes]), 256, 0, st>>>(d_t, d_boxes, d_pg, nboxes, pg[nboxes], g, h->d_box_map, D, ncomp);
   }
-  if (pa[nboxes] > 0) {
-    k_add_source<<<nblk(pa[nboxes]), 256, 0, st>>>(d_t, d_a, d_boxes, d_pa, nboxes, pa[nboxes], ng, M);
-  }
   if (pz[nboxes] > 0) {
-    k_zero_views<<<nblk(pz[nboxes]), 256, 0, st>>>(d_t, d_pz, nboxes, pz[nboxes]);
+    k_add_reset<<<nblk(pz[nboxes]), 256, 0, st>>>(d_t, d_a, d_boxes, d_pz, nboxes, pz[nboxes], ng, M);
   }
   PMP_TRY(h, cudaGetLastError());
   PMP_TRY(h, cudaStreamSynchronize(st));

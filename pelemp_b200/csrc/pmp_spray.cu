@@ -1203,7 +1203,7 @@ int pmp_spray_create(const pmp_spray_config* cfg, pmp_spray** out)
   if (cudaSetDevice(h->device) != cudaSuccess ||
       cudaMalloc(&h->d_status, sizeof(DevStatus)) != cudaSuccess ||
       cudaMemset(h->d_status, 0, sizeof(DevStatus)) != cudaSuccess ||
-      cudaMallocHost(&h->h_status, sizeof(DevStatus)) != cudaSuccess ||
+      cudaMallocHost(&h->h_status, sizeof(DevStatus) + pmp_spray::kSmall) != cudaSuccess ||
       cudaHostAlloc(&h->err_host, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
       cudaHostGetDevicePointer(&h->err_dev, h->err_host, 0) != cudaSuccess ||
       cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess ||
