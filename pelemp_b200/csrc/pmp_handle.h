@@ -117,7 +117,12 @@ struct pmp_spray {
   // re-binning exchanges the store
   bool packed = false;
   long long total = 0;
-  pmp::KeptBuffer store, spare, row_keys, perm_b, fb_b, map_b, sort_scratch, transit;
+  pmp::KeptBuffer store, spare, row_keys, perm_b, fb_b, map_b, sort_scratch, transit, counts;
+  // sort by counting (cell_sort.cuh): `counted`: counts holds the staged rows,
+  // each once; `ranked`: of some staged rows the rank is kept, not the index;
+  // the leading zero_cells entries of counts are zero
+  bool counted = false, ranked = false;
+  long long zero_cells = 0;
   double* soa = nullptr;  // (3 + NR) arrays of length total
   int* ids = nullptr;
   long long* perm() const { return static_cast<long long*>(perm_b.p); }  // slot -> caller's index in its box
@@ -132,9 +137,11 @@ struct pmp_spray {
   unsigned long long table_clock = 0;
   int cur_table = -1;  // slot of the last prepared call's table
   pmp::DevStatus* d_status = nullptr;
-  pmp::DevStatus* h_status = nullptr;  // page-locked, kSmall bytes more behind it
+  pmp::DevStatus* h_status = nullptr;  // page-locked, 2 * kSmall bytes more behind it
   static constexpr size_t kSmall = 64;
   void* h_small() const { return h_status + 1; }  // for the few bytes an operation reads back
+  // raised by a count that found a crowded cell (written by kernels)
+  int* crowded() const { return reinterpret_cast<int*>(static_cast<char*>(h_small()) + kSmall); }
   // the first device error code, written by the kernels into page-locked
   // host memory mapped into the device (err_dev: its device address)
   int* err_host = nullptr;
@@ -217,6 +224,7 @@ int run_update(
 int ensure_packed(pmp_spray* h, cudaStream_t st);
 int keep(pmp_spray* h, KeptBuffer& b, size_t bytes);
 size_t store_bytes(const pmp_spray* h, long long n);
+int count_cells(pmp_spray* h, long long cells, cudaStream_t st);
 // soa and ids for n droplets in the store buffer
 void store_attach(pmp_spray* h, long long n);
 void store_layout(pmp_spray* h);

@@ -26,6 +26,7 @@
 #include <cstring>
 #include <vector>
 
+#include "cell_sort.cuh"
 #include "pmp_handle.h"
 #include "spray_fp64.cuh"
 
@@ -539,55 +540,96 @@ __global__ void __launch_bounds__(256) k_add_reset(const View32* tmp, const View
 // --------------------------------------------------------------------------
 // redistribute
 
+struct Wrap {
+  double lo[3], hi[3], dxi[3];
+};
+
 // Sort key of a droplet: its new box o above `shift` bits of its cell's
 // place in the box's sort order (pmp::brick_key); dead droplets and droplets
 // in no box get box nb, so that they sort last.  K / V: 32-bit keys and slot
 // indices when the key fits 32 bits and the count 2^31, else 64-bit.
-template <typename K, typename V>
-__global__ void k_rebin_keys(double* px, double* py, double* pz, const int* id, long long n, const int* map, Domain D,
-                             double plo0, double plo1, double plo2, double phi0, double phi1, double phi2, double dxi0,
-                             double dxi1, double dxi2, const pmp_box* boxes, int nb, int shift, K* keys, V* idx)
+// COUNT: the live droplets are counted into their cells, the others get key
+// kNoCell, and the ranks take the indices' place.  Two droplets a thread, each
+// of the dependent loads (id and position, owner, box, count) for both at
+// once; the position of a dead droplet is loaded for nothing.
+constexpr int kRebinPer = 2;
+template <typename K, typename V, bool COUNT>
+__global__ void __launch_bounds__(256) k_rebin_keys(double* px, double* py, double* pz, const int* id, long long n,
+                                                    const int* map, const Domain D, const Wrap w, const pmp_box* boxes,
+                                                    int nb, int shift, K* keys, V* idx, unsigned* counts, int* crowded)
 {
-  const long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (s >= n) {
-    return;
-  }
-  idx[s] = (V)s;
-  const K dead = (K)nb << shift;
-  if (!(id[s] > 0)) {
-    keys[s] = dead;
-    return;
-  }
+  const long long s0 = blockIdx.x * (256LL * kRebinPer) + threadIdx.x;
   double* p[3] = {px, py, pz};
-  const double plo[3] = {plo0, plo1, plo2}, phi[3] = {phi0, phi1, phi2}, dxi[3] = {dxi0, dxi1, dxi2};
-  int c[3];
+  int alive[kRebinPer], o[kRebinPer], c[kRebinPer][3];
+  double x[kRebinPer][3];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    double x = p[d][s];
-    if (D.periodic[d]) {
-      const double L = phi[d] - plo[d];
-      const double x0 = x;
-      for (int it = 0; it < 64 && x >= phi[d]; ++it) {
-        x -= L;
-      }
-      for (int it = 0; it < 64 && x < plo[d]; ++it) {
-        x += L;
-      }
-      if (x != x0) {
-        p[d][s] = x;
-      }
+  for (int u = 0; u < kRebinPer; ++u) {
+    const long long s = s0 + 256 * u;
+    alive[u] = s < n ? id[s] : 0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      x[u][d] = s < n ? p[d][s] : 0.;
     }
-    c[d] = static_cast<int>(floor(__dmul_rn(__dsub_rn(x, plo[d]), dxi[d])));
   }
-  const int o = owner(map, D, c);
-  if (o < 0) {
-    keys[s] = dead;
-    return;
+#pragma unroll
+  for (int u = 0; u < kRebinPer; ++u) {
+    o[u] = -1;
+    if (alive[u] > 0) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        double y = x[u][d];
+        if (D.periodic[d]) {
+          const double L = w.hi[d] - w.lo[d];
+          for (int it = 0; it < 64 && y >= w.hi[d]; ++it) {
+            y -= L;
+          }
+          for (int it = 0; it < 64 && y < w.lo[d]; ++it) {
+            y += L;
+          }
+          if (y != x[u][d]) {
+            p[d][s0 + 256 * u] = y;
+          }
+        }
+        c[u][d] = static_cast<int>(floor(__dmul_rn(__dsub_rn(y, w.lo[d]), w.dxi[d])));
+      }
+      o[u] = owner(map, D, c[u]);
+    }
   }
-  const pmp_box& bx = boxes[o];
-  const int ex = bx.hi[0] - bx.lo[0] + 1, ey = bx.hi[1] - bx.lo[1] + 1;
-  const unsigned long long local = pmp::brick_key(c[0] - bx.lo[0], c[1] - bx.lo[1], c[2] - bx.lo[2], ex, ey);
-  keys[s] = ((K)o << shift) | (K)local;
+  K key[kRebinPer];
+  Counted q[kRebinPer];
+#pragma unroll
+  for (int u = 0; u < kRebinPer; ++u) {
+    key[u] = COUNT ? (K)kNoCell : (K)nb << shift;
+    if (o[u] >= 0) {
+      const pmp_box& bx = boxes[o[u]];
+      const int ex = bx.hi[0] - bx.lo[0] + 1, ey = bx.hi[1] - bx.lo[1] + 1;
+      const unsigned long long local =
+        pmp::brick_key(c[u][0] - bx.lo[0], c[u][1] - bx.lo[1], c[u][2] - bx.lo[2], ex, ey);
+      key[u] = ((K)o[u] << shift) | (K)local;
+    }
+    if (COUNT) {
+      q[u] = count_cell(counts, (unsigned)key[u]);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kRebinPer; ++u) {
+    const long long s = s0 + 256 * u;
+    const V v = COUNT ? (V)rank_of(q[u], (unsigned)key[u], crowded) : (V)s;
+    if (s < n) {
+      keys[s] = key[u];
+      idx[s] = v;
+    }
+  }
+}
+
+// begin[b] of counted droplets: the first slot of box b's first cell (b = nb:
+// their number)
+__global__ void k_box_starts(const unsigned* starts, int nb, int shift, long long* begin)
+{
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b <= nb) {
+    begin[b] = starts[(long long)b << shift];
+  }
 }
 
 // begin[b]: the first sorted position of box b (b = nb: the dead)
@@ -945,12 +987,33 @@ extern "C" int pmp_spray_transfer_source(pmp_spray* h, const pmp_box_view* tmp_s
   return PMP_OK;
 }
 
+static Wrap wrap_of(const pmp_spray* h)
+{
+  Wrap w;
+  for (int d = 0; d < 3; ++d) {
+    w.lo[d] = h->geom.plo[d];
+    w.hi[d] = h->geom.phi[d];
+    w.dxi[d] = 1. / h->geom.dx[d];
+  }
+  return w;
+}
+
+// the box bounds on the host
+static int read_bounds(pmp_spray* h, cudaStream_t st, const long long* d_begin, std::vector<long long>& begin)
+{
+  PMP_TRY(h, cudaMemcpyAsync(begin.data(), d_begin, sizeof(long long) * begin.size(), cudaMemcpyDeviceToHost, st));
+  if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
+    return set_err(h, PMP_ERR_CUDA, "redistribute: kernel failed");
+  }
+  return PMP_OK;
+}
+
 // The re-binning's keys, their sort and the box bounds (begin, host copy),
-// with K-bit keys over bits [0, end_bit) and V-bit slot indices; the sorted
-// indices (the gather order) stay in sort_scratch at RebinLayout::perm.
+// with K-bit keys over bits [0, end_bit) and V-bit slot indices; *order: the
+// sorted indices (the gather order), in sort_scratch, *d_begin the bounds.
 template <typename K, typename V>
 static int rebin_sort(pmp_spray* h, cudaStream_t st, long long n, int nb, int shift, int end_bit,
-                      std::vector<long long>& begin)
+                      std::vector<long long>& begin, const void** order, const long long** d_bounds)
 {
   size_t tbytes = 0;
   if (n > 0) {
@@ -969,23 +1032,57 @@ static int rebin_sort(pmp_spray* h, cudaStream_t st, long long n, int nb, int sh
   V* perm = reinterpret_cast<V*>(base + L.perm);
   long long* d_begin = reinterpret_cast<long long*>(base + L.begin);
   pmp_box* d_boxes = reinterpret_cast<pmp_box*>(base + L.boxes);
-  const pmp_geometry& g = h->geom;
   PMP_TRY(h, cudaMemcpyAsync(d_boxes, h->boxes.data(), sizeof(pmp_box) * nb, cudaMemcpyHostToDevice, st));
-  const Domain D = domain_of(h);
   if (n > 0) {
-    k_rebin_keys<K, V><<<nblk(n), 256, 0, st>>>(h->soa, h->soa + n, h->soa + 2 * n, h->ids, n, h->d_box_map, D,
-                                                g.plo[0], g.plo[1], g.plo[2], g.phi[0], g.phi[1], g.phi[2],
-                                                1. / g.dx[0], 1. / g.dx[1], 1. / g.dx[2], d_boxes, nb, shift, keys,
-                                                idx);
+    k_rebin_keys<K, V, false><<<nblk(n, 256 * kRebinPer), 256, 0, st>>>(h->soa, h->soa + n, h->soa + 2 * n, h->ids, n, h->d_box_map,
+                                                       domain_of(h), wrap_of(h), d_boxes, nb, shift, keys, idx, nullptr,
+                                                       nullptr);
     cub::DeviceRadixSort::SortPairs(base + L.tmp, tbytes, keys, keys2, idx, perm, (int)n, 0, end_bit, st);
     k_box_bounds<K><<<nblk(nb + 1, 64), 64, 0, st>>>(keys2, n, nb, shift, d_begin);
   } else {
     PMP_TRY(h, cudaMemsetAsync(d_begin, 0, sizeof(long long) * (nb + 1), st));
   }
-  PMP_TRY(h, cudaMemcpyAsync(begin.data(), d_begin, sizeof(long long) * (nb + 1), cudaMemcpyDeviceToHost, st));
-  if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
-    return set_err(h, PMP_ERR_CUDA, "redistribute: kernel failed");
+  *order = perm;
+  *d_bounds = d_begin;
+  return read_bounds(h, st, d_begin, begin);
+}
+
+// The same by counting (cell_sort.cuh); *crowded: a cell holds too many
+// droplets, and nothing was sorted.
+static int rebin_count(pmp_spray* h, cudaStream_t st, long long n, int nb, int shift, long long cells,
+                       std::vector<long long>& begin, const void** order, const long long** d_bounds, bool* crowded)
+{
+  auto up = [](size_t b) { return align256(b); };
+  const CellSortLayout L = cell_sort_layout(cells, n);
+  const size_t ranks = L.total + up(sizeof(unsigned) * n), bounds = ranks + up(sizeof(int) * n);
+  const size_t boxes = bounds + up(sizeof(long long) * (nb + 1));
+  int rc = keep(h, h->sort_scratch, boxes + sizeof(pmp_box) * nb);
+  if (rc == PMP_OK) {
+    rc = count_cells(h, cells, st);
   }
+  if (rc != PMP_OK) {
+    return rc;
+  }
+  char* base = static_cast<char*>(h->sort_scratch.p);
+  unsigned* counts = static_cast<unsigned*>(h->counts.p);
+  unsigned* keys = reinterpret_cast<unsigned*>(base + L.total);
+  int* rank = reinterpret_cast<int*>(base + ranks);
+  long long* d_begin = reinterpret_cast<long long*>(base + bounds);
+  pmp_box* d_boxes = reinterpret_cast<pmp_box*>(base + boxes);
+  PMP_TRY(h, cudaMemcpyAsync(d_boxes, h->boxes.data(), sizeof(pmp_box) * nb, cudaMemcpyHostToDevice, st));
+  k_rebin_keys<unsigned, int, true><<<nblk(n, 256 * kRebinPer), 256, 0, st>>>(h->soa, h->soa + n, h->soa + 2 * n, h->ids, n, h->d_box_map,
+                                                             domain_of(h), wrap_of(h), d_boxes, nb, shift, keys, rank,
+                                                             counts, h->crowded());
+  cell_sort(counts, cells, keys, rank, n, base, st);
+  k_box_starts<<<nblk(nb + 1), 256, 0, st>>>(reinterpret_cast<unsigned*>(base), nb, shift, d_begin);
+  rc = read_bounds(h, st, d_begin, begin);
+  if (rc != PMP_OK) {
+    return rc;
+  }
+  h->zero_cells = cells;
+  *crowded = *h->crowded() != 0;
+  *order = base + L.order;
+  *d_bounds = d_begin;
   return PMP_OK;
 }
 
@@ -1028,10 +1125,19 @@ extern "C" int pmp_spray_redistribute(pmp_spray* h, long long* removed, void* st
   }
   std::vector<long long> begin(nb + 1, 0);
   const bool narrow = end_bit <= 32 && n < (1LL << 31);
-  const int rc2 = narrow ? rebin_sort<unsigned, int>(h, st, n, nb, shift, end_bit, begin)
-                         : rebin_sort<unsigned long long, long long>(h, st, n, nb, shift, end_bit, begin);
-  if (rc2 != PMP_OK) {
-    return rc2;
+  const void* order = nullptr;
+  const long long* d_begin = nullptr;
+  const long long cells = padded_cells(nb, shift);
+  bool crowded = true;
+  if (narrow && counting_pays(cells, n)) {
+    rc = rebin_count(h, st, n, nb, shift, cells, begin, &order, &d_begin, &crowded);
+  }
+  if (rc == PMP_OK && crowded) {
+    rc = narrow ? rebin_sort<unsigned, int>(h, st, n, nb, shift, end_bit, begin, &order, &d_begin)
+                : rebin_sort<unsigned long long, long long>(h, st, n, nb, shift, end_bit, begin, &order, &d_begin);
+  }
+  if (rc != PMP_OK) {
+    return rc;
   }
   const long long live = begin[nb];
   // gather into the spare store (grown when too small), which then becomes
@@ -1043,14 +1149,11 @@ extern "C" int pmp_spray_redistribute(pmp_spray* h, long long* removed, void* st
   double* soa2 = static_cast<double*>(h->spare.p);
   int* ids2 = reinterpret_cast<int*>(soa2 + (long long)nc * live);
   if (live > 0) {
-    const RebinLayout Lr = rebin_layout(n, nb, narrow ? 4 : 8, narrow ? 4 : 8, 0);
-    const void* perm = static_cast<char*>(h->sort_scratch.p) + Lr.perm;
-    const long long* d_begin = reinterpret_cast<const long long*>(static_cast<char*>(h->sort_scratch.p) + Lr.begin);
     if (narrow) {
-      k_gather_soa<<<nblk(live), 256, 0, st>>>(h->soa, n, h->ids, static_cast<const int*>(perm), live, nc,
+      k_gather_soa<<<nblk(live), 256, 0, st>>>(h->soa, n, h->ids, static_cast<const int*>(order), live, nc,
                                                soa2, ids2);
     } else {
-      k_gather_soa<<<nblk(live), 256, 0, st>>>(h->soa, n, h->ids, static_cast<const long long*>(perm), live, nc,
+      k_gather_soa<<<nblk(live), 256, 0, st>>>(h->soa, n, h->ids, static_cast<const long long*>(order), live, nc,
                                                soa2, ids2);
     }
     // each box's new order is its caller order (h->perm_b holds >= n >= live slots)

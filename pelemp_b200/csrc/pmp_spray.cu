@@ -1203,7 +1203,7 @@ int pmp_spray_create(const pmp_spray_config* cfg, pmp_spray** out)
   if (cudaSetDevice(h->device) != cudaSuccess ||
       cudaMalloc(&h->d_status, sizeof(DevStatus)) != cudaSuccess ||
       cudaMemset(h->d_status, 0, sizeof(DevStatus)) != cudaSuccess ||
-      cudaMallocHost(&h->h_status, sizeof(DevStatus) + pmp_spray::kSmall) != cudaSuccess ||
+      cudaMallocHost(&h->h_status, sizeof(DevStatus) + 2 * pmp_spray::kSmall) != cudaSuccess ||
       cudaHostAlloc(&h->err_host, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
       cudaHostGetDevicePointer(&h->err_dev, h->err_host, 0) != cudaSuccess ||
       cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess ||
@@ -1448,6 +1448,7 @@ int pmp_spray_set_grids(pmp_spray* h, int nboxes, const pmp_box* boxes)
   h->grids_version += 1;
   h->staged.assign(nboxes, pmp::StagedBox{});
   h->staged_rows = 0;
+  h->counted = h->ranked = false;
   pmp::store_layout(h);
   h->box_set.assign(nboxes, false);
   return PMP_OK;

@@ -27,6 +27,7 @@
 #include <cstring>
 #include <vector>
 
+#include "cell_sort.cuh"
 #include "pmp_handle.h"
 
 namespace pmp {
@@ -97,12 +98,43 @@ __device__ __forceinline__ unsigned long long sort_key(const KeyOf& k, double x,
 }
 
 // Where a staging kernel leaves each row's key and index (narrow keys; null:
-// formed from the rows when they are packed)
+// formed from the rows when they are packed); with counts, the row is counted
+// into its cell and its rank takes the index's place
 struct KeyOut {
   unsigned* keys;
   int* idx;
   long long row0;  // index of the kernel's first row
+  unsigned* counts;
+  int* crowded;
 };
+
+// A thread's row in the keys, before and after the CTA writes its rows (all
+// lanes call both); valid: the thread has a row, i its number among the kernel's
+struct RowKey {
+  unsigned key;
+  Counted count;
+};
+__device__ __forceinline__ RowKey begin_key(const KeyOut& out, const KeyOf& key, bool valid, const double* pos)
+{
+  RowKey k{};
+  if (out.keys) {
+    k.key = valid ? (unsigned)sort_key(key, pos[0], pos[1], pos[2]) : kNoCell;
+    if (out.counts) {
+      k.count = count_cell(out.counts, k.key);
+    }
+  }
+  return k;
+}
+__device__ __forceinline__ void end_key(const KeyOut& out, const RowKey& k, bool valid, long long i)
+{
+  if (out.keys) {
+    const int v = out.counts ? rank_of(k.count, k.key, out.crowded) : (int)(out.row0 + i);
+    if (valid) {
+      out.keys[i] = k.key;
+      out.idx[i] = v;
+    }
+  }
+}
 
 __device__ __forceinline__ double pack_ints(int lo, int hi) { return __hiloint2double(hi, lo); }
 
@@ -136,17 +168,16 @@ __global__ void __launch_bounds__(kTile) k_aos_to_rows(const double* aos, long l
     tile[i / R::kWords][i % R::kWords] = __ldcs(src + i);
   }
   __syncthreads();
-  if ((int)threadIdx.x < m) {
-    double* t = tile[threadIdx.x];
+  double* t = tile[threadIdx.x];
+  const bool valid = (int)threadIdx.x < m;
+  if (valid) {
     const int id = __double2loint(t[R::kReals]);
     t[R::kReals] = pack_ints(id, (int)(s0 + threadIdx.x));
-    if (out.keys) {
-      out.keys[s0 + threadIdx.x] = (unsigned)sort_key(key, t[0], t[1], t[2]);
-      out.idx[s0 + threadIdx.x] = (int)(out.row0 + s0 + threadIdx.x);
-    }
   }
+  const RowKey k = begin_key(out, key, valid, t);
   __syncthreads();
   tile_to_rows<NF>(tile, rows + s0 * R::kStride, m);
+  end_key(out, k, valid, s0 + threadIdx.x);
 }
 
 // component arrays -> rows; a null component is zero.  caller: the droplets'
@@ -161,20 +192,19 @@ __global__ void __launch_bounds__(kTile) k_columns_to_rows(const __grid_constant
   const long long s0 = (long long)blockIdx.x * kTile;
   const int m = (int)min((long long)kTile, n - s0);
   const long long s = s0 + threadIdx.x;
-  if ((int)threadIdx.x < m) {
+  const bool valid = (int)threadIdx.x < m;
+  double* t = tile[threadIdx.x];
+  if (valid) {
 #pragma unroll
     for (int c = 0; c < R::kReals; ++c) {
-      tile[threadIdx.x][c] = C.c[c] ? __ldcs(C.c[c] + s) : 0.;
+      t[c] = C.c[c] ? __ldcs(C.c[c] + s) : 0.;
     }
-    double* t = tile[threadIdx.x];
     t[R::kReals] = pack_ints(C.id[s], caller ? (int)caller[s] : (int)s);
-    if (out.keys) {
-      out.keys[s] = (unsigned)sort_key(key, t[0], t[1], t[2]);
-      out.idx[s] = (int)(out.row0 + s);
-    }
   }
+  const RowKey k = begin_key(out, key, valid, t);
   __syncthreads();
   tile_to_rows<NF>(tile, rows + s0 * R::kStride, m);
+  end_key(out, k, valid, s);
 }
 
 // One box's staging rows, in the order of the packed store (box by box).
@@ -422,7 +452,21 @@ KeyOut key_out(const pmp_spray* h, long long row)
 {
   const long long cap = (long long)(h->row_keys.bytes / (2 * sizeof(unsigned)));
   unsigned* keys = static_cast<unsigned*>(h->row_keys.p);
-  return {keys + row, reinterpret_cast<int*>(keys + cap) + row, row};
+  return {keys + row, reinterpret_cast<int*>(keys + cap) + row, row, nullptr, nullptr};
+}
+
+long long sort_cells(const pmp_spray* h) { return padded_cells((long long)h->boxes.size(), h->sort_shift); }
+
+// Whether the rows of a hand-over are counted into their cells while they are
+// staged: decided at its first box, of n droplets, as if the others held as
+// many; cell_sorted() looks at the whole.
+bool count_first(const pmp_spray* h, long long n)
+{
+  return narrow_keys(h) && counting_pays(sort_cells(h), n * (long long)h->boxes.size());
+}
+bool cell_sorted(const pmp_spray* h, long long m)
+{
+  return h->counted && *h->crowded() == 0 && counting_pays(sort_cells(h), m);
 }
 
 // Room for n more staging rows in the spare buffer (and their keys); the live
@@ -462,10 +506,13 @@ int stage_room(pmp_spray* h, long long n)
       if (e == cudaSuccess) {
         e = cudaMemcpy(to.keys + at, from.keys + s.row, sizeof(unsigned) * s.n, cudaMemcpyDeviceToDevice);
       }
+      if (e == cudaSuccess && h->ranked) {
+        e = cudaMemcpy(to.idx + at, from.idx + s.row, sizeof(int) * s.n, cudaMemcpyDeviceToDevice);
+      }
       at += s.n;
     }
   }
-  if (e == cudaSuccess && at > 0) {
+  if (e == cudaSuccess && at > 0 && !h->ranked) {
     k_fill_keys<<<nblk(at, 256), 256>>>(nullptr, to.idx, 0, at, 0);
     e = cudaGetLastError();
   }
@@ -497,6 +544,7 @@ int unpack(pmp_spray* h, int skip)
   const int nc = h->ncomp();
   const long long T = h->total;
   h->staged_rows = 0;
+  h->counted = h->ranked = false;
   for (int b = 0; b < nb; ++b) {
     h->staged[b] = StagedBox{};
   }
@@ -664,6 +712,25 @@ void store_attach(pmp_spray* h, long long n)
   h->ids = reinterpret_cast<int*>(h->soa + (long long)h->ncomp() * n);
 }
 
+// Zeroed counts of `cells` cells, for a sort on st, which leaves them zero
+// again: `zero_cells` says how many are (0 while they are in use).
+int count_cells(pmp_spray* h, long long cells, cudaStream_t st)
+{
+  const void* before = h->counts.p;
+  const int rc = keep(h, h->counts, sizeof(unsigned) * (size_t)cells);
+  if (rc != PMP_OK) {
+    h->zero_cells = 0;
+    return rc;
+  }
+  if (h->counts.p != before || h->zero_cells < cells) {
+    h->zero_cells = 0;
+    PMP_TRY(h, cudaMemsetAsync(h->counts.p, 0, sizeof(unsigned) * (size_t)cells, st));
+  }
+  h->zero_cells = 0;
+  *h->crowded() = 0;
+  return PMP_OK;
+}
+
 // Sort-key layout of new grids: bits of a cell's place in its box, and of the
 // box above them.
 void store_layout(pmp_spray* h)
@@ -697,10 +764,11 @@ void store_free(pmp_spray* h)
 {
   store_reset(h);
   for (KeptBuffer* b : {&h->store, &h->spare, &h->row_keys, &h->perm_b, &h->fb_b, &h->map_b, &h->sort_scratch,
-                        &h->transit}) {
+                        &h->transit, &h->counts}) {
     cudaFree(b->p);
     *b = KeptBuffer{};
   }
+  h->zero_cells = 0;
 }
 
 // Box offsets and the CTA -> (box, first slot) map of the packed droplets,
@@ -784,10 +852,23 @@ int ensure_packed(pmp_spray* h, cudaStream_t st)
       // rows given up carry the key of no box, above every other
       const long long m = h->staged_rows;
       const int bits = m == n ? end_bit : 32;
-      rc = keep(h, h->sort_scratch, sort_bytes<unsigned, int>(m, bits));
+      const long long cells = sort_cells(h);
+      const bool by_cell = m == n && cell_sorted(h, m);
+      rc = keep(h, h->sort_scratch, by_cell ? cell_sort_layout(cells, m).total : sort_bytes<unsigned, int>(m, bits));
       const KeyOut k = key_out(h, 0);
       const int* order = nullptr;
-      if (rc == PMP_OK) {
+      if (rc == PMP_OK && by_cell) {
+        char* buf = static_cast<char*>(h->sort_scratch.p);
+        h->counted = false;
+        cell_sort(static_cast<unsigned*>(h->counts.p), cells, k.keys, k.idx, m, buf, st);
+        PMP_TRY(h, cudaGetLastError());
+        h->zero_cells = cells;
+        order = reinterpret_cast<const int*>(buf + cell_sort_layout(cells, m).order);
+      } else if (rc == PMP_OK) {
+        if (h->ranked) {  // counted, and not sorted by it
+          k_fill_keys<<<nblk(m, 256), 256, 0, st>>>(nullptr, k.idx, 0, m, 0);
+          h->counted = h->ranked = false;
+        }
         rc = sort_rows<unsigned, int>(h, k.keys, k.idx, m, bits, 0, st, &order);
       }
       if (rc == PMP_OK) {
@@ -829,6 +910,7 @@ int ensure_packed(pmp_spray* h, cudaStream_t st)
     s = StagedBox{};
   }
   h->staged_rows = 0;
+  h->counted = h->ranked = false;
   if (capturing) {
     PMP_TRY(h, cudaStreamSynchronize(st));
     return PMP_OK;
@@ -865,6 +947,9 @@ int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
   }
   const long long n = p->n;
   StagedBox& s = h->staged[box];
+  if (s.n > 0) {
+    h->counted = false;  // with the rows that are given up
+  }
   if (s.n > 0 && s.row + s.n == h->staged_rows) {
     h->staged_rows = s.row;  // its rows are the last ones
   } else if (s.n > 0 && narrow_keys(h)) {
@@ -898,7 +983,25 @@ int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
   const int nr = h->nr();
   double* rows = staged_row(h, h->staged_rows);
   const KeyOf key = key_of(h, box, false);
-  const KeyOut out = narrow_keys(h) ? key_out(h, h->staged_rows) : KeyOut{};
+  KeyOut out = narrow_keys(h) ? key_out(h, h->staged_rows) : KeyOut{};
+  if (h->staged_rows == 0) {
+    h->ranked = false;
+    h->counted = count_first(h, n);
+    if (h->counted) {
+      rc = count_cells(h, sort_cells(h), nullptr);
+      if (rc != PMP_OK) {
+        h->counted = false;
+        return rc;
+      }
+    }
+  }
+  const bool counting = h->counted;
+  h->counted = false;  // until the box is in
+  if (counting) {
+    out.counts = static_cast<unsigned*>(h->counts.p);
+    out.crowded = h->crowded();
+    h->ranked = true;
+  }
   const cudaMemcpyKind kind = p->where == PMP_WHERE_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
   DeviceRanges ranges(h->device);
   Transit transit(h);
@@ -958,6 +1061,7 @@ int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
   s.n = n;
   s.row = h->staged_rows;
   h->staged_rows += n;
+  h->counted = counting;
   h->box_set[box] = true;
   return PMP_OK;
 }

@@ -147,6 +147,64 @@ def test_packed_order_is_stable_by_cell():
         assert np.array_equal(got["id"], d[2][order]) and np.array_equal(got["rdata"], d[1][:, order])
 
 
+@pytest.mark.parametrize("counts,crowd,again", [
+    ((2048, 2048), 0, None),  # as many as one launch sorts
+    ((2048, 2049), 0, None),  # one more, the first box too few to expect it
+    ((2049, 2048), 0, None),  # counted
+    ((2049, 0), 0, None),  # counted, and too few of them in the end
+    ((40000, 1), 0, None),
+    ((9000, 3000), 64, None),  # the fullest cell that is sorted by counting
+    ((9000, 3000), 65, None),
+    ((9000, 3000), 9000, None),  # one cell holds a box
+    ((100, 9000), 0, None),  # staging rows exchanged with ranks in them
+    ((3000, 5000), 0, (0, 4000)),  # rows given up
+    ((3000, 5000), 0, (1, 4000)),  # rows given up at the end
+    ((200000, 150000), 0, None),  # a CTA's cells hold more than its tile
+])
+def test_sorted_by_cell_and_stable(counts, crowd, again):
+    """Packed, then re-binned: by new box, then by cell, in the order handed over.  Droplets lie in
+    either box and are dead or alive."""
+    prob = level(2)
+    rng = np.random.default_rng(5)
+    sp = from_problem(prob, set_droplets=False)
+    dx = prob.dx[0]
+    (lo, _), (_, hi) = prob.boxes
+    drs = [droplets(rng, n, 2, lo, hi, dx) for n in counts]
+    if crowd:
+        # one cell with `crowd` droplets of box 0, and no others
+        pos = drs[0][0]
+        cell = np.floor(pos / dx).astype(int)
+        pos[0, np.all(cell == [[3], [4], [5]], axis=0)] += dx
+        pos[:, rng.permutation(counts[0])[:crowd]] = (np.array([[3], [4], [5]]) + rng.random((3, crowd))) * dx
+        if crowd < counts[0]:
+            cell = np.floor(drs[1][0] / dx).astype(int)
+            drs[1][0][0, np.all(cell == [[3], [4], [5]], axis=0)] += dx
+    for d in drs:
+        if d[2].size > 1:
+            d[2][rng.random(d[2].size) < 0.1] *= -1
+    for _ in range(2):
+        for b, d in enumerate(drs):
+            sp.set_particles(b, *d)
+        if again:
+            drs[again[0]] = droplets(rng, again[1], 2, lo, hi, dx)
+            sp.set_particles(again[0], *drs[again[0]])
+        sp.est_timestep(0.5)
+        for b, d in enumerate(drs):
+            got = sp.get_particles(b)
+            assert np.array_equal(got["id"], d[2]) and np.array_equal(got["rdata"], d[1])
+        pos, rd = (np.concatenate([d[i] for d in drs], axis=1) for i in (0, 1))
+        ids = np.concatenate([d[2] for d in drs])
+        c = np.floor(pos * (1.0 / prob.dx)[:, None]).astype(np.int64)
+        key = ((c[0] // 16 * 16 + c[2]) * 16 + c[1]) * 16 + c[0] % 16
+        key[ids <= 0] = 1 << 20
+        order = np.argsort(key, kind="stable")[:np.count_nonzero(ids > 0)]
+        assert sp.redistribute() == np.count_nonzero(ids <= 0)
+        split = np.count_nonzero(key[order] < 4096)
+        for b, sel in enumerate((order[:split], order[split:])):
+            got = sp.get_particles(b)
+            assert np.array_equal(got["id"], ids[sel]) and np.array_equal(got["rdata"], rd[:, sel])
+
+
 def test_refused():
     prob = level(1)
     sp = from_problem(prob, set_droplets=False)
