@@ -56,7 +56,7 @@ int launch_gas_records(int ns, const KParams& P, int b0, int nb, int max_cells, 
   if (nb <= 0 || max_cells <= 0) {
     return PMP_OK;
   }
-  const dim3 grid((unsigned)std::min((max_cells + 255) / 256, 128), (unsigned)nb);
+  const dim3 grid = gas_rec_grid(max_cells, nb);
 #define PMP_REC_CASE(S)                                     \
   if (ns == S) {                                            \
     if (P.pelec) {                                          \

@@ -1128,7 +1128,7 @@ int pmp::launch_gas_records64(const pmp_spray* h, const KParams& P, int b0, int 
   if (nb <= 0 || max_cells <= 0 || h->mode != PMP_MODE_FP64) {
     return PMP_OK;
   }
-  const dim3 grid((unsigned)std::min((max_cells + 255) / 256, 128), (unsigned)nb);
+  const dim3 grid = pmp::gas_rec_grid(max_cells, nb);
 #define PMP_REC_CASE(S)                                                  \
   if (h->nspec == S) {                                                   \
     if (h->pelec) {                                                      \

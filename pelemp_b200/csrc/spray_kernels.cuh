@@ -1025,32 +1025,68 @@ static __global__ void __launch_bounds__(256) k_select_small(const __grid_consta
   }
 }
 
-// The FP32 gas records of boxes [b0, b0 + gridDim.y) (BoxEntry::gr), one
-// thread per cell of the grown box, from the FP64 state: the mixed and
-// learned updates then gather 2-3 16-byte records per stencil cell instead of
-// 5 + NS FP64 planes, with rho*Y / rho divided once per cell.
+// The gas records of boxes [b0, b0 + gridDim.y): a thread per cell of the grown
+// box (gas_rec_grid), whose loads are all in flight together, and the CTA's
+// records written as one run of 16-byte words from shared memory (a thread's
+// own record is 48 or 64 bytes, so that its stores would each leave half
+// sectors to L2).  One exact reciprocal of rho a cell.  Bound by memory
+// bandwidth: FP64 records of 64 boxes of 32^3 with one fuel (3.5M cells)
+// 101 -> 72 us, 6.3 TB/s; FP32 records of 8 boxes of 64 x 64 x 32 with two
+// (1.5M cells), beside the selection of the small droplets, 95 -> 64 us;
+// before, up to 128 CTAs a box went over its cells in a loop, with a division
+// a species and a thread's own stores.
+inline dim3 gas_rec_grid(int max_cells, int nb) { return dim3((unsigned)((max_cells + 255) / 256), (unsigned)nb); }
+
+// the cell of a thread and its state; false beyond the grown box.  n: its cells
+__device__ __forceinline__ bool gas_rec_cell(const BoxEntry& B, const double*& q, int& n)
+{
+  const unsigned nx = B.state_hi[0] - B.state_lo[0] + 1;
+  const unsigned ny = B.state_hi[1] - B.state_lo[1] + 1;
+  const unsigned nz = B.state_hi[2] - B.state_lo[2] + 1;
+  n = (int)(nx * ny * nz);
+  const unsigned c = blockIdx.x * 256u + threadIdx.x;
+  const unsigned t = c / nx;
+  const unsigned k = t / ny;
+  const int i = (int)(c - t * nx), j = (int)(t - k * ny);
+  q = B.st + ((i + B.state_lo[0] - B.st_lo[0]) + (j + B.state_lo[1] - B.st_lo[1]) * B.st_j32 +
+              ((int)k + B.state_lo[2] - B.st_lo[2]) * B.st_k32);
+  return (int)c < n;
+}
+
+// tile[r] of the CTA's cells -> records of `W` 16-byte words, at `out`
+template <int W, int PITCH, typename T>
+__device__ __forceinline__ void write_records(const T (*tile)[PITCH], T* out, int n)
+{
+  const int c0 = blockIdx.x * 256, m = min(256, n - c0);
+  __syncthreads();
+  for (int w = threadIdx.x; w < m * W; w += 256) {
+    out[(long long)c0 * W + w] = tile[w / W][w % W];
+  }
+}
+
+// FP32 records (BoxEntry::gr) from the FP64 state: the mixed and learned
+// updates then gather 2-3 16-byte words per stencil cell instead of 5 + NS
+// FP64 planes, with rho*Y / rho divided once per cell.
 template <int NS, bool PELEC = false>
 __global__ void __launch_bounds__(256) k_gas_records(const __grid_constant__ KParams P, int b0)
 {
   constexpr int R4 = gas_rec4(NS);
+  __shared__ float4 tile[256][R4 | 1];
   const BoxEntry& B = P.boxes[b0 + blockIdx.y];
-  const int nx = B.state_hi[0] - B.state_lo[0] + 1;
-  const int ny = B.state_hi[1] - B.state_lo[1] + 1;
-  const int nz = B.state_hi[2] - B.state_lo[2] + 1;
-  const int n = nx * ny * nz;
-  for (int c = blockIdx.x * 256 + threadIdx.x; c < n; c += gridDim.x * 256) {
-    const int i = c % nx;
-    const int t = c / nx;
-    const int j = t % ny;
-    const int k = t / ny;
-    const double* q = B.st + ((i + B.state_lo[0] - B.st_lo[0]) + (j + B.state_lo[1] - B.st_lo[1]) * B.st_j32 +
-                              (k + B.state_lo[2] - B.st_lo[2]) * B.st_k32);
+  const double* q;
+  int n;
+  const bool valid = gas_rec_cell(B, q, n);
+  if ((int)blockIdx.x * 256 >= n) {
+    return;
+  }
+  if (valid) {
     const double rho = __ldg(q + P.c_rho * B.st_n32);
     float v[4 * R4];
     v[0] = (float)rho;
+    double ry[NS];
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      v[5 + s] = (float)(__ldg(q + (P.c_spec + P.spec_perm[s]) * B.st_n32) / rho);
+      ry[s] = __ldg(q + (P.c_spec + P.spec_perm[s]) * B.st_n32);
     }
     if (!PELEC) {
       v[1] = (float)__ldg(q + P.c_T * B.st_n32);
@@ -1077,76 +1113,95 @@ __global__ void __launch_bounds__(256) k_gas_records(const __grid_constant__ KPa
       const double e = __ldg(q + P.c_eng * B.st_n32) * inv_rho - ke;
       v[1] = (float)ey2t<NS>(P.m, e, Yc, __ldg(q + P.c_T * B.st_n32));
     }
+    // rho*Y / rho by the reciprocal (the quotient's bits, or in an unusual
+    // cell the division itself); a quotient too small for that to be exact
+    // is zero in FP32
+    MathFast M;
+    const Divisor d = M.divisor(rho);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      M.check_finite(ry[s]);
+      v[5 + s] = ry[s] == 0. ? (float)ry[s] : (float)M.div(ry[s], d);
+    }
+    if (M.odd) {
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        v[5 + s] = (float)(ry[s] / rho);
+      }
+    }
 #pragma unroll
     for (int s = 5 + NS; s < 4 * R4; ++s) {
       v[s] = 0.f;
     }
-    float4* r = B.gr + (long long)c * R4;
 #pragma unroll
     for (int m = 0; m < R4; ++m) {
-      r[m] = make_float4(v[4 * m], v[4 * m + 1], v[4 * m + 2], v[4 * m + 3]);
+      tile[threadIdx.x][m] = make_float4(v[4 * m], v[4 * m + 1], v[4 * m + 2], v[4 * m + 3]);
     }
   }
+  write_records<R4>(tile, B.gr, n);
 }
 
-// The FP64 gas records of boxes [b0, b0 + gridDim.y) (BoxEntry::gr64): per
-// cell of the grown box, rho, T, the velocity and the mass fractions formed
-// with exactly the operations of update_one's plane gather (PeleC: velocity
-// from momentum, T by EY2T from the cell's energy with its T as the guess),
-// so that the gathered sums are bit-identical.  Each cell is then converted
-// once per call instead of once per droplet and stencil corner (the PeleC
-// EOS inversion and the 1 / rho division included).
+// FP64 records (BoxEntry::gr64): rho, T, the velocity and the mass fractions
+// formed with exactly the operations of update_one's plane gather (PeleC:
+// velocity from momentum, T by EY2T from the cell's energy with its T as the
+// guess), so that the gathered sums are bit-identical.  Each cell is then
+// converted once per call instead of once per droplet and stencil corner (the
+// PeleC EOS inversion and the 1 / rho division included).
 template <int NS, bool PELEC>
 __global__ void __launch_bounds__(256) k_gas_records64(const __grid_constant__ KParams P, int b0)
 {
   constexpr int R2 = gas_rec2(NS);
+  __shared__ double2 tile[256][R2 | 1];
   const BoxEntry& B = P.boxes[b0 + blockIdx.y];
-  const int nx = B.state_hi[0] - B.state_lo[0] + 1;
-  const int ny = B.state_hi[1] - B.state_lo[1] + 1;
-  const int nz = B.state_hi[2] - B.state_lo[2] + 1;
-  const int n = nx * ny * nz;
-  for (int c = blockIdx.x * 256 + threadIdx.x; c < n; c += gridDim.x * 256) {
-    const int i = c % nx;
-    const int t = c / nx;
-    const int j = t % ny;
-    const int k = t / ny;
-    const double* q = B.st + ((i + B.state_lo[0] - B.st_lo[0]) + (j + B.state_lo[1] - B.st_lo[1]) * B.st_j32 +
-                              (k + B.state_lo[2] - B.st_lo[2]) * B.st_k32);
+  const double* q;
+  int n;
+  const bool valid = gas_rec_cell(B, q, n);
+  if ((int)blockIdx.x * 256 >= n) {
+    return;
+  }
+  if (valid) {
     const double cur_rho = __ldg(q + P.c_rho * B.st_n32);
-    const double inv_rho = 1. / cur_rho;
     double v[2 * R2];
     v[0] = cur_rho;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      v[5 + s] = __dmul_rn(__ldg(q + (P.c_spec + s) * B.st_n32), inv_rho);
+      v[5 + s] = __ldg(q + (P.c_spec + s) * B.st_n32);
     }
-    if (!PELEC) {
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        v[2 + d] = __ldg(q + (P.c_mom + d) * B.st_n32);
-      }
-      v[1] = __ldg(q + P.c_T * B.st_n32);
-    } else {
+    for (int d = 0; d < 3; ++d) {
+      v[2 + d] = __ldg(q + (P.c_mom + d) * B.st_n32);
+    }
+    v[1] = __ldg(q + P.c_T * B.st_n32);
+    MathFast M;
+    double inv_rho = M.inv(cur_rho);
+    if (M.odd) {
+      inv_rho = 1. / cur_rho;
+    }
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      v[5 + s] = __dmul_rn(v[5 + s], inv_rho);
+    }
+    if (PELEC) {
       double ke = 0.;
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        const double vel = __dmul_rn(__ldg(q + (P.c_mom + d) * B.st_n32), inv_rho);
+        const double vel = __dmul_rn(v[2 + d], inv_rho);
         v[2 + d] = vel;
         ke = __dadd_rn(ke, __dmul_rn(vel, vel) / 2.);
       }
       const double intEng = __dsub_rn(__dmul_rn(__ldg(q + P.c_eng * B.st_n32), inv_rho), ke);
-      v[1] = ey2t<NS>(P.m, intEng, v + 5, __ldg(q + P.c_T * B.st_n32));
+      v[1] = ey2t<NS>(P.m, intEng, v + 5, v[1]);
     }
 #pragma unroll
     for (int s = 5 + NS; s < 2 * R2; ++s) {
       v[s] = 0.;
     }
-    double2* r = B.gr64 + (long long)c * R2;
 #pragma unroll
     for (int m = 0; m < R2; ++m) {
-      r[m] = make_double2(v[2 * m], v[2 * m + 1]);
+      tile[threadIdx.x][m] = make_double2(v[2 * m], v[2 * m + 1]);
     }
   }
+  write_records<R2>(tile, B.gr64, n);
 }
 
 template <int NS, int NF, int BLOCK, bool PELEC = false>

@@ -101,3 +101,27 @@ def test_rare_states_match_the_oracle(oracle):
     pg, _, _ = gpu_run(prob, 2)
     po, _ = oracle_run(oracle, prob, 2)
     assert_bitwise(pg, po)
+
+
+@pytest.mark.parametrize("mode", [capi.PMP_MODE_FP64, capi.PMP_MODE_MIXED])
+def test_gas_records_of_unusual_cells(mode, oracle):
+    """Boxes whose grown cells fill no whole CTA, a third of the cells with a density whose significand
+    is all ones (the division itself instead of the reciprocal), zeros among the species."""
+    prob = W.config2(n=3000, steps=1, ncells=(26, 18, 14), box=(13, 18, 14))
+    rng = np.random.default_rng(4)
+    shape = prob.state[0].shape[1:]
+    odd = rng.random((14 + 6, 18 + 6, 26 + 6)) < 1 / 3
+    for (lo, _), st in zip(prob.boxes, prob.state):
+        i = lo[0]  # the same cells in the overlap of the grown boxes
+        m = odd[:shape[0], :shape[1], i:i + shape[2]]
+        Y = st[4:9] / st[3]
+        st[3] = np.where(m, np.nextafter(0.5, 0.0), st[3])
+        st[4:9] = Y * st[3]
+    pg, _, _ = gpu_run(prob, 1, mode=mode)
+    po, _ = oracle_run(oracle, prob, 1)
+    if mode == capi.PMP_MODE_FP64:
+        assert_bitwise(pg, po)
+    else:  # the mixed form's bound
+        for a, b in zip(pg, po):
+            for row in (capi.PSTATE_T, capi.PSTATE_DIA):
+                assert np.max(np.abs(a["rdata"][row] / b["rdata"][row] - 1)) <= 1e-4
