@@ -11,8 +11,11 @@
 // and by launches when each product, activation and column sum is a kernel
 // of its own: 25 launches and 350 us a step, the split-K weight gradients
 // 45 us each (32 CTAs, FP32 atomics) and the column sums 11 us each (64
-// CTAs).  Now 33 us for the rows and 4 us for the update (256 threads a CTA
-// with 4 x 4 outputs each: 36 us); 42 % of the issue slots, the waits are on
+// CTAs).  Now 29 us for the rows and 4 us for the update (256 threads a CTA
+// with 4 x 4 outputs each: 36 us; weights staged a word at a time and before
+// the tuples are asked for: 31 us).  Of the 55k cycles of a tile, 4k are its
+// loads, 7k each 64 x 64 product with its activation or its derivative, 3.4k
+// each 64 x 64 weight gradient; 42 % of the issue slots, the waits are on
 // shared memory.  Every product's sums run in the order of the reduction index, as
 // an FP32 multiply-add chain; only the gradients' sum over rows is split (64
 // rows, then the CTAs' partials).
@@ -90,6 +93,24 @@ struct TrainSmem {
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float at4(const float4& v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); }
+
+__device__ __forceinline__ void st4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
+
+// batch row r's tuple (want, and there is one)
+__device__ __forceinline__ void load_row(const TrainBatch& T, long long r, float4 (&t)[4], bool want)
+{
+  if (!want || !T.tuples || r >= T.rows) {
+    return;
+  }
+  const long long i = T.random ? (long long)(mix64(T.seed ^ mix64((unsigned long long)T.step * 1315423911ULL + r)) %
+                                             (unsigned long long)T.ntuples)
+                               : T.base + r;
+  const float4* o = reinterpret_cast<const float4*>(T.tuples + i * 16);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    t[q] = __ldg(o + q);
+  }
+}
 
 // rows [r][n] = sum_k A[r][k] W[n][k] of a hidden layer, bias and SiLU: this
 // thread's rows 2 ty + i and columns tx + 16 j (the W rows of 16 neighbouring
@@ -218,14 +239,31 @@ __global__ void __launch_bounds__(kTrainThreads) k_train_rows(const __grid_const
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   // weight gradients: the CTA's halves take half of the rows each
   const int ht = tid & 255, wy = ht >> 4, hr0 = (tid >> 8) * (kTrainRows / 2);
-  for (int i = tid; i < 64 * 64; i += kTrainThreads) {
-    S.W2[(i >> 6) * kTP + (i & 63)] = w[kP_W2 + i];
-    S.W3[(i >> 6) * kTP + (i & 63)] = w[kP_W3 + i];
-    if (i < 64 * 16) {
-      S.W1[(i >> 4) * kTX + (i & 15)] = w[kP_W1 + i];
+  // the first tile's tuples and the weights, 16 bytes a load, are asked for
+  // together
+  const long long tiles = (T.rows + kTrainRows - 1) / kTrainRows;
+  float4 t4[4] = {};
+  load_row(T, (long long)blockIdx.x * kTrainRows + tid, t4, tid < kTrainRows);
+  {
+    static_assert(kTrainThreads == 512, "W2 and W3 twice, W1 half, W4 a quarter");
+    const float4* g = reinterpret_cast<const float4*>(w);
+    float4 a[6];
+    a[0] = __ldg(g + kP_W2 / 4 + tid);
+    a[1] = __ldg(g + kP_W2 / 4 + 512 + tid);
+    a[2] = __ldg(g + kP_W3 / 4 + tid);
+    a[3] = __ldg(g + kP_W3 / 4 + 512 + tid);
+    a[4] = tid < 256 ? __ldg(g + kP_W1 / 4 + tid) : make_float4(0.f, 0.f, 0.f, 0.f);
+    a[5] = tid < 128 ? __ldg(g + kP_W4 / 4 + tid) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int o = (tid >> 4) * kTP + 4 * (tid & 15);
+    st4(S.W2 + o, a[0]);
+    st4(S.W2 + o + 32 * kTP, a[1]);
+    st4(S.W3 + o, a[2]);
+    st4(S.W3 + o + 32 * kTP, a[3]);
+    if (tid < 256) {
+      st4(S.W1 + (tid >> 2) * kTX + 4 * (tid & 3), a[4]);
     }
-    if (i < 8 * 64) {
-      S.W4[(i >> 6) * kTP + (i & 63)] = w[kP_W4 + i];
+    if (tid < 128) {
+      st4(S.W4 + o, a[5]);
     }
   }
   if (tid < 64) {
@@ -241,29 +279,22 @@ __global__ void __launch_bounds__(kTrainThreads) k_train_rows(const __grid_const
   }
   float g2[4][4] = {}, g3[4][4] = {}, g1[4] = {}, g4[2] = {};
   float gb1 = 0.f, gb2 = 0.f, gb3 = 0.f, gb4 = 0.f;
-  const long long tiles = (T.rows + kTrainRows - 1) / kTrainRows;
+  double sq = 0.;
   for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const long long r0 = tile * kTrainRows;
     __syncthreads();  // the previous tile's readers are done
     if (T.tuples) {
       if (tid < kTrainRows) {
-        const long long r = r0 + tid;
         float x[16] = {};
         float ell = 0.f, g = 0.f;
-        if (r < T.rows) {
-          const long long i =
-            T.random ? (long long)(mix64(T.seed ^ mix64((unsigned long long)T.step * 1315423911ULL + r)) %
-                                   (unsigned long long)T.ntuples)
-                     : T.base + r;
-          const float4* o = reinterpret_cast<const float4*>(T.tuples + i * 16);
+        if (r0 + tid < T.rows) {
           float t[16];
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const float4 v = __ldg(o + q);
-            t[4 * q] = v.x;
-            t[4 * q + 1] = v.y;
-            t[4 * q + 2] = v.z;
-            t[4 * q + 3] = v.w;
+            t[4 * q] = t4[q].x;
+            t[4 * q + 1] = t4[q].y;
+            t[4 * q + 2] = t4[q].z;
+            t[4 * q + 3] = t4[q].w;
           }
 #pragma unroll
           for (int k = 0; k < kLearnIn; ++k) {
@@ -277,6 +308,7 @@ __global__ void __launch_bounds__(kTrainThreads) k_train_rows(const __grid_const
             S.Y[tid * 8 + k] = t[kLearnIn + k];
           }
         }
+        load_row(T, r0 + (long long)gridDim.x * kTrainRows + tid, t4, true);  // of the CTA's next tile
         S.bell[tid] = ell;
         S.bg[tid] = g;
 #pragma unroll
@@ -343,7 +375,7 @@ __global__ void __launch_bounds__(kTrainThreads) k_train_rows(const __grid_const
         } else {
           const double a = yp * nrm.y_std[k] + nrm.y_mean[k];
           const double t = S.Y[r * 8 + k] * nrm.y_std[k] + nrm.y_mean[k];
-          atomicAdd(&S.val[k], (a - t) * (a - t));
+          sq += (a - t) * (a - t);
         }
       }
       if (BACK) {
@@ -400,6 +432,12 @@ __global__ void __launch_bounds__(kTrainThreads) k_train_rows(const __grid_const
     gb1 += col_part(S.dH, kTP, tid & 63, tid >> 6);
   }
   if (!BACK) {
+    // the lanes of an output: 4 in a warp
+    sq += __shfl_xor_sync(0xffffffffu, sq, 8);
+    sq += __shfl_xor_sync(0xffffffffu, sq, 16);
+    if ((tid & 31) < kLearnOut) {
+      atomicAdd(&S.val[tid & 31], sq);
+    }
     __syncthreads();
     if (tid < kLearnOut) {
       atomicAdd(&val[tid], S.val[tid]);

@@ -322,17 +322,26 @@ __global__ void __launch_bounds__(256) k_tuple_stats(const float* t, long long n
 // shared memory, and a thread sums one 4 x 4 block of entries over half of
 // them: 8 loads for 16 multiply-adds (one entry a thread converted both
 // factors for every product: 115 us for 131k tuples, bound by the conversions).
+// The CTA adds its two halves and leaves partial sums out[blockIdx.x][...],
+// which k_base_sum adds in order; with atomics from every half and neighbouring
+// blocks' reads 32 bytes apart (two passes over the banks) 71 us, now 43 + 5.
 constexpr int kBaseCols = kBaseTerms + kLearnOut;
 constexpr int kBaseTri = kBaseTerms * (kBaseTerms + 1) / 2;
 constexpr int kBaseEntries = kBaseTri + kBaseTerms * kLearnOut;
 constexpr int kBaseTiles = (kBaseCols + 3) / 4;
 constexpr int kBaseBlocks = kBaseTiles * (kBaseTiles + 1) / 2;
 constexpr int kBaseThreads = (2 * kBaseBlocks + 31) / 32 * 32;
+constexpr int kBasePitch = 4 * kBaseTiles + 2;  // 16-byte rows, 8 of them in different banks
+constexpr int kBaseCtas = 296;
+// place of column k in a staged row: the first pairs of every 4 columns, then
+// the second, so that neighbouring blocks read neighbouring 16 bytes
+__device__ __forceinline__ constexpr int base_at(int k) { return (k & 2) * kBaseTiles + (k >> 2) * 2 + (k & 1); }
 __global__ void __launch_bounds__(kBaseThreads) k_base_normal(const float* t, long long n, long long stride,
                                                               const __grid_constant__ LearnNorm nrm, double* out)
 {
   constexpr int kChunk = 64;  // tuples staged per pass
-  __shared__ double F[kChunk][4 * kBaseTiles];
+  __shared__ __align__(16) double F[kChunk][kBasePitch];
+  static_assert(kChunk * kBasePitch >= 16 * kBaseBlocks, "holds the second half's sums");
   // block (ta, tb), ta <= tb, and half of the rows
   const int half = threadIdx.x / kBaseBlocks;
   int ta = 0, tb = threadIdx.x % kBaseBlocks;
@@ -361,11 +370,11 @@ __global__ void __launch_bounds__(kBaseThreads) k_base_normal(const float* t, lo
       }
 #pragma unroll
       for (int k = 0; k < kBaseTerms; ++k) {
-        row[k] = i < m ? (double)f[k] : 0.;
+        row[base_at(k)] = i < m ? (double)f[k] : 0.;
       }
 #pragma unroll
       for (int k = kBaseTerms; k < 4 * kBaseTiles; ++k) {
-        row[k] = k < kBaseCols ? (double)o[kLearnIn + k - kBaseTerms] : 0.;
+        row[base_at(k)] = k < kBaseCols ? (double)o[kLearnIn + k - kBaseTerms] : 0.;
       }
     }
     __syncthreads();
@@ -375,8 +384,8 @@ __global__ void __launch_bounds__(kBaseThreads) k_base_normal(const float* t, lo
         double x[4], y[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          x[i] = F[r][4 * ta + i];
-          y[i] = F[r][4 * tb + i];
+          x[i] = F[r][base_at(4 * ta + i)];
+          y[i] = F[r][base_at(4 * tb + i)];
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -388,7 +397,17 @@ __global__ void __launch_bounds__(kBaseThreads) k_base_normal(const float* t, lo
       }
     }
   }
-  if (half < 2) {
+  __syncthreads();
+  double* other = &F[0][0] + threadIdx.x % kBaseBlocks;
+  if (half == 1) {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      other[e * kBaseBlocks] = acc[e / 4][e % 4];
+    }
+  }
+  __syncthreads();
+  if (half == 0) {
+    out += (long long)blockIdx.x * kBaseEntries;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
 #pragma unroll
@@ -397,10 +416,33 @@ __global__ void __launch_bounds__(kBaseThreads) k_base_normal(const float* t, lo
         if (a < kBaseTerms && b < kBaseCols && a <= b) {
           const int e = b < kBaseTerms ? a * kBaseTerms - a * (a - 1) / 2 + (b - a)
                                        : kBaseTri + a * kLearnOut + (b - kBaseTerms);
-          atomicAdd(&out[e], acc[i][j]);
+          out[e] = acc[i][j] + other[(4 * i + j) * kBaseBlocks];
         }
       }
     }
+  }
+}
+
+// out[e] = sum of the partial sums part[0 .. n)[e], eight at a time
+__global__ void __launch_bounds__(256) k_base_sum(const double* part, int n, double* out)
+{
+  __shared__ double sums[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
+  double v = 0.;
+  if (e < kBaseEntries) {
+#pragma unroll 4
+    for (int b = w; b < n; b += 8) {
+      v += part[(long long)b * kBaseEntries + e];
+    }
+  }
+  sums[w][lane] = v;
+  __syncthreads();
+  if (w == 0 && e < kBaseEntries) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) {
+      v += sums[k][lane];
+    }
+    out[e] = v;
   }
 }
 
@@ -1546,16 +1588,15 @@ static bool solve_baseline(const double* acc, LearnNorm& nrm);
 static bool fit_baseline(LearnState* L, long long n, LearnNorm& nrm)
 {
   const long long stride = std::max(1LL, (n + 8000000LL - 1) / 8000000LL);
-  double* d_acc = nullptr;
-  if (cudaMalloc(&d_acc, sizeof(double) * kBaseEntries) != cudaSuccess) {
-    return false;
-  }
-  cudaMemset(d_acc, 0, sizeof(double) * kBaseEntries);
+  // the sums and partial sums lie where the training's partial gradients will
+  static_assert(sizeof(double) * kBaseEntries * (kBaseCtas + 1) <= sizeof(float) * kP_N * (size_t)kTrainCtas, "room");
+  double* d_acc = reinterpret_cast<double*>(L->part);
   const long long rows = (n + stride - 1) / stride;
-  k_base_normal<<<(int)std::min<long long>(296, (rows + 63) / 64), kBaseThreads>>>(L->tuples, n, stride, nrm, d_acc);
+  const int ctas = (int)std::min<long long>(kBaseCtas, (rows + 63) / 64);
+  k_base_normal<<<ctas, kBaseThreads>>>(L->tuples, n, stride, nrm, d_acc + kBaseEntries);
+  k_base_sum<<<(kBaseEntries + 31) / 32, 256>>>(d_acc + kBaseEntries, ctas, d_acc);
   std::vector<double> acc(kBaseEntries);
   const bool ok = cudaMemcpy(acc.data(), d_acc, sizeof(double) * kBaseEntries, cudaMemcpyDeviceToHost) == cudaSuccess;
-  cudaFree(d_acc);
   return ok && solve_baseline(acc.data(), nrm);
 }
 
