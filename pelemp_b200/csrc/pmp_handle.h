@@ -14,8 +14,8 @@ namespace pmp {
 constexpr int kBlock = 128;
 // cells of margin in the sort key around a box: droplets that left it by up to
 // this much (a state has 3 ghost cells as a rule) still sort by their own cell.
-// 4 keeps the key of a 32^3 box within 16 bits, two radix passes (8: three,
-// 14 us of a hand-over of 100k droplets)
+// 4 keeps the key of a 32^3 box within 16 bits: 65536 cells to count over
+// (8: twice as many), or two radix passes instead of three
 constexpr int kSortPad = 4;
 
 // Device memory that the handle keeps between calls and exchanges for more

@@ -5,18 +5,19 @@
 // A box's droplets are handed over into staging rows (one 128- or 160-byte
 // row per droplet: the reals, the id and the caller's index) and a sort key
 // each (box, then cell), whatever the caller's layout.  The first operation
-// that needs the droplets packs all boxes at once: one radix sort over every
-// box, one gather of whole rows into the store's component arrays.  A row is
-// whole 32-byte sectors, so the gather in sorted (random) order moves no byte
-// it does not use, where gathering 8 bytes from each of 14-17 component
-// arrays read four times the data; write-back to records goes the same way
-// round.  Staging rows, store, sort arrays and maps stay with the handle
-// between calls (KeptBuffer), so that a caller who hands its droplets over
-// for every call allocates nothing in the steady state.  Measured, hand-over,
-// FP64 update and write-back: 2M two-fuel droplets in 8 boxes 56.0 -> 4.25 ms
-// (3.48 ms of it the update; with a cudaMalloc and cudaFree per array and box
-// the allocator took 46 ms and moving droplets 1.8 ms), 0.78M droplets in 64
-// uneven boxes 72.9 -> 2.37 ms, 8M droplets in the mixed form 79.9 -> 4.89 ms.
+// that needs the droplets packs all boxes at once: one sort over every box (by
+// counting into cells, cell_sort.cuh, or a radix sort), one gather of whole
+// rows into the store's component arrays.  A row is whole 32-byte sectors, so
+// the gather in sorted (random) order moves no byte it does not use, where
+// gathering 8 bytes from each of 14-17 component arrays read four times the
+// data; write-back to records goes the same way round.  Staging rows, store,
+// sort arrays and maps stay with the handle between calls (KeptBuffer), so
+// that a caller who hands its droplets over for every call allocates nothing
+// in the steady state.  Measured, hand-over, update and write-back: 2M
+// two-fuel droplets in 8 boxes, FP64, 56.0 -> 2.82 ms (2.15 ms of it the
+// update; with a cudaMalloc and cudaFree per array and box the allocator took
+// 46 ms and moving droplets 1.8 ms), 0.78M droplets in 64 uneven boxes
+// 72.9 -> 2.24 ms, 8M droplets in the mixed form 79.9 -> 4.31 ms.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
