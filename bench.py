@@ -278,19 +278,19 @@ KERNEL = {"fp64": "spray_update_fp64<5,2,128>", "mixed": "spray_update_mixed<5,2
 # x this.  The mixed and learned kernels move less than the 184 algorithmic
 # bytes per droplet: their gathers read the FP32 gas records (written by a
 # separate pass) instead of the FP64 state.
-DRAM_BYTES_PER_DROPLET = {"fp64": 175.6, "mixed": 158.3, "learned": 153.6}
+DRAM_BYTES_PER_DROPLET = {"fp64": 164.8, "mixed": 157.8, "learned": 153.4}
 # Pipe utilisation of each form's update kernel in the same captures (% of
 # the pipe's peak while the SM is active: sm__inst_executed_pipe_*; issue:
 # smsp__issue_active), and its measured pipe peaks: the compute side of the
 # roofline.  The kernels are bound by instruction issue and latency, not by
 # one pipe.
 PIPE_PCT = {
-    "mixed": {"issue": 60.23, "xu": 39.97, "fma": 23.11, "alu": 23.52, "fp64": 11.94, "lsu": 16.02,
+    "mixed": {"issue": 65.85, "xu": 43.23, "fma": 27.25, "alu": 28.24, "fp64": 9.96, "lsu": 14.73,
               "tensor": 0.0},
-    "fp64": {"issue": 47.17, "xu": 13.48, "fma": 6.19, "alu": 16.31, "fp64": 32.35, "lsu": 9.86,
+    "fp64": {"issue": 52.83, "xu": 7.63, "fma": 9.41, "alu": 22.16, "fp64": 45.30, "lsu": 9.79,
              "tensor": 0.0},
-    "learned": {"issue": 47.10, "xu": 38.67, "fma": 16.86, "alu": 19.74, "fp64": 7.84, "lsu": 10.02,
-                "tensor": 5.41},
+    "learned": {"issue": 48.51, "xu": 40.47, "fma": 18.03, "alu": 20.75, "fp64": 6.07, "lsu": 10.97,
+                "tensor": 5.91},
 }
 
 
@@ -300,10 +300,7 @@ def compute_roofline(form, peaks):
     out = {"pipes_pct_of_peak": PIPE_PCT.get(form),
            "pipes_source": "ncu capture of the same kernel: one MKD launch of 2M droplets at config-2 density "
                            "(sm__inst_executed_pipe_*.avg.pct_of_peak_sustained_active, "
-                           "smsp__issue_active, sm__pipe_tensor_cycles_active), taken before the FP64 "
-                           "divisions of the FP32 forms' state update were cut and the mixed form's B_T "
-                           "fixed point stopped at its noise floor (the mixed MKD launch is 17 % shorter "
-                           "since)"}
+                           "smsp__issue_active, sm__pipe_tensor_cycles_active)"}
     if peaks is not None:
         out["peaks"] = peaks
         out["peaks_source"] = ("pmp_measure_peaks on this GPU: loop kernels of independent DFMA, FFMA and "

@@ -11,7 +11,7 @@
 // dependent chain alone (57 elementary functions and 60 divisions per
 // sub-cycle, 7300 instructions a droplet of which 34 % FP64; the warps waited
 // 3.3 cycles per issue on fixed latencies).  Measured, update kernel of 2M
-// two-fuel droplets, 4 sub-cycles: 3.48 -> 2.19 ms (5500 instructions, 41 %
+// two-fuel droplets, 4 sub-cycles: 3.48 -> 2.15 ms (5200 instructions, 41 %
 // FP64); 100k one-fuel droplets 81 -> 36 us; 800 droplets (the latency of one)
 // 29 -> 14 us.  Species loops left rolled (mass fractions in shared memory,
 // code 8 % smaller) measured 4 % slower.
