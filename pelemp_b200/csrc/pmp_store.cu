@@ -717,13 +717,14 @@ void store_attach(pmp_spray* h, long long n)
 // again: `zero_cells` says how many are (0 while they are in use).
 int count_cells(pmp_spray* h, long long cells, cudaStream_t st)
 {
-  const void* before = h->counts.p;
+  const KeptBuffer before = h->counts;
   const int rc = keep(h, h->counts, sizeof(unsigned) * (size_t)cells);
   if (rc != PMP_OK) {
     h->zero_cells = 0;
     return rc;
   }
-  if (h->counts.p != before || h->zero_cells < cells) {
+  // another buffer may lie at the old one's address: its size differs
+  if (h->counts.p != before.p || h->counts.bytes != before.bytes || h->zero_cells < cells) {
     h->zero_cells = 0;
     PMP_TRY(h, cudaMemsetAsync(h->counts.p, 0, sizeof(unsigned) * (size_t)cells, st));
   }

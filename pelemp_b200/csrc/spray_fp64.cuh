@@ -13,7 +13,8 @@
 //
 // Exactness: this file is compiled with -fmad=false and evaluates every
 // expression in the reference's order with the project math library, the
-// same functions the CPU oracle uses.  Each droplet's new state and its
+// same functions the CPU oracle uses, or with math_fast64.cuh, which returns
+// the same bits.  Each droplet's new state and its
 // deposit increments are therefore bit-identical to the oracle's; only the
 // order in which atomics add the increments into a cell differs.
 #pragma once

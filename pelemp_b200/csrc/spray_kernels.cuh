@@ -912,7 +912,7 @@ __device__ __forceinline__ void prefetch_droplet(const KParams& P, long long s)
 }
 
 // capacities of the gather tiles, in cells: FP64 records (the FP64 forms,
-// 5 CTAs per SM) and FP32 records (the mixed form, 7 CTAs per SM)
+// 4 CTAs per SM) and FP32 records (the mixed form, 7 CTAs per SM)
 #ifndef PMP_TILE64_CELLS
 #define PMP_TILE64_CELLS 192
 #endif
