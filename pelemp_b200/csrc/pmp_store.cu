@@ -649,6 +649,21 @@ struct Transit {
   }
 };
 
+// Kernels that a hand-over has launched on the legacy stream and not waited
+// for.  Whatever way the call returns, they have run by then: the next
+// operation packs on its own stream, which may be one that the legacy stream
+// does not order.
+struct InFlight {
+  bool launched = false;
+  cudaError_t wait()
+  {
+    const cudaError_t e = launched ? cudaStreamSynchronize(nullptr) : cudaSuccess;
+    launched = false;
+    return e;
+  }
+  ~InFlight() { wait(); }
+};
+
 // columns of nreal components of n doubles, then n ids, in one buffer
 Columns columns_in(void* base, int nreal, long long n)
 {
@@ -941,7 +956,9 @@ int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
   cudaSetDevice(h->device);
   pmp::quiesce(h);
   int rc = PMP_OK;
+  InFlight flight;
   if (h->packed) {
+    flight.launched = true;
     rc = unpack(h, box);
     if (rc != PMP_OK) {
       return rc;
@@ -957,6 +974,7 @@ int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
   } else if (s.n > 0 && narrow_keys(h)) {
     // given up: the key above every box's
     const KeyOut k = key_out(h, 0);
+    flight.launched = true;
     k_fill_keys<<<nblk(s.n, 256), 256>>>(k.keys, k.idx, s.row, s.n, 0xffffffffu);
     PMP_TRY(h, cudaGetLastError());
   }
@@ -971,12 +989,14 @@ int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
     return set_err(h, PMP_ERR_INVALID, "2^31 droplets or more in one box", box);
   }
   if (n == 0) {
+    PMP_TRY(h, flight.wait());
     h->box_set[box] = true;
     return PMP_OK;
   }
   if (p->layout != PMP_LAYOUT_SOA && p->layout != PMP_LAYOUT_AOS) {
     return set_err(h, PMP_ERR_INVALID, "unknown particle layout");
   }
+  flight.launched = true;
   rc = stage_room(h, n);
   if (rc != PMP_OK) {
     return rc;
@@ -1059,7 +1079,7 @@ int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
   }
   PMP_TRY(h, cudaGetLastError());
   // the caller's arrays are read when the call returns
-  PMP_TRY(h, cudaStreamSynchronize(nullptr));
+  PMP_TRY(h, flight.wait());
   s.n = n;
   s.row = h->staged_rows;
   h->staged_rows += n;
