@@ -615,6 +615,11 @@ int pmp_measure_peaks(int device, double* fp64_tflops, double* fp32_tflops,
 int pmp_debug_math(int fn, const double* x, const double* y, long long n,
                    double* fast, double* plain, int* odd);
 
+/* Check of what a call without memory leaves behind (no counterpart in the
+ * reference): the k-th allocation of the droplet store from now on fails
+ * (k = 0: none). */
+int pmp_spray_debug_fail_alloc(pmp_spray* h, int k);
+
 #ifdef __cplusplus
 }
 #endif

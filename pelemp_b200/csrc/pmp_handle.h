@@ -127,7 +127,7 @@ struct pmp_spray {
   int* ids = nullptr;
   long long* perm() const { return static_cast<long long*>(perm_b.p); }  // slot -> caller's index in its box
   std::vector<long long> box_begin;
-  int ncta = 0;
+  int ncta = 0;  // CTAs of the map below; < 0: the map is to be built again
   int* d_cta_box = nullptr;
   long long* d_cta_start = nullptr;
   long long* d_box_begin = nullptr;
@@ -152,6 +152,12 @@ struct pmp_spray {
   cudaStream_t last_stream = nullptr;
   cudaEvent_t ev_done = nullptr;
   bool pending = false;
+  // the packing of the droplets is enqueued on pack_stream, up to ev_pack, and
+  // the host has not waited for it since
+  bool packing = false;
+  cudaStream_t pack_stream = nullptr;
+  cudaEvent_t ev_pack = nullptr;
+  int fail_alloc = 0;  // pmp_spray_debug_fail_alloc
   // the mixed form's FP64 list kernel runs on `side` beside the mixed kernel
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_sel = nullptr;
@@ -223,6 +229,7 @@ int run_update(
 // pack the staged droplets if needed, on st
 int ensure_packed(pmp_spray* h, cudaStream_t st);
 int keep(pmp_spray* h, KeptBuffer& b, size_t bytes);
+cudaError_t store_alloc(pmp_spray* h, void** p, size_t bytes);
 size_t store_bytes(const pmp_spray* h, long long n);
 int count_cells(pmp_spray* h, long long cells, cudaStream_t st);
 // soa and ids for n droplets in the store buffer

@@ -988,6 +988,10 @@ int update_host_overlapped(
 
 void pmp::quiesce(pmp_spray* h)
 {
+  if (h->packing) {
+    cudaEventSynchronize(h->ev_pack);
+    h->packing = false;
+  }
   if (h->pending && h->ev_done) {
     cudaEventSynchronize(h->ev_done);
     h->pending = false;
@@ -1012,6 +1016,7 @@ int pmp::sync_status(pmp_spray* h)
   PMP_CUDA(h, cudaMemsetAsync(h->d_status, 0, sizeof(DevStatus), st));
   PMP_CUDA(h, cudaStreamSynchronize(st));
   h->pending = false;
+  h->packing = h->packing && h->pack_stream != st;
   const long long T = h->total;
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, h->ev0, h->ev1) == cudaSuccess) {
@@ -1065,7 +1070,7 @@ int pmp::prepare_update(
 int pmp::install_rebinned(pmp_spray* h, const std::vector<long long>& box_begin, cudaStream_t st)
 {
   h->box_begin = box_begin;
-  h->ncta = 0;
+  h->ncta = -1;
   pmp::batch_reset(h);
   return build_cta_map(h, st);
 }
@@ -1207,7 +1212,8 @@ int pmp_spray_create(const pmp_spray_config* cfg, pmp_spray** out)
       cudaHostAlloc(&h->err_host, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
       cudaHostGetDevicePointer(&h->err_dev, h->err_host, 0) != cudaSuccess ||
       cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess ||
-      cudaEventCreateWithFlags(&h->ev_done, cudaEventDisableTiming) != cudaSuccess) {
+      cudaEventCreateWithFlags(&h->ev_done, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->ev_pack, cudaEventDisableTiming) != cudaSuccess) {
     pmp_spray_destroy(h);
     return PMP_ERR_CUDA;
   }
@@ -1258,6 +1264,9 @@ int pmp_spray_destroy(pmp_spray* h)
   cudaFreeHost(h->err_host);
   if (h->ev_done) {
     cudaEventDestroy(h->ev_done);
+  }
+  if (h->ev_pack) {
+    cudaEventDestroy(h->ev_pack);
   }
   if (h->ev0) {
     cudaEventDestroy(h->ev0);

@@ -487,14 +487,14 @@ int stage_room(pmp_spray* h, long long n)
   // so that many boxes exchange the buffer a few times only
   size_t rows = (size_t)(live > 0 ? 2 * (live + n) : n);
   KeptBuffer nw, nk;
-  if (cudaMalloc(&nw.p, rows * rb) != cudaSuccess) {
+  if (store_alloc(h, &nw.p, rows * rb) != cudaSuccess) {
     cudaGetLastError();
     rows = (size_t)(live + n);
-    PMP_TRY(h, cudaMalloc(&nw.p, rows * rb));
+    PMP_TRY(h, store_alloc(h, &nw.p, rows * rb));
   }
   nw.bytes = rows * rb;
   nk.bytes = rows * kb;
-  cudaError_t e = cudaMalloc(&nk.p, nk.bytes);
+  cudaError_t e = store_alloc(h, &nk.p, nk.bytes);
   const KeptBuffer old_rows = h->spare, old_keys = h->row_keys;
   const KeyOut from = key_out(h, 0);
   h->row_keys = nk;
@@ -703,6 +703,17 @@ size_t sort_bytes(long long m, int end_bit)
 
 }  // namespace
 
+// Every allocation of the store; the fail_alloc-th from now fails as cudaMalloc
+// does without memory.
+cudaError_t store_alloc(pmp_spray* h, void** p, size_t bytes)
+{
+  if (h->fail_alloc > 0 && --h->fail_alloc == 0) {
+    *p = nullptr;
+    return cudaErrorMemoryAllocation;
+  }
+  return cudaMalloc(p, bytes);
+}
+
 // A kept buffer of at least `bytes`: exchanged when too small, and when it is
 // large and mostly unused (its content is not kept).
 int keep(pmp_spray* h, KeptBuffer& b, size_t bytes)
@@ -714,7 +725,7 @@ int keep(pmp_spray* h, KeptBuffer& b, size_t bytes)
   cudaFree(b.p);
   b = KeptBuffer{};
   const size_t want = std::max(bytes, (size_t)256);
-  PMP_TRY(h, cudaMalloc(&b.p, want));
+  PMP_TRY(h, store_alloc(h, &b.p, want));
   b.bytes = want;
   return PMP_OK;
 }
@@ -789,7 +800,8 @@ void store_free(pmp_spray* h)
 }
 
 // Box offsets and the CTA -> (box, first slot) map of the packed droplets,
-// and the fallback list, enqueued on st.
+// and the fallback list, enqueued on st.  When it fails, the map counts as not
+// built (ncta < 0), and the next ensure_packed builds it.
 int build_cta_map(pmp_spray* h, cudaStream_t st)
 {
   const int nb = (int)h->boxes.size();
@@ -798,11 +810,12 @@ int build_cta_map(pmp_spray* h, cudaStream_t st)
     const long long n = h->box_begin[b + 1] - h->box_begin[b];
     first[b + 1] = first[b] + (int)((n + kBlock - 1) / kBlock);
   }
-  h->ncta = first[nb];
+  const int ncta = first[nb];
+  h->ncta = -1;
   // {box_begin[nb + 1], first[nb + 1]} uploaded, then cta_start, cta_box
   const size_t bb = sizeof(long long) * (nb + 1), fb = align256(sizeof(int) * (nb + 1));
-  const size_t cs = align256(bb + fb), cb = align256(sizeof(long long) * h->ncta);
-  int rc = keep(h, h->map_b, cs + cb + sizeof(int) * (size_t)h->ncta);
+  const size_t cs = align256(bb + fb), cb = align256(sizeof(long long) * ncta);
+  int rc = keep(h, h->map_b, cs + cb + sizeof(int) * (size_t)ncta);
   if (rc == PMP_OK) {
     rc = keep(h, h->fb_b, sizeof(long long) * (size_t)std::max(h->total, 1LL));
   }
@@ -817,39 +830,23 @@ int build_cta_map(pmp_spray* h, cudaStream_t st)
   h->d_box_begin = reinterpret_cast<long long*>(base);
   h->d_cta_start = reinterpret_cast<long long*>(base + cs);
   h->d_cta_box = reinterpret_cast<int*>(base + cs + cb);
-  if (h->ncta > 0) {
-    k_cta_map<<<nblk(h->ncta, 256), 256, 0, st>>>(h->d_box_begin, reinterpret_cast<const int*>(base + bb), nb, h->ncta,
-                                                  h->d_cta_box, h->d_cta_start);
+  if (ncta > 0) {
+    k_cta_map<<<nblk(ncta, 256), 256, 0, st>>>(h->d_box_begin, reinterpret_cast<const int*>(base + bb), nb, ncta,
+                                               h->d_cta_box, h->d_cta_start);
     PMP_TRY(h, cudaGetLastError());
   }
+  h->ncta = ncta;
   h->packed = true;
   return PMP_OK;
 }
 
-// The staged boxes packed into the store on st.  No work of the handle is
-// pending (whoever staged droplets waited for it).
-int ensure_packed(pmp_spray* h, cudaStream_t st)
+namespace {
+
+// The staged boxes packed into the store, enqueued on st.  No work of the
+// handle is pending (whoever staged droplets waited for it).
+int pack(pmp_spray* h, cudaStream_t st)
 {
-  if (h->packed) {
-    return PMP_OK;
-  }
   const int nb = (int)h->boxes.size();
-  for (int b = 0; b < nb; ++b) {
-    if (!h->box_set[b]) {
-      return set_err(h, PMP_ERR_INVALID, "set_particles was not called for every box", b);
-    }
-  }
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  PMP_TRY(h, cudaStreamIsCapturing(st, &cap));
-  const bool capturing = cap != cudaStreamCaptureStatusNone;
-  if (capturing) {
-    // packing is not part of the caller's graph: it runs at once, beside the
-    // capture, where the capture's mode lets a call allocate
-    void* p = nullptr;
-    PMP_TRY(h, cudaMalloc(&p, 256));
-    cudaFree(p);
-    st = nullptr;
-  }
   h->box_begin.assign(nb + 1, 0);
   for (int b = 0; b < nb; ++b) {
     h->box_begin[b + 1] = h->box_begin[b] + h->staged[b].n;
@@ -928,14 +925,58 @@ int ensure_packed(pmp_spray* h, cudaStream_t st)
   }
   h->staged_rows = 0;
   h->counted = h->ranked = false;
+  return PMP_OK;
+}
+
+}  // namespace
+
+// The droplets packed, and their map built, in the order of st.
+int ensure_packed(pmp_spray* h, cudaStream_t st)
+{
+  for (int b = 0; !h->packed && b < (int)h->boxes.size(); ++b) {
+    if (!h->box_set[b]) {
+      return set_err(h, PMP_ERR_INVALID, "set_particles was not called for every box", b);
+    }
+  }
+  const bool built = h->packed && h->ncta >= 0;
+  if (built && !(h->packing && st != h->pack_stream)) {
+    return PMP_OK;
+  }
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  PMP_TRY(h, cudaStreamIsCapturing(st, &cap));
+  const bool capturing = cap != cudaStreamCaptureStatusNone;
+  if (built) {
+    // packed by a call on another stream, which may have been refused after that
+    if (capturing) {
+      quiesce(h);  // a capture takes no event from outside
+      return PMP_OK;
+    }
+    PMP_TRY(h, cudaStreamWaitEvent(st, h->ev_pack, 0));
+    return PMP_OK;
+  }
+  if (capturing) {
+    // packing is not part of the caller's graph: it runs at once, beside the
+    // capture, where the capture's mode lets a call allocate
+    void* p = nullptr;
+    PMP_TRY(h, cudaMalloc(&p, 256));
+    cudaFree(p);
+    st = nullptr;
+  }
+  const int rc = h->packed ? build_cta_map(h, st) : pack(h, st);
+  if (rc != PMP_OK) {
+    // no kernel of it may still read rows that the caller replaces next
+    cudaStreamSynchronize(st);
+    cudaGetLastError();
+    return rc;
+  }
   if (capturing) {
     PMP_TRY(h, cudaStreamSynchronize(st));
     return PMP_OK;
   }
   // entry points on other streams wait for the store
-  PMP_TRY(h, cudaEventRecord(h->ev_done, st));
-  h->last_stream = st;
-  h->pending = true;
+  PMP_TRY(h, cudaEventRecord(h->ev_pack, st));
+  h->pack_stream = st;
+  h->packing = true;
   return PMP_OK;
 }
 
@@ -1177,6 +1218,15 @@ int pmp_spray_get_particles(pmp_spray* h, int box, pmp_particles* out)
   }
   // the droplets are there when the call returns
   PMP_TRY(h, cudaStreamSynchronize(nullptr));
+  return PMP_OK;
+}
+
+int pmp_spray_debug_fail_alloc(pmp_spray* h, int k)
+{
+  if (!h || k < 0) {
+    return PMP_ERR_INVALID;
+  }
+  h->fail_alloc = k;
   return PMP_OK;
 }
 

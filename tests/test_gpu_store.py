@@ -7,7 +7,9 @@ import numpy as np
 import pytest
 
 from pelemp_b200 import capi, spray
+from pelemp_b200 import workloads as W
 from pelemp_b200.spray import from_problem
+from tests.gpu_util import assert_bitwise, device_sources, device_state, gpu_run
 from tests.test_gpu_handover import droplets, level
 
 pytestmark = pytest.mark.gpu
@@ -64,3 +66,97 @@ def test_emptied_box_and_another_stream(case, counts):
     assert sp.est_timestep(0.5, stream=side.cuda_stream) == expected_dt(prob, drs)
     torch.cuda.synchronize()
     check(sp, drs)
+
+
+@pytest.mark.parametrize("mode", [capi.PMP_MODE_FP64, capi.PMP_MODE_MIXED])
+def test_update_after_a_refused_one_on_another_stream(mode):
+    """An update is refused after it packed the droplets on a held stream; the next one runs on another."""
+    import torch
+    prob = W.config2(n=20_000, steps=1, ncells=(32, 16, 16), box=(16, 16, 16))
+    want, _, ref = gpu_run(prob, 1, mode=mode)
+    sp = from_problem(prob, mode=mode)
+    st_keep, st_v = device_state(prob)
+    held, other = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(held):
+        torch.cuda._sleep(HOLD)
+    for do_move in (1, 0):
+        src, src_v = device_sources(prob)
+        torch.cuda.current_stream().synchronize()
+        if do_move:
+            with pytest.raises(spray.SprayError):  # the views do not cover this many ghost cells
+                sp.update_particles(st_v, src_v, prob.flow_dt, 0.0, prob.state_ghosts + 1, prob.source_ghosts, 0, 0,
+                                    1, prob.spray_cfl_lev, held.cuda_stream)
+        sp.update_particles(st_v, src_v, prob.flow_dt, 0.0, prob.state_ghosts, prob.source_ghosts, 0, 0, do_move,
+                            prob.spray_cfl_lev, other.cuda_stream)
+    assert_bitwise([sp.get_particles(b) for b in range(len(prob.boxes))], want)
+    del st_keep, ref
+
+
+def fail_alloc(sp, k):
+    assert spray.lib().pmp_spray_debug_fail_alloc(sp._h, k) == capi.PMP_OK
+
+
+def by_cell(prob, drs):
+    """The droplets of `drs` by new box, then by cell, in their order (boxes of 16^3 cells along x)."""
+    pos, rd, ids = (np.concatenate([d[i] for d in drs], axis=-1) for i in range(3))
+    c = np.floor(pos * (1.0 / prob.dx)[:, None]).astype(np.int64)
+    key = ((c[0] // 16 * 16 + c[2]) * 16 + c[1]) * 16 + c[0] % 16
+    order = np.argsort(key, kind="stable")
+    return [(pos[:, o], rd[:, o], ids[o]) for o in (order[key[order] // 4096 == b] for b in range(len(prob.boxes)))]
+
+
+@pytest.mark.parametrize("n", [100, 60_000])
+@pytest.mark.parametrize("call", ["set", "pack", "redistribute"])
+def test_allocation_fails(call, n):
+    """Each allocation of a call fails in turn, on a held stream: the call succeeds without it or reports
+    an error, and after that the droplets are handed over again, packed and re-binned as if nothing had
+    happened."""
+    import torch
+    prob = level(2)
+    (lo, _), (_, hi) = prob.boxes
+    side = torch.cuda.Stream()
+    failed = 0
+    for k in range(1, 12):
+        rng = np.random.default_rng(k)
+        sp = from_problem(prob, set_droplets=False)
+        # box 0 is given droplets of both boxes, so that re-binning changes the boxes' counts
+        drs = [droplets(rng, n, 2, lo, hi, prob.dx[0]), droplets(rng, 0, 2, lo, hi, prob.dx[0])]
+        if call == "set":
+            fail_alloc(sp, k)
+        try:
+            for b, d in enumerate(drs):
+                sp.set_particles(b, *d)
+        except spray.SprayError:
+            failed += 1
+            fail_alloc(sp, 0)
+            for b, d in enumerate(drs):
+                sp.set_particles(b, *d)
+        fail_alloc(sp, k if call == "pack" else 0)
+        if call == "pack":
+            with torch.cuda.stream(side):
+                torch.cuda._sleep(HOLD // 10)
+            try:
+                sp.est_timestep(0.5, stream=side.cuda_stream)
+            except spray.SprayError:
+                failed += 1
+                fail_alloc(sp, 0)
+                drs[0] = droplets(rng, n, 2, lo, hi, prob.dx[0])
+                sp.set_particles(0, *drs[0])
+        check(sp, drs)
+        if call == "redistribute":
+            sp.est_timestep(0.5)
+        fail_alloc(sp, k if call == "redistribute" else 0)
+        try:
+            sp.redistribute(stream=side.cuda_stream)
+        except spray.SprayError:
+            assert call == "redistribute"
+            failed += 1
+            fail_alloc(sp, 0)
+            assert sp.est_timestep(0.5) == expected_dt(prob, drs)
+            sp.redistribute()
+        fail_alloc(sp, 0)
+        check(sp, by_cell(prob, drs))
+        assert sp.est_timestep(0.5, stream=side.cuda_stream) == expected_dt(prob, drs)
+        sp.close()
+    assert failed > 0
