@@ -230,8 +230,9 @@ int run_update(
 int ensure_packed(pmp_spray* h, cudaStream_t st);
 int keep(pmp_spray* h, KeptBuffer& b, size_t bytes);
 cudaError_t store_alloc(pmp_spray* h, void** p, size_t bytes);
+cudaError_t try_keep(pmp_spray* h, KeptBuffer& b, size_t bytes);
 size_t store_bytes(const pmp_spray* h, long long n);
-int count_cells(pmp_spray* h, long long cells, cudaStream_t st);
+int count_cells(pmp_spray* h, long long cells, cudaStream_t st, bool* have);
 // soa and ids for n droplets in the store buffer
 void store_attach(pmp_spray* h, long long n);
 void store_layout(pmp_spray* h);

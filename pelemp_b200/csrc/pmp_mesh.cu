@@ -1047,20 +1047,19 @@ static int rebin_sort(pmp_spray* h, cudaStream_t st, long long n, int nb, int sh
   return read_bounds(h, st, d_begin, begin);
 }
 
-// The same by counting (cell_sort.cuh); *crowded: a cell holds too many
-// droplets, and nothing was sorted.
+// The same by counting (cell_sort.cuh); *sorted: false when a cell holds too
+// many droplets, or there is no memory for the counts, and nothing was sorted.
 static int rebin_count(pmp_spray* h, cudaStream_t st, long long n, int nb, int shift, long long cells,
-                       std::vector<long long>& begin, const void** order, const long long** d_bounds, bool* crowded)
+                       std::vector<long long>& begin, const void** order, const long long** d_bounds, bool* sorted)
 {
   auto up = [](size_t b) { return align256(b); };
   const CellSortLayout L = cell_sort_layout(cells, n);
   const size_t ranks = L.total + up(sizeof(unsigned) * n), bounds = ranks + up(sizeof(int) * n);
   const size_t boxes = bounds + up(sizeof(long long) * (nb + 1));
-  int rc = keep(h, h->sort_scratch, boxes + sizeof(pmp_box) * nb);
-  if (rc == PMP_OK) {
-    rc = count_cells(h, cells, st);
-  }
-  if (rc != PMP_OK) {
+  *sorted = false;
+  bool have = try_keep(h, h->sort_scratch, boxes + sizeof(pmp_box) * nb) == cudaSuccess;
+  int rc = have ? count_cells(h, cells, st, &have) : PMP_OK;
+  if (rc != PMP_OK || !have) {
     return rc;
   }
   char* base = static_cast<char*>(h->sort_scratch.p);
@@ -1080,7 +1079,7 @@ static int rebin_count(pmp_spray* h, cudaStream_t st, long long n, int nb, int s
     return rc;
   }
   h->zero_cells = cells;
-  *crowded = *h->crowded() != 0;
+  *sorted = *h->crowded() == 0;
   *order = base + L.order;
   *d_bounds = d_begin;
   return PMP_OK;
@@ -1128,11 +1127,11 @@ extern "C" int pmp_spray_redistribute(pmp_spray* h, long long* removed, void* st
   const void* order = nullptr;
   const long long* d_begin = nullptr;
   const long long cells = padded_cells(nb, shift);
-  bool crowded = true;
+  bool sorted = false;
   if (narrow && counting_pays(cells, n)) {
-    rc = rebin_count(h, st, n, nb, shift, cells, begin, &order, &d_begin, &crowded);
+    rc = rebin_count(h, st, n, nb, shift, cells, begin, &order, &d_begin, &sorted);
   }
-  if (rc == PMP_OK && crowded) {
+  if (rc == PMP_OK && !sorted) {
     rc = narrow ? rebin_sort<unsigned, int>(h, st, n, nb, shift, end_bit, begin, &order, &d_begin)
                 : rebin_sort<unsigned long long, long long>(h, st, n, nb, shift, end_bit, begin, &order, &d_begin);
   }

@@ -716,17 +716,26 @@ cudaError_t store_alloc(pmp_spray* h, void** p, size_t bytes)
 
 // A kept buffer of at least `bytes`: exchanged when too small, and when it is
 // large and mostly unused (its content is not kept).
-int keep(pmp_spray* h, KeptBuffer& b, size_t bytes)
+cudaError_t try_keep(pmp_spray* h, KeptBuffer& b, size_t bytes)
 {
   const bool idle = b.bytes > ((size_t)256 << 20) && b.bytes / 4 > bytes;
   if (b.p && b.bytes >= bytes && !idle) {
-    return PMP_OK;
+    return cudaSuccess;
   }
   cudaFree(b.p);
   b = KeptBuffer{};
   const size_t want = std::max(bytes, (size_t)256);
-  PMP_TRY(h, store_alloc(h, &b.p, want));
+  const cudaError_t e = store_alloc(h, &b.p, want);
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // reported here, not by the next call
+    return e;
+  }
   b.bytes = want;
+  return cudaSuccess;
+}
+int keep(pmp_spray* h, KeptBuffer& b, size_t bytes)
+{
+  PMP_TRY(h, try_keep(h, b, bytes));
   return PMP_OK;
 }
 
@@ -740,14 +749,15 @@ void store_attach(pmp_spray* h, long long n)
 }
 
 // Zeroed counts of `cells` cells, for a sort on st, which leaves them zero
-// again: `zero_cells` says how many are (0 while they are in use).
-int count_cells(pmp_spray* h, long long cells, cudaStream_t st)
+// again: `zero_cells` says how many are (0 while they are in use).  *have:
+// false when there is no memory for them (the radix sort needs none).
+int count_cells(pmp_spray* h, long long cells, cudaStream_t st, bool* have)
 {
   const KeptBuffer before = h->counts;
-  const int rc = keep(h, h->counts, sizeof(unsigned) * (size_t)cells);
-  if (rc != PMP_OK) {
+  *have = try_keep(h, h->counts, sizeof(unsigned) * (size_t)cells) == cudaSuccess;
+  if (!*have) {
     h->zero_cells = 0;
-    return rc;
+    return PMP_OK;
   }
   // another buffer may lie at the old one's address: its size differs
   if (h->counts.p != before.p || h->counts.bytes != before.bytes || h->zero_cells < cells) {
@@ -867,8 +877,9 @@ int pack(pmp_spray* h, cudaStream_t st)
       const long long m = h->staged_rows;
       const int bits = m == n ? end_bit : 32;
       const long long cells = sort_cells(h);
-      const bool by_cell = m == n && cell_sorted(h, m);
-      rc = keep(h, h->sort_scratch, by_cell ? cell_sort_layout(cells, m).total : sort_bytes<unsigned, int>(m, bits));
+      const bool by_cell = m == n && cell_sorted(h, m) &&
+                           try_keep(h, h->sort_scratch, cell_sort_layout(cells, m).total) == cudaSuccess;
+      rc = by_cell ? PMP_OK : keep(h, h->sort_scratch, sort_bytes<unsigned, int>(m, bits));
       const KeyOut k = key_out(h, 0);
       const int* order = nullptr;
       if (rc == PMP_OK && by_cell) {
@@ -1051,7 +1062,7 @@ int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
     h->ranked = false;
     h->counted = count_first(h, n);
     if (h->counted) {
-      rc = count_cells(h, sort_cells(h), nullptr);
+      rc = count_cells(h, sort_cells(h), nullptr, &h->counted);
       if (rc != PMP_OK) {
         h->counted = false;
         return rc;

@@ -160,3 +160,33 @@ def test_allocation_fails(call, n):
         assert sp.est_timestep(0.5, stream=side.cuda_stream) == expected_dt(prob, drs)
         sp.close()
     assert failed > 0
+
+
+def on_device(d):
+    import torch
+    return tuple(torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in d)
+
+
+@pytest.mark.parametrize("call,k,counts", [
+    ("set", 3, (60_000, 40)),  # the counts, after the rows and their keys
+    ("pack", 3, (60_000, 40)),  # the passes' arrays, after the store and the caller's indices
+    ("redistribute", 1, (40, 60_000)),  # not counted before: the passes' arrays,
+    ("redistribute", 2, (40, 60_000)),  # the counts
+])
+def test_no_memory_to_count_with(call, k, counts):
+    """The sort by counting is a choice: a call for whose counts or passes there is no memory sorts
+    without them."""
+    prob = level(2)
+    rng = np.random.default_rng(1)
+    drs = [droplets(rng, n, 2, lo, hi, prob.dx[0]) for n, (lo, hi) in zip(counts, prob.boxes)]
+    sp = from_problem(prob, set_droplets=False)
+    for _ in range(2):
+        fail_alloc(sp, k if call == "set" else 0)
+        for b, d in enumerate(drs):
+            sp.set_particles(b, *on_device(d))
+        fail_alloc(sp, k if call == "pack" else 0)
+        assert sp.est_timestep(0.5) == expected_dt(prob, drs)
+        check(sp, drs)
+        fail_alloc(sp, k if call == "redistribute" else 0)
+        assert sp.redistribute() == 0
+        check(sp, by_cell(prob, drs))
