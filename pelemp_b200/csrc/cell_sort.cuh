@@ -32,7 +32,8 @@ constexpr int kSumCells = 4096;        // cells of a CTA of the first two passes
 constexpr int kOrderCells = 256;       // of the last
 constexpr int kOrderTile = 4096;       // droplets it holds in shared memory
 constexpr long long kOneTile = 4096;   // droplets that the radix sort takes in one launch
-constexpr long long kFewCells = 1LL << 22;  // cells (16 MB of counts)
+constexpr long long kFewCells = 1LL << 22;   // cells (16 MB of counts)
+constexpr long long kMostCells = 1LL << 27;  // (512 MB)
 constexpr unsigned kNoCell = ~0u;      // key of a droplet that is not sorted
 
 // Count a droplet (key kNoCell: none); all 32 lanes call.  A run of lanes of
@@ -108,7 +109,8 @@ __global__ void __launch_bounds__(256) k_cell_sums(const uint4* counts, unsigned
 }
 
 // starts[c]: droplets of the cells before c (one more entry: of all cells).
-// Each CTA adds the sums before its own by itself: at most 2048, from L2.
+// Each CTA adds the sums before its own by itself, from L2: at most 32768
+// (kMostCells; 2 GB of reads, in a re-binning of 5.3 ms).
 __global__ void __launch_bounds__(256) k_cell_starts(uint4* counts, const unsigned* sums, unsigned* starts)
 {
   __shared__ unsigned part[8], wsum[8];
@@ -250,10 +252,13 @@ inline long long padded_cells(long long boxes, int shift)
 // in one launch, 4097 in 19 by counting (45 by a radix sort of several
 // launches); 64k droplets over 4.2M cells, whose passes take 20 us, 211 us of
 // GPU time in 73 (radix) and 215 in 38 from the last staging on (counting),
-// fewer droplets the other way round.
+// fewer droplets the other way round.  Beyond kMostCells it was not measured
+// (k_cell_starts reads a number of sums that grows with their square): a whole
+// re-binning by counting and by radix sort, half a droplet a cell, 1.05M droplets
+// 159 and 200 us, 8.5M 748 and 865, 16.9M 1396 and 1619, 67M 5293 and 6003.
 inline bool counting_pays(long long cells, long long n)
 {
-  return n > kOneTile && cells <= 64 * n && (cells <= kFewCells || cells <= 2 * n);
+  return n > kOneTile && cells <= 64 * n && (cells <= kFewCells || cells <= 2 * n) && cells <= kMostCells;
 }
 
 // The passes' arrays within a buffer: starts, sums, slots, order.

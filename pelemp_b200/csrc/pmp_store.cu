@@ -459,11 +459,19 @@ KeyOut key_out(const pmp_spray* h, long long row)
 long long sort_cells(const pmp_spray* h) { return padded_cells((long long)h->boxes.size(), h->sort_shift); }
 
 // Whether the rows of a hand-over are counted into their cells while they are
-// staged: decided at its first box, of n droplets, as if the others held as
-// many; cell_sorted() looks at the whole.
+// staged: decided at its first box, of n droplets, as if there were as many in
+// all as in the last hand-over; cell_sorted() looks at the whole.  In a handle's
+// first one the other boxes count as full as this one, which says little: the
+// counts are then at most kGuessedCells (64 MB).  512 boxes of 64^3 cells with
+// 300k droplets in the first and 50 in each of the others: without these bounds
+// 1 GB of counts, cleared and left for the radix sort in every pass.
+constexpr long long kGuessedCells = 1LL << 24;
 bool count_first(const pmp_spray* h, long long n)
 {
-  return narrow_keys(h) && counting_pays(sort_cells(h), n * (long long)h->boxes.size());
+  const long long cells = sort_cells(h);
+  const bool known = h->last_total >= 0;
+  return narrow_keys(h) && counting_pays(cells, known ? std::max(n, h->last_total) : n * (long long)h->boxes.size()) &&
+         (known || cells <= kGuessedCells);
 }
 bool cell_sorted(const pmp_spray* h, long long m)
 {
@@ -936,6 +944,7 @@ int pack(pmp_spray* h, cudaStream_t st)
   }
   h->staged_rows = 0;
   h->counted = h->ranked = false;
+  h->last_total = n;
   return PMP_OK;
 }
 

@@ -190,3 +190,45 @@ def test_no_memory_to_count_with(call, k, counts):
         fail_alloc(sp, k if call == "redistribute" else 0)
         assert sp.redistribute() == 0
         check(sp, by_cell(prob, drs))
+
+
+def held_mib():
+    import torch
+    torch.cuda.synchronize()
+    free, total = torch.cuda.mem_get_info()
+    return (total - free) / 2**20
+
+
+def boxes_of(side, nb):
+    """A level of nb[0] x nb[1] x nb[2] boxes of side^3 cells, one fuel, without droplets."""
+    prob = W.config1(n=10, steps=1)
+    prob.boxes = [(tuple(side * c for c in (i, j, k)), tuple(side * c + side - 1 for c in (i, j, k)))
+                  for k in range(nb[2]) for j in range(nb[1]) for i in range(nb[0])]
+    prob.domain_hi = tuple(side * n - 1 for n in nb)
+    prob.phi = prob.dx * side * np.array(nb)
+    return prob
+
+
+def test_memory_of_a_dense_first_box():
+    """Droplets nearly all in the first of many large boxes.  What 326k droplets need: rows and keys
+    (136 bytes, for up to twice as many), store, indices and lists (120 + 24), a sort (under 64):
+    155 MB; a cell counted for each place of 512 padded boxes: 1 GB."""
+    prob = boxes_of(64, (8, 8, 8))
+    rng = np.random.default_rng(6)
+    counts = [300_000] + [50] * 511
+    drs = [droplets(rng, n, 1, lo, hi, prob.dx[0]) for n, (lo, hi) in zip(counts, prob.boxes)]
+    sp = from_problem(prob, set_droplets=False)
+    for b, d in enumerate(drs):
+        sp.set_particles(b, *on_device((d[0][:, :1], d[1][:, :1], d[2][:1])))
+    sp.est_timestep(0.5)  # the kernels are loaded
+    sp.close()
+    sp = from_problem(prob, set_droplets=False)
+    before = held_mib()
+    dev = [on_device(d) for d in drs]
+    own = held_mib() - before
+    for _ in range(3):
+        for b, d in enumerate(dev):
+            sp.set_particles(b, *d)
+        assert sp.est_timestep(0.5) == expected_dt(prob, drs)
+        assert held_mib() - before - own < 300
+        sp.set_grids(prob.boxes)
