@@ -123,6 +123,7 @@ struct pmp_spray {
   // the leading zero_cells entries of counts are zero
   bool counted = false, ranked = false;
   long long zero_cells = 0;
+  int crowd_skip = 0;  // sorts that do not try to count (cell_sort.cuh)
   long long last_total = -1;  // droplets of the last packing (-1: none yet)
   double* soa = nullptr;  // (3 + NR) arrays of length total
   int* ids = nullptr;

@@ -1080,6 +1080,9 @@ static int rebin_count(pmp_spray* h, cudaStream_t st, long long n, int nb, int s
   }
   h->zero_cells = cells;
   *sorted = *h->crowded() == 0;
+  if (!*sorted) {
+    found_crowded(h);
+  }
   *order = base + L.order;
   *d_bounds = d_begin;
   return PMP_OK;
@@ -1128,7 +1131,7 @@ extern "C" int pmp_spray_redistribute(pmp_spray* h, long long* removed, void* st
   const long long* d_begin = nullptr;
   const long long cells = padded_cells(nb, shift);
   bool sorted = false;
-  if (narrow && counting_pays(cells, n)) {
+  if (narrow && counting_pays(cells, n) && try_counting(h)) {
     rc = rebin_count(h, st, n, nb, shift, cells, begin, &order, &d_begin, &sorted);
   }
   if (rc == PMP_OK && !sorted) {

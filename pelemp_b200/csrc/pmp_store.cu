@@ -885,6 +885,9 @@ int pack(pmp_spray* h, cudaStream_t st)
       const long long m = h->staged_rows;
       const int bits = m == n ? end_bit : 32;
       const long long cells = sort_cells(h);
+      if (h->counted && *h->crowded() != 0) {
+        found_crowded(h);
+      }
       const bool by_cell = m == n && cell_sorted(h, m) &&
                            try_keep(h, h->sort_scratch, cell_sort_layout(cells, m).total) == cudaSuccess;
       rc = by_cell ? PMP_OK : keep(h, h->sort_scratch, sort_bytes<unsigned, int>(m, bits));
@@ -1069,7 +1072,7 @@ int pmp_spray_set_particles(pmp_spray* h, int box, const pmp_particles* p)
   KeyOut out = narrow_keys(h) ? key_out(h, h->staged_rows) : KeyOut{};
   if (h->staged_rows == 0) {
     h->ranked = false;
-    h->counted = count_first(h, n);
+    h->counted = count_first(h, n) && try_counting(h);
     if (h->counted) {
       rc = count_cells(h, sort_cells(h), nullptr, &h->counted);
       if (rc != PMP_OK) {

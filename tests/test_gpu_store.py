@@ -232,3 +232,42 @@ def test_memory_of_a_dense_first_box():
         assert sp.est_timestep(0.5) == expected_dt(prob, drs)
         assert held_mib() - before - own < 300
         sp.set_grids(prob.boxes)
+
+
+def kernels_of(call):
+    """Names of the kernels that a call launches."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    return [e.key for e in prof.key_averages()]
+
+
+def test_crowded_cells_are_not_counted_again():
+    """A level with an injector: a third of the droplets in two cells for 20 passes, then spread, then
+    crowded again.  The order is right every time; a sort that follows a crowded one does not count, and
+    once the droplets have spread counting comes back."""
+    prob = level(2)
+    rng = np.random.default_rng(9)
+    n = 9000
+    sp = from_problem(prob, set_droplets=False)
+    counted = []
+    for i in range(60):
+        drs = [droplets(rng, n, 2, lo, hi, prob.dx[0]) for lo, hi in prob.boxes]
+        if i < 20 or i >= 50:
+            drs[0][0][:, :n // 3] = (np.array([[3], [4], [5]]) + rng.random((3, n // 3))) * prob.dx[0]
+            drs[0][0][0, :n // 6] += 4 * prob.dx[0]
+        sp.set_grids(prob.boxes)
+        for b, d in enumerate(drs):
+            sp.set_particles(b, *d)
+        names = kernels_of(lambda: (sp.est_timestep(0.5), sp.redistribute())) if i in (1, 2, 19, 48, 49) else None
+        if names is None:
+            sp.redistribute()
+        else:
+            counted.append(any("k_cell_scatter" in k for k in names))
+            assert any("k_rows_to_store" in k for k in names)
+        check(sp, by_cell(prob, drs))
+    # passes 1, 2: after a crowded one; 19: one of every 16 sorts tries, two sorts a pass; 48, 49: spread
+    assert counted[:2] == [False, False] and counted[3:] == [True, True]
