@@ -12,8 +12,11 @@
 // gathering 8 bytes from each of 14-17 component arrays read four times the
 // data; write-back to records goes the same way round.  Staging rows, store,
 // sort arrays and maps stay with the handle between calls (KeptBuffer), so
-// that a caller who hands its droplets over for every call allocates nothing
-// in the steady state.  Measured, hand-over, update and write-back: 2M
+// that a caller who hands its droplets over for every call, in device memory
+// that the kernels read directly, allocates nothing in the steady state
+// (droplets that come another way pass through a buffer, given back when it is
+// above 64 MB).  A buffer above 256 MB of which a packing leaves three quarters
+// idle is given back.  Measured, hand-over, update and write-back: 2M
 // two-fuel droplets in 8 boxes, FP64, 56.0 -> 2.82 ms (2.15 ms of it the
 // update; with a cudaMalloc and cudaFree per array and box the allocator took
 // 46 ms and moving droplets 1.8 ms), 0.78M droplets in 64 uneven boxes
@@ -492,8 +495,12 @@ int stage_room(pmp_spray* h, long long n)
     live += s.n;
   }
   // the first boxes of a hand-over say little about the rest of it: doubling,
-  // so that many boxes exchange the buffer a few times only
+  // so that many boxes exchange the buffer a few times only, up to what the last
+  // hand-over came to
   size_t rows = (size_t)(live > 0 ? 2 * (live + n) : n);
+  if (live > 0 && h->last_total >= live + n) {
+    rows = std::min(rows, (size_t)h->last_total);
+  }
   KeptBuffer nw, nk;
   if (store_alloc(h, &nw.p, rows * rb) != cudaSuccess) {
     cudaGetLastError();
@@ -722,12 +729,14 @@ cudaError_t store_alloc(pmp_spray* h, void** p, size_t bytes)
   return cudaMalloc(p, bytes);
 }
 
+// a buffer of which `bytes` are used is large and mostly unused
+static bool idle(const KeptBuffer& b, size_t bytes) { return b.bytes > ((size_t)256 << 20) && b.bytes / 4 > bytes; }
+
 // A kept buffer of at least `bytes`: exchanged when too small, and when it is
-// large and mostly unused (its content is not kept).
+// idle (its content is not kept).
 cudaError_t try_keep(pmp_spray* h, KeptBuffer& b, size_t bytes)
 {
-  const bool idle = b.bytes > ((size_t)256 << 20) && b.bytes / 4 > bytes;
-  if (b.p && b.bytes >= bytes && !idle) {
+  if (b.p && b.bytes >= bytes && !idle(b, bytes)) {
     return cudaSuccess;
   }
   cudaFree(b.p);
@@ -951,6 +960,29 @@ int pack(pmp_spray* h, cudaStream_t st)
   return PMP_OK;
 }
 
+// What n packed droplets leave idle of the buffers that a hand-over fills,
+// which grow with it and go through keep() only in a re-binning, or not at all:
+// given back.  The packing on st still reads them.
+void give_back(pmp_spray* h, long long n, cudaStream_t st)
+{
+  const size_t m = (size_t)n;
+  const bool rows = idle(h->spare, m * row_bytes(h)), counts = idle(h->counts, m * 2 * sizeof(unsigned));
+  if (!rows && !counts) {
+    return;
+  }
+  cudaStreamSynchronize(st);
+  if (rows) {
+    cudaFree(h->spare.p);
+    cudaFree(h->row_keys.p);
+    h->spare = h->row_keys = KeptBuffer{};
+  }
+  if (counts) {
+    cudaFree(h->counts.p);
+    h->counts = KeptBuffer{};
+    h->zero_cells = 0;
+  }
+}
+
 }  // namespace
 
 // The droplets packed, and their map built, in the order of st.
@@ -985,7 +1017,11 @@ int ensure_packed(pmp_spray* h, cudaStream_t st)
     cudaFree(p);
     st = nullptr;
   }
-  const int rc = h->packed ? build_cta_map(h, st) : pack(h, st);
+  const bool packing = !h->packed;
+  const int rc = packing ? pack(h, st) : build_cta_map(h, st);
+  if (rc == PMP_OK && packing) {
+    give_back(h, h->total, st);
+  }
   if (rc != PMP_OK) {
     // no kernel of it may still read rows that the caller replaces next
     cudaStreamSynchronize(st);

@@ -271,3 +271,32 @@ def test_crowded_cells_are_not_counted_again():
         check(sp, by_cell(prob, drs))
     # passes 1, 2: after a crowded one; 19: one of every 16 sorts tries, two sorts a pass; 48, 49: spread
     assert counted[:2] == [False, False] and counted[3:] == [True, True]
+
+
+def test_memory_after_a_large_hand_over():
+    """8M droplets, then 8000, by a handle that lives on.  What stays of the large one are buffers of up to
+    256 MB each: the caller's indices, the update's list and the sort's arrays (8, 8 and under 32 bytes a
+    droplet: 384 MB)."""
+    import torch
+    prob = boxes_of(64, (2, 2, 2))
+    big = 1_000_000
+    dx = prob.dx[0]
+    lo = torch.tensor([b[0] for b in prob.boxes], device="cuda", dtype=torch.float64)
+    pos = (torch.rand((3, big), device="cuda", dtype=torch.float64) * 64)
+    rd = torch.rand((11, big), device="cuda", dtype=torch.float64)
+    ids = torch.arange(1, big + 1, device="cuda", dtype=torch.int32)
+    at = torch.empty_like(pos)
+    sp = from_problem(prob, set_droplets=False)
+    torch.cuda.synchronize()
+    before = held_mib()
+    held = []
+    for n in (big, 1000, 1000, big):
+        sp.set_grids(prob.boxes)
+        for b in range(8):
+            at.copy_((pos + lo[b][:, None]) * dx)
+            sp.set_particles(b, at[:, :n].contiguous(), rd[:, :n].contiguous(), ids[:n].contiguous())
+        assert sp.est_timestep(0.5) == float((0.5 / ((rd[:3, :n] * (1.0 / prob.dx[0])).amax(0))).min())
+        torch.cuda.empty_cache()
+        held.append(held_mib() - before)
+    print("MiB held after 8M, 8k, 8k, 8M droplets:", [round(v) for v in held])
+    assert held[0] > 1500 and max(held[1:3]) < 512 and held[3] < held[0] + 64
