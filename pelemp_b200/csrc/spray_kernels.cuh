@@ -682,7 +682,9 @@ __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, 
         wf[1][dir] = (float)ssv[1][dir];
       }
       const StencilAt<float4> S = stencil_at<R4>(B, static_cast<const float4*>(B.gr), tile32, ijk, ssv);
-      state_ok = S.in;
+      // a position that is not a number gives no cell a weight: it is the source
+      // cell that is outside, as in the FP64 form
+      state_ok = S.in || ssv[0][0] != ssv[0][0] || ssv[0][1] != ssv[0][1] || ssv[0][2] != ssv[0][2];
       if (S.in) {
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk) {
