@@ -3,9 +3,17 @@
 //
 // MathPlain evaluates pmp_math.h and `/` as they stand.  MathFast returns the
 // same values for ordinary arguments without a branch: an argument that
-// pmp_math.h sends down a rare path, a divisor or quotient whose exponent is
-// not in the middle of the range, sets `odd`, and the caller then evaluates
-// the whole droplet sub-cycle again with MathPlain (redo_subcycle).
+// pmp_math.h sends down a rare path, or a divisor whose exponent is not in the
+// middle of the range, sets `odd`, and the caller then evaluates the whole
+// droplet sub-cycle again with MathPlain (redo_subcycle).
+// Dividends are not checked.  A quotient has the bits of IEEE division when the
+// dividend's magnitude is within 2^+-600, and a zero dividend gives +0 (-0 too).
+// Of a smaller dividend the last bits can differ (a - b q is rounded), of a
+// larger or infinite one the quotient can be NaN.  The droplets' bits do not
+// depend on it: an infinite or NaN gas state reaches a checked divisor (the
+// mixture's weight, the pressure) or check_finite (the Reynolds number), a
+// droplet's temperature, diameter and fractions reach the density's reciprocal
+// or a logarithm, and a tiny mass fraction is a term of sums of ordinary ones.
 // Why: each branch ends a basic block, so that in the plain form every
 // exponential, logarithm and division of the droplet physics ran its
 // dependent chain alone (57 elementary functions and 60 divisions per
@@ -32,7 +40,7 @@
 //    rounding correctly unless b's significand is all ones (Markstein), where
 //    1/b is known.
 // tests/test_gpu_math.py compares every function with the plain one, bit for
-// bit.
+// bit, and droplets with rare dividends with the oracle.
 #pragma once
 
 #include "pmp_math.h"

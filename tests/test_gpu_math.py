@@ -125,3 +125,44 @@ def test_gas_records_of_unusual_cells(mode, oracle):
         for a, b in zip(pg, po):
             for row in (capi.PSTATE_T, capi.PSTATE_DIA):
                 assert np.max(np.abs(a["rdata"][row] / b["rdata"][row] - 1)) <= 1e-4
+
+
+@pytest.mark.parametrize("fn", [DIV, NEAR1, DIVK])
+def test_dividends(fn):
+    """Bits of quotients over the dividends' stated range; zeros of either sign give +0."""
+    rng = np.random.default_rng(20 + fn)
+    for lo, hi in ((-600, -300), (300, 600)):
+        x, y = bits(rng, N, lo, hi), bits(rng, N, -290, 290)
+        x[1::3] *= -1.0
+        assert same(*evaluate(fn, x, y))
+    fast, plain, odd = evaluate(fn, [0.0, -0.0] * 64, bits(rng, 128, -290, 290))
+    assert np.array_equal(fast[~odd], plain[~odd]) and not np.signbit(fast[~odd]).any()
+
+
+TINY = np.array([1e-100, 1e-181, 1e-200, 1e-290, 1e-300, 1e-310, 5e-324, 0.0, -0.0])
+
+
+@pytest.mark.parametrize("where", ["liquid", "gas"])
+def test_tiny_fractions_match_the_oracle(where, oracle):
+    """Mass fractions far below the dividends' range, subnormal, zero and -0: the droplets' bits, the
+    zeros' signs among them."""
+    prob = W.config2(n=6000, steps=2, ncells=(32, 16, 16), box=(16, 16, 16))
+    rng = np.random.default_rng(1)
+    if where == "liquid":
+        for p in prob.parts:
+            n = p["id"].size
+            v, first = rng.choice(TINY, n), rng.integers(0, 2, n) == 0
+            p["rdata"][5:7] = np.where(first, v, 1.0 - v), np.where(first, 1.0 - v, v)
+    else:
+        shape = prob.state[0].shape[1:]
+        for s in range(5):
+            tiny = rng.choice(TINY, (shape[0], shape[1], 32 + 6))
+            m = rng.random(tiny.shape) < 0.3
+            for (lo, _), st in zip(prob.boxes, prob.state):  # the same cells in the overlap of the grown boxes
+                part = (slice(None), slice(None), slice(lo[0], lo[0] + shape[2]))
+                st[4 + s] = np.where(m[part], tiny[part], st[4 + s])
+    pg, _, _ = gpu_run(prob, 2)
+    po, _ = oracle_run(oracle, prob, 2)
+    assert_bitwise(pg, po)
+    for a, b in zip(pg, po):
+        assert np.array_equal(np.signbit(a["rdata"]), np.signbit(b["rdata"]))
