@@ -279,8 +279,8 @@ int pmp_spray_update(
  * copies overlap the update: the boxes go in up to 8 groups, each group's
  * update starting once its views are on the device and its sources copied
  * back while later groups run (page-locked host memory lets all three
- * proceed at once).  The FP64 form with a non-default launch shape or CUDA
- * graph, and the learned form with its audit on, copy, update and copy back
+ * proceed at once).  The FP64 form with a launch shape other than the grid of
+ * 128 threads or a CUDA graph, and the learned form with its audit on, copy, update and copy back
  * in sequence.  Stream-ordered like pmp_spray_update: with page-locked host
  * views the call returns before the copies run, so the caller synchronises
  * the stream (or calls pmp_spray_sync) before it reads the host source or
@@ -452,7 +452,7 @@ int pmp_spray_redistribute(pmp_spray* h, long long* removed, void* stream);
  * work of an update (box table upload, status reset, kernels, status
  * read-back) in a CUDA graph on an internal stream and replays it while the
  * call's arguments repeat (PMP_MODE_FP64 and PMP_MODE_MIXED, not with
- * PMP_LAUNCH_PER_BOX).  The default is GRID, 128 threads, 96 registers, no
+ * PMP_LAUNCH_PER_BOX).  The default is GRID, 128 threads, 128 registers, no
  * graph.  PMP_MODE_MIXED and PMP_MODE_LEARNED use their own launch. */
 enum { PMP_LAUNCH_GRID = 0, PMP_LAUNCH_PERSISTENT = 1, PMP_LAUNCH_PER_BOX = 2 };
 typedef struct pmp_launch_config {
@@ -479,10 +479,10 @@ int pmp_spray_get_launch(const pmp_spray* h, pmp_launch_config* cfg);
  * the given views (arguments as pmp_spray_update), keeps the fastest in the
  * handle and, when cache_path is not NULL, records it in that text file
  * under a key of device name, species and fuel counts, droplet count (to a
- * power of two), box count, do_move and sub-cycle count; a later call with
- * the same key reads it back without timing.  Droplets are restored after
- * every trial and deposits go to scratch arrays: the handle's droplets and
- * the caller's source are left as they were. */
+ * power of two), box count, do_move, sub-cycle count and the kernels'
+ * revision; a later call with the same key reads it back without timing.
+ * Droplets are restored after every trial and deposits go to scratch arrays:
+ * the handle's droplets and the caller's source are left as they were. */
 int pmp_spray_autotune(
   pmp_spray* h, const pmp_box_view* state, const pmp_box_view* source,
   int nboxes, double flow_dt, int state_ghosts, int source_ghosts,

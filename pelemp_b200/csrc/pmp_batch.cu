@@ -148,8 +148,8 @@ int batch_prepare(pmp_spray* h, const WorkMap** map)
   BatchState& B = h->batch;
   const pmp_launch_config& c = B.cfg;
   *map = nullptr;
-  if (c.kind == PMP_LAUNCH_GRID && c.block == 128 && c.regs == 96) {
-    return PMP_OK;  // the default launch uses the handle's own CTA map
+  if (c.kind == PMP_LAUNCH_GRID && c.block == 128) {
+    return PMP_OK;  // the handle's own CTA map
   }
   const int chunk = c.kind == PMP_LAUNCH_PERSISTENT ? c.chunk : c.block;
   int rc = get_map(h, chunk, map);
@@ -189,7 +189,7 @@ int batch_enqueue_fp64(pmp_spray* h, const KParams& P, int nboxes, cudaStream_t 
     return rc;
   }
   if (!m) {
-    return dispatch_fp64_default(ns, nf, P, h->ncta, st);
+    return dispatch_fp64_map(ns, nf, c.regs, P, h->ncta, st);
   }
   if (m->nitems == 0) {
     return PMP_OK;
@@ -347,6 +347,9 @@ extern "C" int pmp_spray_get_launch(const pmp_spray* h, pmp_launch_config* cfg)
 
 namespace {
 
+// of the kernels that a cache file's times belong to: counted up when they change
+constexpr int kKernelRevision = 2;
+
 std::string tune_key(pmp_spray* h, int nboxes, int do_move, int num_iter)
 {
   cudaDeviceProp prop;
@@ -359,8 +362,8 @@ std::string tune_key(pmp_spray* h, int nboxes, int do_move, int num_iter)
   }
   const int lg = h->total > 0 ? (int)std::floor(std::log2((double)h->total)) : 0;
   char b[256];
-  snprintf(b, sizeof(b), "%s|ns=%d|nf=%d|n=2^%d|boxes=%d|move=%d|iter=%d", name.c_str(), h->nspec, h->nfuel, lg,
-           nboxes, do_move, num_iter);
+  snprintf(b, sizeof(b), "%s|ns=%d|nf=%d|n=2^%d|boxes=%d|move=%d|iter=%d|rev=%d", name.c_str(), h->nspec, h->nfuel, lg,
+           nboxes, do_move, num_iter, kKernelRevision);
   return b;
 }
 
@@ -499,8 +502,8 @@ extern "C" int pmp_spray_autotune(
     return PMP_OK;
   };
   const pmp_launch_config cands[] = {
-    {PMP_LAUNCH_GRID, 128, 96, 128, 0, 0},        {PMP_LAUNCH_GRID, 64, 96, 64, 0, 0},
-    {PMP_LAUNCH_GRID, 128, 128, 128, 0, 0},       {PMP_LAUNCH_GRID, 256, 128, 256, 0, 0},
+    {PMP_LAUNCH_GRID, 128, 128, 128, 0, 0},       {PMP_LAUNCH_GRID, 64, 96, 64, 0, 0},
+    {PMP_LAUNCH_GRID, 128, 96, 128, 0, 0},        {PMP_LAUNCH_GRID, 256, 128, 256, 0, 0},
     {PMP_LAUNCH_PERSISTENT, 128, 96, 128, 0, 0},  {PMP_LAUNCH_PERSISTENT, 128, 96, 512, 0, 0},
     {PMP_LAUNCH_PERSISTENT, 128, 96, 2048, 0, 0}, {PMP_LAUNCH_PERSISTENT, 64, 96, 512, 0, 0},
     {PMP_LAUNCH_PERSISTENT, 128, 128, 512, 0, 0}, {PMP_LAUNCH_PERSISTENT, 256, 128, 1024, 0, 0},

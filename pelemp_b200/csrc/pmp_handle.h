@@ -62,7 +62,7 @@ struct WorkMap {
 };
 
 struct BatchState {
-  pmp_launch_config cfg{PMP_LAUNCH_GRID, 128, 96, 512, 0, 0};
+  pmp_launch_config cfg{PMP_LAUNCH_GRID, 128, 128, 512, 0, 0};
   std::vector<WorkMap> maps;
   int* d_counter = nullptr;
   int sm_count = 0;
@@ -218,7 +218,8 @@ int prepare_update(
   double flow_dt, int state_ghosts, int source_ghosts, int is_ghost, int do_move,
   double spray_cfl_lev, cudaStream_t st, KParams& P);
 int run_fp64_list(int ns, int nf, const KParams& P, long long total, cudaStream_t st);
-int dispatch_fp64_default(int ns, int nf, const KParams& P, int ncta, cudaStream_t st);
+// the grid of 128 threads over the handle's own CTA map
+int dispatch_fp64_map(int ns, int nf, int regs, const KParams& P, int ncta, cudaStream_t st);
 // the device work of one update after prepare: the per-call fallback count
 // reset, timing events, kernels (no synchronisation, no status read-back)
 int enqueue_update(pmp_spray* h, const KParams& P, int nboxes, cudaStream_t st);

@@ -414,18 +414,17 @@ int tile_at_bndry(const pmp_box& b, const pmp_geometry& g)
   return at;
 }
 
-template <int NS, int NF>
-void launch_fp64(const KParams& P, int ncta, cudaStream_t st)
+// regs: the register cap of the launch shape
+int dispatch_fp64(int ns, int nf, int regs, const KParams& P, int ncta, cudaStream_t st)
 {
-  pmp::spray_update_fp64<NS, NF, kBlock><<<ncta, kBlock, 0, st>>>(P);
-}
-
-int dispatch_fp64(int ns, int nf, const KParams& P, int ncta, cudaStream_t st)
-{
-#define PMP_CASE(S, F)          \
-  if (ns == S && nf == F) {     \
-    launch_fp64<S, F>(P, ncta, st); \
-    return PMP_OK;              \
+#define PMP_CASE(S, F)                                                       \
+  if (ns == S && nf == F) {                                                  \
+    if (regs == 96) {                                                        \
+      pmp::spray_update_fp64<S, F, kBlock, 5><<<ncta, kBlock, 0, st>>>(P);   \
+    } else {                                                                 \
+      pmp::spray_update_fp64<S, F, kBlock><<<ncta, kBlock, 0, st>>>(P);      \
+    }                                                                        \
+    return PMP_OK;                                                           \
   }
   PMP_CASE(3, 1)
   PMP_CASE(5, 1)
@@ -934,7 +933,7 @@ int update_host_overlapped_impl(
       } else if (P.pelec) {
         rc = dispatch_fp64_pelec(NS, NF, Q, n, st);
       } else {
-        rc = dispatch_fp64(NS, NF, Q, n, st);
+        rc = dispatch_fp64(NS, NF, h->batch.cfg.regs, Q, n, st);
       }
       if (rc == PMP_ERR_UNSUPPORTED) {
         return set_err(h, rc, "no kernel for this species / fuel count");
@@ -1150,9 +1149,9 @@ int pmp::launch_gas_records64(const pmp_spray* h, const KParams& P, int b0, int 
   return PMP_ERR_UNSUPPORTED;
 }
 
-int pmp::dispatch_fp64_default(int ns, int nf, const KParams& P, int ncta, cudaStream_t st)
+int pmp::dispatch_fp64_map(int ns, int nf, int regs, const KParams& P, int ncta, cudaStream_t st)
 {
-  return dispatch_fp64(ns, nf, P, ncta, st);
+  return dispatch_fp64(ns, nf, regs, P, ncta, st);
 }
 
 int pmp::run_fp64_list(int ns, int nf, const KParams& P, long long total, cudaStream_t st)
@@ -1527,10 +1526,10 @@ int pmp_spray_update_host(
   // copies overlapped with the update, except for the FP64 form's launch
   // shapes and graphs and the learned form's audit (whole-map launches)
   const pmp_launch_config& lc = h->batch.cfg;
-  const bool default_fp64 = lc.kind == PMP_LAUNCH_GRID && lc.block == 128 && lc.regs == 96 && !lc.use_graph;
+  const bool map_fp64 = lc.kind == PMP_LAUNCH_GRID && lc.block == 128 && !lc.use_graph;  // over the handle's map
   const bool overlapped = h->mode == PMP_MODE_MIXED ||
                           (h->mode == PMP_MODE_LEARNED && !pmp::learn_audit_on(h)) ||
-                          (h->mode == PMP_MODE_FP64 && (h->pelec || default_fp64));
+                          (h->mode == PMP_MODE_FP64 && (h->pelec || map_fp64));
   if (overlapped) {
     return update_host_overlapped(h, state, source, dst.data(), dsr.data(), nboxes, flow_dt,
                                   state_ghosts, source_ghosts, is_ghost, do_move, spray_cfl_lev, st);

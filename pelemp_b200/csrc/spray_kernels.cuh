@@ -955,8 +955,9 @@ __device__ __forceinline__ void fp64_cta(const KParams& P)
   flush_counters(P, c);
 }
 
-template <int NS, int NF, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, PMP_FP64_MIN_BLOCKS) spray_update_fp64(const __grid_constant__ KParams P)
+// MINB: CTAs per SM, for the register cap (128: 4, the default; 96: 5)
+template <int NS, int NF, int BLOCK, int MINB = PMP_FP64_MIN_BLOCKS>
+__global__ void __launch_bounds__(BLOCK, MINB) spray_update_fp64(const __grid_constant__ KParams P)
 {
   fp64_cta<NS, NF, BLOCK, false>(P);
 }

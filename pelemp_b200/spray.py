@@ -360,8 +360,11 @@ class SprayParticleContainer:
         return n.value
 
     # --- launch shape, CUDA graph, autotuner (batched form) ---------------
-    def set_launch(self, kind=capi.PMP_LAUNCH_GRID, block=128, regs=96, chunk=512, ctas_per_sm=0,
+    def set_launch(self, kind=capi.PMP_LAUNCH_GRID, block=128, regs=None, chunk=512, ctas_per_sm=0,
                    use_graph=False):
+        """regs None: the cap of the default launch (128) for its kind and block, 96 for the others."""
+        if regs is None:
+            regs = 128 if kind == capi.PMP_LAUNCH_GRID and block == 128 else 96
         cfg = capi.LaunchConfig(kind, block, regs, chunk, ctas_per_sm, int(use_graph))
         self._check(lib().pmp_spray_set_launch(self._h, C.byref(cfg)))
 
