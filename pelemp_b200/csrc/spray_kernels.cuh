@@ -246,7 +246,7 @@ __device__ __forceinline__ Rec load_rec(const Rec* p)
 // the box's state.
 template <int NS, int NF, bool PELEC>
 __device__ __forceinline__ bool gather_fp64(const KParams& P, const BoxEntry& B, const int* ijk, const double (&ssv)[2][3],
-                                            GasVals<NS, NF>& gpv, const CellTile<double2>* tile64)
+                                            GasVals<NS, NF>& gpv)
 {
   bool state_ok = true;
   gpv.rho = 0.;
@@ -266,90 +266,79 @@ __device__ __forceinline__ bool gather_fp64(const KParams& P, const BoxEntry& B,
   }
   gpv.eng_src = 0.;
   gpv.mass_src = 0.;
-        const int tb = tile_base(tile64, ijk);
-  #pragma unroll
-        for (int kk = -1; kk < 1; ++kk) {
-  #pragma unroll
-          for (int jj = -1; jj < 1; ++jj) {
-  #pragma unroll
-            for (int ii = -1; ii < 1; ++ii) {
-              const double cw = __dmul_rn(__dmul_rn(ssv[ii + 1][0], ssv[jj + 1][1]), ssv[kk + 1][2]);
-              if (cw > 0.) {
-                const int ci = ijk[0] + ii;
-                const int cj = ijk[1] + jj;
-                const int ck = ijk[2] + kk;
-                if (!in_box(B.state_lo, B.state_hi, ci, cj, ck)) {
-                  state_ok = false;
-                } else if (B.gr64) {
-                  // the cell's record holds the same per-cell terms the plane
-                  // gather below forms (k_gas_records64), so the sums are equal
-                  constexpr int R2 = gas_rec2(NS);
-                  double rec[2 * R2];
-                  if (tb >= 0) {
-                    const double2* r = tile64->rec + (tb + (kk + 1) * tile64->nxy + (jj + 1) * tile64->nx + (ii + 1)) * R2;
-  #pragma unroll
-                    for (int m = 0; m < R2; ++m) {
-                      const double2 v = r[m];
-                      rec[2 * m] = v.x;
-                      rec[2 * m + 1] = v.y;
-                    }
-                  } else {
-                    load_gas_rec64<R2>(B, ci, cj, ck, rec);
-                  }
-                  gpv.rho = __dadd_rn(gpv.rho, __dmul_rn(cw, rec[0]));
-  #pragma unroll
-                  for (int n = 0; n < NS; ++n) {
-                    gpv.Y[n] = __dadd_rn(gpv.Y[n], __dmul_rn(cw, rec[5 + n]));
-                  }
-  #pragma unroll
-                  for (int dir = 0; dir < 3; ++dir) {
-                    gpv.vel[dir] = __dadd_rn(gpv.vel[dir], __dmul_rn(cw, rec[2 + dir]));
-                  }
-                  gpv.T = __dadd_rn(gpv.T, __dmul_rn(cw, rec[1]));
-                } else {
-                  const double* q = B.st + ((ci - B.st_lo[0]) + (cj - B.st_lo[1]) * B.st_j32 + (ck - B.st_lo[2]) * B.st_k32);
-                  const double cur_rho = __ldg(q + P.c_rho * B.st_n32);
-                  gpv.rho = __dadd_rn(gpv.rho, __dmul_rn(cw, cur_rho));
-                  const double inv_rho = 1. / cur_rho;
-                  if (!PELEC) {
-  #pragma unroll
-                    for (int n = 0; n < NS; ++n) {
-                      const double cur_mf = __dmul_rn(__ldg(q + (P.c_spec + n) * B.st_n32), inv_rho);
-                      gpv.Y[n] = __dadd_rn(gpv.Y[n], __dmul_rn(cw, cur_mf));
-                    }
-  #pragma unroll
-                    for (int dir = 0; dir < 3; ++dir) {
-                      gpv.vel[dir] =
-                        __dadd_rn(gpv.vel[dir], __dmul_rn(cw, __ldg(q + (P.c_mom + dir) * B.st_n32)));
-                    }
-                    gpv.T = __dadd_rn(gpv.T, __dmul_rn(cw, __ldg(q + P.c_T * B.st_n32)));
-                  } else {
-                    // PeleC branch (SprayInterpolation.H:111-146): velocity from
-                    // momentum, T from the internal energy (eos.EY2T, the cell's
-                    // T as the guess)
-                    double mass_frac[NS];
-  #pragma unroll
-                    for (int n = 0; n < NS; ++n) {
-                      const double cur_mf = __dmul_rn(__ldg(q + (P.c_spec + n) * B.st_n32), inv_rho);
-                      gpv.Y[n] = __dadd_rn(gpv.Y[n], __dmul_rn(cw, cur_mf));
-                      mass_frac[n] = cur_mf;
-                    }
-                    double ke = 0.;
-  #pragma unroll
-                    for (int dir = 0; dir < 3; ++dir) {
-                      const double vel = __dmul_rn(__ldg(q + (P.c_mom + dir) * B.st_n32), inv_rho);
-                      gpv.vel[dir] = __dadd_rn(gpv.vel[dir], __dmul_rn(cw, vel));
-                      ke = __dadd_rn(ke, __dmul_rn(vel, vel) / 2.);
-                    }
-                    const double intEng = __dsub_rn(__dmul_rn(__ldg(q + P.c_eng * B.st_n32), inv_rho), ke);
-                    const double T_i = ey2t<NS>(P.m, intEng, mass_frac, __ldg(q + P.c_T * B.st_n32));
-                    gpv.T = __dadd_rn(gpv.T, __dmul_rn(cw, T_i));
-                  }
-                }
+#pragma unroll
+  for (int kk = -1; kk < 1; ++kk) {
+#pragma unroll
+    for (int jj = -1; jj < 1; ++jj) {
+#pragma unroll
+      for (int ii = -1; ii < 1; ++ii) {
+        const double cw = __dmul_rn(__dmul_rn(ssv[ii + 1][0], ssv[jj + 1][1]), ssv[kk + 1][2]);
+        if (cw > 0.) {
+          const int ci = ijk[0] + ii;
+          const int cj = ijk[1] + jj;
+          const int ck = ijk[2] + kk;
+          if (!in_box(B.state_lo, B.state_hi, ci, cj, ck)) {
+            state_ok = false;
+          } else if (B.gr64) {
+            // the cell's record holds the same per-cell terms the plane
+            // gather below forms (k_gas_records64), so the sums are equal
+            constexpr int R2 = gas_rec2(NS);
+            double rec[2 * R2];
+            load_gas_rec64<R2>(B, ci, cj, ck, rec);
+            gpv.rho = __dadd_rn(gpv.rho, __dmul_rn(cw, rec[0]));
+#pragma unroll
+            for (int n = 0; n < NS; ++n) {
+              gpv.Y[n] = __dadd_rn(gpv.Y[n], __dmul_rn(cw, rec[5 + n]));
+            }
+#pragma unroll
+            for (int dir = 0; dir < 3; ++dir) {
+              gpv.vel[dir] = __dadd_rn(gpv.vel[dir], __dmul_rn(cw, rec[2 + dir]));
+            }
+            gpv.T = __dadd_rn(gpv.T, __dmul_rn(cw, rec[1]));
+          } else {
+            const double* q = B.st + ((ci - B.st_lo[0]) + (cj - B.st_lo[1]) * B.st_j32 + (ck - B.st_lo[2]) * B.st_k32);
+            const double cur_rho = __ldg(q + P.c_rho * B.st_n32);
+            gpv.rho = __dadd_rn(gpv.rho, __dmul_rn(cw, cur_rho));
+            const double inv_rho = 1. / cur_rho;
+            if (!PELEC) {
+#pragma unroll
+              for (int n = 0; n < NS; ++n) {
+                const double cur_mf = __dmul_rn(__ldg(q + (P.c_spec + n) * B.st_n32), inv_rho);
+                gpv.Y[n] = __dadd_rn(gpv.Y[n], __dmul_rn(cw, cur_mf));
               }
+#pragma unroll
+              for (int dir = 0; dir < 3; ++dir) {
+                gpv.vel[dir] =
+                  __dadd_rn(gpv.vel[dir], __dmul_rn(cw, __ldg(q + (P.c_mom + dir) * B.st_n32)));
+              }
+              gpv.T = __dadd_rn(gpv.T, __dmul_rn(cw, __ldg(q + P.c_T * B.st_n32)));
+            } else {
+              // PeleC branch (SprayInterpolation.H:111-146): velocity from
+              // momentum, T from the internal energy (eos.EY2T, the cell's
+              // T as the guess)
+              double mass_frac[NS];
+#pragma unroll
+              for (int n = 0; n < NS; ++n) {
+                const double cur_mf = __dmul_rn(__ldg(q + (P.c_spec + n) * B.st_n32), inv_rho);
+                gpv.Y[n] = __dadd_rn(gpv.Y[n], __dmul_rn(cw, cur_mf));
+                mass_frac[n] = cur_mf;
+              }
+              double ke = 0.;
+#pragma unroll
+              for (int dir = 0; dir < 3; ++dir) {
+                const double vel = __dmul_rn(__ldg(q + (P.c_mom + dir) * B.st_n32), inv_rho);
+                gpv.vel[dir] = __dadd_rn(gpv.vel[dir], __dmul_rn(cw, vel));
+                ke = __dadd_rn(ke, __dmul_rn(vel, vel) / 2.);
+              }
+              const double intEng = __dsub_rn(__dmul_rn(__ldg(q + P.c_eng * B.st_n32), inv_rho), ke);
+              const double T_i = ey2t<NS>(P.m, intEng, mass_frac, __ldg(q + P.c_T * B.st_n32));
+              gpv.T = __dadd_rn(gpv.T, __dmul_rn(cw, T_i));
             }
           }
         }
+      }
+    }
+  }
   return state_ok;
 }
 
@@ -407,24 +396,22 @@ __device__ __forceinline__ void gather_fp64_inner(const StencilAt<double2>& S, c
 template <int NS, int NF, bool PELEC, class Math>
 __device__ __forceinline__ void define_gas(Math& M, const KParams& P, GasVals<NS, NF>& gpv, double* cBoilT)
 {
-        double mw_mix = 0.;
-  #pragma unroll
-        for (int n = 0; n < NS; ++n) {
-          mw_mix = __dadd_rn(mw_mix, M.divk(gpv.Y[n], P.m.mw_kg[n], P.m.inv_mw_kg[n]));
-        }
-        gpv.p = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(gpv.rho, kRuCgs), mw_mix), gpv.T), Units<PELEC>::ru);
-        gpv.mw_mix = M.inv(mw_mix);
-              {
-          const double RU = kRuCgs * Units<PELEC>::ru;
-          const double PATM = kPatmCgs * Units<PELEC>::pres;
-          const double lp = M.log(M.div(PATM, gpv.p));
-  #pragma unroll
-          for (int spf = 0; spf < NF; ++spf) {
-                  const double cc = M.inv(
-        __dadd_rn(M.divk(__dmul_rn(lp, RU), P.f.hboil_mw[spf], P.f.inv_hboil_mw[spf]), P.f.inv_boilT[spf]));
-      cBoilT[spf] = dmin(P.f.critT[spf], cc);
-          }
-        }
+  double mw_mix = 0.;
+#pragma unroll
+  for (int n = 0; n < NS; ++n) {
+    mw_mix = __dadd_rn(mw_mix, M.divk(gpv.Y[n], P.m.mw_kg[n], P.m.inv_mw_kg[n]));
+  }
+  gpv.p = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(gpv.rho, kRuCgs), mw_mix), gpv.T), Units<PELEC>::ru);
+  gpv.mw_mix = M.inv(mw_mix);
+  const double RU = kRuCgs * Units<PELEC>::ru;
+  const double PATM = kPatmCgs * Units<PELEC>::pres;
+  const double lp = M.log(M.div(PATM, gpv.p));
+#pragma unroll
+  for (int spf = 0; spf < NF; ++spf) {
+    const double cc =
+      M.inv(__dadd_rn(M.divk(__dmul_rn(lp, RU), P.f.hboil_mw[spf], P.f.inv_hboil_mw[spf]), P.f.inv_boilT[spf]));
+    cBoilT[spf] = dmin(P.f.critT[spf], cc);
+  }
 }
 
 // trilinear_interp (SprayInterpolation.H:158-199)
@@ -492,7 +479,7 @@ __device__ __noinline__ bool redo_subcycle(const KParams& P, const BoxEntry& B, 
   stencil_factors(fx, bflags, ssv);
   GasVals<NS, NF> gpv;
   double cBoilT[NF];
-  if (!gather_fp64<NS, NF, PELEC>(P, B, ijk, ssv, gpv, nullptr)) {
+  if (!gather_fp64<NS, NF, PELEC>(P, B, ijk, ssv, gpv)) {
     return false;
   }
   define_gas<NS, NF, PELEC>(M, P, gpv, cBoilT);
@@ -618,7 +605,7 @@ __device__ __forceinline__ void update_one(const KParams& P, const DevParts& D, 
           gpv = GasVals<NS, NF>{};
         }
       } else {
-        state_ok = gather_fp64<NS, NF, PELEC>(P, B, ijk, ssv, gpv, tile64);
+        state_ok = gather_fp64<NS, NF, PELEC>(P, B, ijk, ssv, gpv);
       }
       if (!state_ok) {
         set_error(P, PMP_ERR_STATE_BOX, b, s);
