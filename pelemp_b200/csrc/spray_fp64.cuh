@@ -454,7 +454,9 @@ __device__ __forceinline__ int spray_source_fp64(
         const double Sc_skin = M.div(mu_skin, rhoDtotal);
         double logB, pBM07;
         M.log1p_pow07(B_M, logB, pBM07);
-        const double invFM = M.div(B_M, logB * pBM07);
+        // B_M < 0 where vapour condenses; its logarithm has its sign, so the
+        // magnitudes' quotient has the same bits, and its divisor is positive
+        const double invFM = M.div(fabs(B_M), fabs(logB * pBM07));
         const double Sh_0 = 1. + powR * M.cbrt(1. + Reyn * Sc_skin);
         const double Sh_num = 2. + (Sh_0 - 2.) * invFM;
         const double mdotcoeff = PMP_PI * dia_part * Sh_num * logB;
