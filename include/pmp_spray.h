@@ -619,6 +619,8 @@ int pmp_debug_math(int fn, const double* x, const double* y, long long n,
  * reference): the k-th allocation of the droplet store from now on fails
  * (k = 0: none). */
 int pmp_spray_debug_fail_alloc(pmp_spray* h, int k);
+/* Allocations that the droplet store has made. */
+int pmp_spray_debug_allocs(const pmp_spray* h, long long* n);
 
 #ifdef __cplusplus
 }

@@ -159,7 +159,8 @@ struct pmp_spray {
   bool packing = false;
   cudaStream_t pack_stream = nullptr;
   cudaEvent_t ev_pack = nullptr;
-  int fail_alloc = 0;  // pmp_spray_debug_fail_alloc
+  int fail_alloc = 0;    // pmp_spray_debug_fail_alloc
+  long long allocs = 0;  // of the droplet store
   // the mixed form's FP64 list kernel runs on `side` beside the mixed kernel
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_sel = nullptr;

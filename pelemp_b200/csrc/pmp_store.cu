@@ -491,14 +491,18 @@ int stage_room(pmp_spray* h, long long n)
     return PMP_OK;
   }
   long long live = 0;
+  bool whole = true;  // every box is handed over: no rows were unpacked or given up
   for (const StagedBox& s : h->staged) {
     live += s.n;
+    whole = whole && !s.kept;
   }
+  whole = whole && live == h->staged_rows;
   // the first boxes of a hand-over say little about the rest of it: doubling,
   // so that many boxes exchange the buffer a few times only, up to what the last
-  // hand-over came to
+  // hand-over came to (boxes handed over again also need the rows that they give
+  // up: 64 boxes one by one, without the doubling, exchange the buffer 64 times)
   size_t rows = (size_t)(live > 0 ? 2 * (live + n) : n);
-  if (live > 0 && h->last_total >= live + n) {
+  if (whole && live > 0 && h->last_total >= live + n) {
     rows = std::min(rows, (size_t)h->last_total);
   }
   KeptBuffer nw, nk;
@@ -726,6 +730,7 @@ cudaError_t store_alloc(pmp_spray* h, void** p, size_t bytes)
     *p = nullptr;
     return cudaErrorMemoryAllocation;
   }
+  h->allocs += 1;
   return cudaMalloc(p, bytes);
 }
 
@@ -1286,6 +1291,15 @@ int pmp_spray_debug_fail_alloc(pmp_spray* h, int k)
     return PMP_ERR_INVALID;
   }
   h->fail_alloc = k;
+  return PMP_OK;
+}
+
+int pmp_spray_debug_allocs(const pmp_spray* h, long long* n)
+{
+  if (!h || !n) {
+    return PMP_ERR_INVALID;
+  }
+  *n = h->allocs;
   return PMP_OK;
 }
 

@@ -300,3 +300,33 @@ def test_memory_after_a_large_hand_over():
         held.append(held_mib() - before)
     print("MiB held after 8M, 8k, 8k, 8M droplets:", [round(v) for v in held])
     assert held[0] > 1500 and max(held[1:3]) < 512 and held[3] < held[0] + 64
+
+
+def allocs(sp):
+    n = C.c_longlong()
+    assert spray.lib().pmp_spray_debug_allocs(sp._h, C.byref(n)) == capi.PMP_OK
+    return n.value
+
+
+def test_allocations_of_repeated_hand_overs():
+    """64 boxes of 300 droplets: handed over, then again box by box without new grids, then with them.  A
+    pass allocates a few buffers at most (rows and keys are exchanged as they double), then none."""
+    prob = boxes_of(8, (4, 4, 4))
+    rng = np.random.default_rng(2)
+    drs = [droplets(rng, 300, 1, lo, hi, prob.dx[0]) for lo, hi in prob.boxes]
+    dev = [on_device(d) for d in drs]
+    sp = from_problem(prob, set_droplets=False)
+    made = []
+    for i in range(7):
+        if i > 3:
+            sp.set_grids(prob.boxes)
+        before = allocs(sp)
+        for b, d in enumerate(dev):
+            sp.set_particles(b, *d)
+        assert sp.est_timestep(0.5) == expected_dt(prob, drs)
+        made.append(allocs(sp) - before)
+    check(sp, drs)
+    print("allocations of the passes:", made)
+    # the first: 8 exchanges of two buffers, counts, and one each of store, indices, sort, map and list;
+    # the second: two exchanges while the boxes give their rows up, and the sort's
+    assert made[0] <= 22 and made[1] <= 6 and made[3:] == [0] * 4
