@@ -148,7 +148,7 @@ struct BoxEntry {
   int src_lo[3], src_hi[3];       // tilebox grown by source_ghosts
   int sr_alo[3], sr_ahi[3];       // allocated bounds of the source view
   int at_bounds;
-  int pad;
+  int rec_cta;                    // CTAs of the boxes before this one in the gas-record pass
   long long p_begin, p_end;       // droplet slots of this box
   // the strides again as 32-bit ints (every view is checked to span fewer
   // than 2^31 elements), for cheaper index arithmetic in the update kernels

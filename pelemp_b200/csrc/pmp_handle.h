@@ -190,11 +190,11 @@ struct pmp_spray {
   void* mesh_scratch = nullptr;
   size_t mesh_scratch_bytes = 0;
   // gas records of the grown boxes (BoxEntry::gr, FP32, mixed and learned
-  // forms; BoxEntry::gr64, FP64 form): capacity in bytes, and the largest
-  // grown box (cells) of the last prepared update
+  // forms; BoxEntry::gr64, FP64 form): capacity in bytes, and the pass's CTAs
+  // before each box of the last prepared update
   void* gas_rec = nullptr;
   size_t gas_rec_bytes = 0;
-  int gas_rec_max_cells = 0;
+  std::vector<int> gas_rec_cta;
   int nr() const { return PMP_PSTATE_NUM(nfuel); }
   int ncomp() const { return 3 + nr(); }
 };

@@ -51,18 +51,18 @@ int launch_select_small(const KParams& P, long long s0, long long s1, cudaStream
   return PMP_OK;
 }
 
-int launch_gas_records(int ns, const KParams& P, int b0, int nb, int max_cells, cudaStream_t st)
+int launch_gas_records(int ns, const KParams& P, int b0, int nb, const int* rec_cta, cudaStream_t st)
 {
-  if (nb <= 0 || max_cells <= 0) {
+  if (nb <= 0 || rec_cta[b0 + nb] == rec_cta[b0]) {
     return PMP_OK;
   }
-  const dim3 grid = gas_rec_grid(max_cells, nb);
+  const dim3 grid = gas_rec_grid(rec_cta, b0, nb);
 #define PMP_REC_CASE(S)                                     \
   if (ns == S) {                                            \
     if (P.pelec) {                                          \
-      k_gas_records<S, true><<<grid, 256, 0, st>>>(P, b0);  \
+      k_gas_records<S, true><<<grid, 256, 0, st>>>(P, b0, nb);  \
     } else {                                                \
-      k_gas_records<S><<<grid, 256, 0, st>>>(P, b0);        \
+      k_gas_records<S><<<grid, 256, 0, st>>>(P, b0, nb);        \
     }                                                       \
     return PMP_OK;                                          \
   }

@@ -21,9 +21,9 @@ namespace pmp {
 int launch_mixed(int ns, int nf, const KParams& P, int ncta, int block, cudaStream_t st);
 // the mixed form's droplets below 2 um of slots [s0, s1) onto the fallback list
 int launch_select_small(const KParams& P, long long s0, long long s1, cudaStream_t st);
-// FP32 gas records (BoxEntry::gr) of boxes [b0, b0 + nb); max_cells = the
-// largest grown box's cell count
-int launch_gas_records(int ns, const KParams& P, int b0, int nb, int max_cells, cudaStream_t st);
+// FP32 gas records (BoxEntry::gr) of boxes [b0, b0 + nb); rec_cta: the pass's
+// CTAs before each box (nboxes + 1)
+int launch_gas_records(int ns, const KParams& P, int b0, int nb, const int* rec_cta, cudaStream_t st);
 }  // namespace pmp
 
 using pmp::BoxEntry;
@@ -516,7 +516,7 @@ int prepare_update_impl(
   const bool rec32 = h->mode == PMP_MODE_MIXED || h->mode == PMP_MODE_LEARNED;
   const int R = rec32 ? pmp::gas_rec4(NS) : pmp::gas_rec2(NS);
   size_t rec_total = 0;
-  h->gas_rec_max_cells = 0;
+  h->gas_rec_cta.assign(nboxes + 1, 0);
   for (int b = 0; b < nboxes; ++b) {
     long long cells = 1;
     for (int d = 0; d < 3; ++d) {
@@ -525,7 +525,7 @@ int prepare_update_impl(
     if (cells * R >= (1LL << 31)) {
       return set_err(h, PMP_ERR_INVALID, "a grown box holds 2^31 gas-record words or more", b);
     }
-    h->gas_rec_max_cells = std::max(h->gas_rec_max_cells, (int)cells);
+    h->gas_rec_cta[b + 1] = h->gas_rec_cta[b] + pmp::gas_rec_ctas(cells);
     rec_total += (size_t)cells * R;
   }
   if (16 * rec_total > h->gas_rec_bytes) {
@@ -606,6 +606,7 @@ int prepare_update_impl(
       rec_off += (size_t)nx * ny * nz * R;
     }
     e.at_bounds = tile_at_bndry(bx, h->geom);
+    e.rec_cta = h->gas_rec_cta[b];
     e.p_begin = h->box_begin[b];
     e.p_end = h->box_begin[b + 1];
   }
@@ -764,7 +765,7 @@ int enqueue_mixed(pmp_spray* h, const KParams& Q, int n, long long s0, long long
     rc = dispatch_fp64_list(h->nspec, h->nfuel, R, h->total, h->side);
   }
   if (rc == PMP_OK && es == cudaSuccess) {
-    rc = pmp::launch_gas_records(h->nspec, Q, b0, nb, h->gas_rec_max_cells, st);
+    rc = pmp::launch_gas_records(h->nspec, Q, b0, nb, h->gas_rec_cta.data(), st);
     if (rc != PMP_OK) {
       rc = set_err(h, rc, "no gas-record kernel for this species count");
     }
@@ -915,7 +916,7 @@ int update_host_overlapped_impl(
     if (n > 0) {
       // the mixed form builds its gas records inside enqueue_mixed
       if (h->mode != PMP_MODE_MIXED) {
-        rc = h->mode == PMP_MODE_LEARNED ? pmp::launch_gas_records(NS, P, b0, b1 - b0, h->gas_rec_max_cells, st)
+        rc = h->mode == PMP_MODE_LEARNED ? pmp::launch_gas_records(NS, P, b0, b1 - b0, h->gas_rec_cta.data(), st)
                                          : pmp::launch_gas_records64(h, P, b0, b1 - b0, st);
         if (rc != PMP_OK) {
           return set_err(h, rc, "no gas-record kernel for this species count");
@@ -1087,7 +1088,7 @@ int pmp::enqueue_update(pmp_spray* h, const KParams& P, int nboxes, cudaStream_t
     const int NF = h->nfuel;
     int rc = PMP_OK;
     if (h->mode == PMP_MODE_LEARNED) {
-      rc = pmp::launch_gas_records(NS, P, 0, nboxes, h->gas_rec_max_cells, st);
+      rc = pmp::launch_gas_records(NS, P, 0, nboxes, h->gas_rec_cta.data(), st);
       if (rc == PMP_OK) {
         rc = enqueue_learned(h, P, 0, h->ncta, 0, h->total, st);
       }
@@ -1128,17 +1129,17 @@ int pmp::run_update(
 
 int pmp::launch_gas_records64(const pmp_spray* h, const KParams& P, int b0, int nb, cudaStream_t st)
 {
-  const int max_cells = h->gas_rec_max_cells;
-  if (nb <= 0 || max_cells <= 0 || h->mode != PMP_MODE_FP64) {
+  const int* rec_cta = h->gas_rec_cta.data();
+  if (nb <= 0 || h->mode != PMP_MODE_FP64 || rec_cta[b0 + nb] == rec_cta[b0]) {
     return PMP_OK;
   }
-  const dim3 grid = pmp::gas_rec_grid(max_cells, nb);
+  const dim3 grid = pmp::gas_rec_grid(rec_cta, b0, nb);
 #define PMP_REC_CASE(S)                                                  \
   if (h->nspec == S) {                                                   \
     if (h->pelec) {                                                      \
-      pmp::k_gas_records64<S, true><<<grid, 256, 0, st>>>(P, b0);        \
+      pmp::k_gas_records64<S, true><<<grid, 256, 0, st>>>(P, b0, nb);        \
     } else {                                                             \
-      pmp::k_gas_records64<S, false><<<grid, 256, 0, st>>>(P, b0);       \
+      pmp::k_gas_records64<S, false><<<grid, 256, 0, st>>>(P, b0, nb);       \
     }                                                                    \
     return PMP_OK;                                                       \
   }

@@ -22,6 +22,8 @@
 //    (grid-stride; the list length is read on the device).
 #pragma once
 
+#include <algorithm>
+
 #include "spray_fp64.cuh"
 #include "spray_mixed.cuh"
 
@@ -1015,26 +1017,63 @@ static __global__ void __launch_bounds__(256) k_select_small(const __grid_consta
   }
 }
 
-// The gas records of boxes [b0, b0 + gridDim.y): a thread per cell of the grown
-// box (gas_rec_grid), whose loads are all in flight together, and the CTA's
-// records written as one run of 16-byte words from shared memory (a thread's
-// own record is 48 or 64 bytes, so that its stores would each leave half
-// sectors to L2).  One exact reciprocal of rho a cell.  Bound by memory
+// The gas records of boxes [b0, b0 + nb): a thread per cell of the grown box,
+// whose loads are all in flight together, and the CTA's records written as one
+// run of 16-byte words from shared memory (a thread's own record is 48 or 64
+// bytes, so that its stores would each leave half sectors to L2).  One exact reciprocal of rho a cell.  Bound by memory
 // bandwidth: FP64 records of 64 boxes of 32^3 with one fuel (3.5M cells)
 // 101 -> 72 us, 6.3 TB/s; FP32 records of 8 boxes of 64 x 64 x 32 with two
 // (1.5M cells), beside the selection of the small droplets, 95 -> 64 us;
 // before, up to 128 CTAs a box went over its cells in a loop, with a division
 // a species and a thread's own stores.
-inline dim3 gas_rec_grid(int max_cells, int nb) { return dim3((unsigned)((max_cells + 255) / 256), (unsigned)nb); }
+// The grid is a row per box, as long as the largest box's CTAs, or, where that
+// would be over 1.4 times the CTAs that the boxes need, those in one row
+// (BoxEntry::rec_cta).  A CTA without cells costs 0.7 ns (500 boxes of 8^3 beside
+// one of 128^3: 3.4 ms by rows, 0.10 in one), one with cells 5, and 5 % more
+// where it looks for its box (512 boxes of 16^3: 212 us by one row, 202 by rows).
+inline int gas_rec_ctas(long long cells) { return cells > 0 ? (int)((cells + 255) / 256) : 0; }
+// rec_cta: the CTAs before each box
+inline dim3 gas_rec_grid(const int* rec_cta, int b0, int nb)
+{
+  const int all = rec_cta[b0 + nb] - rec_cta[b0];
+  int most = 0;
+  for (int b = b0; b < b0 + nb; ++b) {
+    most = std::max(most, rec_cta[b + 1] - rec_cta[b]);
+  }
+  return nb <= 65535 && (double)most * nb <= 1.4 * all ? dim3((unsigned)most, (unsigned)nb) : dim3((unsigned)all);
+}
 
-// the cell of a thread and its state; false beyond the grown box.  n: its cells
-__device__ __forceinline__ bool gas_rec_cell(const BoxEntry& B, const double*& q, int& n)
+// The box of this CTA among boxes [b0, b0 + nb), and its number in the box.  In
+// one row it is the last box that begins at or before the CTA, found 32 boxes a
+// look (each warp for itself).
+__device__ __forceinline__ int gas_rec_box(const KParams& P, int b0, int nb, int* tile)
+{
+  if ((int)gridDim.y == nb) {
+    *tile = (int)blockIdx.x;
+    return b0 + (int)blockIdx.y;
+  }
+  const int lane = threadIdx.x & 31;
+  const int item = __ldg(&P.boxes[b0].rec_cta) + (int)blockIdx.x;
+  while (nb > 1) {
+    const int step = (nb + 31) / 32;
+    const bool before = lane * step < nb && __ldg(&P.boxes[b0 + lane * step].rec_cta) <= item;
+    const int k = 31 - __clz((int)__ballot_sync(0xffffffffu, before));
+    b0 += k * step;
+    nb = min(step, nb - k * step);
+  }
+  *tile = item - __ldg(&P.boxes[b0].rec_cta);
+  return b0;
+}
+
+// the cell of a thread of the box's CTA `tile` and its state; false beyond the
+// grown box.  n: its cells
+__device__ __forceinline__ bool gas_rec_cell(const BoxEntry& B, int tile, const double*& q, int& n)
 {
   const unsigned nx = B.state_hi[0] - B.state_lo[0] + 1;
   const unsigned ny = B.state_hi[1] - B.state_lo[1] + 1;
   const unsigned nz = B.state_hi[2] - B.state_lo[2] + 1;
   n = (int)(nx * ny * nz);
-  const unsigned c = blockIdx.x * 256u + threadIdx.x;
+  const unsigned c = tile * 256u + threadIdx.x;
   const unsigned t = c / nx;
   const unsigned k = t / ny;
   const int i = (int)(c - t * nx), j = (int)(t - k * ny);
@@ -1043,14 +1082,14 @@ __device__ __forceinline__ bool gas_rec_cell(const BoxEntry& B, const double*& q
   return (int)c < n;
 }
 
-// tile[r] of the CTA's cells -> records of `W` 16-byte words, at `out`
+// rec[r] of the cells of the box's CTA `tile` -> records of `W` 16-byte words, at `out`
 template <int W, int PITCH, typename T>
-__device__ __forceinline__ void write_records(const T (*tile)[PITCH], T* out, int n)
+__device__ __forceinline__ void write_records(const T (*rec)[PITCH], T* out, int tile, int n)
 {
-  const int c0 = blockIdx.x * 256, m = min(256, n - c0);
+  const int c0 = tile * 256, m = min(256, n - c0);
   __syncthreads();
   for (int w = threadIdx.x; w < m * W; w += 256) {
-    out[(long long)c0 * W + w] = tile[w / W][w % W];
+    out[(long long)c0 * W + w] = rec[w / W][w % W];
   }
 }
 
@@ -1058,15 +1097,16 @@ __device__ __forceinline__ void write_records(const T (*tile)[PITCH], T* out, in
 // updates then gather 2-3 16-byte words per stencil cell instead of 5 + NS
 // FP64 planes, with rho*Y / rho divided once per cell.
 template <int NS, bool PELEC = false>
-__global__ void __launch_bounds__(256) k_gas_records(const __grid_constant__ KParams P, int b0)
+__global__ void __launch_bounds__(256) k_gas_records(const __grid_constant__ KParams P, int b0, int nb)
 {
   constexpr int R4 = gas_rec4(NS);
-  __shared__ float4 tile[256][R4 | 1];
-  const BoxEntry& B = P.boxes[b0 + blockIdx.y];
+  __shared__ float4 rec[256][R4 | 1];
+  int tile;
+  const BoxEntry& B = P.boxes[gas_rec_box(P, b0, nb, &tile)];
   const double* q;
   int n;
-  const bool valid = gas_rec_cell(B, q, n);
-  if ((int)blockIdx.x * 256 >= n) {
+  const bool valid = gas_rec_cell(B, tile, q, n);
+  if (tile * 256 >= n) {
     return;
   }
   if (valid) {
@@ -1125,10 +1165,10 @@ __global__ void __launch_bounds__(256) k_gas_records(const __grid_constant__ KPa
     }
 #pragma unroll
     for (int m = 0; m < R4; ++m) {
-      tile[threadIdx.x][m] = make_float4(v[4 * m], v[4 * m + 1], v[4 * m + 2], v[4 * m + 3]);
+      rec[threadIdx.x][m] = make_float4(v[4 * m], v[4 * m + 1], v[4 * m + 2], v[4 * m + 3]);
     }
   }
-  write_records<R4>(tile, B.gr, n);
+  write_records<R4>(rec, B.gr, tile, n);
 }
 
 // FP64 records (BoxEntry::gr64): rho, T, the velocity and the mass fractions
@@ -1138,15 +1178,16 @@ __global__ void __launch_bounds__(256) k_gas_records(const __grid_constant__ KPa
 // converted once per call instead of once per droplet and stencil corner (the
 // PeleC EOS inversion and the 1 / rho division included).
 template <int NS, bool PELEC>
-__global__ void __launch_bounds__(256) k_gas_records64(const __grid_constant__ KParams P, int b0)
+__global__ void __launch_bounds__(256) k_gas_records64(const __grid_constant__ KParams P, int b0, int nb)
 {
   constexpr int R2 = gas_rec2(NS);
-  __shared__ double2 tile[256][R2 | 1];
-  const BoxEntry& B = P.boxes[b0 + blockIdx.y];
+  __shared__ double2 rec[256][R2 | 1];
+  int tile;
+  const BoxEntry& B = P.boxes[gas_rec_box(P, b0, nb, &tile)];
   const double* q;
   int n;
-  const bool valid = gas_rec_cell(B, q, n);
-  if ((int)blockIdx.x * 256 >= n) {
+  const bool valid = gas_rec_cell(B, tile, q, n);
+  if (tile * 256 >= n) {
     return;
   }
   if (valid) {
@@ -1188,10 +1229,10 @@ __global__ void __launch_bounds__(256) k_gas_records64(const __grid_constant__ K
     }
 #pragma unroll
     for (int m = 0; m < R2; ++m) {
-      tile[threadIdx.x][m] = make_double2(v[2 * m], v[2 * m + 1]);
+      rec[threadIdx.x][m] = make_double2(v[2 * m], v[2 * m + 1]);
     }
   }
-  write_records<R2>(tile, B.gr64, n);
+  write_records<R2>(rec, B.gr64, tile, n);
 }
 
 template <int NS, int NF, int BLOCK, bool PELEC = false>
