@@ -505,6 +505,10 @@ int stage_room(pmp_spray* h, long long n)
   if (whole && live > 0 && h->last_total >= live + n) {
     rows = std::min(rows, (size_t)h->last_total);
   }
+  if (live == 0 && h->last_total < 0) {
+    // a handle's first: as if every box held as many, within 64 MB
+    rows = std::max(rows, std::min(rows * h->boxes.size(), ((size_t)64 << 20) / rb));
+  }
   KeptBuffer nw, nk;
   if (store_alloc(h, &nw.p, rows * rb) != cudaSuccess) {
     cudaGetLastError();
