@@ -261,9 +261,17 @@ inline long long padded_cells(long long boxes, int shift)
 // (k_cell_starts reads a number of sums that grows with their square): a whole
 // re-binning by counting and by radix sort, half a droplet a cell, 1.05M droplets
 // 159 and 200 us, 8.5M 748 and 865, 16.9M 1396 and 1619, 67M 5293 and 6003.
-inline bool counting_pays(long long cells, long long n)
+// At the other end the last pass decides, which is quadratic in a cell's droplets
+// and holds 16 a cell in shared memory.  One box of 32^3 and of 64^3, droplets a
+// cell of the grids (`held`), radix sort and counting: hand-over and packing 16 a
+// cell 181 and 163 us, 20: 196 and 216, 31: 245 and 317 (8M: 1183 and 1536);
+// re-binning, whose key kernel costs as much as the sort, 20: 156 and 147, 24: 162
+// and 161, 31: 175 and 208 (8M: 738 and 996).
+constexpr int kDenseStaged = 16, kDenseRebin = 24;
+inline bool counting_pays(long long cells, long long n, long long held, int dense)
 {
-  return n > kOneTile && cells <= 64 * n && (cells <= kFewCells || cells <= 2 * n) && cells <= kMostCells;
+  return n > kOneTile && cells <= 64 * n && (cells <= kFewCells || cells <= 2 * n) && cells <= kMostCells &&
+         n <= dense * held;
 }
 
 // Whether a sort that counting_pays for tries it: not for a while after one

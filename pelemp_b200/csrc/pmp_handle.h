@@ -112,6 +112,7 @@ struct pmp_spray {
   long long staged_rows = 0;
   std::vector<bool> box_set;
   int sort_shift = 0, sort_bits = 1;  // sort keys of the grids: a cell's bits, and the box's above them
+  long long grid_cells = 0;           // cells of the grids
   // packed droplets: component arrays of length total and ids, in `store`;
   // `spare` holds the staging rows, and the re-binned droplets, with which a
   // re-binning exchanges the store

@@ -1131,7 +1131,7 @@ extern "C" int pmp_spray_redistribute(pmp_spray* h, long long* removed, void* st
   const long long* d_begin = nullptr;
   const long long cells = padded_cells(nb, shift);
   bool sorted = false;
-  if (narrow && counting_pays(cells, n) && try_counting(h)) {
+  if (narrow && counting_pays(cells, n, h->grid_cells, kDenseRebin) && try_counting(h)) {
     rc = rebin_count(h, st, n, nb, shift, cells, begin, &order, &d_begin, &sorted);
   }
   if (rc == PMP_OK && !sorted) {

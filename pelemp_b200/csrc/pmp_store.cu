@@ -473,12 +473,12 @@ bool count_first(const pmp_spray* h, long long n)
 {
   const long long cells = sort_cells(h);
   const bool known = h->last_total >= 0;
-  return narrow_keys(h) && counting_pays(cells, known ? std::max(n, h->last_total) : n * (long long)h->boxes.size()) &&
-         (known || cells <= kGuessedCells);
+  const long long total = known ? std::max(n, h->last_total) : n * (long long)h->boxes.size();
+  return narrow_keys(h) && counting_pays(cells, total, h->grid_cells, kDenseStaged) && (known || cells <= kGuessedCells);
 }
 bool cell_sorted(const pmp_spray* h, long long m)
 {
-  return h->counted && *h->crowded() == 0 && counting_pays(sort_cells(h), m);
+  return h->counted && *h->crowded() == 0 && counting_pays(sort_cells(h), m, h->grid_cells, kDenseStaged);
 }
 
 // Room for n more staging rows in the spare buffer (and their keys); the live
@@ -800,9 +800,11 @@ int count_cells(pmp_spray* h, long long cells, cudaStream_t st, bool* have)
 void store_layout(pmp_spray* h)
 {
   int sh = 0;
+  h->grid_cells = 0;
   for (const pmp_box& bx : h->boxes) {
     int ext[3];
     sort_extent(bx, ext);
+    h->grid_cells += (long long)(bx.hi[0] - bx.lo[0] + 1) * (bx.hi[1] - bx.lo[1] + 1) * (bx.hi[2] - bx.lo[2] + 1);
     const unsigned long long cells = brick_key_count(ext[0], ext[1], ext[2]);
     while (sh < 40 && (1ULL << sh) < cells) {
       ++sh;

@@ -330,3 +330,43 @@ def test_allocations_of_repeated_hand_overs():
     # the first: 8 exchanges of two buffers, counts, and one each of store, indices, sort, map and list;
     # the second: two exchanges while the boxes give their rows up, and the sort's
     assert made[0] <= 22 and made[1] <= 6 and made[3:] == [0] * 4
+
+
+@pytest.mark.parametrize("per_cell,staged,rebinned", [(12, True, True), (20, False, True), (30, False, False)])
+def test_dense_levels_are_not_counted(per_cell, staged, rebinned):
+    """Which sort a level of evenly dense cells takes, and that its order is right."""
+    prob = level(2)
+    rng = np.random.default_rng(per_cell)
+    drs = [droplets(rng, per_cell * 4096, 2, lo, hi, prob.dx[0]) for lo, hi in prob.boxes]
+    dev = [on_device(d) for d in drs]
+    sp = from_problem(prob, set_droplets=False)
+    for _ in range(2):
+        sp.set_grids(prob.boxes)
+        for b, d in enumerate(dev):
+            sp.set_particles(b, *d)
+        pack = kernels_of(lambda: sp.est_timestep(0.5))
+        rebin = kernels_of(lambda: sp.redistribute())
+        assert any("k_cell_scatter" in k for k in pack) == staged
+        assert any("k_cell_scatter" in k for k in rebin) == rebinned
+        check(sp, by_cell(prob, drs))
+
+
+@pytest.mark.parametrize("each", [17, 40, 64])
+def test_dense_layer_is_counted(each):
+    """Two layers of cells with up to 64 droplets each and none elsewhere: more in a block's 256 cells than
+    its tile holds, counted all the same."""
+    prob = level(2)
+    rng = np.random.default_rng(each)
+    drs = []
+    for lo, hi in prob.boxes:
+        pos, rd, ids = droplets(rng, 512 * each, 2, lo, hi, prob.dx[0])
+        cell = rng.permutation(np.repeat(np.arange(512), each))
+        pos = (np.stack([cell % 16 + lo[0], cell // 16 % 16, cell // 256]) + rng.random(pos.shape)) * prob.dx[0]
+        drs.append((pos, rd, ids))
+    dev = [on_device(d) for d in drs]
+    sp = from_problem(prob, set_droplets=False)
+    for b, d in enumerate(dev):
+        sp.set_particles(b, *d)
+    names = kernels_of(lambda: sp.est_timestep(0.5)) + kernels_of(lambda: sp.redistribute())
+    assert sum("k_cell_order" in k for k in names) == 2
+    check(sp, by_cell(prob, drs))
