@@ -1014,7 +1014,14 @@ int ensure_packed(pmp_spray* h, cudaStream_t st)
   if (built) {
     // packed by a call on another stream, which may have been refused after that
     if (capturing) {
-      quiesce(h);  // a capture takes no event from outside
+      // a capture takes no event from outside, and a wait for one is allowed
+      // beside it in the relaxed mode alone
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      PMP_TRY(h, cudaThreadExchangeStreamCaptureMode(&mode));
+      const cudaError_t e = cudaEventSynchronize(h->ev_pack);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      PMP_TRY(h, e);
+      h->packing = false;
       return PMP_OK;
     }
     PMP_TRY(h, cudaStreamWaitEvent(st, h->ev_pack, 0));

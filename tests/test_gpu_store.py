@@ -370,3 +370,47 @@ def test_dense_layer_is_counted(each):
     names = kernels_of(lambda: sp.est_timestep(0.5)) + kernels_of(lambda: sp.redistribute())
     assert sum("k_cell_order" in k for k in names) == 2
     check(sp, by_cell(prob, drs))
+
+
+@pytest.mark.parametrize("refused", [False, True])
+def test_capture_after_an_update_on_another_stream(refused):
+    """The droplets are packed by an update on one stream, which only the caller has waited for, and the
+    next update is captured on another (captures in which calls that wait are not allowed)."""
+    import torch
+    prob = W.config2(n=20_000, steps=2, ncells=(32, 16, 16), box=(16, 16, 16))
+    st_keep, st_v = device_state(prob)
+    src, src_v = device_sources(prob)
+    side = torch.cuda.Stream()
+
+    def update(sp, do_move, stream, ghosts=prob.state_ghosts):
+        sp.update_particles(st_v, src_v, prob.flow_dt, 0.0, ghosts, prob.source_ghosts, 0, 0, do_move,
+                            prob.spray_cfl_lev, stream.cuda_stream, sync=False)
+
+    warm = from_problem(prob)  # the buffers that an update keeps are the handle's own, the kernels are loaded
+    update(warm, 0, side)
+    want = from_problem(prob)
+    for do_move in ((0, 1) if not refused else (1,)):
+        update(want, do_move, side)
+    want.sync()
+    sp = from_problem(prob)
+    update(sp, 0, side)
+    sp.sync()
+    for b, p in enumerate(prob.parts):
+        sp.set_particles(b, p["pos"], p["rdata"], p["id"])
+    torch.cuda.synchronize()
+    if refused:
+        with pytest.raises(spray.SprayError):
+            update(sp, 0, side, prob.state_ghosts + 1)
+    else:
+        update(sp, 0, side)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        update(sp, 1, torch.cuda.current_stream())
+    g.replay()
+    torch.cuda.synchronize()
+    sp.sync()
+    assert_bitwise([sp.get_particles(b) for b in range(len(prob.boxes))],
+                   [want.get_particles(b) for b in range(len(prob.boxes))])
+    del g, st_keep
+    warm.close()
