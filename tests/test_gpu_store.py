@@ -382,8 +382,8 @@ def test_capture_after_an_update_on_another_stream(refused):
     src, src_v = device_sources(prob)
     side = torch.cuda.Stream()
 
-    def update(sp, do_move, stream, ghosts=prob.state_ghosts):
-        sp.update_particles(st_v, src_v, prob.flow_dt, 0.0, ghosts, prob.source_ghosts, 0, 0, do_move,
+    def update(sp, do_move, stream, ghosts=prob.source_ghosts):
+        sp.update_particles(st_v, src_v, prob.flow_dt, 0.0, prob.state_ghosts, ghosts, 0, 0, do_move,
                             prob.spray_cfl_lev, stream.cuda_stream, sync=False)
 
     warm = from_problem(prob)  # the buffers that an update keeps are the handle's own, the kernels are loaded
@@ -399,8 +399,8 @@ def test_capture_after_an_update_on_another_stream(refused):
         sp.set_particles(b, p["pos"], p["rdata"], p["id"])
     torch.cuda.synchronize()
     if refused:
-        with pytest.raises(spray.SprayError):
-            update(sp, 0, side, prob.state_ghosts + 1)
+        with pytest.raises(spray.SprayError):  # the source views do not cover this many ghost cells
+            update(sp, 0, side, prob.source_ghosts + 1)
     else:
         update(sp, 0, side)
     torch.cuda.synchronize()
