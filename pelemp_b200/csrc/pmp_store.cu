@@ -499,11 +499,17 @@ int stage_room(pmp_spray* h, long long n)
   whole = whole && live == h->staged_rows;
   // the first boxes of a hand-over say little about the rest of it: doubling,
   // so that many boxes exchange the buffer a few times only, up to what the last
-  // hand-over came to (boxes handed over again also need the rows that they give
+  // hand-over came to, or to what the boxes so far let expect and a quarter more
+  // than they need (boxes handed over again also need the rows that they give
   // up: 64 boxes one by one, without the doubling, exchange the buffer 64 times)
   size_t rows = (size_t)(live > 0 ? 2 * (live + n) : n);
-  if (whole && live > 0 && h->last_total >= live + n) {
-    rows = std::min(rows, (size_t)h->last_total);
+  if (whole && live > 0) {
+    const long long nb = (long long)h->boxes.size();
+    const long long so_far = 1 + std::count(h->box_set.begin(), h->box_set.end(), true);
+    const long long all = h->last_total >= live + n ? h->last_total
+                          : so_far >= nb            ? live + n
+                                                    : std::max((live + n) * 5 / 4, (live + n) / so_far * nb + nb);
+    rows = std::min(rows, (size_t)all);
   }
   if (live == 0 && h->last_total < 0) {
     // a handle's first: as if every box held as many, within 64 MB

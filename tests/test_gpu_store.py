@@ -414,3 +414,30 @@ def test_capture_after_an_update_on_another_stream(refused):
                    [want.get_particles(b) for b in range(len(prob.boxes))])
     del g, st_keep
     warm.close()
+
+
+@pytest.mark.parametrize("sizes", ["like", "growing", "shrinking"])
+def test_rows_of_a_first_hand_over(sizes):
+    """What a level's first hand-over takes for its staging rows: exactly the rows of like boxes, a quarter
+    more at most than those of growing ones, exchanged a few times."""
+    prob = boxes_of(32, (4, 2, 2))
+    like = 60_000
+    counts = {"like": [like] * 16, "growing": [8_000 * (b + 1) for b in range(16)],
+              "shrinking": [8_000 * (16 - b) for b in range(16)]}[sizes]
+    rng = np.random.default_rng(4)
+    big = [on_device(d) for d in (droplets(rng, max(counts), 1, lo, hi, prob.dx[0]) for lo, hi in prob.boxes)]
+    warm, _ = filled(boxes_of(32, (4, 2, 2)), [100] * 16, nf=1)
+    warm.est_timestep(0.5)
+    warm.close()
+    sp = from_problem(prob, set_droplets=False)
+    before, made = held_mib(), allocs(sp)
+    for b, (d, n) in enumerate(zip(big, counts)):
+        sp.set_particles(b, d[0][:, :n].contiguous(), d[1][:, :n].contiguous(), d[2][:n].contiguous())
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held, made = held_mib() - before, allocs(sp) - made
+    need = 136 * sum(counts) / 2**20
+    print("%s: %d allocations, %.0f MiB held for %.0f of rows and keys" % (sizes, made, held, need))
+    # the counts (4 MB), and the driver's granules of 2 MB
+    assert held < {"like": 1.02, "growing": 1.27, "shrinking": 2.02}[sizes] * need + 12 and made <= 15
