@@ -619,8 +619,9 @@ int pmp_debug_math(int fn, const double* x, const double* y, long long n,
  * reference): the k-th allocation of the droplet store from now on fails
  * (k = 0: none). */
 int pmp_spray_debug_fail_alloc(pmp_spray* h, int k);
-/* Allocations that the droplet store has made. */
-int pmp_spray_debug_allocs(const pmp_spray* h, long long* n);
+/* Allocations that the droplet store has made, and sorts by counting that it
+ * has run (packings and re-binnings). */
+int pmp_spray_debug_store(const pmp_spray* h, long long* allocs, long long* cell_sorts);
 
 #ifdef __cplusplus
 }

@@ -162,6 +162,7 @@ struct pmp_spray {
   cudaEvent_t ev_pack = nullptr;
   int fail_alloc = 0;    // pmp_spray_debug_fail_alloc
   long long allocs = 0;  // of the droplet store
+  long long cell_sorts = 0;  // sorts by counting
   // the mixed form's FP64 list kernel runs on `side` beside the mixed kernel
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_sel = nullptr;

@@ -1073,6 +1073,7 @@ static int rebin_count(pmp_spray* h, cudaStream_t st, long long n, int nb, int s
                                                              domain_of(h), wrap_of(h), d_boxes, nb, shift, keys, rank,
                                                              counts, h->crowded());
   cell_sort(counts, cells, keys, rank, n, base, st);
+  h->cell_sorts += 1;
   k_box_starts<<<nblk(nb + 1), 256, 0, st>>>(reinterpret_cast<unsigned*>(base), nb, shift, d_begin);
   rc = read_bounds(h, st, d_begin, begin);
   if (rc != PMP_OK) {

@@ -923,6 +923,7 @@ int pack(pmp_spray* h, cudaStream_t st)
         char* buf = static_cast<char*>(h->sort_scratch.p);
         h->counted = false;
         cell_sort(static_cast<unsigned*>(h->counts.p), cells, k.keys, k.idx, m, buf, st);
+        h->cell_sorts += 1;
         PMP_TRY(h, cudaGetLastError());
         h->zero_cells = cells;
         order = reinterpret_cast<const int*>(buf + cell_sort_layout(cells, m).order);
@@ -1313,12 +1314,13 @@ int pmp_spray_debug_fail_alloc(pmp_spray* h, int k)
   return PMP_OK;
 }
 
-int pmp_spray_debug_allocs(const pmp_spray* h, long long* n)
+int pmp_spray_debug_store(const pmp_spray* h, long long* allocs, long long* cell_sorts)
 {
-  if (!h || !n) {
+  if (!h || !allocs || !cell_sorts) {
     return PMP_ERR_INVALID;
   }
-  *n = h->allocs;
+  *allocs = h->allocs;
+  *cell_sorts = h->cell_sorts;
   return PMP_OK;
 }
 

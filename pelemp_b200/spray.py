@@ -83,7 +83,7 @@ _SIGS = {
     "pmp_learn_debug_solve_baseline": [C.c_void_p, C.c_void_p],
     "pmp_debug_math": [C.c_int, C.c_void_p, C.c_void_p, C.c_longlong, C.c_void_p, C.c_void_p, C.c_void_p],
     "pmp_spray_debug_fail_alloc": [C.c_void_p, C.c_int],
-    "pmp_spray_debug_allocs": [C.c_void_p, C.POINTER(C.c_longlong)],
+    "pmp_spray_debug_store": [C.c_void_p, C.POINTER(C.c_longlong), C.POINTER(C.c_longlong)],
     "pmp_measure_peaks": [C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double), C.POINTER(C.c_double)],
 }
 
